@@ -79,6 +79,8 @@ __constant__ int f_oy[8] = {0, 0, 1, -1, 1, 1, -1, -1};
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ void st2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
 __device__ __forceinline__ float at4(const float4& v, int j) { return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w; }
 
 __device__ __forceinline__ int find_terrain(const int* tile0, int nterr, int tile) {
@@ -203,37 +205,40 @@ __device__ __forceinline__ void hydro_tile(const TerrainHot& td, const CUtensorM
     const float* FR = sm + H_FR * H_RC;
     const float* FT = sm + H_FT * H_RC;
     const float* FB = sm + H_FB * H_RC;
+    // Pairs of horizontally adjacent cells, a row of the tile per warp: 8-byte
+    // shared loads and global stores, both cells in one f32x2 instruction
+    // (cell_hydro2).  Neighbours outside the grid read rock 0, flux 0 and
+    // total height FAR_HEIGHT from the tile (see the fill above); the
+    // closed-boundary outflow zeroing runs in edge tiles.
+    float* const rock_o = c.thermal ? td.b_ero : td.out[S_ROCK];  // no thermal pass: eroded rock is final
 #pragma unroll 1
-    for (int k = 0; k < G::CPT; ++k) {
+    for (int k = 0; k < G::CPT / 2; ++k) {
         const int q = tid + k * NTH;
-        const int ix = q % TW, iy = q / TW;
+        const int ix = (q % (TW / 2)) * 2, iy = q / (TW / 2);
         const int x = tx0 + ix, y = ty0 + iy;
         const int si = (1 + iy) * RW + HX + ix;
         const size_t gi = (size_t)y * n + x;
-        // neighbours outside the grid read rock 0, flux 0 and total height
-        // FAR_HEIGHT from the tile (see the fill above); the closed-boundary
-        // outflow zeroing runs in edge tiles
-        float b = B[si], d1 = D[si];
-        float bl = B[si - 1], br = B[si + 1], bb = B[si - RW], bt = B[si + RW];
-        float w_c = b + d1;
-        float wl = bl + D[si - 1];
-        float wr = br + D[si + 1];
-        float wt = bt + D[si + RW];
-        float wb = bb + D[si - RW];
-        FluxOut o = cell_flux(c, x, y, w_c, d1, FL[si], FR[si], FT[si], FB[si], wl, wr, wt, wb, FR[si - 1], FL[si + 1],
-                              FB[si + RW], FT[si - RW], EDGE);
-        float s = S[si];
-        float Kls0 = c.ks_field ? c.dt * __ldg(c.ks_field + gi) : c.Kls0;
-        cell_erosion(c, Kls0, o.u, o.v, o.vz, b, s, br, bl, bb, bt);
-        td.out[S_FL][gi] = o.fl;
-        td.out[S_FR][gi] = o.fr;
-        td.out[S_FT][gi] = o.ft;
-        td.out[S_FB][gi] = o.fb;
-        td.out[S_WATER][gi] = o.d2 * c.evap;  // sediment_transport's evaporation (glsl/sediment_transport.glsl:75)
-        td.u[gi] = o.u;
-        td.v[gi] = o.v;
-        td.s_ero[gi] = s;
-        (c.thermal ? td.b_ero : td.out[S_ROCK])[gi] = b;  // no thermal pass: eroded rock is final
+        const float2 b = ld2(B + si), d1 = ld2(D + si);
+        const float2 bl = make_float2(B[si - 1], b.x), br = make_float2(b.y, B[si + 2]);
+        const float2 bb = ld2(B + si - RW), bt = ld2(B + si + RW);
+        const float2 wl = add2(bl, make_float2(D[si - 1], d1.x)), wr = add2(br, make_float2(d1.y, D[si + 2]));
+        const float2 wt = add2(bt, ld2(D + si + RW)), wb = add2(bb, ld2(D + si - RW));
+        const float2 fl = ld2(FL + si), fr = ld2(FR + si);
+        const float2 inl = make_float2(FR[si - 1], fr.x), inr = make_float2(fl.y, FL[si + 2]);
+        float2 Kls0 = pf(c.Kls0);
+        if (c.ks_field) Kls0 = mul2(pf(c.dt), __ldg(reinterpret_cast<const float2*>(c.ks_field + gi)));
+        const Hydro2 o = cell_hydro2(c, x, y, EDGE, b, d1, ld2(S + si), fl, fr, ld2(FT + si), ld2(FB + si), wl, wr, wt,
+                                     wb, inl, inr, ld2(FB + si + RW), ld2(FT + si - RW), bl, br, bb, bt, Kls0);
+        st2(td.out[S_FL] + gi, o.fl);
+        st2(td.out[S_FR] + gi, o.fr);
+        st2(td.out[S_FT] + gi, o.ft);
+        st2(td.out[S_FB] + gi, o.fb);
+        // sediment_transport's evaporation (glsl/sediment_transport.glsl:75)
+        st2(td.out[S_WATER] + gi, mul2(o.d2, pf(c.evap)));
+        st2(td.u + gi, o.u);
+        st2(td.v + gi, o.v);
+        st2(td.s_ero + gi, o.s);
+        st2(rock_o + gi, o.b);
     }
 }
 
@@ -390,16 +395,16 @@ __device__ __forceinline__ void transport_tile(const TerrainHot& td, const CUten
     // sediment_transport: semi-Lagrangian gather of eroded sediment (any
     // reach), two cells per pair.  The taps' loads stay in flight across the
     // tile's TMA wait.
-    float2 bx[2], by[2], t00[2], t10[2], t01[2], t11[2];
+    Trace2 tr[2];
+    float2 t00[2], t10[2], t01[2], t11[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-        backtrace2(c, x0 + 2 * h, y, make_float2(at4(u4, 2 * h), at4(u4, 2 * h + 1)),
-                   make_float2(at4(v4, 2 * h), at4(v4, 2 * h + 1)), bx[h], by[h]);
+        tr[h] = backtrace2(c, x0 + 2 * h, y, make_float2(at4(u4, 2 * h), at4(u4, 2 * h + 1)),
+                           make_float2(at4(v4, 2 * h), at4(v4, 2 * h + 1)));
         float tap[4][2];
 #pragma unroll
         for (int l = 0; l < 2; ++l) {
-            const float px = l ? bx[h].y : bx[h].x, py = l ? by[h].y : by[h].x;
-            const int ix = min(max((int)px, 0), n - 1), iy2 = min(max((int)py, 0), n - 1);
+            const int ix = (int)tr[h].ix[l], iy2 = (int)tr[h].iy[l];
             const float* se = td.s_ero + (size_t)iy2 * n + ix;
             tap[0][l] = __ldg(se);
             tap[1][l] = ix + 1 < n ? __ldg(se + 1) : 0.0f;
@@ -412,8 +417,8 @@ __device__ __forceinline__ void transport_tile(const TerrainHot& td, const CUten
         t11[h] = make_float2(tap[3][0], tap[3][1]);
     }
     auto finish_sed = [&]() {
-        const float2 s0 = bilinear_mix2(bx[0], by[0], t00[0], t10[0], t01[0], t11[0]);
-        const float2 s1 = bilinear_mix2(bx[1], by[1], t00[1], t10[1], t01[1], t11[1]);
+        const float2 s0 = bilinear_mix2(tr[0], t00[0], t10[0], t01[0], t11[0]);
+        const float2 s1 = bilinear_mix2(tr[1], t00[1], t10[1], t01[1], t11[1]);
         st4(td.out[S_SED] + gi0, make_float4(s0.x, s0.y, s1.x, s1.y));
     };
     if (!c.thermal) {

@@ -49,6 +49,10 @@ __global__ void k_selftest_division(uint32_t seed_lo, uint32_t seed_hi, unsigned
         const float dd = uniform_exp_float(w[2], w[0], -30, 39);
         if (__float_as_uint(div_recip(dd, SQRT2_F, RCP_SQRT2_F)) != __float_as_uint(__fdiv_rn(dd, SQRT2_F)))
             ++local;
+        // the Newton reciprocal and square root the quotients and roots start from
+        const float rr = uniform_exp_float(w[1], w[2], -100, 99);
+        if (__float_as_uint(rcp_newton(rr)) != __float_as_uint(__frcp_rn(rr))) ++local;
+        if (__float_as_uint(sqrt_newton(rr)) != __float_as_uint(__fsqrt_rn(rr))) ++local;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0 && __float_as_uint(__frcp_rn(SQRT2_F)) != __float_as_uint(RCP_SQRT2_F))
         ++local;

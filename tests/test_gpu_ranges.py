@@ -1,0 +1,76 @@
+"""The fused step against the per-pass kernels on fields from all over the
+float range: water films and fluxes down to subnormals, zeros, values whose
+quotients and roots leave the range of the fused kernels' Newton forms,
+negative heights, infinities and NaN.  The per-pass kernels use the built-in
+division and square root, so every field is compared bit for bit (a NaN
+matches any NaN)."""
+import numpy as np
+import pytest
+
+import hydrogen as H
+
+pytestmark = pytest.mark.gpu
+
+STATE = H.STATE_FIELDS
+
+
+def fields(kind, n, seed):
+    rng = np.random.default_rng(seed)
+
+    def wide(lo, hi, zeros=0.2, signed=False):
+        x = np.exp2(rng.uniform(lo, hi, (n, n)))
+        x = np.where(rng.random((n, n)) < zeros, 0.0, x)
+        if signed:
+            x = np.where(rng.random((n, n)) < 0.5, -x, x)
+        return x.astype(np.float32)
+
+    f = {"rock": (64 * rng.random((n, n))).astype(np.float32), "water": wide(-20, 3), "sediment": wide(-30, 0)}
+    for k in ("flux_l", "flux_r", "flux_t", "flux_b"):
+        f[k] = wide(-20, 4)
+    if kind == "films":  # depths and fluxes through the subnormals
+        f["water"] = wide(-149, -5)
+        for k in ("flux_l", "flux_r", "flux_t", "flux_b"):
+            f[k] = wide(-149, 2, zeros=0.4)
+    elif kind == "dry":
+        f["water"] = wide(-10, 0, zeros=0.9)
+        for k in ("flux_l", "flux_r", "flux_t", "flux_b"):
+            f[k] = wide(-10, 0, zeros=0.9)
+    elif kind == "huge":
+        f["rock"] = wide(-10, 60, signed=True)
+        f["water"] = wide(-10, 90)
+        for k in ("flux_l", "flux_r", "flux_t", "flux_b"):
+            f[k] = wide(-10, 100)
+    elif kind == "negative":  # heights below zero: exhausted cells, H capped by a negative height
+        f["rock"] = (f["rock"] - 60).astype(np.float32)
+        f["sediment"] = wide(-30, 0, signed=True)
+    elif kind == "nonfinite":
+        for k in f:
+            bad = rng.random((n, n)) < 0.002
+            f[k][bad] = rng.choice(np.array([np.inf, -np.inf, np.nan], np.float32), bad.sum())
+    return f
+
+
+@pytest.mark.parametrize("kind", ["ordinary", "films", "dry", "huge", "negative", "nonfinite"])
+@pytest.mark.parametrize("n,thermal,ks1", [(64, True, 0.05), (192, True, 0.0), (128, False, 0.05)])
+def test_fused_equals_plain_over_the_float_range(kind, n, thermal, ks1):
+    f = fields(kind, n, seed=n + len(kind))
+    worlds = []
+    for _ in range(2):
+        w = H.World(n)
+        H.configure(w, "config2")
+        s = H.settings_config2()
+        s.Ks[1] = ks1
+        if not thermal:
+            s.Kspeed[0] = 0.0
+        w.set_erosion(s)
+        w.set_options(H.options(H.RAIN_BERNOULLI, p=0.02, seed=3))
+        for k, v in f.items():
+            w.upload(k, v)
+        worlds.append(w)
+    for step in range(3):
+        for w, mode in zip(worlds, (H.MODE_PLAIN, H.MODE_FUSED)):
+            w.step(1, mode)
+        for k in STATE:
+            a, b = worlds[0].download(k), worlds[1].download(k)
+            assert np.array_equal(a, b, equal_nan=True), \
+                f"step {step + 1} {k}: {np.count_nonzero(~((a == b) | (np.isnan(a) & np.isnan(b))))} cells differ"
