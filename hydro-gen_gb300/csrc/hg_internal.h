@@ -151,34 +151,39 @@ struct RainBase {
 
 // One terrain (world) of a fused launch, without its tensor maps.
 struct TerrainHot {
-    StepConsts c;
+    StepConsts1 c;
     RainBase rain;
     float* out[S_COUNT];
     float* u;
     float* v;
-    float* s_ero;  // eroded sediment of every cell (k_hydro -> k_transport)
+    float* s_ero;  // eroded sediment of every cell (k_hydro -> the next gather)
     float* b_ero;  // eroded rock of every cell (k_hydro -> k_transport, thermal on)
+    const float* s_prev;  // the previous step's s_ero (a chained k_hydro gathers from it)
+    float* s_keep;        // where a chained k_hydro leaves the gathered sediment, or nullptr
+    ptrdiff_t uv_prev;    // the previous step's u and v lie this many floats from u and v
     unsigned long long* step;  // device step counter (steps completed)
     int tiles_x;
-    int tile0;  // first tile of this terrain in the launch
+    int t_rows;  // k_transport: rows a warp marches
 };
 // maps[0..6]: TMA boxes of the step's input rock, water, sediment, fL, fR,
-// fT, fB; maps[7]: eroded rock.  (CUtensorMap makes it 64-byte aligned.)
-constexpr int MAPS_PER_TERRAIN = 8;
+// fT, fB.  (CUtensorMap makes it 64-byte aligned.)
+constexpr int MAPS_PER_TERRAIN = 7;
 struct TerrainDesc {
     CUtensorMap maps[MAPS_PER_TERRAIN];
     TerrainHot h;
-    int tile_off;  // first tile launched (a row slab's), 0 for the whole world
+    int row_lo, row_hi;  // rows to do (a row slab's; all of the world otherwise)
 };
 // A batch launch's terrain records travel as one kernel parameter (read
 // through the constant bank); the tensor maps stay in global memory.
 constexpr int MAX_BATCH = 128;
 struct BatchParams {
     int nterr;
-    int tile0[MAX_BATCH];
+    int tasks;              // k_transport's warps over all terrains
+    int tile0[MAX_BATCH];   // k_hydro: first tile of each terrain
+    int task0[MAX_BATCH];   // k_transport: first warp of each terrain
     TerrainHot t[MAX_BATCH];
 };
-static_assert(sizeof(BatchParams) < 32000, "kernel parameter space");
+static_assert(sizeof(BatchParams) + 2 * sizeof(void*) <= 32764, "kernel parameter space");
 
 // Host view of one terrain for one step direction (inputs -> outputs).
 struct TerrainSrc {
@@ -190,7 +195,18 @@ struct TerrainSrc {
     float* v;
     float* s_ero;
     float* b_ero;
+    const float* s_prev;
+    float* s_keep;
+    ptrdiff_t uv_prev;
     unsigned long long* step;
+};
+
+// A step's place in a run of steps launched together (a chain).  Within a
+// chain a step's sediment gather runs in the next step's k_hydro, and the
+// device step counter stays at the chain's start until its end.
+struct ChainPos {
+    int index;  // steps of the chain before this one
+    bool last;  // the step's results become the state
 };
 
 // Tensor maps encoded once per (buffer, box) and reused.
@@ -208,16 +224,21 @@ struct TmaCache {
 bool fused_tile_ok(int n, int th);
 int fused_tiles(int n, int th);
 // Fills a descriptor (tensor maps from the cache); false if a map cannot be encoded.
-bool fill_desc(TerrainDesc& d, const TerrainSrc& s, int th, int tile0, TmaCache& cache);
-// k_hydro then k_transport over every tile of the batch's terrains; maps
-// holds MAPS_PER_TERRAIN tensor maps per terrain (device memory).
-void launch_fused_table(const BatchParams& bp, const CUtensorMap* maps, int total_tiles, int th, int* err,
-                        cudaStream_t st);
+bool fill_desc(TerrainDesc& d, const TerrainSrc& s, int th, TmaCache& cache);
+// Rows a warp of k_transport marches in a launch over `cells` cells.
+int chunk_rows(size_t cells);
+// Warps it runs for `rows` rows of an n x n terrain.
+int transport_tasks(int n, int rows, int t_rows);
+// One fused step (k_hydro, k_transport) over every tile of the batch's
+// terrains; maps holds MAPS_PER_TERRAIN tensor maps per terrain (device
+// memory); thermal: some terrain has talus passes.
+void launch_fused_table(const BatchParams& bp, const CUtensorMap* maps, int total_tiles, int th, bool thermal,
+                        ChainPos pos, int* err, cudaStream_t st);
 // Same for one terrain whose descriptor travels as a kernel parameter.
-void launch_fused_one(const TerrainDesc& td, int th, int* err, cudaStream_t st);
-// One kernel of the fused step (which 0: k_hydro, 1: k_transport) over tiles
-// [tile_lo, tile_lo + tiles) of a single world.
-void launch_fused_half(const TerrainDesc& td, int th, int which, int tile_lo, int tiles, int* err, cudaStream_t st);
+void launch_fused_one(const TerrainDesc& td, int th, ChainPos pos, int* err, cudaStream_t st);
+// One kernel of an unchained fused step (which 0: k_hydro, 1: k_transport)
+// over the descriptor's rows (whole tile rows) of a single world.
+void launch_fused_half(const TerrainDesc& td, int th, int which, int* err, cudaStream_t st);
 
 // ---- adjoint (hg_adjoint.cu) ----------------------------------------------------------
 // A step's state or its adjoint: rock, water, sediment, fL, fR, fT, fB.

@@ -456,7 +456,11 @@ int build_plan(Plan* p) {
             }
             s.u = w->u;
             s.v = w->v;
-            s.s_ero = w->s_ero;
+            // chained steps alternate between two buffers of eroded sediment
+            // (the second is a scratch plane of the per-pass talus passes)
+            float* se[2] = {w->s_ero, reinterpret_cast<float*>(w->td)};
+            s.s_ero = se[dir];
+            s.s_prev = se[dir ^ 1];
             s.b_ero = w->b_ero;
             s.step = w->d_step;
             p->smooth_dst[dir].resize(nt);
@@ -465,7 +469,7 @@ int build_plan(Plan* p) {
                 p->smooth_dst[dir][i] = s.out[S_ROCK];
                 s.out[S_ROCK] = reinterpret_cast<float*>(w->tc);
             }
-            if (!fill_desc(tab[i], s, p->th, tile0[i], w->tma))
+            if (!fill_desc(tab[i], s, p->th, w->tma))
                 return fail(HG_ERR_CUDA, "cuTensorMapEncodeTiled failed for a world buffer");
         }
         p->h_tab[dir] = tab;
@@ -473,10 +477,16 @@ int build_plan(Plan* p) {
             if (!p->bp[dir]) p->bp[dir] = new BatchParams();
             BatchParams& bp = *p->bp[dir];
             bp.nterr = (int)nt;
+            bp.tasks = 0;
+            size_t all = 0;
+            for (hg_world* w : p->worlds) all += cells(w);
             std::vector<CUtensorMap> maps(nt * MAPS_PER_TERRAIN);
             for (size_t i = 0; i < nt; ++i) {
                 bp.tile0[i] = tile0[i];
+                bp.task0[i] = bp.tasks;
                 bp.t[i] = tab[i].h;
+                bp.t[i].t_rows = chunk_rows(all);
+                bp.tasks += transport_tasks(p->worlds[i]->n, p->worlds[i]->n, bp.t[i].t_rows);
                 for (int m = 0; m < MAPS_PER_TERRAIN; ++m) maps[i * MAPS_PER_TERRAIN + m] = tab[i].maps[m];
             }
             if (!p->d_maps[dir]) HG_CUDA(cudaMalloc((void**)&p->d_maps[dir], sizeof(CUtensorMap) * maps.size()));
@@ -521,17 +531,31 @@ int plan_dir(const Plan* p) {
 
 // One fused step in direction `dir`: a single world takes its descriptor as
 // a kernel parameter, a batch launches over the device table.
-void launch_dir(Plan* p, int dir) {
-    if (p->worlds.size() == 1) launch_fused_one(p->h_tab[dir][0], p->th, p->err, p->stream);
-    else launch_fused_table(*p->bp[dir], p->d_maps[dir], p->total, p->th, p->err, p->stream);
+void launch_dir(Plan* p, int dir, ChainPos pos) {
+    if (p->worlds.size() == 1) {
+        launch_fused_one(p->h_tab[dir][0], p->th, pos, p->err, p->stream);
+    } else {
+        bool thermal = false;
+        for (const TerrainDesc& d : p->h_tab[dir]) thermal = thermal || d.h.c.thermal;
+        launch_fused_table(*p->bp[dir], p->d_maps[dir], p->total, p->th, thermal, pos, p->err, p->stream);
+    }
     // smoothing (worlds with Kspeed[1] != 0): the fused kernels left the
     // step's rock in scratch (the per-pass thermal buffer); the per-pass
     // smoothing kernel writes it into the step's rock output
     for (size_t i = 0; i < p->worlds.size(); ++i) {
-        const TerrainHot& h = p->h_tab[dir][i].h;
-        if (h.c.smooth_m == 0.0f) continue;
-        launch_smooth(h.c, h.out[S_ROCK], p->smooth_dst[dir][i], p->stream);
+        const TerrainDesc& d = p->h_tab[dir][i];
+        if (d.h.c.smooth_m == 0.0f) continue;
+        launch_smooth(make_consts(p->worlds[i]), d.h.out[S_ROCK], p->smooth_dst[dir][i], p->stream);
     }
+}
+
+// `count` steps from direction `dir` on, chained (see ChainPos) unless a
+// world smooths its rock between its steps.
+void launch_steps(Plan* p, int dir, int count) {
+    bool chain = true;
+    for (const TerrainDesc& d : p->h_tab[dir]) chain = chain && d.h.c.smooth_m == 0.0f;
+    for (int k = 0; k < count; ++k)
+        launch_dir(p, (dir + k) & 1, chain ? ChainPos{k, k + 1 == count} : ChainPos{0, true});
 }
 
 // Brings a plan up to date (tables, device step counters, the graph that
@@ -550,7 +574,7 @@ int capture_steps(Plan* p, int dir, int which) {
     cudaGraph_t g = nullptr;
     const uint64_t before = g_launches.load();
     HG_CUDA(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
-    for (int k = 0; k < steps; ++k) launch_dir(p, (dir + k) & 1);
+    launch_steps(p, dir, steps);
     cudaError_t e = cudaStreamEndCapture(p->stream, &g);
     p->graph_launches[which] = g_launches.load() - before;  // captured, not run
     g_launches.fetch_sub(p->graph_launches[which]);
@@ -604,17 +628,18 @@ int run_plan(Plan* p, int nsteps, bool use_graph) {
             count_launch(p->graph_launches[0]);
         }
     }
-    for (; k < nsteps; ++k) {
+    if (!ref_rain) launch_steps(p, dir, nsteps - k);  // (k is even: still direction dir)
+    for (; ref_rain && k < nsteps; ++k) {
         const int d = (dir + k) & 1;
-        if (ref_rain)  // the step's input water: the buffers of direction d at the plan's build
-            for (int i = 0; i < nt; ++i) {
-                hg_world* w = p->worlds[i];
-                if (w->opt.rain_mode != HG_RAIN_REFERENCE) continue;
-                const auto& in = d == 0 ? p->key_cur[i] : p->key_alt[i];
-                rain_pass(w, StepConsts{}, w->step + (uint64_t)k + 1, in[S_ROCK], nullptr,
-                          const_cast<float*>(in[S_WATER]), p->stream);
-            }
-        launch_dir(p, d);
+        // the step's input water: the buffers of direction d at the plan's build
+        for (int i = 0; i < nt; ++i) {
+            hg_world* w = p->worlds[i];
+            if (w->opt.rain_mode != HG_RAIN_REFERENCE) continue;
+            const auto& in = d == 0 ? p->key_cur[i] : p->key_alt[i];
+            rain_pass(w, StepConsts{}, w->step + (uint64_t)k + 1, in[S_ROCK], nullptr,
+                      const_cast<float*>(in[S_WATER]), p->stream);
+        }
+        launch_dir(p, d, ChainPos{0, true});
     }
     HG_CUDA(cudaGetLastError());
     for (hg_world* w : p->worlds) {
@@ -1638,10 +1663,10 @@ int hg_fused_pass(hg_world* w, int which) {
     src.s_ero = w->s_ero;
     src.b_ero = w->b_ero;
     TerrainDesc td;
-    if (!fill_desc(td, src, th, 0, w->tma)) return fail(HG_ERR_CUDA, "cuTensorMapEncodeTiled failed for a world buffer");
-    const int tiles_x = w->n / 64;
-    launch_fused_half(td, th, which, (w->row_lo / th) * tiles_x, ((w->row_hi - w->row_lo) / th) * tiles_x, w->err,
-                      st);
+    if (!fill_desc(td, src, th, w->tma)) return fail(HG_ERR_CUDA, "cuTensorMapEncodeTiled failed for a world buffer");
+    td.row_lo = w->row_lo;
+    td.row_hi = w->row_hi;
+    launch_fused_half(td, th, which, w->err, st);
     if (which == 1) {  // the step's outputs become the state (k_transport advanced the device counter)
         for (int f = 0; f < S_COUNT; ++f) std::swap(w->cur[f], w->alt[f]);
         w->step += 1;
@@ -2083,9 +2108,14 @@ int recompute_segment(hg_tape* t, int s, int len, const StepConsts& cst, int th,
         src.v = sl + c;
         src.s_ero = sl + 2 * c;
         src.b_ero = sl + 3 * c;
-        if (!fill_desc(td, src, th, 0, t->tma))
+        // a chain: step j gathers step j - 1's sediment and keeps it in its
+        // input state, which the reverse sweep reads
+        src.uv_prev = -(ptrdiff_t)(kSlotFields * c);
+        src.s_prev = j > 0 ? src.s_ero + src.uv_prev : nullptr;
+        src.s_keep = j > 0 ? const_cast<float*>(src.in[S_SED]) : nullptr;
+        if (!fill_desc(td, src, th, t->tma))
             return fail(HG_ERR_CUDA, "cuTensorMapEncodeTiled failed for a tape buffer");
-        launch_fused_one(td, th, w->err, st);
+        launch_fused_one(td, th, ChainPos{j, j + 1 == len}, w->err, st);
     }
     HG_CUDA(cudaGetLastError());
     return HG_OK;

@@ -1,0 +1,68 @@
+"""Chains of fused steps: several steps in one call (the sediment gather runs
+in the next step's first kernel) against the same steps one call at a time,
+bit for bit, with and without talus passes, by direct launches and by graph,
+for batches of unlike worlds, and where k_transport's strips and chunks end
+unevenly."""
+import numpy as np
+import pytest
+
+import hydrogen as H
+
+pytestmark = pytest.mark.gpu
+
+
+def make(n, cfg="config2", smooth=False, seed=0, graph=H.HG_AUTO, thermal=True):
+    w = H.World(n)
+    w.init_heightmap(H.noise(seed=seed))
+    H.configure(w, cfg)
+    s = H.settings_config2() if thermal else H.settings_config1()
+    if smooth:
+        s.Kspeed[1] = 2.0
+    w.set_erosion(s)
+    w.set_options(H.options(H.RAIN_BERNOULLI, p=0.02, seed=seed, graph=graph))
+    return w
+
+
+def assert_same(a, b, ctx):
+    for f in H.STATE_FIELDS:
+        x, y = a.download(f), b.download(f)
+        assert np.array_equal(x, y), f"{ctx} {f}: {np.count_nonzero(x != y)} cells differ"
+    assert a.step_count == b.step_count
+
+
+@pytest.mark.parametrize("thermal", [True, False])
+@pytest.mark.parametrize("graph", [0, 1])
+@pytest.mark.parametrize("calls", [[2], [3, 1, 2], [5], [9, 8, 3]])
+def test_chained_steps_equal_single_steps(thermal, graph, calls):
+    a, b = make(192, graph=graph, thermal=thermal), make(192, graph=graph, thermal=thermal)
+    for k in calls:
+        a.step(k, H.MODE_FUSED)
+        for _ in range(k):
+            b.step(1, H.MODE_FUSED)
+        assert_same(a, b, f"after {a.step_count} steps")
+
+
+@pytest.mark.parametrize("smooth", [False, True])
+def test_batch_of_unlike_worlds_in_a_chain(smooth):
+    def worlds():
+        return [make(64, seed=1), make(320, seed=2, thermal=False), make(192, seed=3, smooth=smooth),
+                make(128, cfg="config1", seed=4)]
+
+    a, b = worlds(), worlds()
+    batch = H.Batch(a)
+    batch.step(5)
+    batch.step(1)
+    batch.sync()
+    for w in b:
+        w.step(6, H.MODE_PLAIN)
+    for i, (x, y) in enumerate(zip(a, b)):
+        assert_same(x, y, f"terrain {i}")
+    batch.close()
+
+
+@pytest.mark.parametrize("n", [64, 960, 1536])
+def test_strips_and_chunks_against_per_pass(n):
+    a, b = make(n, seed=5), make(n, seed=5)
+    a.step(3, H.MODE_FUSED)
+    b.step(3, H.MODE_PLAIN)
+    assert_same(a, b, f"{n}")
