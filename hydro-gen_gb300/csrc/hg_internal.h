@@ -38,7 +38,9 @@ void launch_thermal_in(const StepConsts& c, const float* rock, const float4* tc,
 void launch_smooth(const StepConsts& c, const float* rock, float* rock_o, cudaStream_t st);
 
 // ---- the reference's terrain generator and rain (hg_terrain.cu) --------------------
-void launch_ref_heightmap(const hg_map_settings& cfg, int n, float* rock, float* dirt, cudaStream_t st);
+// (zero: up to 20 fields to clear in the same launch)
+void launch_ref_heightmap(const hg_map_settings& cfg, int n, float* rock, float* dirt, float* const* zero, int nzero,
+                          cudaStream_t st);
 // water += the reference's rain at frame time `time`; dirt may be nullptr (one layer)
 void launch_ref_rain(const hg_rain_settings& rs, const hg_map_settings& map, float time, int n, const float* rock,
                      const float* dirt, float* water, cudaStream_t st);
@@ -68,6 +70,8 @@ struct RenderInput {
     const float* sed0;
     const float* sed1;   // nullptr: one-layer world
     float4* hm;          // n*n packed heightmap texels (written)
+    float* total;        // n*n totals (written)
+    float2* ground;      // n*n (rock, dirt) (written)
     float2* sed;         // n*n packed sediment texels (written when displayed)
 };
 // packs the heightmap and renders width x height pixels into rgba_dev

@@ -5,7 +5,9 @@
 //   k_pack_heightmap   the world's fields as the shader's heightmap texels
 //                      (rock, dirt, water, total = rock + dirt + water) and
 //                      the sediment texels (rock, dirt), one float4 / float2
-//                      per cell, so a bilinear tap is one 16-byte load
+//                      per cell, so a bilinear tap is one 16-byte load; and
+//                      the two planes the marches read: the total, and
+//                      (rock, dirt)
 //   k_render           one thread per pixel: primary march on the total
 //                      height, water refraction / reflection marches, shadow
 //                      march, material shading, fog, sky, gamma
@@ -113,10 +115,11 @@ __device__ __forceinline__ float rm_exp(float x) { return rm_exp2(x * 1.44269504
 
 constexpr float MAX_DIST = 2048.0f;  // glsl/rendering.glsl:40-41
 constexpr int MAX_STEPS = 1024;
-constexpr int KIND_TOTAL = 3, KIND_TERRAIN = 4;
 
 struct Scene {
     const float4* hm;  // (rock, dirt, water, total)
+    const float* total;    // the marches' planes: total, (rock, dirt)
+    const float2* ground;
     const float2* sed;
     int n;
     float max_height;
@@ -158,33 +161,32 @@ __device__ __forceinline__ float4 tex_bilinear(const Scene& S, float px, float p
     return r;
 }
 
-// the march's height at (px, py): rock + dirt (terrain rays) or the total
-// (primary rays), the same bilinear channels tex_bilinear gives
-__device__ __forceinline__ float tex_height(const Scene& S, float px, float py, bool terrain) {
-    if (!(px > -2.0f && px < (float)S.n + 1.0f && py > -2.0f && py < (float)S.n + 1.0f))
-        return terrain ? 0.0f + 0.0f : 0.0f;
-    const int ix = (int)px, iy = (int)py;
-    const float fx = fract_(px), fy = fract_(py);
-    const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float4 a, b, c, d;
-    if ((unsigned)ix < (unsigned)(S.n - 1) && (unsigned)iy < (unsigned)(S.n - 1)) {
-        const float4* q = S.hm + (size_t)iy * S.n + ix;
-        a = __ldg(q);
-        b = __ldg(q + 1);
-        c = __ldg(q + S.n);
-        d = __ldg(q + S.n + 1);
-    } else {
-        auto t = [&](int x, int y) {
-            return (x >= 0 && x < S.n && y >= 0 && y < S.n) ? __ldg(S.hm + (size_t)y * S.n + x) : z;
-        };
-        a = t(ix, iy);
-        b = t(ix + 1, iy);
-        c = t(ix, iy + 1);
-        d = t(ix + 1, iy + 1);
+// The march's height at (px, py): rock + dirt (terrain rays) or the total
+// (primary rays), the same bilinear channels tex_bilinear gives.  The march
+// was held by the load pipe (75 % busy with four 16-byte taps a step) and by
+// issue slots (72 %): it reads a plane of totals or of (rock, dirt) pairs, a
+// quarter or half of the texel, and takes the texel index from an add of 2^23
+// that rounds toward zero (an index outside [0, n - 2], a negative or NaN
+// coordinate too, fails the unsigned test and goes the general way).
+template <bool TERRAIN>
+__device__ __forceinline__ float tex_height(const Scene& S, float px, float py) {
+    const float wx = __fadd_rz(px, 0x1p23f), wy = __fadd_rz(py, 0x1p23f);
+    const uint32_t ix = __float_as_uint(wx) - 0x4b000000u, iy = __float_as_uint(wy) - 0x4b000000u;
+    if ((ix < (uint32_t)(S.n - 1)) & (iy < (uint32_t)(S.n - 1))) {  // all four taps inside
+        const float fx = px - (wx - 0x1p23f), fy = py - (wy - 0x1p23f);
+        const size_t q = (size_t)iy * S.n + ix;
+        if (TERRAIN) {
+            const float2* p = S.ground + q;
+            const float2 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + S.n), d = __ldg(p + S.n + 1);
+            const float2 w = pf(fx), h = gmix2(gmix2(a, b, w), gmix2(c, d, w), pf(fy));
+            return h.x + h.y;
+        }
+        const float* p = S.total + q;
+        const float a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + S.n), d = __ldg(p + S.n + 1);
+        return gmix(gmix(a, b, fx), gmix(c, d, fx), fy);
     }
-    if (terrain)
-        return gmix(gmix(a.x, b.x, fx), gmix(c.x, d.x, fx), fy) + gmix(gmix(a.y, b.y, fx), gmix(c.y, d.y, fx), fy);
-    return gmix(gmix(a.w, b.w, fx), gmix(c.w, d.w, fx), fy);
+    const float4 t = tex_bilinear(S, px, py);
+    return TERRAIN ? t.x + t.y : t.w;
 }
 
 __device__ __forceinline__ float2 sed_bilinear(const Scene& S, float px, float py) {
@@ -207,33 +209,37 @@ struct Ray {
     float4 terr;
 };
 
-// raymarch (glsl/rendering.glsl:462-516)
-__device__ __noinline__ Ray raymarch(const Scene S, V3 o, V3 d, float max_d, int max_iter, int kind) {
-    float dist = 0.001f, d_dist = 0.1f;
-    const bool terrain = kind == KIND_TERRAIN;
-    if (terrain) {
-        dist = 0.0f;
-        d_dist = 0.1e-12f;
-    }
+// raymarch (glsl/rendering.glsl:462-516).  TERRAIN: the ray follows rock +
+// dirt; PENUMBRA: it keeps the smallest 12 d_dist / dist (shadow rays, the
+// only ones whose w is read), else w is 1 or 0.
+template <bool TERRAIN, bool PENUMBRA>
+__device__ __noinline__ Ray raymarch(const Scene S, V3 o, V3 d, float max_d, int max_iter) {
+    float dist = TERRAIN ? 0.0f : 0.001f, d_dist = TERRAIN ? 0.1e-12f : 0.1f;
     float min_sdf = 1.0f;
+    const bool up = d.y >= 0.0f, down = d.y < 0.0f;
     // each step needs only the marched height; the full texel (terr) is
     // sampled again where the ray stops
     V3 last = o;
     bool sampled = false;
     for (int i = 0; i < max_iter; ++i) {
         const V3 sp = add(o, scl(d, dist));
-        const float t_height = tex_height(S, sp.x, sp.z, terrain);
         last = sp;
         sampled = true;
-        if ((sp.y > S.max_height && d.y >= 0.0f) || (sp.y <= 0.0f && d.y < 0.0f)) break;
-        const float d_height = sp.y - t_height;
+        if ((up & (sp.y > S.max_height)) | (down & (sp.y <= 0.0f))) break;
+        const float d_height = sp.y - tex_height<TERRAIN>(S, sp.x, sp.z);
         if (fabsf(d_height) <= 0.05f) {
             const V3 q = sub(sp, scl(d, 0.05f));
             return Ray{q, 0.0f, dist - 0.05f, tex_bilinear(S, q.x, q.z)};
         } else if (d_height < 0.0f) {
             return Ray{add(o, scl(d, dist)), min_sdf, dist, tex_bilinear(S, sp.x, sp.z)};
         }
-        min_sdf = gmin(min_sdf, 12.0f * d_dist / dist);
+        if (PENUMBRA) {
+            const float num = 12.0f * d_dist;
+            float q;
+            if (num_range(num) & den_range(dist) & (fabsf(num) <= 0x1p80f)) q = div_recip(num, dist, rcp_newton(dist));
+            else q = num / dist;
+            min_sdf = fminf(min_sdf, q);
+        }
         if (dist > max_d) return Ray{sp, min_sdf, max_d, tex_bilinear(S, sp.x, sp.z)};
         d_dist = S.prec * d_height;
         dist += d_dist;
@@ -325,7 +331,7 @@ __device__ __noinline__ Shade shade(const Scene S, const Ray ray, V3 normal, boo
     const float shadow_diff = S.max_height - ray.pos.y;
     const float shadow_scale = shadow_diff / -S.light.y;
     const float shadow_max = len(scl(S.light, shadow_scale));
-    const Ray shadow = raymarch(S, ray.pos, neg(S.light), shadow_max, MAX_STEPS / 2, KIND_TERRAIN);
+    const Ray shadow = raymarch<true, true>(S, ray.pos, neg(S.light), shadow_max, MAX_STEPS / 2);
     const float amb_factor = gclamp(0.5f + 0.5f * -normal.y, 0.0f, 1.0f);
     V3 ambient, diffuse;
     if (is_water) {
@@ -367,12 +373,12 @@ __device__ V3 refract_ray(V3 n, V3 d, float eta) {
 __device__ V3 water_color(const Scene& S, const Ray& w_ray, V3 dir, float sundot) {
     const V3 w_norm = water_normal(S, w_ray.pos.x, w_ray.pos.z);
     const V3 refract_dir = refract_ray(w_norm, dir, 1.0f / 1.3f);
-    Ray t_ray = raymarch(S, w_ray.pos, neg(refract_dir), MAX_DIST / 8.0f, MAX_STEPS / 4, KIND_TERRAIN);
+    Ray t_ray = raymarch<true, false>(S, w_ray.pos, neg(refract_dir), MAX_DIST / 8.0f, MAX_STEPS / 4);
     const float water_vol = t_ray.dist;
     t_ray.dist += w_ray.dist;
     const V3 t_shad = terrain_color(S, t_ray, dir, sundot);
     const V3 w_refl = reflect(dir, w_norm);
-    Ray wrefl_ray = raymarch(S, w_ray.pos, w_refl, MAX_DIST, MAX_STEPS, KIND_TERRAIN);
+    Ray wrefl_ray = raymarch<true, false>(S, w_ray.pos, w_refl, MAX_DIST, MAX_STEPS);
     const Shade w_shad = shade(S, w_ray, w_norm, true);
     V3 water_col = w_shad.rgb;
     const float refl_sundot = gclamp(dot(w_refl, neg(S.light)), 0.0f, 1.0f);
@@ -443,7 +449,7 @@ __global__ void __launch_bounds__(128, 8) k_render(const RenderArgs a) {
     const float4 re = to_world(a, make_float4(cx, cy, 1.0f, 1.0f));
     const V3 dir = normalize(v3(re.x - rs.x, re.y - rs.y, re.z - rs.z));
 
-    const Ray ray = raymarch(S, a.pos, dir, MAX_DIST, MAX_STEPS, KIND_TOTAL);
+    const Ray ray = raymarch<false, false>(S, a.pos, dir, MAX_DIST, MAX_STEPS);
     const float sundot = gclamp(dot(dir, neg(S.light)), 0.0f, 1.0f);
     const float pxz = ray.pos.x * 1.0f, pzz = ray.pos.z * 1.0f;
     const float water_h = gmin(1.0f, smoothstep(1e-4f, 1.0f, ray.terr.z));
@@ -485,10 +491,13 @@ __global__ void __launch_bounds__(128, 8) k_render(const RenderArgs a) {
 __global__ void k_pack_heightmap(const float* __restrict__ rock, const float* __restrict__ dirt,
                                  const float* __restrict__ water, const float* __restrict__ s0,
                                  const float* __restrict__ s1, size_t count, float4* __restrict__ hm,
-                                 float2* __restrict__ sed) {
+                                 float* __restrict__ total, float2* __restrict__ ground, float2* __restrict__ sed) {
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
         const float r = rock[i], g = dirt ? dirt[i] : 0.0f, b = water[i];
-        hm[i] = make_float4(r, g, b, r + g + b);
+        const float t = r + g + b;
+        hm[i] = make_float4(r, g, b, t);
+        total[i] = t;
+        ground[i] = make_float2(r, g);
         if (sed) sed[i] = make_float2(s0[i], s1 ? s1[i] : 0.0f);
     }
 }
@@ -532,12 +541,12 @@ int render_image(const RenderInput& in, const hg_camera& cam, int width, int hei
     const size_t cells = (size_t)in.n * in.n;
     const int blocks = (int)std::min<size_t>((cells + 255) / 256, 152 * 16);
     k_pack_heightmap<<<blocks, 256, 0, st>>>(in.rock, in.dirt, in.water, in.sed0, in.sed1, cells, in.hm,
-                                             cam.display_sediment ? in.sed : nullptr);
+                                             in.total, in.ground, cam.display_sediment ? in.sed : nullptr);
     count_launch();
     // the light direction, normalize(vec3(0, -0.7, 1)), in float as the kernel would
     const float lx = 0.0f, ly = -0.7f, lz = 1.0f;
     const float ll = std::sqrt(lx * lx + ly * ly + lz * lz);
-    a.S = Scene{in.hm, in.sed, in.n, in.max_height, cam.prec, V3{lx / ll, ly / ll, lz / ll}};
+    a.S = Scene{in.hm, in.total, in.ground, in.sed, in.n, in.max_height, cam.prec, V3{lx / ll, ly / ll, lz / ll}};
     a.pos = V3{cam.pos[0], cam.pos[1], cam.pos[2]};
     a.draw_water = cam.draw_water;
     a.display_sediment = cam.display_sediment;

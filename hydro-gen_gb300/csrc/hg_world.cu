@@ -122,7 +122,7 @@ struct hg_world {
     double* red_d = nullptr;  // FP64 partials + result
     std::vector<hg_tape*> tapes;     // live tapes of this world (freed with it)
     hg::Particles* parts = nullptr;  // particle mode: droplets and momentum map
-    float4* r_hm = nullptr;          // ray-marcher: packed heightmap texels
+    float4* r_hm = nullptr;          // ray-marcher: packed heightmap texels and the marches' planes
     float2* r_sed = nullptr;         // ray-marcher: packed sediment texels
     uint8_t* r_rgba = nullptr;       // hg_render: device image
     float* r_rgb = nullptr;
@@ -960,20 +960,22 @@ int reset_particles(hg_world* w) {
     return HG_OK;
 }
 
-// every state field (and the dirt layer's) back to zero
-int zero_state(hg_world* w) {
-    size_t bytes = cells(w) * sizeof(float);
+// every state field (and the dirt layer's) that starts a world at zero
+std::vector<float*> state_fields(const hg_world* w) {
+    std::vector<float*> v;
     for (int f = 0; f < S_COUNT; ++f) {
-        HG_CUDA(cudaMemsetAsync(w->cur[f], 0, bytes, w->stream));
-        HG_CUDA(cudaMemsetAsync(w->alt[f], 0, bytes, w->stream));
+        v.push_back(w->cur[f]);
+        v.push_back(w->alt[f]);
     }
-    HG_CUDA(cudaMemsetAsync(w->u, 0, bytes, w->stream));
-    HG_CUDA(cudaMemsetAsync(w->v, 0, bytes, w->stream));
-    HG_CUDA(cudaMemsetAsync(w->vz, 0, bytes, w->stream));
+    for (float* p : {w->u, w->v, w->vz}) v.push_back(p);
     for (int k = 0; k < 2 && w->layers == 2; ++k) {
-        HG_CUDA(cudaMemsetAsync(w->dirt[k], 0, bytes, w->stream));
-        HG_CUDA(cudaMemsetAsync(w->sdirt[k], 0, bytes, w->stream));
+        v.push_back(w->dirt[k]);
+        v.push_back(w->sdirt[k]);
     }
+    return v;
+}
+int zero_state(hg_world* w) {
+    for (float* p : state_fields(w)) HG_CUDA(cudaMemsetAsync(p, 0, cells(w) * sizeof(float), w->stream));
     if (w->parts) return reset_particles(w);
     return HG_OK;
 }
@@ -1025,8 +1027,12 @@ int hg_init_reference_heightmap(hg_world* w, const hg_map_settings* s) {
     int rc = check_map_settings(s);
     if (rc != HG_OK) return rc;
     DeviceGuard g(w->device);
-    if ((rc = zero_state(w)) != HG_OK) return rc;
-    launch_ref_heightmap(*s, w->n, w->cur[S_ROCK], w->layers == 2 ? w->dirt[0] : nullptr, w->stream);
+    if (w->parts && (rc = reset_particles(w)) != HG_OK) return rc;
+    float* dirt = w->layers == 2 ? w->dirt[0] : nullptr;
+    std::vector<float*> zero = state_fields(w);  // all but what the generator writes
+    zero.erase(std::remove_if(zero.begin(), zero.end(), [&](float* p) { return p == w->cur[S_ROCK] || p == dirt; }),
+               zero.end());
+    launch_ref_heightmap(*s, w->n, w->cur[S_ROCK], dirt, zero.data(), (int)zero.size(), w->stream);
     HG_CUDA(cudaGetLastError());
     w->map = *s;
     w->version += 1;
@@ -1091,10 +1097,13 @@ int hg_render_device(hg_world* w, const hg_camera* cam, int width, int height, u
     if (!(cam->prec > 0.0f) || !std::isfinite(cam->prec)) return fail(HG_ERR_INVALID, "prec must be positive");
     DeviceGuard g(w->device);
     const size_t bytes = cells(w);
-    if (!w->r_hm) HG_CUDA(cudaMalloc((void**)&w->r_hm, bytes * sizeof(float4)));
+    // heightmap texels, (rock, dirt) plane, total plane: 7 floats a cell
+    if (!w->r_hm) HG_CUDA(cudaMalloc((void**)&w->r_hm, bytes * 7 * sizeof(float)));
+    float2* ground = reinterpret_cast<float2*>(w->r_hm + bytes);
+    float* total = reinterpret_cast<float*>(ground + bytes);
     if (cam->display_sediment && !w->r_sed) HG_CUDA(cudaMalloc((void**)&w->r_sed, bytes * sizeof(float2)));
     RenderInput in{w->n, w->map.max_height, w->map.hmap_dims[0], w->cur[S_ROCK], w->layers == 2 ? w->dirt[0] : nullptr,
-                   w->cur[S_WATER], w->cur[S_SED], w->layers == 2 ? w->sdirt[0] : nullptr, w->r_hm, w->r_sed};
+                   w->cur[S_WATER], w->cur[S_SED], w->layers == 2 ? w->sdirt[0] : nullptr, w->r_hm, total, ground, w->r_sed};
     int rc = render_image(in, *cam, width, height, rgba_dev, rgb_dev, w->stream);
     if (rc != HG_OK) return fail(rc, "singular view or perspective matrix");
     HG_CUDA(cudaGetLastError());
