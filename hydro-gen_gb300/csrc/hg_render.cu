@@ -92,7 +92,8 @@ __device__ __forceinline__ float rm_log2(float x) {
         m *= 0.5f;
         e += 1;
     }
-    const float s = (m - 1.0f) / (m + 1.0f);
+    // the divisor lies in [1.7, 2.5]: the correctly rounded quotient without a range check
+    const float s = div_recip(m - 1.0f, m + 1.0f, rcp_newton(m + 1.0f));
     const float s2 = s * s;
     float q = 1.0f / 9.0f;
     q = q * s2 + 1.0f / 7.0f;
@@ -103,14 +104,18 @@ __device__ __forceinline__ float rm_log2(float x) {
     return (float)e + ln_m * 1.44269504088896341f;
 }
 
-// pow(x, y) for the shader's bases: NaN below 0 (GLSL leaves it undefined),
-// 0^y = 0 (y > 0) or 1 (y == 0), otherwise exp2(y log2 x)
-__device__ __forceinline__ float rm_pow(float x, float y) {
-    if (!(x >= 0.0f)) return __int_as_float(0x7fc00000);
-    if (x == 0.0f) return y > 0.0f ? 0.0f : (y == 0.0f ? 1.0f : __int_as_float(0x7f800000));
-    if (x == __int_as_float(0x7f800000)) return y > 0.0f ? x : (y == 0.0f ? 1.0f : 0.0f);
-    return rm_exp2(y * rm_log2(x));
+// pow(x, y) for the shader's bases and exponents (y > 0): NaN below 0 (GLSL
+// leaves it undefined), 0^y = 0, otherwise exp2(y log2 x).  lg is rm_log2(x)
+// (of 1 where x is not a positive finite number), shared by the powers of one
+// base.
+__device__ __forceinline__ float pow_log(float x) {
+    return rm_log2(x > 0.0f && x < __int_as_float(0x7f800000) ? x : 1.0f);
 }
+__device__ __forceinline__ float rm_pow_lg(float x, float lg, float y) {
+    const float p = rm_exp2(y * lg);
+    return !(x >= 0.0f) ? __int_as_float(0x7fc00000) : x > 0.0f && x < __int_as_float(0x7f800000) ? p : x;
+}
+__device__ __forceinline__ float rm_pow(float x, float y) { return rm_pow_lg(x, pow_log(x), y); }
 __device__ __forceinline__ float rm_exp(float x) { return rm_exp2(x * 1.44269504088896341f); }
 
 constexpr float MAX_DIST = 2048.0f;  // glsl/rendering.glsl:40-41
@@ -168,25 +173,47 @@ __device__ __forceinline__ float4 tex_bilinear(const Scene& S, float px, float p
 // quarter or half of the texel, and takes the texel index from an add of 2^23
 // that rounds toward zero (an index outside [0, n - 2], a negative or NaN
 // coordinate too, fails the unsigned test and goes the general way).
-template <bool TERRAIN>
-__device__ __forceinline__ float tex_height(const Scene& S, float px, float py) {
+__device__ __forceinline__ float plane_mix(float a, float b, float fx) { return gmix(a, b, fx); }
+__device__ __forceinline__ float2 plane_mix(float2 a, float2 b, float fx) { return gmix2(a, b, pf(fx)); }
+template <class T>
+__device__ __forceinline__ T plane_bilinear(const T* __restrict__ plane, int n, float px, float py, T zero) {
     const float wx = __fadd_rz(px, 0x1p23f), wy = __fadd_rz(py, 0x1p23f);
     const uint32_t ix = __float_as_uint(wx) - 0x4b000000u, iy = __float_as_uint(wy) - 0x4b000000u;
-    if ((ix < (uint32_t)(S.n - 1)) & (iy < (uint32_t)(S.n - 1))) {  // all four taps inside
-        const float fx = px - (wx - 0x1p23f), fy = py - (wy - 0x1p23f);
-        const size_t q = (size_t)iy * S.n + ix;
-        if (TERRAIN) {
-            const float2* p = S.ground + q;
-            const float2 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + S.n), d = __ldg(p + S.n + 1);
-            const float2 w = pf(fx), h = gmix2(gmix2(a, b, w), gmix2(c, d, w), pf(fy));
-            return h.x + h.y;
-        }
-        const float* p = S.total + q;
-        const float a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + S.n), d = __ldg(p + S.n + 1);
-        return gmix(gmix(a, b, fx), gmix(c, d, fx), fy);
+    T a, b, c, d;
+    float fx, fy;
+    if ((ix < (uint32_t)(n - 1)) & (iy < (uint32_t)(n - 1))) {  // all four taps inside
+        fx = px - (wx - 0x1p23f);
+        fy = py - (wy - 0x1p23f);
+        const T* p = plane + (size_t)iy * n + ix;
+        a = __ldg(p);
+        b = __ldg(p + 1);
+        c = __ldg(p + n);
+        d = __ldg(p + n + 1);
+    } else {
+        // every tap is outside the map beyond these bounds (and for NaN)
+        if (!(px > -2.0f && px < (float)n + 1.0f && py > -2.0f && py < (float)n + 1.0f)) return zero;
+        const int jx = (int)px, jy = (int)py;
+        fx = fract_(px);
+        fy = fract_(py);
+        auto t = [&](int x, int y) { return (x >= 0 && x < n && y >= 0 && y < n) ? __ldg(plane + (size_t)y * n + x) : zero; };
+        a = t(jx, jy);
+        b = t(jx + 1, jy);
+        c = t(jx, jy + 1);
+        d = t(jx + 1, jy + 1);
     }
-    const float4 t = tex_bilinear(S, px, py);
-    return TERRAIN ? t.x + t.y : t.w;
+    return plane_mix(plane_mix(a, b, fx), plane_mix(c, d, fx), fy);
+}
+__device__ __forceinline__ float2 tex_ground(const Scene& S, float px, float py) {
+    return plane_bilinear(S.ground, S.n, px, py, make_float2(0.0f, 0.0f));
+}
+__device__ __forceinline__ float tex_total(const Scene& S, float px, float py) {
+    return plane_bilinear(S.total, S.n, px, py, 0.0f);
+}
+template <bool TERRAIN>
+__device__ __forceinline__ float tex_height(const Scene& S, float px, float py) {
+    if (!TERRAIN) return tex_total(S, px, py);
+    const float2 h = tex_ground(S, px, py);
+    return h.x + h.y;
 }
 
 __device__ __forceinline__ float2 sed_bilinear(const Scene& S, float px, float py) {
@@ -212,40 +239,57 @@ struct Ray {
 // raymarch (glsl/rendering.glsl:462-516).  TERRAIN: the ray follows rock +
 // dirt; PENUMBRA: it keeps the smallest 12 d_dist / dist (shadow rays, the
 // only ones whose w is read), else w is 1 or 0.
+//
+// A step has one exit test; which of the shader's exits it was is settled
+// after the loop (their order decides where several hold).
 template <bool TERRAIN, bool PENUMBRA>
 __device__ __noinline__ Ray raymarch(const Scene S, V3 o, V3 d, float max_d, int max_iter) {
+    const float nan = __int_as_float(0x7fffffff);  // compares false: a limit that does not apply
+    const float top = d.y >= 0.0f ? S.max_height : nan, bottom = d.y < 0.0f ? 0.0f : nan;
     float dist = TERRAIN ? 0.0f : 0.001f, d_dist = TERRAIN ? 0.1e-12f : 0.1f;
-    float min_sdf = 1.0f;
-    const bool up = d.y >= 0.0f, down = d.y < 0.0f;
-    // each step needs only the marched height; the full texel (terr) is
-    // sampled again where the ray stops
-    V3 last = o;
-    bool sampled = false;
+    float min_sdf = 1.0f, dh = 0.0f;
+    V3 sp = o;
+    bool out = true;  // left the height range, or ran out of steps
+    auto penumbra = [&]() {
+        const float num = 12.0f * d_dist;
+        float q = div_recip(num, dist, rcp_newton(dist));
+        if (!(num_range(num) & den_range(dist) & (fabsf(num) <= 0x1p80f))) q = num / dist;
+        min_sdf = fminf(min_sdf, q);
+    };
+#pragma unroll 1
     for (int i = 0; i < max_iter; ++i) {
-        const V3 sp = add(o, scl(d, dist));
-        last = sp;
-        sampled = true;
-        if ((up & (sp.y > S.max_height)) | (down & (sp.y <= 0.0f))) break;
-        const float d_height = sp.y - tex_height<TERRAIN>(S, sp.x, sp.z);
-        if (fabsf(d_height) <= 0.05f) {
-            const V3 q = sub(sp, scl(d, 0.05f));
-            return Ray{q, 0.0f, dist - 0.05f, tex_bilinear(S, q.x, q.z)};
-        } else if (d_height < 0.0f) {
-            return Ray{add(o, scl(d, dist)), min_sdf, dist, tex_bilinear(S, sp.x, sp.z)};
-        }
-        if (PENUMBRA) {
-            const float num = 12.0f * d_dist;
-            float q;
-            if (num_range(num) & den_range(dist) & (fabsf(num) <= 0x1p80f)) q = div_recip(num, dist, rcp_newton(dist));
-            else q = num / dist;
-            min_sdf = fminf(min_sdf, q);
-        }
-        if (dist > max_d) return Ray{sp, min_sdf, max_d, tex_bilinear(S, sp.x, sp.z)};
-        d_dist = S.prec * d_height;
+        sp = add(o, scl(d, dist));
+        dh = sp.y - tex_height<TERRAIN>(S, sp.x, sp.z);
+        out = (sp.y > top) | (sp.y <= bottom);
+        if (out | (dh <= 0.05f) | (dist > max_d)) break;  // (a NaN height goes on)
+        out = true;
+        if (PENUMBRA) penumbra();
+        d_dist = S.prec * dh;
         dist += d_dist;
     }
-    const float4 terr = sampled ? tex_bilinear(S, last.x, last.z) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    return Ray{add(o, scl(d, max_d)), min_sdf, max_d, terr};
+    // each step needs only the marched height; the full texel is sampled
+    // where the ray stops (nothing reads a shadow ray's)
+    Ray r;
+    float2 at = make_float2(sp.x, sp.z);
+    r.w = min_sdf;
+    r.dist = max_d;
+    if (out) {
+        r.pos = add(o, scl(d, max_d));
+    } else if (fabsf(dh) <= 0.05f) {
+        r.pos = sub(sp, scl(d, 0.05f));
+        at = make_float2(r.pos.x, r.pos.z);
+        r.w = 0.0f;
+        r.dist = dist - 0.05f;
+    } else if (dh < 0.0f) {
+        r.pos = sp;
+        r.dist = dist;
+    } else {
+        if (PENUMBRA) penumbra();
+        r.w = min_sdf;
+        r.pos = sp;
+    }
+    r.terr = PENUMBRA || max_iter < 1 ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : tex_bilinear(S, at.x, at.y);
+    return r;
 }
 
 __device__ __forceinline__ float fog_mix(float f) { return gclamp(f * f, 0.0f, 1.0f); }
@@ -286,8 +330,8 @@ __device__ __forceinline__ V3 sky_base() { return v3(0.3f, 0.5f, 0.85f); }
 
 // get_img_normal (:160-172): terrain normal from rock + dirt
 __device__ V3 terrain_normal(const Scene& S, float x, float z) {
-    const float4 r = tex_bilinear(S, x + 1.0f, z + 0.0f), l = tex_bilinear(S, x + -1.0f, z + 0.0f);
-    const float4 b = tex_bilinear(S, x + 0.0f, z + -1.0f), t = tex_bilinear(S, x + 0.0f, z + 1.0f);
+    const float2 r = tex_ground(S, x + 1.0f, z + 0.0f), l = tex_ground(S, x + -1.0f, z + 0.0f);
+    const float2 b = tex_ground(S, x + 0.0f, z + -1.0f), t = tex_ground(S, x + 0.0f, z + 1.0f);
     const float dx = r.x + r.y - l.x - l.y;
     const float dz = t.x + t.y - b.x - b.y;
     return normalize(cross(v3(2.0f, dx, 0.0f), v3(0.0f, dz, 2.0f)));
@@ -295,8 +339,8 @@ __device__ V3 terrain_normal(const Scene& S, float x, float z) {
 
 // get_img_normal_w (:148-157): water surface normal from the total height
 __device__ V3 water_normal(const Scene& S, float x, float z) {
-    const float dx = tex_bilinear(S, x + 1.0f, z + 0.0f).w - tex_bilinear(S, x + -1.0f, z + 0.0f).w;
-    const float dz = tex_bilinear(S, x + 0.0f, z + 1.0f).w - tex_bilinear(S, x + 0.0f, z + -1.0f).w;
+    const float dx = tex_total(S, x + 1.0f, z + 0.0f) - tex_total(S, x + -1.0f, z + 0.0f);
+    const float dz = tex_total(S, x + 0.0f, z + 1.0f) - tex_total(S, x + 0.0f, z + -1.0f);
     return normalize(cross(v3(2.0f, dx, 0.0f), v3(0.0f, dz, 2.0f)));
 }
 
@@ -309,16 +353,18 @@ __device__ V3 fog_color(V3 col, float ray_dist, float sundot) {
 }
 
 // get_sky_color (:182-220)
-__device__ V3 sky_color(V3 dir, float sundot) {
+__device__ __noinline__ V3 sky_color(V3 dir, float sundot) {
     const float diry = dir.y;
     const float dd = diry * diry * 0.37f;
     const V3 s = sky_base();
     V3 col = v3(s.x - dd, s.y - dd, s.z - dd);
-    col = mix3(col, scl(v3(0.7f, 0.75f, 0.85f), 0.85f), rm_pow(1.0f - gmax(diry, 0.0f), 4.0f));
-    col = add(col, scl(scl(v3(1.0f, 0.7f, 0.4f), 0.25f), rm_pow(sundot, 5.0f)));
-    col = add(col, scl(scl(v3(1.0f, 0.8f, 0.6f), 0.25f), rm_pow(sundot, 64.0f)));
-    col = add(col, scl(scl(v3(1.0f, 0.8f, 0.6f), 0.2f), rm_pow(sundot, 512.0f)));
-    return mix3(col, scl(v3(0.4f, 0.65f, 1.0f), 0.68f), rm_pow(1.0f - gmax(diry, 0.0f), 16.0f));
+    const float hz = 1.0f - gmax(diry, 0.0f);
+    const float lh = pow_log(hz), ls = pow_log(sundot);
+    col = mix3(col, scl(v3(0.7f, 0.75f, 0.85f), 0.85f), rm_pow_lg(hz, lh, 4.0f));
+    col = add(col, scl(scl(v3(1.0f, 0.7f, 0.4f), 0.25f), rm_pow_lg(sundot, ls, 5.0f)));
+    col = add(col, scl(scl(v3(1.0f, 0.8f, 0.6f), 0.25f), rm_pow_lg(sundot, ls, 64.0f)));
+    col = add(col, scl(scl(v3(1.0f, 0.8f, 0.6f), 0.2f), rm_pow_lg(sundot, ls, 512.0f)));
+    return mix3(col, scl(v3(0.4f, 0.65f, 1.0f), 0.68f), rm_pow_lg(hz, lh, 16.0f));
 }
 
 struct Shade {
@@ -352,11 +398,12 @@ __device__ __noinline__ Shade shade(const Scene S, const Ray ray, V3 normal, boo
 }
 
 // get_terrain_color (:289-302)
-__device__ V3 terrain_color(const Scene& S, const Ray& ray, V3 dir, float sundot) {
+// sky: sky_color(dir, sundot)
+__device__ V3 terrain_color(const Scene& S, const Ray& ray, float sundot, V3 sky) {
     const V3 normal = terrain_normal(S, ray.pos.x, ray.pos.z);
     V3 col = shade(S, ray, normal, false).rgb;
     col = fog_color(col, ray.dist, sundot);
-    return mix3(col, sky_color(dir, sundot), fog_mix(ray.dist / MAX_DIST));
+    return mix3(col, sky, fog_mix(ray.dist / MAX_DIST));
 }
 
 // refractCameraRay (:304-317)
@@ -370,13 +417,13 @@ __device__ V3 refract_ray(V3 n, V3 d, float eta) {
 }
 
 // get_water_color (:319-391)
-__device__ V3 water_color(const Scene& S, const Ray& w_ray, V3 dir, float sundot) {
+__device__ V3 water_color(const Scene& S, const Ray& w_ray, V3 dir, float sundot, V3 sky) {
     const V3 w_norm = water_normal(S, w_ray.pos.x, w_ray.pos.z);
     const V3 refract_dir = refract_ray(w_norm, dir, 1.0f / 1.3f);
     Ray t_ray = raymarch<true, false>(S, w_ray.pos, neg(refract_dir), MAX_DIST / 8.0f, MAX_STEPS / 4);
     const float water_vol = t_ray.dist;
     t_ray.dist += w_ray.dist;
-    const V3 t_shad = terrain_color(S, t_ray, dir, sundot);
+    const V3 t_shad = terrain_color(S, t_ray, sundot, sky);
     const V3 w_refl = reflect(dir, w_norm);
     Ray wrefl_ray = raymarch<true, false>(S, w_ray.pos, w_refl, MAX_DIST, MAX_STEPS);
     const Shade w_shad = shade(S, w_ray, w_norm, true);
@@ -392,7 +439,7 @@ __device__ V3 water_color(const Scene& S, const Ray& w_ray, V3 dir, float sundot
     } else {
         wrefl_ray.dist += w_ray.dist;
         water_col = mix3(t_shad, water_col, gmin(1.0f, water_vol / 2.0f));
-        water_col = mix3(water_col, terrain_color(S, wrefl_ray, w_refl, refl_sundot), w_shad.w);
+        water_col = mix3(water_col, terrain_color(S, wrefl_ray, refl_sundot, wrefl_skycol), w_shad.w);
         water_col = mix3(t_shad, water_col, fresnel);
         water_col = mix3(water_col, wrefl_skycol, fog_mix(wrefl_ray.dist / MAX_DIST));
     }
@@ -453,17 +500,18 @@ __global__ void __launch_bounds__(128, 8) k_render(const RenderArgs a) {
     const float sundot = gclamp(dot(dir, neg(S.light)), 0.0f, 1.0f);
     const float pxz = ray.pos.x * 1.0f, pzz = ray.pos.z * 1.0f;
     const float water_h = gmin(1.0f, smoothstep(1e-4f, 1.0f, ray.terr.z));
+    const V3 sky = sky_color(dir, sundot);
     V3 color;
     if (pxz < 0.0f || pxz >= (float)S.n || pzz < 0.0f || pzz >= (float)S.n) {
-        color = sky_color(dir, sundot);
+        color = sky;
     } else if (ray.dist >= MAX_DIST) {
-        color = sky_color(dir, sundot);
+        color = sky;
     } else if (water_h > 1e-12f && a.draw_water) {
-        V3 wc = water_color(S, ray, dir, sundot);
+        V3 wc = water_color(S, ray, dir, sundot, sky);
         wc = fog_color(wc, ray.dist, sundot);
-        color = mix3(wc, sky_color(dir, sundot), fog_mix(ray.dist / MAX_DIST));
+        color = mix3(wc, sky, fog_mix(ray.dist / MAX_DIST));
     } else {
-        color = terrain_color(S, ray, dir, sundot);
+        color = terrain_color(S, ray, sundot, sky);
     }
     if (a.display_sediment) {
         const float2 sd = sed_bilinear(S, ray.pos.x, ray.pos.z);
