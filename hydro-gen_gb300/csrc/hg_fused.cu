@@ -64,10 +64,10 @@ constexpr int HX = 4;            // halo columns: 16-byte aligned TMA boxes
 constexpr int RW = TW + 2 * HX;  // 72
 enum { H_B = 0, H_D, H_FL, H_FR, H_FT, H_FB, H_S, H_N };
 
-// Geometry of a 64 x TH tile: TH = 16 with 256 threads or TH = 8 with 128.
+// Geometry of a 64 x TH tile, TH = 16 or 8: 256 threads with two pairs of cells or one.
 template <int TH>
 struct Geo {
-    static constexpr int NTH = TH * 16;
+    static constexpr int NTH = 256;
     static constexpr int H_RH = TH + 2, H_BOX = RW * H_RH;
     static constexpr int H_RC = ((H_BOX + 31) / 32) * 32;  // 128-byte aligned array stride
     static constexpr int CPT = TW * TH / NTH;             // cells per thread in k_hydro (4)
@@ -325,7 +325,7 @@ __device__ __forceinline__ void hydro_block(const TerrainHot& td, const CUtensor
 // Batch form: the terrain records are a kernel parameter (constant bank),
 // the block finds its terrain by binary search.
 template <int TH, bool CHAIN>
-__global__ void __launch_bounds__(Geo<TH>::NTH, TH == 16 ? 4 : 8) k_hydro(const __grid_constant__ BatchParams bp,
+__global__ void __launch_bounds__(Geo<TH>::NTH, 4) k_hydro(const __grid_constant__ BatchParams bp,
                                                         const CUtensorMap* __restrict__ maps, int index, int* err) {
     const int t = find_terrain(bp.tile0, bp.nterr, blockIdx.x);
     const unsigned tile = blockIdx.x - bp.tile0[t], tiles_x = bp.t[t].tiles_x;
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(Geo<TH>::NTH, TH == 16 ? 4 : 8) k_hydro(const 
 // Single-world form: the whole descriptor, tensor maps included, is a kernel
 // parameter.  SPLIT as for hydro_block: the host picks it by world size.
 template <int TH, bool SPLIT, bool CHAIN>
-__global__ void __launch_bounds__(Geo<TH>::NTH, TH == 16 ? 4 : 8) k_hydro1(const __grid_constant__ TerrainDesc td, int index, int* err) {
+__global__ void __launch_bounds__(Geo<TH>::NTH, 4) k_hydro1(const __grid_constant__ TerrainDesc td, int index, int* err) {
     hydro_block<TH, SPLIT, CHAIN>(td.h, td.maps, blockIdx.x * TW, td.row_lo + blockIdx.y * TH, index, err);
 }
 
@@ -482,6 +482,75 @@ __global__ void __launch_bounds__(32 * T_WARPS, SED ? T_BLOCKS_SED : T_BLOCKS)
     if (w < tasks) transport_task<SED>(td.h, w, td.row_lo, td.row_hi, steps);
 }
 
+// A small world's k_transport: a block takes 8 rows of a strip, one warp per
+// row (and one for the row above and below), so a launch is one pass over
+// short straight code instead of a march of several rows per warp: there the
+// time is latency, and chunks of few rows recompute half of their outflows.
+// Rows exchange the outflows they send each other through shared memory.
+constexpr int R_ROWS = 8, R_WARPS = R_ROWS + 2;
+template <bool SED>
+__device__ __forceinline__ void transport_rows(const TerrainHot& td, int strip, int y0) {
+    __shared__ float2 to_up[R_WARPS][3][32], to_down[R_WARPS][3][32];  // T, RT, LT / B, RB, LB at the receiving column
+    const unsigned FULL = 0xffffffffu;
+    const StepConsts1& c = td.c;
+    const int n = c.n;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int x = strip * SW - 2 + 2 * lane, y = y0 - 1 + warp;
+    const bool in = x >= 0 && x < n;
+    const bool own = in && lane >= 1 && lane <= SW / 2 && warp >= 1 && warp <= R_ROWS;
+    const size_t gi = (size_t)y * n + x;
+    float2 u, v;
+    if (SED && own) {
+        u = ldg2(td.u + gi);
+        v = ldg2(td.v + gi);
+    }
+    if (!c.thermal) {
+        if (SED && own) st2(td.out[S_SED] + gi, gather_sediment(c, td.s_ero, x, y, u, v));
+        return;
+    }
+    auto rock = [&](int r) { return in && r >= 0 && r < n ? ldg2(td.b_ero + (size_t)r * n + x) : pf(FAR_HEIGHT); };
+    const float2 c0 = rock(y - 1), c1 = rock(y), c2 = rock(y + 1);
+    float2 sed;
+    if (SED && own) sed = gather_sediment(c, td.s_ero, x, y, u, v);
+    float2 o[8];
+    if (y >= 0 && y < n) {
+        const RockRow dn = rock_row(c0), md = rock_row(c1), up = rock_row(c2);
+        float2 dm[8] = {sub2(md.c, md.l), sub2(md.c, md.r), sub2(md.c, up.c), sub2(md.c, dn.c),
+                        sub2(md.c, up.l), sub2(md.c, up.r), sub2(md.c, dn.l), sub2(md.c, dn.r)};
+        cell_thermal_outflows_dh2(c.dt, c.Kalpha0, c.Kspeed0, c.talus_x_cross, c.talus_b_diag, c.fast_div, md.c, dm, o);
+    }
+    if (!in || y < 0 || y >= n) {
+#pragma unroll
+        for (int d = 0; d < 8; ++d) o[d] = pf(0.0f);
+    }
+    auto from_left = [&](float2 a) { return make_float2(__shfl_up_sync(FULL, a.y, 1), a.x); };
+    auto from_right = [&](float2 a) { return make_float2(a.y, __shfl_down_sync(FULL, a.x, 1)); };
+    to_up[warp][0][lane] = o[2];
+    to_up[warp][1][lane] = from_left(o[5]);
+    to_up[warp][2][lane] = from_right(o[4]);
+    to_down[warp][0][lane] = o[3];
+    to_down[warp][1][lane] = from_left(o[7]);
+    to_down[warp][2][lane] = from_right(o[6]);
+    const float2 lr = add2(from_left(o[1]), from_right(o[0]));
+    float2 osum = sub2(pf(0.0f), o[0]);
+#pragma unroll
+    for (int d = 1; d < 8; ++d) osum = sub2(osum, o[d]);
+    __syncthreads();
+    if (!own) return;
+    // the shader's order: L, R, T, B, LT, RT, LB, RB
+    float2 inf = add2(add2(lr, to_down[warp + 1][0][lane]), to_up[warp - 1][0][lane]);
+    inf = add2(add2(inf, to_down[warp + 1][1][lane]), to_down[warp + 1][2][lane]);
+    inf = add2(add2(inf, to_up[warp - 1][1][lane]), to_up[warp - 1][2][lane]);
+    st2(td.out[S_ROCK] + gi, add2(c1, add2(osum, inf)));
+    if (SED) st2(td.out[S_SED] + gi, sed);
+}
+
+template <bool SED>
+__global__ void __launch_bounds__(32 * R_WARPS, 2) k_transport_rows(const __grid_constant__ TerrainDesc td, int steps) {
+    transport_rows<SED>(td.h, blockIdx.x, td.row_lo + blockIdx.y * R_ROWS);
+    if (SED && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *td.h.step += (unsigned long long)steps;
+}
+
 // ---------------------------------------------------------------------------
 // tensor maps
 // ---------------------------------------------------------------------------
@@ -590,7 +659,21 @@ void launch_hydro_table(const BatchParams& bp, const CUtensorMap* maps, int tile
     count_launch();
 }
 
+// Worlds up to this side run k_transport_rows: a step with talus takes, in
+// three worlds in turn / alone, 3.4 / 8.3 us at 256² (marching: 4.6 / 11.2),
+// 5.0 / 10.4 at 448² (6.0 / 12.4), 11.7 / 18.3 at 768² (12.4 / 21.8); at
+// 1024² marching takes 19.8 / 29.1 against 22.8 / 26.1, from 1536² on less
+// both ways.
+constexpr int ROWS_MAX_N = 768;
+
 void launch_transport1(const TerrainDesc& td, bool last, int steps, cudaStream_t st) {
+    if (td.h.c.n <= ROWS_MAX_N) {
+        const dim3 grid(strips(td.h.c.n), (td.row_hi - td.row_lo) / R_ROWS);
+        if (last) k_transport_rows<true><<<grid, 32 * R_WARPS, 0, st>>>(td, steps);
+        else k_transport_rows<false><<<grid, 32 * R_WARPS, 0, st>>>(td, 0);
+        count_launch();
+        return;
+    }
     const int tasks = transport_tasks(td.h.c.n, td.row_hi - td.row_lo, td.h.t_rows);
     if (last) k_transport1<true><<<task_blocks(tasks), 32 * T_WARPS, 0, st>>>(td, tasks, steps);
     else k_transport1<false><<<task_blocks(tasks), 32 * T_WARPS, 0, st>>>(td, tasks, 0);

@@ -679,6 +679,14 @@ int fused_run(Plan** plans, const std::vector<hg_world*>& worlds, Tuning& tune, 
         HG_CUDA(cudaEventCreate(&e0));
         HG_CUDA(cudaEventCreate(&e1));
         double best = 1e30;
+        // tiles of 8 rows give a launch more blocks and each thread one pair:
+        // less latency, which is what a small launch takes, but more halo to
+        // load.  Two steps from an idle queue show the latency and not the
+        // cost beside other work (1024² without talus: 12.2 us a step at 16
+        // rows, 15.2 at 8, three worlds in turn), so larger ones stay at 16.
+        size_t all = 0;
+        for (hg_world* w : worlds) all += cells(w);
+        const bool small = all <= (size_t)640 * 640;
         for (int cand = 0; cand < 4; ++cand) {
             int th = cand < 2 ? 16 : 8, graph = cand & 1;
             int dir = 0;
@@ -692,6 +700,7 @@ int fused_run(Plan** plans, const std::vector<hg_world*>& worlds, Tuning& tune, 
             float ms = 0;
             cudaEventElapsedTime(&ms, e0, e1);
             tune.ms[cand] = ms / 2.0;
+            if (th == 8 && !small) continue;
             if (tune.ms[cand] < best) { best = tune.ms[cand]; tune.th = th; tune.graph = graph; }
         }
         cudaEventDestroy(e0);
