@@ -86,6 +86,10 @@ struct Particles {
 
 using namespace hg;
 
+namespace hg {
+struct FusedGroup;
+}
+
 struct hg_world {
     int n = 0;
     int row_lo = 0, row_hi = 0;  // rows the per-pass kernels compute (hg_set_rows; all by default)
@@ -116,7 +120,7 @@ struct hg_world {
     bool dev_step_valid = false;           // d_step == step
     uint64_t version = 1;                  // bumps whenever settings, options or Ks change
     TmaCache tma;
-    hg::Plan* plans[2] = {};               // fused plans of this world alone, tile height 16 / 8
+    hg::FusedGroup* self = nullptr;        // this world alone as a group: its fused plans
     hg::Tuning tuning;                     // autotuned fused-step variant
     float* red_f = nullptr;   // min/max partials + result
     double* red_d = nullptr;  // FP64 partials + result
@@ -133,13 +137,24 @@ namespace hg {
 void release_tapes(hg_world* w);
 }  // namespace hg
 
+namespace hg {
+// Worlds whose fused steps share launches, with their plans (tile height 16
+// / 8) and stream.
+struct FusedGroup {
+    std::vector<hg_world*> worlds;
+    Plan* plans[2] = {};
+    cudaStream_t st = nullptr;
+};
+}  // namespace hg
+
 struct hg_batch {
     std::vector<hg_world*> worlds;
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev = nullptr;
     int* err = nullptr;
-    hg::Plan* plans[2] = {};
+    hg::FusedGroup groups[2];          // the table launches' groups of worlds (the second may be empty)
+    cudaStream_t stream2 = nullptr;    // the second group's stream
     hg::Tuning tuning;
 };
 
@@ -262,7 +277,9 @@ void free_world(hg_world* w) {
         cudaFree(w->sdirt[k]);
     }
     cudaFree(w->s_ero); cudaFree(w->b_ero); cudaFree(w->err); cudaFree(w->d_step);
-    for (Plan*& p : w->plans) destroy_plan(p);
+    if (w->self)
+        for (Plan*& p : w->self->plans) destroy_plan(p);
+    delete w->self;
     cudaFree(w->red_f); cudaFree(w->red_d);
     delete w->parts;
     w->parts = nullptr;
@@ -650,71 +667,120 @@ int run_plan(Plan* p, int nsteps, bool use_graph) {
     return HG_OK;
 }
 
-// Fused steps over `worlds` with the autotuned (or requested) variant.  The
+Plan* plan_for(FusedGroup& g, int th, int* err) {
+    Plan*& p = g.plans[th == 16 ? 0 : 1];
+    if (!p) {
+        p = new Plan();
+        p->worlds = g.worlds;
+        p->th = th;
+        p->stream = g.st;
+        p->err = err;
+    }
+    return p;
+}
+
+// The other groups' streams go on after the first group's.
+int fork_groups(FusedGroup* groups, int ngroups, cudaEvent_t ev) {
+    if (ngroups == 1) return HG_OK;
+    HG_CUDA(cudaEventRecord(ev, groups[0].st));
+    for (int g = 1; g < ngroups; ++g) HG_CUDA(cudaStreamWaitEvent(groups[g].st, ev, 0));
+    return HG_OK;
+}
+
+int check_groups(const FusedGroup* groups, int ngroups) {
+    for (int g = 0; g < ngroups; ++g)
+        for (const hg_world* w : groups[g].worlds) {
+            if (!fused_tile_ok(w->n, 16)) return fail(HG_ERR_UNSUPPORTED, "fused mode needs n divisible by 64");
+            if (w->layers != 1) return fail(HG_ERR_UNSUPPORTED, "the fused step covers one-layer worlds");
+        }
+    return HG_OK;
+}
+
+// Builds the groups' plans of both tile heights and captures their graphs.
+int fused_prepare(FusedGroup* groups, int ngroups, cudaEvent_t ev, int* err) {
+    int rc = check_groups(groups, ngroups), dir = 0;
+    if (rc == HG_OK) rc = fork_groups(groups, ngroups, ev);
+    for (int g = 0; g < ngroups && rc == HG_OK; ++g)
+        for (int th : {16, 8})
+            if (rc == HG_OK) rc = prepare_plan(plan_for(groups[g], th, err), true, &dir);
+    return rc;
+}
+
+// Fused steps over the groups' worlds with the autotuned (or requested) variant.  The
 // first call with at least 8 steps and no tuned choice times two steps of
 // each variant (tile height 16/8 x direct launches/graph replay); every
 // variant gives identical fields, so tuning steps are ordinary steps.  Graph
 // replay runs kLongGraph steps per replay while that many remain, then two.
-int fused_run(Plan** plans, const std::vector<hg_world*>& worlds, Tuning& tune, int req_th, int req_graph,
-              cudaStream_t st, int* err, int nsteps) {
-    for (hg_world* w : worlds) {
-        if (!fused_tile_ok(w->n, 16)) return fail(HG_ERR_UNSUPPORTED, "fused mode needs n divisible by 64");
-        if (w->layers != 1) return fail(HG_ERR_UNSUPPORTED, "the fused step covers one-layer worlds");
-    }
+// Groups run concurrently on their streams, forked from and joined to the
+// first group's (ev: one event, reused).
+int fused_run(FusedGroup* groups, int ngroups, cudaEvent_t ev, Tuning& tune, int req_th, int req_graph, int* err,
+              int nsteps) {
+    size_t all = 0;
+    int nworlds = 0;
+    for (int g = 0; g < ngroups; ++g)
+        for (hg_world* w : groups[g].worlds) {
+            all += cells(w);
+            nworlds += 1;
+        }
+    const int checked = check_groups(groups, ngroups);
+    if (checked != HG_OK) return checked;
     if (req_th != HG_AUTO && req_th != 16 && req_th != 8)
         return fail(HG_ERR_UNSUPPORTED, "fused tile height must be 16 or 8");
-    auto plan_for = [&](int th) -> Plan* {
-        Plan*& p = plans[th == 16 ? 0 : 1];
-        if (!p) {
-            p = new Plan();
-            p->worlds = worlds;
-            p->th = th;
-            p->stream = st;
-            p->err = err;
+    const cudaStream_t st = groups[0].st;
+    auto run_all = [&](int th, int count, bool graph) -> int {
+        int rc = fork_groups(groups, ngroups, ev);
+        for (int g = 0; g < ngroups && rc == HG_OK; ++g) rc = run_plan(plan_for(groups[g], th, err), count, graph);
+        for (int g = 1; g < ngroups; ++g) {
+            HG_CUDA(cudaEventRecord(ev, groups[g].st));
+            HG_CUDA(cudaStreamWaitEvent(st, ev, 0));
         }
-        return p;
+        return rc;
     };
     if (req_th == HG_AUTO && req_graph == HG_AUTO && tune.th == 0 && nsteps >= 8) {
-        cudaEvent_t e0, e1;
-        HG_CUDA(cudaEventCreate(&e0));
-        HG_CUDA(cudaEventCreate(&e1));
-        double best = 1e30;
         // tiles of 8 rows give a launch more blocks and each thread one pair:
         // less latency, which is what a small launch takes, but more halo to
-        // load.  Two steps from an idle queue show the latency and not the
-        // cost beside other work (1024² without talus: 12.2 us a step at 16
-        // rows, 15.2 at 8, three worlds in turn), so larger ones stay at 16.
-        size_t all = 0;
-        for (hg_world* w : worlds) all += cells(w);
+        // load (1024² without talus: 12.2 us a step at 16 rows, 15.2 at 8,
+        // three worlds in turn), so larger ones stay at 16.
         const bool small = all <= (size_t)640 * 640;
-        for (int cand = 0; cand < 4; ++cand) {
-            int th = cand < 2 ? 16 : 8, graph = cand & 1;
-            int dir = 0;
-            int rc0 = prepare_plan(plan_for(th), graph != 0, &dir);  // host work outside the timed span
-            if (rc0 != HG_OK) { cudaEventDestroy(e0); cudaEventDestroy(e1); return rc0; }
-            cudaEventRecord(e0, st);
-            int rc = run_plan(plan_for(th), 2, graph != 0);
-            cudaEventRecord(e1, st);
-            if (rc != HG_OK) { cudaEventDestroy(e0); cudaEventDestroy(e1); return rc; }
-            HG_CUDA(cudaEventSynchronize(e1));
-            float ms = 0;
-            cudaEventElapsedTime(&ms, e0, e1);
-            tune.ms[cand] = ms / 2.0;
-            if (th == 8 && !small) continue;
-            if (tune.ms[cand] < best) { best = tune.ms[cand]; tune.th = th; tune.graph = graph; }
+        // Host work (plans, graph captures) first; then the candidates are
+        // queued without a wait between them, so that each one's launches
+        // overlap the steps before it as they do in a run.
+        int rc = fused_prepare(groups, ngroups, ev, err);
+        if (rc != HG_OK) return rc;
+        cudaEvent_t mark[5] = {};
+        for (cudaEvent_t& e : mark)
+            if (rc == HG_OK && cudaEventCreate(&e) != cudaSuccess) rc = HG_ERR_CUDA;
+        if (rc == HG_OK) cudaEventRecord(mark[0], st);
+        for (int cand = 0; cand < 4 && rc == HG_OK; ++cand) {
+            rc = run_all(cand < 2 ? 16 : 8, 2, (cand & 1) != 0);
+            cudaEventRecord(mark[cand + 1], st);
         }
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
+        if (rc == HG_OK && cudaEventSynchronize(mark[4]) != cudaSuccess) rc = HG_ERR_CUDA;
+        double best = 1e30;
+        for (int cand = 0; cand < 4 && rc == HG_OK; ++cand) {
+            float ms = 0;
+            cudaEventElapsedTime(&ms, mark[cand], mark[cand + 1]);
+            tune.ms[cand] = ms / 2.0;
+            if (cand >= 2 && !small) continue;
+            if (tune.ms[cand] < best) {
+                best = tune.ms[cand];
+                tune.th = cand < 2 ? 16 : 8;
+                tune.graph = cand & 1;
+            }
+        }
+        for (cudaEvent_t e : mark)
+            if (e) cudaEventDestroy(e);
+        if (rc != HG_OK) return rc == HG_ERR_CUDA ? cuda_fail(cudaGetLastError(), "autotuning") : rc;
         nsteps -= 8;
         char m[160];
-        std::snprintf(m, sizeof m, "autotuner: %zu world(s), tile 64x%d, graph %s (ms/step: %.4f %.4f %.4f %.4f)",
-                      worlds.size(), tune.th, tune.graph ? "on" : "off", tune.ms[0], tune.ms[1], tune.ms[2],
+        std::snprintf(m, sizeof m, "autotuner: %d world(s), tile 64x%d, graph %s (ms/step: %.4f %.4f %.4f %.4f)",
+                      nworlds, tune.th, tune.graph ? "on" : "off", tune.ms[0], tune.ms[1], tune.ms[2],
                       tune.ms[3]);
         log_msg(HG_LOG_INFO, m);
     }
     int th = req_th != HG_AUTO ? req_th : (tune.th ? tune.th : 16);
     int graph = req_graph != HG_AUTO ? req_graph : (tune.th ? tune.graph : 1);
-    return run_plan(plan_for(th), nsteps, graph != 0);
+    return run_all(th, nsteps, graph != 0);
 }
 
 float* field_ptr(hg_world* w, int field) {
@@ -1581,8 +1647,12 @@ int hg_step(hg_world* w, int nsteps, int mode) {
         int rc = fused2_steps(w, nsteps);
         if (rc != HG_OK) return rc;
     } else if (nsteps > 0) {
-        std::vector<hg_world*> one{w};
-        int rc = fused_run(w->plans, one, w->tuning, w->opt.tile_y, w->opt.graph, st, w->err, nsteps);
+        if (!w->self) {
+            w->self = new FusedGroup();
+            w->self->worlds = {w};
+            w->self->st = st;
+        }
+        int rc = fused_run(w->self, 1, nullptr, w->tuning, w->opt.tile_y, w->opt.graph, w->err, nsteps);
         if (rc != HG_OK) return rc;
     }
     HG_CUDA(cudaGetLastError());
@@ -1731,6 +1801,10 @@ int hg_world_tuning(const hg_world* w, int* tile_y, int* graph, double ms[4]) {
 
 // ---- batches ---------------------------------------------------------------------
 
+namespace {
+constexpr size_t kTwoGroupCells = (size_t)3 << 20;
+}
+
 int hg_batch_create(hg_world* const* worlds, int count, hg_batch** out) {
     if (!out) return fail(HG_ERR_INVALID, "null output pointer");
     *out = nullptr;
@@ -1748,16 +1822,33 @@ int hg_batch_create(hg_world* const* worlds, int count, hg_batch** out) {
     b->worlds.assign(worlds, worlds + count);
     b->device = worlds[0]->device;
     cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream2, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaMalloc((void**)&b->err, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(b->err, 0, sizeof(int));
     if (e != cudaSuccess) {
         if (b->stream) cudaStreamDestroy(b->stream);
+        if (b->stream2) cudaStreamDestroy(b->stream2);
         if (b->ev) cudaEventDestroy(b->ev);
         cudaFree(b->err);
         delete b;
         return cuda_fail(e, "batch creation");
     }
+    // Two groups of like size (largest world first, each to the lighter
+    // group): one's k_hydro, bound by memory, overlaps the other's talus
+    // pass, bound by issue slots.  Below a step of about 50 us the fork and
+    // join cost more.
+    size_t total = 0, load[2] = {0, 0};
+    for (hg_world* w : b->worlds) total += cells(w);
+    std::vector<hg_world*> order = b->worlds;
+    std::stable_sort(order.begin(), order.end(), [](const hg_world* x, const hg_world* y) { return x->n > y->n; });
+    for (hg_world* w : order) {
+        const int g = total >= kTwoGroupCells && load[1] < load[0] ? 1 : 0;
+        b->groups[g].worlds.push_back(w);
+        load[g] += cells(w);
+    }
+    b->groups[0].st = b->stream;
+    b->groups[1].st = b->stream2;
     *out = b;
     return HG_OK;
 }
@@ -1766,9 +1857,11 @@ int hg_batch_destroy(hg_batch* b) {
     if (!b) return HG_OK;
     DeviceGuard g(b->device);
     cudaStreamSynchronize(b->stream);
-    for (Plan*& p : b->plans) destroy_plan(p);
+    for (FusedGroup& g : b->groups)
+        for (Plan*& p : g.plans) destroy_plan(p);
     cudaEventDestroy(b->ev);
     cudaStreamDestroy(b->stream);
+    cudaStreamDestroy(b->stream2);
     cudaFree(b->err);
     delete b;
     return HG_OK;
@@ -1796,6 +1889,7 @@ int hg_batch_step(hg_batch* b, int nsteps, int mode) {
         return HG_OK;
     }
     const hg_step_options& o = b->worlds[0]->opt;
+    const int ngroups = b->groups[1].worlds.empty() ? 1 : 2;
     const bool autotune = o.tile_y == HG_AUTO && o.graph == HG_AUTO;
     auto join_worlds = [&]() -> int {  // batch stream after every world's stream
         for (hg_world* w : b->worlds) {
@@ -1817,18 +1911,23 @@ int hg_batch_step(hg_batch* b, int nsteps, int mode) {
         return HG_OK;
     };
     if (autotune && b->tuning.th == 0 && nsteps >= 12) {
-        // Two untimed steps of per-world launches build (and capture) the
-        // worlds' own plans; the next two are timed.  fused_run then times the
-        // table variants; the faster form serves every later call.
+        // The table plans first (host work), then two untimed steps of
+        // per-world launches build and capture the worlds' own plans; the
+        // next two are timed, and fused_run times the table variants right
+        // behind them; the faster form serves every later call.
         cudaEvent_t e0, e1;
         HG_CUDA(cudaEventCreate(&e0));
         HG_CUDA(cudaEventCreate(&e1));
-        int rc = per_world(2);
+        int rc = join_worlds();
+        if (rc == HG_OK) rc = fused_prepare(b->groups, ngroups, b->ev, b->err);
+        if (rc == HG_OK) rc = release_worlds();
+        if (rc == HG_OK) rc = per_world(2);
         if (rc == HG_OK) rc = join_worlds();
         if (rc == HG_OK) rc = cudaEventRecord(e0, b->stream) == cudaSuccess ? release_worlds() : HG_ERR_CUDA;
         if (rc == HG_OK) rc = per_world(2);
         if (rc == HG_OK) rc = join_worlds();
         if (rc == HG_OK && cudaEventRecord(e1, b->stream) != cudaSuccess) rc = HG_ERR_CUDA;
+        if (rc == HG_OK) rc = fused_run(b->groups, ngroups, b->ev, b->tuning, o.tile_y, o.graph, b->err, 8);
         if (rc == HG_OK && cudaEventSynchronize(e1) != cudaSuccess) rc = HG_ERR_CUDA;
         float ms = 0;
         if (rc == HG_OK) cudaEventElapsedTime(&ms, e0, e1);
@@ -1836,11 +1935,7 @@ int hg_batch_step(hg_batch* b, int nsteps, int mode) {
         cudaEventDestroy(e1);
         if (rc != HG_OK) return rc == HG_ERR_CUDA ? cuda_fail(cudaGetLastError(), "batch tuning") : rc;
         b->tuning.ms_per_world = ms / 2.0;
-        nsteps -= 4;
-        if ((rc = join_worlds()) != HG_OK) return rc;
-        rc = fused_run(b->plans, b->worlds, b->tuning, o.tile_y, o.graph, b->stream, b->err, 8);
-        if (rc != HG_OK) return rc;
-        nsteps -= 8;
+        nsteps -= 12;
         double best = 1e30;
         for (double m : b->tuning.ms) best = std::min(best, m);
         b->tuning.per_world = b->tuning.ms_per_world < best ? 1 : 0;
@@ -1855,7 +1950,7 @@ int hg_batch_step(hg_batch* b, int nsteps, int mode) {
     // one table launch per kernel for every world: ordered after the worlds' streams
     int rc = join_worlds();
     if (rc != HG_OK) return rc;
-    rc = fused_run(b->plans, b->worlds, b->tuning, o.tile_y, o.graph, b->stream, b->err, nsteps);
+    rc = fused_run(b->groups, ngroups, b->ev, b->tuning, o.tile_y, o.graph, b->err, nsteps);
     int rc2 = release_worlds();
     return rc != HG_OK ? rc : rc2;
 }
