@@ -109,27 +109,6 @@ __device__ __forceinline__ RainStep rain_for(const RainBase& rb, unsigned long l
     return r;
 }
 
-// sediment_transport of the cells (x, y) and (x + 1, y): semi-Lagrangian
-// gather of the eroded sediment se (any reach)
-__device__ __forceinline__ float2 gather_sediment(const StepConsts1& c, const float* __restrict__ se, int x, int y,
-                                                  float2 u, float2 v) {
-    const int n = c.n;
-    const Trace2 tr = backtrace2(c, x, y, u, v);
-    float tap[4][2];
-#pragma unroll
-    for (int l = 0; l < 2; ++l) {
-        const int ix = (int)tr.ix[l], iy = (int)tr.iy[l];
-        const float* p = se + (size_t)iy * n + ix;
-        const bool hx = ix + 1 < n, hy = iy + 1 < n;
-        tap[0][l] = __ldg(p);
-        tap[1][l] = hx ? __ldg(p + 1) : 0.0f;
-        tap[2][l] = hy ? __ldg(p + n) : 0.0f;
-        tap[3][l] = hx & hy ? __ldg(p + n + 1) : 0.0f;
-    }
-    return bilinear_mix2(tr, make_float2(tap[0][0], tap[0][1]), make_float2(tap[1][0], tap[1][1]),
-                         make_float2(tap[2][0], tap[2][1]), make_float2(tap[3][0], tap[3][1]));
-}
-
 // ---------------------------------------------------------------------------
 // k_hydro
 // ---------------------------------------------------------------------------
@@ -265,7 +244,7 @@ __device__ __forceinline__ void hydro_tile(const TerrainHot& td, const CUtensorM
     const float* FB = sm + H_FB * H_RC;
     // Pairs of horizontally adjacent cells, a row of the tile per warp: 8-byte
     // shared loads and global stores, both cells in one f32x2 instruction
-    // (cell_hydro2).  Neighbours outside the grid read rock 0, flux 0 and
+    // (cell_flux2, cell_erosion_pair).  Neighbours outside the grid read rock 0, flux 0 and
     // total height FAR_HEIGHT from the tile (see the fill above); the
     // closed-boundary outflow zeroing runs in edge tiles.
     float* const rock_o = c.thermal ? td.b_ero : td.out[S_ROCK];  // no thermal pass: eroded rock is final
@@ -287,8 +266,10 @@ __device__ __forceinline__ void hydro_tile(const TerrainHot& td, const CUtensorM
         const float2 s = !CHAIN ? ld2(S + si) : k == 0 ? sed[0] : sed[PAIRS - 1];
         float2 Kls0 = pf(c.Kls0);
         if (c.ks_field) Kls0 = mul2(pf(c.dt), __ldg(reinterpret_cast<const float2*>(c.ks_field + gi)));
-        const Hydro2 o = cell_hydro2(c, x, y, EDGE, b, d1, s, fl, fr, ld2(FT + si), ld2(FB + si), wl, wr, wt,
-                                     wb, inl, inr, ld2(FB + si + RW), ld2(FT + si - RW), bl, br, bb, bt, Kls0);
+        const Flux2 o = cell_flux2(c, x, y, EDGE, add2(b, d1), d1, fl, fr, ld2(FT + si), ld2(FB + si), wl, wr, wt, wb,
+                                   inl, inr, ld2(FB + si + RW), ld2(FT + si - RW));
+        float2 be = b, se = s;
+        cell_erosion_pair(c, Kls0, o.vz, o.len, be, se, br, bl, bb, bt);
         st2(td.out[S_FL] + gi, o.fl);
         st2(td.out[S_FR] + gi, o.fr);
         st2(td.out[S_FT] + gi, o.ft);
@@ -297,8 +278,8 @@ __device__ __forceinline__ void hydro_tile(const TerrainHot& td, const CUtensorM
         st2(td.out[S_WATER] + gi, mul2(o.d2, pf(c.evap)));
         st2(td.u + gi, o.u);
         st2(td.v + gi, o.v);
-        st2(td.s_ero + gi, o.s);
-        st2(rock_o + gi, o.b);
+        st2(td.s_ero + gi, se);
+        st2(rock_o + gi, be);
     }
 }
 

@@ -1,7 +1,11 @@
 // Per-pass kernels: one kernel per GLSL pass of the grid step, FP32
-// structure-of-arrays fields, one cell per thread (rows of 32 cells per warp,
-// so every field access of a warp is a 128-byte coalesced line), Jacobi
-// ping-pong between passes as in the reference (src/erosion.cpp:158-200).
+// structure-of-arrays fields, two adjacent cells per thread (rows of 64 cells
+// per warp, 8-byte accesses, both cells in f32x2 instructions; the maps' side
+// is even), Jacobi ping-pong between passes as in the reference
+// (src/erosion.cpp:158-200).  Bound by issue slots (flux, talus outflows: 83
+// and 86 % busy with one cell per thread and built-in divisions) or by the
+// launch at sides around 1000; a step with talus at 1000²: 52 us with one
+// cell per thread, TIME with two.
 #include "hg_internal.h"
 
 namespace hg {
@@ -28,6 +32,16 @@ __global__ void k_rain(StepConsts c, RainStep r, float* __restrict__ water) {
     *p = d;
 }
 
+// the thread's pair of cells (x, y), (x + 1, y); false past the map or the rows
+__device__ __forceinline__ bool pair_at(const StepConsts& c, int& x, int& y, size_t& i) {
+    x = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    y = blockIdx.y * blockDim.y + threadIdx.y;
+    i = at(c.n, x, y);
+    return x < c.n && y >= c.row_lo && y < c.row_hi;
+}
+__device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ void st2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
+
 // glsl/hydro_flux.glsl:77-166
 __global__ void k_flux(StepConsts c, const float* __restrict__ rock, const float* __restrict__ water,
                        const float* __restrict__ fl, const float* __restrict__ fr,
@@ -35,92 +49,82 @@ __global__ void k_flux(StepConsts c, const float* __restrict__ rock, const float
                        float* __restrict__ water_o, float* __restrict__ fl_o, float* __restrict__ fr_o,
                        float* __restrict__ ft_o, float* __restrict__ fb_o, float* __restrict__ u_o,
                        float* __restrict__ v_o, float* __restrict__ vz_o) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y * blockDim.y + threadIdx.y;
+    int x, y;
+    size_t i;
+    if (!pair_at(c, x, y, i)) return;
     const int n = c.n;
-    if (x >= n || y < c.row_lo || y >= c.row_hi) return;
-    size_t i = at(n, x, y);
-    auto total = [&](int xx, int yy) -> float {
-        if (xx < 0 || xx >= n || yy < 0 || yy >= n) return FAR_HEIGHT;
-        size_t j = at(n, xx, yy);
-        return rock[j] + water[j];
-    };
-    float d1 = water[i];
-    float w_c = rock[i] + d1;
-    float inl = x > 0 ? fr[i - 1] : 0.0f;
-    float inr = x < n - 1 ? fl[i + 1] : 0.0f;
-    float int_ = y < n - 1 ? fb[i + n] : 0.0f;
-    float inb = y > 0 ? ft[i - n] : 0.0f;
-    FluxOut o = cell_flux(c, x, y, w_c, d1, fl[i], fr[i], ft[i], fb[i], total(x - 1, y), total(x + 1, y),
-                          total(x, y + 1), total(x, y - 1), inl, inr, int_, inb);
-    fl_o[i] = o.fl; fr_o[i] = o.fr; ft_o[i] = o.ft; fb_o[i] = o.fb;
-    water_o[i] = o.d2;
-    u_o[i] = o.u; v_o[i] = o.v; vz_o[i] = o.vz;
+    const bool hl = x > 0, hr = x + 2 < n, hb = y > 0, ht = y < n - 1;
+    const float2 d1 = ld2(water + i), w = add2(ld2(rock + i), d1);
+    const float2 f_l = ld2(fl + i), f_r = ld2(fr + i);
+    const float2 wl = make_float2(hl ? rock[i - 1] + water[i - 1] : FAR_HEIGHT, w.x);
+    const float2 wr = make_float2(w.y, hr ? rock[i + 2] + water[i + 2] : FAR_HEIGHT);
+    const float2 wt = ht ? add2(ld2(rock + i + n), ld2(water + i + n)) : pf(FAR_HEIGHT);
+    const float2 wb = hb ? add2(ld2(rock + i - n), ld2(water + i - n)) : pf(FAR_HEIGHT);
+    const float2 inl = make_float2(hl ? fr[i - 1] : 0.0f, f_r.x), inr = make_float2(f_l.y, hr ? fl[i + 2] : 0.0f);
+    const Flux2 o = cell_flux2(c, x, y, true, w, d1, f_l, f_r, ld2(ft + i), ld2(fb + i), wl, wr, wt, wb, inl, inr,
+                               ht ? ld2(fb + i + n) : pf(0.0f), hb ? ld2(ft + i - n) : pf(0.0f));
+    st2(fl_o + i, o.fl);
+    st2(fr_o + i, o.fr);
+    st2(ft_o + i, o.ft);
+    st2(fb_o + i, o.fb);
+    st2(water_o + i, o.d2);
+    st2(u_o + i, o.u);
+    st2(v_o + i, o.v);
+    st2(vz_o + i, o.vz);
 }
 
 // glsl/hydro_erosion.glsl:37-92
 __global__ void k_erosion(StepConsts c, const float* __restrict__ u, const float* __restrict__ v,
                           const float* __restrict__ vz, const float* __restrict__ rock,
                           float* __restrict__ rock_o, float* __restrict__ sed) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y * blockDim.y + threadIdx.y;
+    int x, y;
+    size_t i;
+    if (!pair_at(c, x, y, i)) return;
     const int n = c.n;
-    if (x >= n || y < c.row_lo || y >= c.row_hi) return;
-    size_t i = at(n, x, y);
-    float br = x < n - 1 ? rock[i + 1] : 0.0f;
-    float bl = x > 0 ? rock[i - 1] : 0.0f;
-    float bb = y > 0 ? rock[i - n] : 0.0f;
-    float bt = y < n - 1 ? rock[i + n] : 0.0f;
-    float b = rock[i], s = sed[i];
-    float Kls0 = c.ks_field ? c.dt * c.ks_field[i] : c.Kls0;
-    cell_erosion(c, Kls0, u[i], v[i], vz[i], b, s, br, bl, bb, bt);
-    rock_o[i] = b;
-    sed[i] = s;
+    float2 b = ld2(rock + i), s = ld2(sed + i);
+    const float2 bl = make_float2(x > 0 ? rock[i - 1] : 0.0f, b.x), br = make_float2(b.y, x + 2 < n ? rock[i + 2] : 0.0f);
+    const float2 bb = y > 0 ? ld2(rock + i - n) : pf(0.0f), bt = y < n - 1 ? ld2(rock + i + n) : pf(0.0f);
+    const float2 Kls0 = c.ks_field ? mul2(pf(c.dt), ld2(c.ks_field + i)) : pf(c.Kls0);
+    cell_erosion_pair(c, Kls0, ld2(vz + i), speed2(ld2(u + i), ld2(v + i)), b, s, br, bl, bb, bt);
+    st2(rock_o + i, b);
+    st2(sed + i, s);
 }
 
 // glsl/sediment_transport.glsl:66-93
 __global__ void k_sediment(StepConsts c, const float* __restrict__ u, const float* __restrict__ v,
                            const float* __restrict__ sed, float* __restrict__ sed_o,
                            float* __restrict__ water) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int n = c.n;
-    if (x >= n || y < c.row_lo || y >= c.row_hi) return;
-    size_t i = at(n, x, y);
-    float px, py;
-    backtrace(c, x, y, u[i], v[i], px, py);
-    int ix = (int)px, iy = (int)py;
-    auto tap = [&](int xx, int yy) -> float {
-        return (xx >= 0 && xx < n && yy >= 0 && yy < n) ? sed[at(n, xx, yy)] : 0.0f;
-    };
-    sed_o[i] = bilinear_mix(px, py, tap(ix, iy), tap(ix + 1, iy), tap(ix, iy + 1), tap(ix + 1, iy + 1));
-    water[i] = water[i] * c.evap;
+    int x, y;
+    size_t i;
+    if (!pair_at(c, x, y, i)) return;
+    st2(sed_o + i, gather_sediment(c, sed, x, y, ld2(u + i), ld2(v + i)));
+    st2(water + i, mul2(ld2(water + i), pf(c.evap)));
 }
-
-__constant__ int c_ox[8] = {-1, 1, 0, 0, -1, 1, -1, 1};
-__constant__ int c_oy[8] = {0, 0, 1, -1, 1, 1, -1, -1};
 
 // glsl/thermal_erosion.glsl:28-115, layer 0
 __global__ void k_thermal_out(StepConsts c, const float* __restrict__ rock, float4* __restrict__ tc,
                               float4* __restrict__ td) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y * blockDim.y + threadIdx.y;
+    int x, y;
+    size_t i;
+    if (!pair_at(c, x, y, i)) return;
     const int n = c.n;
-    if (x >= n || y < c.row_lo || y >= c.row_hi) return;
-    size_t i = at(n, x, y);
-    float b = rock[i];
-    float nb[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        int xx = x + c_ox[k], yy = y + c_oy[k];
-        nb[k] = (xx < 0 || xx >= n || yy < 0 || yy >= n) ? FAR_HEIGHT : rock[at(n, xx, yy)];
-    }
-    ThermalOut t = cell_thermal_ref(c, b, nb);
-    float o[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) o[k] = (t.mask >> k & 1u) ? t.S * (b - nb[k]) / t.bk : 0.0f;
-    tc[i] = make_float4(o[0], o[1], o[2], o[3]);
-    td[i] = make_float4(o[4], o[5], o[6], o[7]);
+    const bool hl = x > 0, hr = x + 2 < n;
+    auto row = [&](bool ok, size_t j, float2& m, float2& l, float2& r) {
+        m = ok ? ld2(rock + j) : pf(FAR_HEIGHT);
+        l = make_float2(ok && hl ? rock[j - 1] : FAR_HEIGHT, m.x);
+        r = make_float2(m.y, ok && hr ? rock[j + 2] : FAR_HEIGHT);
+    };
+    float2 b, bl, br, t, tl, tr, d, dl, dr;
+    row(true, i, b, bl, br);
+    row(y < n - 1, i + n, t, tl, tr);
+    row(y > 0, i - n, d, dl, dr);
+    float2 dm[8] = {sub2(b, bl), sub2(b, br), sub2(b, t), sub2(b, d), sub2(b, tl), sub2(b, tr), sub2(b, dl), sub2(b, dr)};
+    float2 o[8];
+    cell_thermal_outflows_dh2(c.dt, c.Kalpha0, c.Kspeed0, c.talus_x_cross, c.talus_b_diag, c.fast_div, b, dm, o);
+    tc[i] = make_float4(o[0].x, o[1].x, o[2].x, o[3].x);
+    tc[i + 1] = make_float4(o[0].y, o[1].y, o[2].y, o[3].y);
+    td[i] = make_float4(o[4].x, o[5].x, o[6].x, o[7].x);
+    td[i + 1] = make_float4(o[4].y, o[5].y, o[6].y, o[7].y);
 }
 
 // glsl/thermal_transport.glsl:31-65, layer 0
@@ -161,6 +165,7 @@ __global__ void k_smooth(StepConsts c, const float* __restrict__ rock, float* __
 }
 
 dim3 grid_for(int n) { return dim3((n + BX - 1) / BX, (n + BY - 1) / BY); }
+dim3 pairs_for(int n) { return dim3((n / 2 + BX - 1) / BX, (n + BY - 1) / BY); }
 
 }  // namespace
 
@@ -173,25 +178,25 @@ void launch_rain(const StepConsts& c, const RainStep& r, float* water, cudaStrea
 void launch_flux(const StepConsts& c, const float* rock, const float* water, const float* fl, const float* fr,
                  const float* ft, const float* fb, float* water_o, float* fl_o, float* fr_o, float* ft_o,
                  float* fb_o, float* u, float* v, float* vz, cudaStream_t st) {
-    k_flux<<<grid_for(c.n), dim3(BX, BY), 0, st>>>(c, rock, water, fl, fr, ft, fb, water_o, fl_o, fr_o, ft_o,
+    k_flux<<<pairs_for(c.n), dim3(BX, BY), 0, st>>>(c, rock, water, fl, fr, ft, fb, water_o, fl_o, fr_o, ft_o,
                                                    fb_o, u, v, vz);
     count_launch();
 }
 
 void launch_erosion(const StepConsts& c, const float* u, const float* v, const float* vz, const float* rock,
                     float* rock_o, float* sed_inout, cudaStream_t st) {
-    k_erosion<<<grid_for(c.n), dim3(BX, BY), 0, st>>>(c, u, v, vz, rock, rock_o, sed_inout);
+    k_erosion<<<pairs_for(c.n), dim3(BX, BY), 0, st>>>(c, u, v, vz, rock, rock_o, sed_inout);
     count_launch();
 }
 
 void launch_sediment(const StepConsts& c, const float* u, const float* v, const float* sed, float* sed_o,
                      float* water_inout, cudaStream_t st) {
-    k_sediment<<<grid_for(c.n), dim3(BX, BY), 0, st>>>(c, u, v, sed, sed_o, water_inout);
+    k_sediment<<<pairs_for(c.n), dim3(BX, BY), 0, st>>>(c, u, v, sed, sed_o, water_inout);
     count_launch();
 }
 
 void launch_thermal_out(const StepConsts& c, const float* rock, float4* tc, float4* td, cudaStream_t st) {
-    k_thermal_out<<<grid_for(c.n), dim3(BX, BY), 0, st>>>(c, rock, tc, td);
+    k_thermal_out<<<pairs_for(c.n), dim3(BX, BY), 0, st>>>(c, rock, tc, td);
     count_launch();
 }
 
