@@ -53,15 +53,13 @@
 #include <vector>
 
 #include "hg_internal.h"
+#include "hg_tile.cuh"
 #include "hg_tma.cuh"
 
 namespace hg {
 
 namespace {
 
-constexpr int TW = 64;
-constexpr int HX = 4;            // halo columns: 16-byte aligned TMA boxes
-constexpr int RW = TW + 2 * HX;  // 72
 enum { H_B = 0, H_D, H_FL, H_FR, H_FT, H_FB, H_S, H_N };
 
 // Geometry of a 64 x TH tile, TH = 16 or 8: 256 threads with two pairs of cells or one.
@@ -72,12 +70,6 @@ struct Geo {
     static constexpr int H_RC = ((H_BOX + 31) / 32) * 32;  // 128-byte aligned array stride
     static constexpr int CPT = TW * TH / NTH;             // cells per thread in k_hydro (4)
 };
-
-__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-__device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
-__device__ __forceinline__ float2 ldg2(const float* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
-__device__ __forceinline__ void st2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
 
 __device__ __forceinline__ int find_terrain(const int* tile0, int nterr, int tile) {
     int lo = 0, hi = nterr - 1;
@@ -112,31 +104,6 @@ __device__ __forceinline__ RainStep rain_for(const RainBase& rb, unsigned long l
 // ---------------------------------------------------------------------------
 // k_hydro
 // ---------------------------------------------------------------------------
-// Sets the cells of a staged box that lie outside the grid to v.  The box
-// (ROWS x RW cells, row 0 at global row gy0, column 0 at global column
-// gx0 = tx0 - HX) reaches past the grid only through its HX outer columns
-// on either side and its HALO outer rows on either side, so only those
-// are visited (a corner cell twice, with the same value).
-template <int ROWS, int HALO, int NTH>
-__device__ __forceinline__ void fill_outside(float* box, int gx0, int gy0, int n, float v, int tid) {
-    constexpr int SIDE = ROWS * 2 * HX;  // the outer columns of every row
-    constexpr int CAP = 2 * HALO * RW;   // the outer rows
-    for (int i = tid; i < SIDE + CAP; i += NTH) {
-        int r, col;
-        if (i < SIDE) {
-            r = i / (2 * HX);
-            const int k = i % (2 * HX);
-            col = k < HX ? k : RW - 2 * HX + k;
-        } else {
-            const int j = i - SIDE, rr = j / RW;
-            col = j % RW;
-            r = rr < HALO ? rr : ROWS - 2 * HALO + rr;
-        }
-        const int gx = gx0 + col, gy = gy0 + r;
-        if (gx < 0 || gx >= n || gy < 0 || gy >= n) box[r * RW + col] = v;
-    }
-}
-
 // EM: 0 inner tile, 1 edge tile (each its own code), 2 either, told at run
 // time by edge_rt (one code path for both)
 template <int TH, int EM, bool CHAIN>
@@ -333,28 +300,18 @@ __global__ void __launch_bounds__(Geo<TH>::NTH, 4) k_hydro1(const __grid_constan
 // one column around it, and those the rock one further), a chunk of R rows
 // recomputes the outflows of two rows.
 // ---------------------------------------------------------------------------
-constexpr int SW = 60;           // columns a warp's strip delivers
 constexpr int T_WARPS = 4;       // warps per block, each with its own strip
 // Blocks per SM: with the gather 5 (96 registers), without 6 (80).  More warps
 // at fewer registers spill, and leave no room for another world's k_hydro
 // beside them (4096², three worlds in turn: 262 us a step at 6 blocks, 299 at
 // 7, 324 at 8).
 constexpr int T_BLOCKS_SED = 5, T_BLOCKS = 6;
-// Warps a launch should have (two rounds of 152 SMs x 24 warps): fewer leave
-// SMs idle at the end of the launch, more recompute more rows.  One step at
+// Most warps a launch should have (two rounds of 152 SMs x 24 warps): fewer
+// leave SMs idle at the end of the launch, more recompute more rows, and just
+// over a round leaves the last one nearly empty.  One step at
 // 4096², alone / among other worlds' steps: one round 331 / 265 us, two 310 /
 // 262, three 302 / 266.
 constexpr int T_FILL = 2 * 152 * T_WARPS * T_BLOCKS;
-__host__ __device__ constexpr int strips(int n) { return (n + SW - 1) / SW; }
-
-// Eroded rock of a row's pair and its pairs one column to the left and right.
-struct RockRow {
-    float2 c, l, r;
-};
-__device__ __forceinline__ RockRow rock_row(float2 c) {
-    const unsigned FULL = 0xffffffffu;
-    return RockRow{c, make_float2(__shfl_up_sync(FULL, c.y, 1), c.x), make_float2(c.y, __shfl_down_sync(FULL, c.x, 1))};
-}
 
 // rows [y0, y1) of strip `strip`; SED: with the sediment gather
 template <bool SED>
@@ -410,8 +367,6 @@ __device__ __forceinline__ void transport_strip(const TerrainHot& td, int strip,
 #pragma unroll
             for (int d = 0; d < 8; ++d) o[d] = zero;
         }
-        auto from_left = [&](float2 a) { return make_float2(__shfl_up_sync(FULL, a.y, 1), a.x); };
-        auto from_right = [&](float2 a) { return make_float2(a.y, __shfl_down_sync(FULL, a.x, 1)); };
         // the row below: its inflows in the shader's order (L, R, T, B, LT,
         // RT, LB, RB), then rock + (its outflows' sum + inflow)
         const float2 rb = from_left(o[7]), lb = from_right(o[6]);
@@ -463,72 +418,19 @@ __global__ void __launch_bounds__(32 * T_WARPS, SED ? T_BLOCKS_SED : T_BLOCKS)
     if (w < tasks) transport_task<SED>(td.h, w, td.row_lo, td.row_hi, steps);
 }
 
-// A small world's k_transport: a block takes 8 rows of a strip, one warp per
-// row (and one for the row above and below), so a launch is one pass over
-// short straight code instead of a march of several rows per warp: there the
-// time is latency, and chunks of few rows recompute half of their outflows.
-// Rows exchange the outflows they send each other through shared memory.
-constexpr int R_ROWS = 8, R_WARPS = R_ROWS + 2;
 template <bool SED>
-__device__ __forceinline__ void transport_rows(const TerrainHot& td, int strip, int y0) {
-    __shared__ float2 to_up[R_WARPS][3][32], to_down[R_WARPS][3][32];  // T, RT, LT / B, RB, LB at the receiving column
-    const unsigned FULL = 0xffffffffu;
-    const StepConsts1& c = td.c;
-    const int n = c.n;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int x = strip * SW - 2 + 2 * lane, y = y0 - 1 + warp;
-    const bool in = x >= 0 && x < n;
-    const bool own = in && lane >= 1 && lane <= SW / 2 && warp >= 1 && warp <= R_ROWS;
-    const size_t gi = (size_t)y * n + x;
-    float2 u, v;
-    if (SED && own) {
-        u = ldg2(td.u + gi);
-        v = ldg2(td.v + gi);
-    }
-    if (!c.thermal) {
-        if (SED && own) st2(td.out[S_SED] + gi, gather_sediment(c, td.s_ero, x, y, u, v));
-        return;
-    }
-    auto rock = [&](int r) { return in && r >= 0 && r < n ? ldg2(td.b_ero + (size_t)r * n + x) : pf(FAR_HEIGHT); };
-    const float2 c0 = rock(y - 1), c1 = rock(y), c2 = rock(y + 1);
-    float2 sed;
-    if (SED && own) sed = gather_sediment(c, td.s_ero, x, y, u, v);
-    float2 o[8];
-    if (y >= 0 && y < n) {
-        const RockRow dn = rock_row(c0), md = rock_row(c1), up = rock_row(c2);
-        float2 dm[8] = {sub2(md.c, md.l), sub2(md.c, md.r), sub2(md.c, up.c), sub2(md.c, dn.c),
-                        sub2(md.c, up.l), sub2(md.c, up.r), sub2(md.c, dn.l), sub2(md.c, dn.r)};
-        cell_thermal_outflows_dh2(c.dt, c.Kalpha0, c.Kspeed0, c.talus_x_cross, c.talus_b_diag, c.fast_div, md.c, dm, o);
-    }
-    if (!in || y < 0 || y >= n) {
-#pragma unroll
-        for (int d = 0; d < 8; ++d) o[d] = pf(0.0f);
-    }
-    auto from_left = [&](float2 a) { return make_float2(__shfl_up_sync(FULL, a.y, 1), a.x); };
-    auto from_right = [&](float2 a) { return make_float2(a.y, __shfl_down_sync(FULL, a.x, 1)); };
-    to_up[warp][0][lane] = o[2];
-    to_up[warp][1][lane] = from_left(o[5]);
-    to_up[warp][2][lane] = from_right(o[4]);
-    to_down[warp][0][lane] = o[3];
-    to_down[warp][1][lane] = from_left(o[7]);
-    to_down[warp][2][lane] = from_right(o[6]);
-    const float2 lr = add2(from_left(o[1]), from_right(o[0]));
-    float2 osum = sub2(pf(0.0f), o[0]);
-#pragma unroll
-    for (int d = 1; d < 8; ++d) osum = sub2(osum, o[d]);
-    __syncthreads();
-    if (!own) return;
-    // the shader's order: L, R, T, B, LT, RT, LB, RB
-    float2 inf = add2(add2(lr, to_down[warp + 1][0][lane]), to_up[warp - 1][0][lane]);
-    inf = add2(add2(inf, to_down[warp + 1][1][lane]), to_down[warp + 1][2][lane]);
-    inf = add2(add2(inf, to_up[warp - 1][1][lane]), to_up[warp - 1][2][lane]);
-    st2(td.out[S_ROCK] + gi, add2(c1, add2(osum, inf)));
-    if (SED) st2(td.out[S_SED] + gi, sed);
-}
-
-template <bool SED>
-__global__ void __launch_bounds__(32 * R_WARPS, 2) k_transport_rows(const __grid_constant__ TerrainDesc td, int steps) {
-    transport_rows<SED>(td.h, blockIdx.x, td.row_lo + blockIdx.y * R_ROWS);
+__global__ void __launch_bounds__(32 * R_WARPS, SED ? 2 : 3) k_transport_rows(const __grid_constant__ TerrainDesc td, int steps) {
+    const TerrainHot& h = td.h;
+    Taps<1> taps;
+    talus_rows(
+        h.c, h.b_ero, h.out[S_ROCK], blockIdx.x, td.row_lo + blockIdx.y * R_ROWS,
+        [&](int x, int y, size_t gi) {
+            const float* const se[1] = {h.s_ero};
+            if (SED) load_taps<1>(h.c, se, x, y, ldg2(h.u + gi), ldg2(h.v + gi), taps);
+        },
+        [&](int, int, size_t gi) {
+            if (SED) st2(h.out[S_SED] + gi, mix_taps(taps, 0));
+        });
     if (SED && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *td.h.step += (unsigned long long)steps;
 }
 
@@ -577,9 +479,20 @@ bool fused_tile_ok(int n, int th) { return (th == 16 || th == 8) && n % TW == 0 
 
 int fused_tiles(int n, int th) { return (n / TW) * (n / th); }
 
-int chunk_rows(size_t cells) {
-    const size_t r = cells / SW / T_FILL;
-    return r < 4 ? 4 : (int)r;
+int chunk_rows(const int* sides, int count) {
+    int most = 0;
+    size_t cells = 0;
+    for (int i = 0; i < count; ++i) {
+        most = sides[i] > most ? sides[i] : most;
+        cells += (size_t)sides[i] * sides[i];
+    }
+    size_t r = cells / SW / T_FILL;
+    for (r = r < 4 ? 4 : r; r < (size_t)most; ++r) {
+        size_t tasks = 0;
+        for (int i = 0; i < count; ++i) tasks += transport_tasks(sides[i], sides[i], (int)r);
+        if (tasks <= (size_t)T_FILL) break;
+    }
+    return (int)r;
 }
 
 int transport_tasks(int n, int rows, int t_rows) { return strips(n) * ((rows + t_rows - 1) / t_rows); }
@@ -602,7 +515,7 @@ bool fill_desc(TerrainDesc& d, const TerrainSrc& s, int th, TmaCache& cache) {
     h.uv_prev = s.uv_prev;
     h.step = s.step;
     h.tiles_x = s.c.n / TW;
-    h.t_rows = chunk_rows((size_t)s.c.n * s.c.n);
+    h.t_rows = chunk_rows(&s.c.n, 1);
     d.row_lo = 0;
     d.row_hi = s.c.n;
     const int in_fields[H_N] = {S_ROCK, S_WATER, S_FL, S_FR, S_FT, S_FB, S_SED};
@@ -639,13 +552,6 @@ void launch_hydro_table(const BatchParams& bp, const CUtensorMap* maps, int tile
     else k_hydro<TH, false><<<tiles, Geo<TH>::NTH, 0, st>>>(bp, maps, 0, err);
     count_launch();
 }
-
-// Worlds up to this side run k_transport_rows: a step with talus takes, in
-// three worlds in turn / alone, 3.4 / 8.3 us at 256² (marching: 4.6 / 11.2),
-// 5.0 / 10.4 at 448² (6.0 / 12.4), 11.7 / 18.3 at 768² (12.4 / 21.8); at
-// 1024² marching takes 19.8 / 29.1 against 22.8 / 26.1, from 1536² on less
-// both ways.
-constexpr int ROWS_MAX_N = 768;
 
 void launch_transport1(const TerrainDesc& td, bool last, int steps, cudaStream_t st) {
     if (td.h.c.n <= ROWS_MAX_N) {

@@ -88,15 +88,13 @@ struct Fused2Bufs {
     float *rock_o, *dirt_o, *water_o, *s0_o, *s1_o, *fl_o, *fr_o, *ft_o, *fb_o;
     float *u, *v;
     float *s0_ero, *s1_ero;  // eroded sediment (rock, dirt)
+    const float *s0_prev, *s1_prev;  // the previous step's, in a chain
     float *b_ero;            // eroded rock (input of the rock talus pass)
     float *rock_mid;         // rock after the rock talus pass (input of the dirt pass)
     float *g_ero;            // eroded dirt (input of the dirt pass)
 };
 struct TmaCache;
 bool fused2_ok(int n);
-int launch_fused2_step(const StepConsts& c, const Talus1& t1, const RainStep& r, const Fused2Bufs& b, TmaCache& tma,
-                       int* err, cudaStream_t st);
-
 // ---- particle erosion (hg_particles.cu) --------------------------------------------
 // Droplets as structure of arrays (Particle, glsl/bindings.glsl:101-110).
 struct Drops {
@@ -135,11 +133,11 @@ void launch_particle_step(const StepConsts& c, const hg_erosion_settings& es, co
                           const PWorld& pw, uint32_t step1, uint64_t seed, bool should_rain, cudaStream_t st);
 // smoothing with the particle branch: in -> out (all of rock, dirt, water, momentum)
 void launch_particle_smooth(const StepConsts& c, float count, const PWorld& in, const PWorld& out, cudaStream_t st);
-struct TmaCache;
 struct Talus1;
 // the particle step's talus passes (rock, then dirt) and smoothing with the
 // particle branch as fused kernels (hg_fused2.cu, n a multiple of 64):
 // in -> out, the rock after its talus pass in rock_mid
+struct TmaCache;
 int launch_particle_thermal_smooth(const StepConsts& c, const Talus1& t1, float count, const PWorld& in,
                                    const PWorld& out, float* rock_mid, TmaCache& tma, int* err, cudaStream_t st);
 
@@ -213,6 +211,11 @@ struct ChainPos {
     bool last;  // the step's results become the state
 };
 
+// One fused two-layer step (hg_fused2.cu).
+struct TmaCache;
+int launch_fused2_step(const StepConsts& c, const Talus1& t1, const RainStep& r, const Fused2Bufs& b, ChainPos pos,
+                       TmaCache& tma, int* err, cudaStream_t st);
+
 // Tensor maps encoded once per (buffer, box) and reused.
 struct TmaCache {
     struct Entry {
@@ -229,8 +232,8 @@ bool fused_tile_ok(int n, int th);
 int fused_tiles(int n, int th);
 // Fills a descriptor (tensor maps from the cache); false if a map cannot be encoded.
 bool fill_desc(TerrainDesc& d, const TerrainSrc& s, int th, TmaCache& cache);
-// Rows a warp of k_transport marches in a launch over `cells` cells.
-int chunk_rows(size_t cells);
+// Rows a warp of k_transport marches in a launch over terrains of these sides.
+int chunk_rows(const int* sides, int count);
 // Warps it runs for `rows` rows of an n x n terrain.
 int transport_tasks(int n, int rows, int t_rows);
 // One fused step (k_hydro, k_transport) over every tile of the batch's

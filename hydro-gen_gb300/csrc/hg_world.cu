@@ -495,14 +495,15 @@ int build_plan(Plan* p) {
             BatchParams& bp = *p->bp[dir];
             bp.nterr = (int)nt;
             bp.tasks = 0;
-            size_t all = 0;
-            for (hg_world* w : p->worlds) all += cells(w);
+            std::vector<int> sides;
+            for (hg_world* w : p->worlds) sides.push_back(w->n);
+            const int rows = chunk_rows(sides.data(), (int)nt);
             std::vector<CUtensorMap> maps(nt * MAPS_PER_TERRAIN);
             for (size_t i = 0; i < nt; ++i) {
                 bp.tile0[i] = tile0[i];
                 bp.task0[i] = bp.tasks;
                 bp.t[i] = tab[i].h;
-                bp.t[i].t_rows = chunk_rows(all);
+                bp.t[i].t_rows = rows;
                 bp.tasks += transport_tasks(p->worlds[i]->n, p->worlds[i]->n, bp.t[i].t_rows);
                 for (int m = 0; m < MAPS_PER_TERRAIN; ++m) maps[i * MAPS_PER_TERRAIN + m] = tab[i].maps[m];
             }
@@ -1490,6 +1491,10 @@ int fused2_steps(hg_world* w, int nsteps) {
     cudaStream_t st = w->stream;
     const size_t cl = cells(w);
     float* scratch = reinterpret_cast<float*>(w->tc);  // 4 n^2 floats
+    // chained steps alternate between two pairs of eroded sediment fields
+    float* prev = reinterpret_cast<float*>(w->td);
+    float* s0e[2] = {w->s_ero, prev};
+    float* s1e[2] = {scratch, prev + cl};
     for (int k = 0; k < nsteps; ++k) {
         const uint64_t step1 = w->step + 1;
         RainStep r = make_rain(w, step1);
@@ -1505,9 +1510,10 @@ int fused2_steps(hg_world* w, int nsteps) {
         b.s0_o = w->alt[S_SED]; b.s1_o = w->sdirt[1];
         b.fl_o = w->alt[S_FL]; b.fr_o = w->alt[S_FR]; b.ft_o = w->alt[S_FT]; b.fb_o = w->alt[S_FB];
         b.u = w->u; b.v = w->v;
-        b.s0_ero = w->s_ero; b.s1_ero = scratch; b.b_ero = w->b_ero;
+        b.s0_ero = s0e[k & 1]; b.s1_ero = s1e[k & 1]; b.b_ero = w->b_ero;
+        b.s0_prev = s0e[~k & 1]; b.s1_prev = s1e[~k & 1];
         b.rock_mid = scratch + cl; b.g_ero = scratch + 2 * cl;
-        int rc = launch_fused2_step(c, t1, r, b, w->tma, w->err, st);
+        int rc = launch_fused2_step(c, t1, r, b, ChainPos{k, k + 1 == nsteps}, w->tma, w->err, st);
         if (rc != HG_OK) return fail(rc, "cuTensorMapEncodeTiled failed for a world buffer");
         for (int f = 0; f < S_COUNT; ++f) std::swap(w->cur[f], w->alt[f]);
         std::swap(w->dirt[0], w->dirt[1]);

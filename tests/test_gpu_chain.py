@@ -66,3 +66,32 @@ def test_strips_and_chunks_against_per_pass(n):
     a.step(3, H.MODE_FUSED)
     b.step(3, H.MODE_PLAIN)
     assert_same(a, b, f"{n}")
+
+
+def make2(n, seed=0, thermal=True, dirt_talus=True):
+    w = H.World(n, layers=2)
+    w.init_reference_heightmap(H.map_settings(hmap_dims=(n, n), seed=0.1 * seed, scale=0.006))
+    s = H.ErosionSettings()
+    H.check(H.lib.hg_default_erosion_settings(H.ctypes.byref(s)))
+    s.d_t, s.G = 0.02, 9.81
+    s.Kalpha[0], s.Kalpha[1] = 0.6, 0.4
+    if not thermal:
+        s.Kspeed[0] = 0.0
+    if not dirt_talus:
+        s.Kspeed[1] = 0.0
+    w.set_erosion(s)
+    w.set_rain(H.rain_uniform(0.5, 1))
+    w.set_options(H.options(H.RAIN_BERNOULLI, p=0.02, seed=seed))
+    return w
+
+
+@pytest.mark.parametrize("n", [64, 192, 832])
+@pytest.mark.parametrize("thermal,dirt_talus", [(True, True), (True, False), (False, True), (False, False)])
+def test_two_layer_chain_against_per_pass(n, thermal, dirt_talus):
+    a, b = make2(n, 1, thermal, dirt_talus), make2(n, 1, thermal, dirt_talus)
+    for k in (3, 1, 4):
+        a.step(k, H.MODE_FUSED)
+        b.step(k, H.MODE_PLAIN)
+        for f in H.STATE_FIELDS + ["dirt", "sediment_dirt"]:
+            x, y = a.download(f), b.download(f)
+            assert np.array_equal(x, y), f"{f} after {a.step_count}: {np.count_nonzero(x != y)} cells differ"
