@@ -4,29 +4,28 @@
 // forward intermediates kept by the segment recompute (velocity u, v and the
 // eroded sediment se of every cell: the fused forward step writes them
 // anyway) and the adjoint A of the step's outputs.  The adjoint of a state is
-// kept as each cell's own terms plus ten packet fields that carry the terms
-// of its neighbours' inputs; a reader adds the neighbours' packets in a
-// fixed order (deterministic), so no separate gather pass runs.  One kernel
-// per step:
-//   k_adj_cell      TMA-staged 64 x 4 tiles of X_j with a one-cell halo,
-//                   this step's rain added in shared memory; one thread per
-//                   cell gathers the cell's adjoint inputs while the tile
-//                   flies, recomputes the forward flux and erosion (the
+// kept as twelve fields (AdjState) from which a reader takes each cell's own
+// terms and adds what its neighbours pass, in a fixed order (deterministic),
+// so no separate gather pass runs.  One kernel per step:
+//   k_adj_cell      64 x 8 tiles of X_j and of A's fields that neighbours
+//                   read, staged by TMA with a one-row halo, this step's rain
+//                   added in shared memory; one thread per pair of cells
+//                   (f32x2) recomputes the forward flux and erosion (the
 //                   operations of hg_device.cuh, so every branch is the
-//                   forward's) and reverses them; it writes its own terms
-//                   and packets, accumulates the Ks gradient and clears its
-//                   sediment-adjoint cell (double buffer); then, with the
-//                   cell's sediment adjoint of step j - 1 now final, it
-//                   reverses that step's semi-Lagrangian gather: a scatter
-//                   to the back-trace's four taps (atomicAdd: the taps are
-//                   data dependent) and the back-trace velocity adjoint
+//                   forward's) and reverses them; it writes the adjoint of
+//                   X_j, accumulates the Ks gradient and clears its
+//                   sediment-adjoint cells (double buffer); then, with the
+//                   sediment adjoint of step j - 1 now final, it reverses
+//                   that step's semi-Lagrangian gather: a scatter to the
+//                   back-trace's four taps (atomicAdd: the taps are data
+//                   dependent) and the back-trace velocity adjoint
 //   k_adj_sediment  the same scatter on its own, for a segment's last step
 //                   (its intermediates exist only after the recompute)
 //   k_adj_final     the gathered rock adjoint of the first state
 //   k_adj_thermal   the talus passes reversed: gathers the output rock's
-//                   adjoint over its box from own terms and packets while
-//                   the eroded rock's box flies, and yields the adjoint of
-//                   the eroded rock, which k_adj_cell then takes
+//                   adjoint over its box while the eroded rock's box flies,
+//                   and yields the adjoint of the eroded rock, which
+//                   k_adj_cell then takes
 //
 // Subgradients: max(0, x) and min(1, q) pass the derivative of the taken
 // argument (ties take the constant side), clamps pass 0 when clamped,
@@ -34,9 +33,10 @@
 // constant, and in water films below FILM_DEPTH the velocity and the flux
 // scale are locally constant.  The formulas follow the shaders cited in hg_device.cuh.  The
 // reversed arithmetic divides through correctly rounded reciprocals
-// (x * (1/y), within two ulps of x / y); the recomputed forward keeps IEEE
-// division, so its values and branches are the forward's own.
+// (x * (1/y), within two ulps of x / y); the recomputed forward's quotients
+// and roots are the forward's own, so its values and branches are too.
 #include "hg_internal.h"
+#include "hg_tile.cuh"
 #include "hg_tma.cuh"
 
 namespace hg {
@@ -55,136 +55,181 @@ __device__ __forceinline__ size_t at(int n, int x, int y) { return (size_t)y * n
 constexpr float FILM_DEPTH = 5e-4f;
 
 // ---- sediment_transport reversed ------------------------------------------------
-// Cell (x, y) of a step whose output sediment adjoint is `a`: scatter to the
-// back-trace taps of dse, back-trace velocity adjoint into du, dv.
-__device__ __forceinline__ void sediment_adjoint(const StepConsts& c, const AdjSlot& sl, int x, int y, size_t i,
-                                                 float a, float ui, float vi, float* dse, float* du, float* dv) {
+// Cells (x, y) and (x + 1, y) of a step whose output sediment adjoint is `a`,
+// with the back-trace's taps of the eroded sediment in q: scatter to the taps
+// of dse, back-trace velocity adjoint into du, dv.  Neighbouring cells mostly
+// trace to neighbouring taps: the column they share is added once.
+__device__ __forceinline__ void sediment_adjoint(const StepConsts& c, const Taps<1>& q, size_t i, float2 a, float* dse,
+                                                 float* du, float* dv) {
     const int n = c.n;
-    const float maxc = (float)(n - 1);
-    float rx = (float)x - ui * c.dt, ry = (float)y - vi * c.dt;
-    float px = gclamp(rx, 0.0f, maxc), py = gclamp(ry, 0.0f, maxc);
-    int ix = min(max((int)px, 0), n - 1), iy = min(max((int)py, 0), n - 1);
-    float fx = px - floorf(px), fy = py - floorf(py);
-    auto S = [&](int xx, int yy) -> float { return (xx < n && yy < n) ? sl.se[at(n, xx, yy)] : 0.0f; };
+    const float2 fx = q.tr.fx, fy = q.tr.fy, ox = sub2(pf(1.0f), fx), oy = sub2(pf(1.0f), fy);
+    const float2 a0 = mul2(a, ox), a1 = mul2(a, fx);
+    float2 w00 = mul2(a0, oy), w01 = mul2(a0, fy);
+    float2 w10 = mul2(a1, oy), w11 = mul2(a1, fy);
+    const int x0 = (int)q.tr.ix[0], y0 = (int)q.tr.iy[0], x1 = (int)q.tr.ix[1], y1 = (int)q.tr.iy[1];
+    const bool shared = x0 + 1 < n && x1 == x0 + 1 && y1 == y0;
+    if (shared) {
+        w10.x += w00.y;
+        w11.x += w01.y;
+        w00.y = w01.y = 0.0f;
+    }
     auto add = [&](int xx, int yy, float v) {
         if (xx < n && yy < n && v != 0.0f) atomicAdd(dse + at(n, xx, yy), v);
     };
-    add(ix, iy, a * (1.0f - fx) * (1.0f - fy));
-    add(ix + 1, iy, a * fx * (1.0f - fy));
-    add(ix, iy + 1, a * (1.0f - fx) * fy);
-    add(ix + 1, iy + 1, a * fx * fy);
-    float s00 = S(ix, iy), s10 = S(ix + 1, iy), s01 = S(ix, iy + 1), s11 = S(ix + 1, iy + 1);
-    float dfx = (s10 - s00) * (1.0f - fy) + (s11 - s01) * fy;
-    float dfy = (s01 * (1.0f - fx) + s11 * fx) - (s00 * (1.0f - fx) + s10 * fx);
-    du[i] = (rx > 0.0f && rx < maxc) ? a * dfx * (-c.dt) : 0.0f;
-    dv[i] = (ry > 0.0f && ry < maxc) ? a * dfy * (-c.dt) : 0.0f;
+    add(x0, y0, w00.x);
+    add(x0 + 1, y0, w10.x);
+    add(x0, y0 + 1, w01.x);
+    add(x0 + 1, y0 + 1, w11.x);
+    add(x1, y1, w00.y);
+    add(x1 + 1, y1, w10.y);
+    add(x1, y1 + 1, w01.y);
+    add(x1 + 1, y1 + 1, w11.y);
+    auto s = [&](int k) { return make_float2(q.t[0][k][0], q.t[0][k][1]); };  // 00, 10, 01, 11
+    const float2 dfx = add2(mul2(sub2(s(1), s(0)), oy), mul2(sub2(s(3), s(2)), fy));
+    const float2 dfy = sub2(add2(mul2(s(2), ox), mul2(s(3), fx)), add2(mul2(s(0), ox), mul2(s(1), fx)));
+    const float2 gx = mul2(mul2(a, dfx), pf(-c.dt)), gy = mul2(mul2(a, dfy), pf(-c.dt));
+    // a point clamped to the grid passes nothing on (the last texel holds only
+    // points at its very edge or beyond)
+    auto inside = [&](int t, float f) { return (t > 0 || f > 0.0f) && t < n - 1; };
+    st2(du + i, make_float2(inside(x0, fx.x) ? gx.x : 0.0f, inside(x1, fx.y) ? gx.y : 0.0f));
+    st2(dv + i, make_float2(inside(y0, fy.x) ? gy.x : 0.0f, inside(y1, fy.y) ? gy.y : 0.0f));
 }
 
 __global__ void k_adj_sediment(StepConsts c, AdjSlot sl, const float* __restrict__ as_, float* __restrict__ dse,
                                float* __restrict__ du, float* __restrict__ dv) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= c.n || y >= c.n) return;
-    size_t i = at(c.n, x, y);
-    sediment_adjoint(c, sl, x, y, i, as_[i], sl.u[i], sl.v[i], dse, du, dv);
+    const int x = 2 * (blockIdx.x * BX + threadIdx.x), y = blockIdx.y * BY + threadIdx.y;
+    const size_t i = at(c.n, x, y);
+    Taps<1> q;
+    const float* const se[1] = {sl.se};
+    load_taps<1>(c, se, x, y, ldg2(sl.u + i), ldg2(sl.v + i), q);
+    sediment_adjoint(c, q, i, ldg2(as_ + i), dse, du, dv);
 }
 
-// Gathered adjoint of a state at cell i: own terms plus the neighbours'
-// packets (L, R, T, B neighbours, fixed order).
-// ROCK false leaves ab alone (the caller has the rock adjoint from elsewhere)
-// and skips the loads only it needs
-template <bool ROCK = true>
-__device__ __forceinline__ void adj_view_at(const AdjView& A, int n, int x, int y, size_t i, float& ab, float& ad,
-                                            float af[4]) {
-    // w = rock + water: a neighbour's height difference toward this cell
-    // (its direction opposite to ours) enters with a minus sign
-    float nbw = 0.0f;
-    if (x > 0) nbw += A.pdh[1][i - 1];      // left neighbour's R
-    if (x < n - 1) nbw += A.pdh[0][i + 1];  // right neighbour's L
-    if (y < n - 1) nbw += A.pdh[3][i + n];  // top neighbour's B
-    if (y > 0) nbw += A.pdh[2][i - n];      // bottom neighbour's T
-    if (ROCK) {
-        float nrm = 0.0f;  // terrain-normal terms of the neighbours
-        if (x > 0) nrm += A.pdx[i - 1];
-        if (x < n - 1) nrm -= A.pdx[i + 1];
-        if (y > 0) nrm += A.pdz[i - n];
-        if (y < n - 1) nrm -= A.pdz[i + n];
-        ab = (A.b[i] - nbw) + nrm;
-    }
-    ad = A.d[i] - nbw;
-#pragma unroll
-    for (int d = 0; d < 4; ++d) af[d] = A.f[d][i];
-    if (x > 0) af[0] += A.pin[1][i - 1];      // left neighbour's inflow from me
-    if (x < n - 1) af[1] += A.pin[0][i + 1];  // right neighbour's inflow from me
-    if (y < n - 1) af[2] += A.pin[3][i + n];  // top neighbour's inflow from me
-    if (y > 0) af[3] += A.pin[2][i - n];      // bottom neighbour's inflow from me
+// A state's adjoint at the cells (x, y), (x + 1, y): own terms plus what the
+// neighbours pass (L, R, T, B neighbours, fixed order).
+// nbw: what the neighbours' height differences toward the cell pass to its total
+// (w = rock + water enters those with a minus sign)
+template <bool EDGE>
+__device__ __forceinline__ float2 adj_nbw(const StepConsts1& c, const AdjState& A, int x, int y, size_t i, float2 h0,
+                                          float2 h1) {
+    const int n = c.n;
+    const float2 z = pf(0.0f), w = pf(c.dt * c.G);
+    const float l = !EDGE || x > 0 ? __ldg(A.h[1] + i - 1) : 0.0f;      // left neighbour's R
+    const float r = !EDGE || x + 2 < n ? __ldg(A.h[0] + i + 2) : 0.0f;  // right neighbour's L
+    const float2 t = !EDGE || y < n - 1 ? ldg2(A.h[3] + i + n) : z;     // top neighbour's B
+    const float2 b = !EDGE || y > 0 ? ldg2(A.h[2] + i - n) : z;         // bottom neighbour's T
+    const float2 s = add2(mul2(w, make_float2(l, h1.x)), mul2(w, make_float2(h0.y, r)));
+    return add2(add2(s, mul2(w, t)), mul2(w, b));
 }
-
-// The gathered rock adjoint alone, with adj_view_at's operations and order.
-__device__ __forceinline__ float adj_rock_at(const AdjView& A, int n, int x, int y, size_t i) {
-    float nbw = 0.0f;
-    if (x > 0) nbw += A.pdh[1][i - 1];
-    if (x < n - 1) nbw += A.pdh[0][i + 1];
-    if (y < n - 1) nbw += A.pdh[3][i + n];
-    if (y > 0) nbw += A.pdh[2][i - n];
-    float nrm = 0.0f;
-    if (x > 0) nrm += A.pdx[i - 1];
-    if (x < n - 1) nrm -= A.pdx[i + 1];
-    if (y > 0) nrm += A.pdz[i - n];
-    if (y < n - 1) nrm -= A.pdz[i + n];
-    return (A.b[i] - nbw) + nrm;
+// the neighbours' terrain-normal terms
+template <bool EDGE>
+__device__ __forceinline__ float2 adj_normal(const AdjState& A, int n, int x, int y, size_t i) {
+    const float2 z = pf(0.0f), nx = ldg2(A.nx + i);
+    const float l = !EDGE || x > 0 ? __ldg(A.nx + i - 1) : 0.0f;
+    const float r = !EDGE || x + 2 < n ? __ldg(A.nx + i + 2) : 0.0f;
+    const float2 b = !EDGE || y > 0 ? ldg2(A.nz + i - n) : z, t = !EDGE || y < n - 1 ? ldg2(A.nz + i + n) : z;
+    return sub2(add2(sub2(make_float2(l, nx.x), make_float2(nx.y, r)), b), t);
 }
 
 // ---- k_adj_cell ------------------------------------------------------------------
-constexpr int TW = 64, TH = 4, HX = 4, RW = TW + 2 * HX, NTH = TW * TH;
+// A warp per row of 32 pairs of cells, in f32x2; the tile is staged with a
+// one-row halo.  Bound by the latency of its loads under too few warps (80
+// registers, 24 warps per SM) before DRAM (131 MB at 1024²): what a thread
+// alone reads goes into shared memory by cp.async and to registers only where
+// it is used, and so do the neighbours' terms.  1024² with talus, per launch:
+// one cell at a time with every neighbour's share stored by itself 45 us (827
+// instructions per cell, 172 MB); pairs with the inputs in registers 44
+// (16 warps per SM); as here 33 (460).  64 x 4 tiles take 1 % longer, 4 blocks
+// per SM 8 % (spills), 2 blocks 10 %.
+constexpr int TH = 8, NTH = TW / 2 * TH;
 constexpr int H_RH = TH + 2, H_BOX = RW * H_RH, H_RC = ((H_BOX + 31) / 32) * 32;
-enum { X_B = 0, X_D, X_S, X_FL, X_FR, X_FT, X_FB, X_N };
+// the pair's own inputs: rock, water, sediment adjoint, back-trace velocity
+// adjoint, Ks, velocity of step j - 1
+enum { O_B = 0, O_D, O_S, O_DU, O_DV, O_KS, O_PU, O_PV, O_N };
+enum { X_B = 0, X_D, X_S, X_FL, X_FR, X_FT, X_FB, X_H, X_P = X_H + 4, X_GU, X_GV, X_N };  // state, adjoint
 
-// Forward flux of one cell with the intermediates its adjoint needs: the
-// operations of cell_flux (hg_device.cuh), so every branch is the forward's.
+__device__ __forceinline__ float2 sel(bool x, bool y, float2 a, float2 b) {
+    return make_float2(x ? a.x : b.x, y ? a.y : b.y);
+}
+__device__ __forceinline__ float2 frcp2(float2 a) { return make_float2(__frcp_rn(a.x), __frcp_rn(a.y)); }
+
+// Forward flux of two cells with the intermediates its adjoint needs: the
+// operations of cell_flux2 (hg_device.cuh), so every branch is the forward's.
 // Directions L, R, T, B; wn[] neighbour totals, in[] neighbours' facing flux.
-struct FluxFwd {
-    float g[4];
-    bool live[4];
-    float sum_out, den, K, arg, vz, u, v;
-    bool scaled;
+// A direction is live where g > 0.
+struct FluxFwd2 {
+    float2 g[4];  // outflows before scaling
+    float2 sum_out, K, arg, vz, u, v, len;
+    float2 rden, rvz, rlen;      // reciprocals, of 1 where no use is made of them
+    bool scaled_x, scaled_y;
 };
-__device__ __forceinline__ FluxFwd flux_fwd(const StepConsts& c, int x, int y, float w_c, float d1, const float f[4],
-                                            const float wn[4], const float in[4], bool border) {
-    FluxFwd o;
-    float ft[4];
+__device__ __forceinline__ FluxFwd2 flux_fwd2(const StepConsts& c, int x, int y, float2 w, float2 d1,
+                                              const float2 f[4], const float2 wn[4], const float2 in[4], bool border) {
+    FluxFwd2 o;
+    const float2 EK = pf(c.EK), dt = pf(c.dt), G = pf(c.G);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        ft[k] = c.EK * f[k] + c.dt * (c.G * (w_c - wn[k]));
-        o.g[k] = gmax(0.0f, ft[k]);
-        o.live[k] = ft[k] > 0.0f;
+        const float2 t = add2(mul2(EK, f[k]), mul2(dt, mul2(G, sub2(w, wn[k]))));
+        o.g[k] = make_float2(fmaxf(0.0f, t.x), fmaxf(0.0f, t.y));
     }
     if (border) {
-        if (x <= 0) { o.g[0] = 0.0f; o.live[0] = false; }
-        else if (x >= c.n - 1) { o.g[1] = 0.0f; o.live[1] = false; }
-        if (y <= 0) { o.g[3] = 0.0f; o.live[3] = false; }
-        else if (y >= c.n - 1) { o.g[2] = 0.0f; o.live[2] = false; }
+        if (x <= 0) o.g[0].x = 0.0f;
+        if (x + 1 >= c.n - 1) o.g[1].y = 0.0f;
+        if (y <= 0) o.g[3] = pf(0.0f);
+        else if (y >= c.n - 1) o.g[2] = pf(0.0f);
     }
-    float sum_in = in[0] + in[1] + in[2] + in[3];
-    o.sum_out = o.g[0] + o.g[1] + o.g[2] + o.g[3];
-    o.den = o.sum_out * c.dt;
-    o.scaled = false;
-    o.K = 1.0f;
-    if (!(d1 >= o.den)) {
-        float q = d1 / o.den;
-        if (q < 1.0f) { o.scaled = true; o.K = q; }
+    const float2 sum_in = add2(add2(add2(in[0], in[1]), in[2]), in[3]);
+    o.sum_out = add2(add2(add2(o.g[0], o.g[1]), o.g[2]), o.g[3]);
+    const float2 den = mul2(o.sum_out, dt);
+    const bool fullx = d1.x >= den.x, fully = d1.y >= den.y;
+    o.K = o.rden = pf(1.0f);
+    o.scaled_x = o.scaled_y = false;
+    if (!(fullx & fully)) {
+        const float2 dn = make_float2(fullx ? 1.0f : den.x, fully ? 1.0f : den.y);
+        float2 q;
+        if (num_range(d1.x) & num_range(d1.y) & den_range(dn.x) & den_range(dn.y)) {
+            o.rden = rcp_newton2(dn);
+            q = div_recip2(d1, make_float2(-dn.x, -dn.y), o.rden);
+        } else {
+            o.rden = frcp2(dn);
+            q = make_float2(d1.x / dn.x, d1.y / dn.y);
+        }
+        o.scaled_x = !fullx && q.x < 1.0f;
+        o.scaled_y = !fully && q.y < 1.0f;
+        o.K = sel(o.scaled_x, o.scaled_y, q, o.K);
     }
-    o.arg = d1 + c.dt * (sum_in - o.sum_out * o.K);
-    float d2 = gmax(0.0f, o.arg);
-    o.vz = d1 + d2;
-    if (o.vz > 0.0f) {
-        o.u = (in[0] - f[0] + f[1] - in[1]) / o.vz;
-        o.v = (in[3] - f[3] + f[2] - in[2]) / o.vz;
+    o.arg = add2(d1, mul2(dt, sub2(sum_in, mul2(o.sum_out, o.K))));
+    o.vz = add2(d1, make_float2(fmaxf(0.0f, o.arg.x), fmaxf(0.0f, o.arg.y)));
+    const float2 nu = sub2(add2(sub2(in[0], f[0]), f[1]), in[1]), nv = sub2(add2(sub2(in[3], f[3]), f[2]), in[2]);
+    const bool wetx = o.vz.x > 0.0f, wety = o.vz.y > 0.0f;
+    const float2 vs = sel(wetx, wety, o.vz, pf(1.0f)), nd = make_float2(-vs.x, -vs.y);
+    o.rvz = rcp_newton2(vs);
+    o.u = sel(wetx, wety, div_recip2(nu, nd, o.rvz), pf(0.0f));
+    o.v = sel(wetx, wety, div_recip2(nv, nd, o.rvz), pf(0.0f));
+    float2 ss = add2(mul2(o.u, o.u), mul2(o.v, o.v));
+    const bool ok = num_range(nu.x) & num_range(nu.y) & num_range(nv.x) & num_range(nv.y) & den_range(vs.x) &
+                    den_range(vs.y) & root_range(ss.x) & root_range(ss.y);
+    if (ok) {
+        o.len = sqrt_newton2(ss);
+        o.rlen = rcp_newton2(sel(o.len.x > 0.0f, o.len.y > 0.0f, o.len, pf(1.0f)));
     } else {
-        o.u = 0.0f; o.v = 0.0f;
+        o.rvz = frcp2(vs);
+        o.u = make_float2(wetx ? nu.x / vs.x : 0.0f, wety ? nu.y / vs.y : 0.0f);
+        o.v = make_float2(wetx ? nv.x / vs.x : 0.0f, wety ? nv.y / vs.y : 0.0f);
+        ss = add2(mul2(o.u, o.u), mul2(o.v, o.v));
+        o.len = make_float2(sqrtf(ss.x), sqrtf(ss.y));
+        o.rlen = frcp2(o.len);
     }
     return o;
 }
+
+// 8 bytes of global memory into shared memory, in flight until copy_async_wait
+// (of the same thread)
+__device__ __forceinline__ void copy_async8(void* dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void prefetch_l2(const float* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 template <bool EDGE>
 __device__ __forceinline__ void adj_tile(const AdjCellArgs& a, float* sm, uint64_t* bar, int tx0, int ty0,
@@ -199,34 +244,33 @@ __device__ __forceinline__ void adj_tile(const AdjCellArgs& a, float* sm, uint64
 #pragma unroll
         for (int f = 0; f < X_N; ++f) tma_load_2d(sm + f * H_RC, &a.maps[f], gx0, gy0, bar);
     }
-    constexpr int RG = (RW / 4) * H_RH;
-    constexpr int RGK = (RG + NTH - 1) / NTH;
-    uint32_t words[RGK][4];
-#pragma unroll
-    for (int k = 0; k < RGK; ++k) {
-        words[k][0] = words[k][1] = words[k][2] = words[k][3] = 0;
-        int q = tid + k * NTH;
-        if (q < RG && r.active && r.bernoulli) {
-            int gx = gx0 + (q % (RW / 4)) * 4, gy = gy0 + q / (RW / 4);
-            if (!EDGE || (gx >= 0 && gx < n && gy >= 0 && gy < n)) rain_words4(r, gx, gy, words[k]);
-        }
-    }
-    // the cell's adjoint inputs, loaded while the tile flies
-    const int ix = tid % TW, iy = tid / TW;
+    // the pair's adjoint inputs, loaded while the tile flies, and the taps of
+    // step j - 1's sediment gather, which the end reverses
+    const int ix = (tid % (TW / 2)) * 2, iy = tid / (TW / 2);
     const int x = tx0 + ix, y = ty0 + iy;
     const size_t i = (size_t)y * n + x;
-    float ab, ad, af[4];
-    if (a.gbe) {  // thermal on: the eroded rock's adjoint (k_adj_thermal)
-        ab = a.gbe[i];
-        adj_view_at<false>(a.A, n, x, y, i, ab, ad, af);
-    } else {
-        adj_view_at(a.A, n, x, y, i, ab, ad, af);
+    const float2 z = pf(0.0f), one = pf(1.0f);
+    float2* own = reinterpret_cast<float2*>(sm + X_N * H_RC) + tid;
+    auto fetch = [&](int k, const float* p) { copy_async8(own + k * NTH, p + i); };
+    if (a.scatter_prev) {
+        fetch(O_PU, a.prev.u);
+        fetch(O_PV, a.prev.v);
+        prefetch_l2(a.prev.se + i);  // near the taps read at the end
     }
-    const float as = a.dse[i];
-    const float DUs = a.du[i], DVs = a.dv[i];
-    const float Ks_i = c.ks_field ? c.ks_field[i] : c.Ks0;
-    // step j - 1's velocity for its sediment reversal at the end
-    const float pu = a.scatter_prev ? a.prev.u[i] : 0.0f, pv = a.scatter_prev ? a.prev.v[i] : 0.0f;
+    fetch(O_B, a.gbe ? a.gbe : a.A.b);  // thermal on: the eroded rock's adjoint (k_adj_thermal)
+    fetch(O_D, a.A.d);
+    fetch(O_S, a.dse);
+    fetch(O_DU, a.du);
+    fetch(O_DV, a.dv);
+    if (c.ks_field) fetch(O_KS, c.ks_field);
+    const float2 Anrm = a.gbe ? z : adj_normal<EDGE>(a.A, n, x, y, i);
+    constexpr int RG = (RW / 4) * H_RH;  // groups of four cells, at most one per thread
+    static_assert(RG <= NTH, "one rain group per thread");
+    uint32_t words[4] = {0, 0, 0, 0};
+    const int rrx = (tid % (RW / 4)) * 4, rry = tid / (RW / 4), rgx = gx0 + rrx, rgy = gy0 + rry;
+    const bool rains = r.active && tid < RG && (!EDGE || (rgx >= 0 && rgx < n && rgy >= 0 && rgy < n));
+    if (rains && r.bernoulli) rain_words4(r, rgx, rgy, words);
+    copy_async_wait();
     bool ok = __syncthreads_and(mbar_wait(bar, 0));
     if (!ok) {
         if (tid == 0) atomicExch(err, 1);
@@ -234,178 +278,201 @@ __device__ __forceinline__ void adj_tile(const AdjCellArgs& a, float* sm, uint64
         return;
     }
     if (r.active) {
-        float* D = sm + X_D * H_RC;
-#pragma unroll
-        for (int k = 0; k < RGK; ++k) {
-            int q = tid + k * NTH;
-            if (q >= RG) continue;
-            int rx = (q % (RW / 4)) * 4, ry = q / (RW / 4);
-            int gx = gx0 + rx, gy = gy0 + ry;
-            if (EDGE && !(gx >= 0 && gx < n && gy >= 0 && gy < n)) continue;
-            float* p = D + ry * RW + rx;
-            p[0] += rain_incr(r, words[k][0]);
-            p[1] += rain_incr(r, words[k][1]);
-            p[2] += rain_incr(r, words[k][2]);
-            p[3] += rain_incr(r, words[k][3]);
+        if (rains) {
+            float* p = sm + X_D * H_RC + rry * RW + rrx;
+            p[0] += rain_incr(r, words[0]);
+            p[1] += rain_incr(r, words[1]);
+            p[2] += rain_incr(r, words[2]);
+            p[3] += rain_incr(r, words[3]);
         }
+        __syncthreads();
     }
-    __syncthreads();
     const float* B = sm + X_B * H_RC;
     const float* D = sm + X_D * H_RC;
-    const float* S = sm + X_S * H_RC;
     const float* F[4] = {sm + X_FL * H_RC, sm + X_FR * H_RC, sm + X_FT * H_RC, sm + X_FB * H_RC};
+    const int si = (1 + iy) * RW + HX + ix;
+    const bool has_l = !EDGE || x > 0, has_r = !EDGE || x + 2 < n;
+    const bool has_b = !EDGE || y > 0, has_t = !EDGE || y < n - 1;
+    auto left = [&](const float* p, float2 m) { return make_float2(p[si - 1], m.x); };
+    auto right = [&](const float* p, float2 m) { return make_float2(m.y, p[si + 2]); };
+    // ---- adjoint of the step's output (0 outside the grid) ---------------
+    float2 Ab, Ad;
+    const float *h = sm + X_H * H_RC, *P = sm + X_P * H_RC, *GU = sm + X_GU * H_RC, *GV = sm + X_GV * H_RC;
     {
-        const int si = (1 + iy) * RW + HX + ix;
-        const bool has_l = !EDGE || x > 0, has_r = !EDGE || x < n - 1;
-        const bool has_b = !EDGE || y > 0, has_t = !EDGE || y < n - 1;
-        // ---- forward recompute: flux --------------------------------------
-        const float b = B[si], d1 = D[si];
-        const float bl = B[si - 1], br = B[si + 1], bb = B[si - RW], bt = B[si + RW];
-        const float f[4] = {F[0][si], F[1][si], F[2][si], F[3][si]};
-        const float wn[4] = {has_l ? bl + D[si - 1] : FAR_HEIGHT, has_r ? br + D[si + 1] : FAR_HEIGHT,
-                             has_t ? bt + D[si + RW] : FAR_HEIGHT, has_b ? bb + D[si - RW] : FAR_HEIGHT};
-        const float in[4] = {has_l ? F[1][si - 1] : 0.0f, has_r ? F[0][si + 1] : 0.0f,
-                             has_t ? F[3][si + RW] : 0.0f, has_b ? F[2][si - RW] : 0.0f};
-        const FluxFwd fw = flux_fwd(c, x, y, b + d1, d1, f, wn, in, EDGE);
-        // ---- forward recompute: erosion speed and tilt ---------------------
-        const float u = fw.u, v = fw.v, vz = fw.vz;
-        const float len = sqrtf(u * u + v * v);
-        float ero = len, dero_dlen = 1.0f, dero_dvz = 0.0f;
-        if (vz < 1e-3f) {
-            float dd = gmax(5e-4f, vz);
-            float tr = (dd - 1e-3f) / (5e-4f - 1e-3f);
-            float t = gclamp(tr, 0.0f, 1.0f);
-            float sm3 = t * t * (3.0f - 2.0f * t);
-            ero = gmix(len, 0.0f, sm3);
-            dero_dlen = 1.0f - sm3;
-            // d(smoothstep)/d(vz): 6 t (1 - t) / (5e-4 - 1e-3)
-            if (vz > 5e-4f && tr > 0.0f && tr < 1.0f) dero_dvz = len * 6.0f * t * (1.0f - t) * 2000.0f;
-        }
-        const float ebr = has_r ? br : 0.0f, ebl = has_l ? bl : 0.0f;
-        const float ebt = has_t ? bt : 0.0f, ebb = has_b ? bb : 0.0f;
-        const float dx = ebr - ebl, dz = ebt - ebb;
-        const float cx = dx * 2.0f - 0.0f * dz, cz = 2.0f * dz - dx * 0.0f;
-        const float L3 = sqrtf(cx * cx + 16.0f + cz * cz);
-        const float ny = -4.0f / L3;
-        const float sin_a = fabsf(sqrtf(1.0f - ny * ny));
-        const float sa = gmax(0.02f, sin_a);
-        const float craw = c.Kc * sa * ero;
-        const float cc = gmax(0.0f, craw);
-        const float Kls = c.dt * Ks_i, Kld = c.Kld0, s = S[si];
-        // ---- erosion reversed ----------------------------------------------
-        a.dse[i] = 0.0f;  // free for the step after next
-        float gb, gs, gc = 0.0f, gKs = 0.0f;
-        if (cc > 0.0f && !(c.Kls1 * cc > 0.0f)) {  // the empty dirt layer ends the layer loop: identity
-            gb = ab;
-            gs = as;
-        } else if (cc > s) {
-            float del = Kls * (cc - s);
-            if (b - del < 0.0f) {  // rock exhausted: b' = 0, s' = s + b
-                gb = as;
-                gs = as;
-            } else {
-                gb = ab;
-                gs = ab * Kls + as * (1.0f - Kls);
-                gc = (as - ab) * Kls;
-                gKs = (as - ab) * (cc - s);
-            }
-        } else {
-            gb = ab;
-            gs = ab * Kld + as * (1.0f - Kld);
-            gc = (as - ab) * Kld;
-        }
-        if (gKs != 0.0f) a.dks[i] += gKs * c.dt;
-        float pdx = 0.0f, pdz = 0.0f, due = 0.0f, dve = 0.0f, gvz = 0.0f;
-        if (craw > 0.0f) {
-            float gsa = gc * c.Kc * ero, gero = gc * c.Kc * sa;
-            if (sin_a > 0.02f) {
-                const float r3 = __frcp_rn(L3);
-                float gny = gsa * (-ny * __frcp_rn(sin_a));
-                float gL3 = gny * (4.0f * r3 * r3);
-                pdx = gL3 * 4.0f * dx * r3;
-                pdz = gL3 * 4.0f * dz * r3;
-            }
-            float glen = gero * dero_dlen;
-            gvz = gero * dero_dvz;
-            if (len > 0.0f) {
-                const float rl = __frcp_rn(len);
-                due = glen * u * rl;
-                dve = glen * v * rl;
-            }
-        }
-        // ---- flux reversed -------------------------------------------------
-        const float DU = DUs + due, DV = DVs + dve;
-        float gin[4] = {0.0f, 0.0f, 0.0f, 0.0f}, gfown[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        if (vz >= FILM_DEPTH) {  // thinner films: velocity locally constant
-            const float rv = __frcp_rn(vz);
-            float gu = DU * rv, gv = DV * rv;
-            gin[0] += gu; gin[1] -= gu;
-            gfown[0] -= gu; gfown[1] += gu;
-            gin[3] += gv; gin[2] -= gv;
-            gfown[3] -= gv; gfown[2] += gv;
-            gvz -= (DU * u + DV * v) * rv;
-        }
-        float gd1 = gvz, gd2 = gvz + ad * c.evap;
-        float garg = fw.arg > 0.0f ? gd2 : 0.0f;
-        gd1 += garg;
-        float gsum_in = c.dt * garg, gsum_outK = -c.dt * garg;
-#pragma unroll
-        for (int d = 0; d < 4; ++d) gin[d] += gsum_in;
-        float gK = gsum_outK * fw.sum_out, gsum_out = gsum_outK * fw.K;
-#pragma unroll
-        for (int d = 0; d < 4; ++d) gK += af[d] * fw.g[d];
-        float gg[4];
-#pragma unroll
-        for (int d = 0; d < 4; ++d) gg[d] = af[d] * fw.K + gsum_out;
-        if (fw.scaled && d1 >= FILM_DEPTH) {  // thinner films: K locally constant
-            const float rd = __frcp_rn(fw.den);
-            gd1 += gK * rd;
-            float gden = -gK * d1 * rd * rd;
-#pragma unroll
-            for (int d = 0; d < 4; ++d) gg[d] += gden * c.dt;
-        }
-        float gw = 0.0f;
-#pragma unroll
-        for (int d = 0; d < 4; ++d) {
-            float gdh = 0.0f;
-            if (fw.live[d]) {
-                gfown[d] += c.EK * gg[d];
-                gdh = c.dt * c.G * gg[d];
-                gw += gdh;
-            }
-            a.pdh[d][i] = gdh;
-            a.pin[d][i] = gin[d];
-            a.rf[d][i] = gfown[d];
-        }
-        a.pdx[i] = pdx;
-        a.pdz[i] = pdz;
-        a.rb[i] = gb + gw;
-        a.rd[i] = gw + gd1;
-        a.rs[i] = gs;
-        // ---- sediment_transport of step j - 1 reversed ----------------------
-        if (a.scatter_prev) sediment_adjoint(c, a.prev, x, y, i, gs, pu, pv, a.dse_prev, a.du, a.dv);
+        const float2 w = pf(c.dt * c.G), h0 = ld2(h + si), h1 = ld2(h + H_RC + si);
+        float2 nbw = add2(mul2(w, left(h + H_RC, h1)), mul2(w, right(h, h0)));
+        nbw = add2(nbw, mul2(w, ld2(h + 3 * H_RC + si + RW)));
+        nbw = add2(nbw, mul2(w, ld2(h + 2 * H_RC + si - RW)));
+        Ab = own[O_B * NTH];
+        if (!a.gbe) Ab = add2(sub2(Ab, nbw), Anrm);
+        Ad = sub2(own[O_D * NTH], nbw);
     }
+    // ---- forward recompute: flux --------------------------------------
+    const float2 b = ld2(B + si), d1 = ld2(D + si);
+    float2 bl = left(B, b), br = right(B, b), bb = ld2(B + si - RW), bt = ld2(B + si + RW);
+    const float2 f[4] = {ld2(F[0] + si), ld2(F[1] + si), ld2(F[2] + si), ld2(F[3] + si)};
+    float2 wn[4] = {add2(bl, left(D, d1)), add2(br, right(D, d1)), add2(bt, ld2(D + si + RW)),
+                    add2(bb, ld2(D + si - RW))};
+    // (outside the grid the staged tile is 0, what the normal and the inflows read there)
+    const float2 in[4] = {left(F[1], f[1]), right(F[0], f[0]), ld2(F[3] + si + RW), ld2(F[2] + si - RW)};
+    if (EDGE) {
+        if (!has_l) wn[0].x = FAR_HEIGHT;
+        if (!has_r) wn[1].y = FAR_HEIGHT;
+        if (!has_t) wn[2] = pf(FAR_HEIGHT);
+        if (!has_b) wn[3] = pf(FAR_HEIGHT);
+    }
+    const FluxFwd2 fw = flux_fwd2(c, x, y, add2(b, d1), d1, f, wn, in, EDGE);
+    // ---- forward recompute: erosion speed and tilt ---------------------
+    const float2 u = fw.u, v = fw.v, vz = fw.vz, len = fw.len;
+    float2 ero = len, dero_dlen = one, dero_dvz = z;
+    if ((vz.x < 1e-3f) | (vz.y < 1e-3f)) {  // (see capacity2; a depth from 1e-3 up has t = 0)
+        constexpr float DD = 5e-4f - 1e-3f, RD = 1.0f / DD;
+        const float2 dd = make_float2(fminf(fmaxf(5e-4f, vz.x), 1e-3f), fminf(fmaxf(5e-4f, vz.y), 1e-3f));
+        const float2 t = div_recip2(add2(dd, pf(-1e-3f)), pf(-DD), pf(RD));
+        const float2 fade = sub2(one, mul2(mul2(t, t), sub2(pf(3.0f), mul2(pf(2.0f), t))));
+        const bool sx = vz.x < 1e-3f, sy = vz.y < 1e-3f;
+        dero_dlen = sel(sx, sy, fade, one);
+        ero = sel(sx, sy, mul2(len, fade), len);
+        // d(smoothstep)/d(vz): 6 t (1 - t) / (5e-4 - 1e-3)
+        const float2 dv = mul2(mul2(mul2(mul2(len, pf(6.0f)), t), sub2(one, t)), pf(2000.0f));
+        dero_dvz = sel(sx && vz.x > 5e-4f && t.x > 0.0f && t.x < 1.0f, sy && vz.y > 5e-4f && t.y > 0.0f && t.y < 1.0f,
+                       dv, z);
+    }
+    const float2 dx = sub2(br, bl), dz = sub2(bt, bb);
+    const float2 cx = add2(dx, dx), cz = add2(dz, dz);
+    const float2 L2 = add2(add2(mul2(cx, cx), pf(16.0f)), mul2(cz, cz));
+    float2 L3 = sqrt_newton2(L2), r3 = rcp_newton2(L3);
+    float2 ny = div_recip2(pf(-4.0f), make_float2(-L3.x, -L3.y), r3);
+    float2 sin_a = sqrt_newton2(sub2(one, mul2(ny, ny)));
+    if (!((L2.x <= 0x1p80f) & (L2.y <= 0x1p80f))) {
+        auto tilt = [](float ddx, float ddz, float& nyl, float& r3l) {
+            const float x1 = ddx * 2.0f - 0.0f * ddz, z1 = 2.0f * ddz - ddx * 0.0f;
+            const float l = sqrtf(x1 * x1 + 16.0f + z1 * z1);
+            nyl = -4.0f / l;
+            r3l = __frcp_rn(l);
+            return fabsf(sqrtf(1.0f - nyl * nyl));
+        };
+        sin_a.x = tilt(dx.x, dz.x, ny.x, r3.x);
+        sin_a.y = tilt(dx.y, dz.y, ny.y, r3.y);
+    }
+    const float2 sa = make_float2(gmax(0.02f, sin_a.x), gmax(0.02f, sin_a.y));
+    const float2 craw = mul2(mul2(pf(c.Kc), sa), ero);
+    const float2 cc = make_float2(fmaxf(0.0f, craw.x), fmaxf(0.0f, craw.y));
+    const float2 s = ld2(sm + X_S * H_RC + si);
+    // ---- erosion reversed ----------------------------------------------
+    st2(a.dse + i, z);  // free for the step after next
+    // dissolve (K = dt Ks) and deposit (K = dt Kd) are one form; identity where
+    // the empty dirt layer ends the layer loop, and where the rock is exhausted
+    // (b' = 0, s' = s + b) both inputs take the sediment's adjoint
+    const float2 e = sub2(cc, s), k1 = mul2(pf(c.Kls1), cc);
+    const bool morex = cc.x > s.x, morey = cc.y > s.y;
+    const bool endx = (cc.x > 0.0f) & !(k1.x > 0.0f), endy = (cc.y > 0.0f) & !(k1.y > 0.0f);
+    const float2 Kls = mul2(pf(c.dt), c.ks_field ? own[O_KS * NTH] : pf(c.Ks0)), K = sel(morex, morey, Kls, pf(c.Kld0));
+    const float2 left_b = sub2(b, mul2(Kls, e));
+    const bool gonex = !endx & morex & (left_b.x < 0.0f), goney = !endy & morey & (left_b.y < 0.0f);
+    const bool keepx = endx | gonex, keepy = endy | goney;
+    const float2 as = own[O_S * NTH], diff = sub2(as, Ab);
+    const float2 gs = sel(keepx, keepy, as, add2(mul2(Ab, K), mul2(as, sub2(one, K))));
+    const float2 gb = sel(gonex, goney, as, Ab);
+    const float2 gc = sel(keepx, keepy, z, mul2(diff, K));
+    const float2 gKs = sel(!keepx & morex, !keepy & morey, mul2(diff, e), z);
+    const bool ks_any = (gKs.x != 0.0f) | (gKs.y != 0.0f);
+    float2 dks = z;
+    if (ks_any) dks = ld2(a.dks + i);  // (added at the end)
+    // capacity reversed
+    const bool cx0 = craw.x > 0.0f, cy0 = craw.y > 0.0f;
+    const float2 gk = mul2(gc, pf(c.Kc));
+    const float2 gsa = mul2(gk, ero), gero = sel(cx0, cy0, mul2(gk, sa), z);
+    const bool tx = cx0 & (sin_a.x > 0.02f), ty = cy0 & (sin_a.y > 0.02f);
+    const float2 rsin = rcp_newton2(sel(tx, ty, sin_a, one));
+    const float2 gny = mul2(gsa, mul2(make_float2(-ny.x, -ny.y), rsin));
+    const float2 gL = mul2(mul2(gny, mul2(mul2(pf(4.0f), r3), r3)), pf(4.0f));
+    st2(a.R.nx + i, sel(tx, ty, mul2(mul2(gL, dx), r3), z));
+    st2(a.R.nz + i, sel(tx, ty, mul2(mul2(gL, dz), r3), z));
+    const float2 glen = mul2(gero, dero_dlen);
+    const bool mx = len.x > 0.0f, my = len.y > 0.0f;
+    const float2 DU = add2(own[O_DU * NTH], sel(mx, my, mul2(mul2(glen, u), fw.rlen), z));
+    const float2 DV = add2(own[O_DV * NTH], sel(mx, my, mul2(mul2(glen, v), fw.rlen), z));
+    float2 gvz = mul2(gero, dero_dvz);
+    // ---- flux reversed -------------------------------------------------
+    const bool wx = vz.x >= FILM_DEPTH, wy = vz.y >= FILM_DEPTH;  // thinner films: velocity locally constant
+    const float2 gu = sel(wx, wy, mul2(DU, fw.rvz), z), gv = sel(wx, wy, mul2(DV, fw.rvz), z);
+    gvz = sel(wx, wy, sub2(gvz, mul2(add2(mul2(DU, u), mul2(DV, v)), fw.rvz)), gvz);
+    st2(a.R.gu + i, gu);
+    st2(a.R.gv + i, gv);
+    const float2 gd2 = add2(gvz, mul2(Ad, pf(c.evap)));
+    const float2 garg = make_float2(fw.arg.x > 0.0f ? gd2.x : 0.0f, fw.arg.y > 0.0f ? gd2.y : 0.0f);
+    float2 gd1 = add2(gvz, garg);
+    st2(a.R.p + i, mul2(pf(c.dt), garg));
+    float2 Af[4];
+    {
+        const float2 EK = pf(c.EK), p = ld2(P + si), nu = ld2(GU + si), nv = ld2(GV + si);
+        // a cell's own flux term: its outflow's energy part and its place in its
+        // own velocity; the neighbour it flows to has it as an inflow
+        Af[0] = add2(sub2(mul2(EK, ld2(h + si)), nu), sub2(left(P, p), left(GU, nu)));
+        Af[1] = add2(add2(mul2(EK, ld2(h + H_RC + si)), nu), add2(right(P, p), right(GU, nu)));
+        Af[2] = add2(add2(mul2(EK, ld2(h + 2 * H_RC + si)), nv), add2(ld2(P + si + RW), ld2(GV + si + RW)));
+        Af[3] = add2(sub2(mul2(EK, ld2(h + 3 * H_RC + si)), nv), sub2(ld2(P + si - RW), ld2(GV + si - RW)));
+    }
+    const float2 gsum_outK = mul2(pf(-c.dt), garg), gsum_out = mul2(gsum_outK, fw.K);
+    float2 gK = mul2(gsum_outK, fw.sum_out);
+#pragma unroll
+    for (int d = 0; d < 4; ++d) gK = add2(gK, mul2(Af[d], fw.g[d]));
+    // K = depth / outflow where it scales (thinner films: locally constant)
+    const bool kx = fw.scaled_x & (d1.x >= FILM_DEPTH), ky = fw.scaled_y & (d1.y >= FILM_DEPTH);
+    float2 gden = z;
+    if (kx | ky) {
+        const float2 rd = fw.rden, g1 = mul2(gK, rd);
+        gden = sel(kx, ky, mul2(mul2(mul2(mul2(make_float2(-gK.x, -gK.y), d1), rd), rd), pf(c.dt)), z);
+        gd1 = sel(kx, ky, add2(gd1, g1), gd1);
+    }
+    const float2 wd = pf(c.dt * c.G);
+    float2 gw = z;
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {
+        float2 gg = add2(mul2(Af[d], fw.K), gsum_out);
+        gg = sel(kx, ky, add2(gg, gden), gg);
+        gg = sel(fw.g[d].x > 0.0f, fw.g[d].y > 0.0f, gg, z);
+        st2(a.R.h[d] + i, gg);
+        gw = add2(gw, mul2(wd, gg));
+    }
+    st2(a.R.b + i, add2(gb, gw));
+    st2(a.R.d + i, add2(gw, gd1));
+    // ---- sediment_transport of step j - 1 reversed ----------------------
+    if (a.scatter_prev) {
+        const float* const se[1] = {a.prev.se};
+        Taps<1> q;
+        load_taps<1>(c, se, x, y, own[O_PU * NTH], own[O_PV * NTH], q);
+        sediment_adjoint(c, q, i, gs, a.dse_prev, a.du, a.dv);
+    } else {
+        st2(a.R.s + i, gs);
+    }
+    if (ks_any) st2(a.dks + i, add2(dks, mul2(gKs, pf(c.dt))));
 }
 
-__global__ void __launch_bounds__(NTH) k_adj_cell(const __grid_constant__ AdjCellArgs a, int* err) {
-    __shared__ __align__(128) float sm[X_N * H_RC];
+constexpr size_t ADJ_SMEM = X_N * H_RC * sizeof(float) + O_N * NTH * sizeof(float2);
+
+__global__ void __launch_bounds__(NTH, 3) k_adj_cell(const __grid_constant__ AdjCellArgs a, int* err) {
+    extern __shared__ __align__(128) float sm[];  // staged tile, then the pairs' own inputs
     __shared__ __align__(8) uint64_t bar;
     if (threadIdx.x == 0) mbar_init(&bar, 1);
     __syncthreads();
     const int n = a.c.n;
-    const int tiles_x = n / TW;
-    const int tx0 = (blockIdx.x % tiles_x) * TW, ty0 = (blockIdx.x / tiles_x) * TH;
-    bool inner = tx0 - HX >= 0 && tx0 + TW + HX <= n && ty0 - 1 >= 0 && ty0 + TH + 1 <= n;
+    const int tx0 = blockIdx.x * TW, ty0 = blockIdx.y * TH;
+    const bool inner = tx0 - HX >= 0 && tx0 + TW + HX <= n && ty0 - 1 >= 0 && ty0 + TH + 1 <= n;
     if (inner) adj_tile<false>(a, sm, &bar, tx0, ty0, err);
     else adj_tile<true>(a, sm, &bar, tx0, ty0, err);
 }
 
 // ---- k_adj_final -----------------------------------------------------------------
-__global__ void k_adj_final(int n, AdjView A, float* __restrict__ out_b) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= n || y >= n) return;
-    out_b[at(n, x, y)] = adj_rock_at(A, n, x, y, at(n, x, y));
+__device__ __forceinline__ float2 adj_rock_pair(const StepConsts1& c, const AdjState& A, int x, int y) {
+    const size_t i = at(c.n, x, y);
+    const float2 nbw = adj_nbw<true>(c, A, x, y, i, ldg2(A.h[0] + i), ldg2(A.h[1] + i));
+    return add2(sub2(ldg2(A.b + i), nbw), adj_normal<true>(A, c.n, x, y, i));
+}
+__global__ void k_adj_final(StepConsts c, AdjState A, float* __restrict__ out_b) {
+    const int x = 2 * (blockIdx.x * BX + threadIdx.x), y = blockIdx.y * BY + threadIdx.y;
+    st2(out_b + at(c.n, x, y), adj_rock_pair(c, A, x, y));
 }
 
 // ---- k_adj_thermal ---------------------------------------------------------------
@@ -432,10 +499,25 @@ __host__ __device__ constexpr int tt_oy(int k) { return (k == 2 || k == 4 || k =
 
 struct ThermalArgs {
     CUtensorMap map_b;  // eroded rock of the step (box TT_RW x TT_BH)
-    AdjView A;          // adjoint of the step's output (own terms + packets)
+    AdjState A;          // adjoint of the step's output (own terms + packets)
     StepConsts c;
     float* g;           // out: adjoint of the eroded rock
 };
+
+__device__ __forceinline__ float adj_rock_at(const StepConsts1& c, const AdjState& A, int n, int x, int y, size_t i) {
+    const float w = c.dt * c.G;
+    float nbw = 0.0f;
+    if (x > 0) nbw += w * A.h[1][i - 1];
+    if (x < n - 1) nbw += w * A.h[0][i + 1];
+    if (y < n - 1) nbw += w * A.h[3][i + n];
+    if (y > 0) nbw += w * A.h[2][i - n];
+    float nrm = 0.0f;
+    if (x > 0) nrm += A.nx[i - 1];
+    if (x < n - 1) nrm -= A.nx[i + 1];
+    if (y > 0) nrm += A.nz[i - n];
+    if (y < n - 1) nrm -= A.nz[i + n];
+    return (A.b[i] - nbw) + nrm;
+}
 
 template <bool EDGE>
 __device__ __forceinline__ void thermal_tile(const ThermalArgs& ta, float* bs, float* as, float* gd, uint64_t* bar,
@@ -455,7 +537,7 @@ __device__ __forceinline__ void thermal_tile(const ThermalArgs& ta, float* bs, f
         const int rx = 2 + q % (TT_RW - 4), ry = q / (TT_RW - 4);
         const int x = gx0 + rx, y = gy0 + ry;
         float v = 0.0f;
-        if (!EDGE || (x >= 0 && x < n && y >= 0 && y < n)) v = adj_rock_at(ta.A, n, x, y, (size_t)y * n + x);
+        if (!EDGE || (x >= 0 && x < n && y >= 0 && y < n)) v = adj_rock_at(c, ta.A, n, x, y, (size_t)y * n + x);
         as[ry * TT_RW + rx] = v;
     }
     bool ok = __syncthreads_and(mbar_wait(bar, 0));
@@ -667,7 +749,7 @@ __global__ void k_descend(float* __restrict__ x, const float* __restrict__ g, si
         x[i] = fminf(fmaxf(x[i] - a * g[i], lo), hi);
 }
 
-dim3 grid_for(int n) { return dim3((n + BX - 1) / BX, (n + BY - 1) / BY); }
+dim3 grid_for(int n) { return dim3(n / (2 * BX), n / BY); }  // n % 64 == 0: every thread has a pair
 
 }  // namespace
 
@@ -683,18 +765,19 @@ void launch_adjoint_sediment(const StepConsts& c, const AdjSlot& slot, const flo
 
 void launch_adjoint_cell(const AdjCellArgs& args, int* err, cudaStream_t st) {
     const int n = args.c.n;
-    k_adj_cell<<<(n / TW) * (n / TH), NTH, 0, st>>>(args, err);
+    cudaFuncSetAttribute(k_adj_cell, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ADJ_SMEM);
+    k_adj_cell<<<dim3(n / TW, n / TH), NTH, ADJ_SMEM, st>>>(args, err);
     count_launch();
 }
 
-void launch_adjoint_final(int n, const AdjView& A, float* out_b, cudaStream_t st) {
-    k_adj_final<<<grid_for(n), dim3(BX, BY), 0, st>>>(n, A, out_b);
+void launch_adjoint_final(const StepConsts& c, const AdjState& A, float* out_b, cudaStream_t st) {
+    k_adj_final<<<grid_for(c.n), dim3(BX, BY), 0, st>>>(c, A, out_b);
     count_launch();
 }
 
 int adjoint_thermal_box_rows() { return TT_BH; }
 
-void launch_adjoint_thermal(const StepConsts& c, const CUtensorMap& map_b, const AdjView& A, float* g, int* err,
+void launch_adjoint_thermal(const StepConsts& c, const CUtensorMap& map_b, const AdjState& A, float* g, int* err,
                             cudaStream_t st) {
     ThermalArgs ta;
     ta.map_b = map_b;

@@ -316,7 +316,6 @@ constexpr int T_FILL = 2 * 152 * T_WARPS * T_BLOCKS;
 // rows [y0, y1) of strip `strip`; SED: with the sediment gather
 template <bool SED>
 __device__ __forceinline__ void transport_strip(const TerrainHot& td, int strip, int y0, int y1) {
-    const unsigned FULL = 0xffffffffu;
     const StepConsts1& c = td.c;
     const int n = c.n;
     const int lane = threadIdx.x & 31;

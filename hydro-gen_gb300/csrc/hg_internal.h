@@ -248,13 +248,6 @@ void launch_fused_one(const TerrainDesc& td, int th, ChainPos pos, int* err, cud
 void launch_fused_half(const TerrainDesc& td, int th, int which, int* err, cudaStream_t st);
 
 // ---- adjoint (hg_adjoint.cu) ----------------------------------------------------------
-// A step's state or its adjoint: rock, water, sediment, fL, fR, fT, fB.
-struct AdjFields {
-    float* b;
-    float* d;
-    float* s;
-    float* f[4];
-};
 // Forward intermediates of one step kept by the segment recompute.
 struct AdjSlot {
     const float* u;
@@ -263,25 +256,26 @@ struct AdjSlot {
 };
 // packet fields of a state adjoint: height-difference terms toward L, R, T,
 // B, inflow terms from L, R, T, B, terrain-normal x and z terms
-constexpr int ADJ_PACKET_FIELDS = 10;
-// Adjoint of a state: each cell's own terms (rock, water, fluxes) plus the
-// packets of the terms of its neighbours' inputs; the sediment adjoint needs
-// no packets.
-struct AdjView {
-    const float* b;
-    const float* d;
-    const float* f[4];
-    const float* pdh[4];
-    const float* pin[4];
-    const float* pdx;
-    const float* pdz;
+// Adjoint of a state, as twelve fields per cell.  b, d, s: what the cell passes
+// to its own rock, water and sediment.  h: the adjoint of its four outflows
+// before scaling, 0 where nothing flows (L, R, T, B); p: of its inflows' sum;
+// gu, gv: of its velocity times its depth; nx, nz: of the terrain normal's
+// height differences.  A reader adds what a cell's neighbours pass to it: with
+// these terms that needs 12 fields against 17 when every neighbour's share is
+// stored by itself.
+struct AdjState {
+    float *b, *d, *s;
+    float* h[4];
+    float *p, *gu, *gv, *nx, *nz;
 };
+constexpr int ADJ_FIELDS = 12;
 // Arguments of k_adj_cell (one kernel parameter).
 struct AdjCellArgs {
-    CUtensorMap maps[7];  // X: rock, water, sediment, fL, fR, fT, fB (64-wide tiles, 1-cell halo)
+    // X: rock, water, sediment, fL, fR, fT, fB; A: h (4), p, gu, gv (64-wide tiles, 1-row halo)
+    CUtensorMap maps[14];
     StepConsts c;
     RainStep rain;
-    AdjView A;            // adjoint of the step's output
+    AdjState A;           // adjoint of the step's output
     float* dse;           // this step's sediment adjoint (read, then cleared)
     float* dse_prev;      // step j - 1's sediment adjoint (scatter target)
     float* du;            // back-trace velocity adjoint: read for step j, written for step j - 1
@@ -289,14 +283,7 @@ struct AdjCellArgs {
     const float* gbe;     // thermal on: adjoint of the eroded rock (replaces A's rock), else nullptr
     AdjSlot prev;         // step j - 1's intermediates
     int scatter_prev;     // reverse step j - 1's sediment pass here (its intermediates exist)
-    float* rb;            // R: own terms of the input adjoint
-    float* rd;
-    float* rs;
-    float* rf[4];
-    float* pdh[4];        // R: packets
-    float* pin[4];
-    float* pdx;
-    float* pdz;
+    AdjState R;           // out: adjoint of the step's input (s only without scatter_prev)
     float* dks;           // per-cell Ks gradient (accumulated)
 };
 bool adjoint_tile_ok(int n);
@@ -307,12 +294,12 @@ void launch_adjoint_sediment(const StepConsts& c, const AdjSlot& slot, const flo
                              float* dv, cudaStream_t st);
 void launch_adjoint_cell(const AdjCellArgs& args, int* err, cudaStream_t st);
 // gathered rock adjoint of a state into out_b
-void launch_adjoint_final(int n, const AdjView& A, float* out_b, cudaStream_t st);
+void launch_adjoint_final(const StepConsts& c, const AdjState& A, float* out_b, cudaStream_t st);
 // reverse of the talus passes: A (adjoint of the step's output, own terms and
 // packets; its rock part is gathered in the kernel) -> g (adjoint of the
 // eroded rock); map_b: boxes 72 x adjoint_thermal_box_rows() of the eroded rock
 int adjoint_thermal_box_rows();
-void launch_adjoint_thermal(const StepConsts& c, const CUtensorMap& map_b, const AdjView& A, float* g, int* err,
+void launch_adjoint_thermal(const StepConsts& c, const CUtensorMap& map_b, const AdjState& A, float* g, int* err,
                             cudaStream_t st);
 // loss = mean((b - target)^2) into *out (device), grad = dloss/db (optional).
 void launch_mse(const float* b, const float* target, size_t count, float* grad, double* part, int nparts,

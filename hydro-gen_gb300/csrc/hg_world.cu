@@ -2030,8 +2030,7 @@ struct hg_tape {
     float* seg = nullptr;    // nbuf x K states: slot j >= 1 the input of a segment's step j,
                              // slot 0 receives the (unused) output of its last step
     float* slots = nullptr;  // nbuf x K x (u, v, eroded sediment, eroded rock) of a segment's steps
-    float* adj = nullptr;    // 2 adjoint states (own terms), alternating A / R
-    float* pk = nullptr;     // their 2 x ADJ_PACKET_FIELDS neighbour packets
+    float* adj = nullptr;    // 2 adjoint states, alternating A / R
     float* aux = nullptr;    // 2 sediment-adjoint buffers, du, dv, rock adjoints for the talus reverse
     float* dks = nullptr;    // per-cell Ks gradient
     unsigned long long* d_step = nullptr;  // step counter of the recompute launches
@@ -2045,17 +2044,22 @@ constexpr int kStateFields = 7;
 constexpr int kSlotFields = 4;  // u, v, eroded sediment, eroded rock
 constexpr int kAuxFields = 5;   // 2 sediment-adjoint buffers, du, dv, eroded-rock adjoint
 
-AdjFields fields_at(float* base, size_t c) {
-    AdjFields f;
+AdjState adj_at(float* base, size_t c) {
+    AdjState f;
     f.b = base;
     f.d = base + c;
     f.s = base + 2 * c;
-    for (int k = 0; k < 4; ++k) f.f[k] = base + (3 + k) * c;
+    for (int k = 0; k < 4; ++k) f.h[k] = base + (3 + k) * c;
+    f.p = base + 7 * c;
+    f.gu = base + 8 * c;
+    f.gv = base + 9 * c;
+    f.nx = base + 10 * c;
+    f.nz = base + 11 * c;
     return f;
 }
 
 void free_tape(hg_tape* t) {
-    cudaFree(t->ckpt); cudaFree(t->seg); cudaFree(t->slots); cudaFree(t->adj); cudaFree(t->pk);
+    cudaFree(t->ckpt); cudaFree(t->seg); cudaFree(t->slots); cudaFree(t->adj);
     cudaFree(t->aux); cudaFree(t->dks); cudaFree(t->d_step);
     for (int b = 0; b < 2; ++b) {
         if (t->ev_rec[b]) cudaEventDestroy(t->ev_rec[b]);
@@ -2089,8 +2093,8 @@ int copy_state_out(hg_world* w, float* dst, cudaStream_t st) {
 
 size_t tape_bytes(size_t c, int nsteps, int K, int nbuf) {
     const size_t nseg = (size_t)(nsteps + K - 1) / K;
-    return (nseg * kStateFields + (size_t)nbuf * K * (kStateFields + kSlotFields) + 2 * kStateFields +
-            2 * ADJ_PACKET_FIELDS + kAuxFields + 1) * c * sizeof(float);
+    return (nseg * kStateFields + (size_t)nbuf * K * (kStateFields + kSlotFields) + 2 * ADJ_FIELDS +
+            kAuxFields + 1) * c * sizeof(float);
 }
 }  // namespace
 
@@ -2148,8 +2152,7 @@ int hg_tape_create(hg_world* w, int nsteps, int ckpt_every, hg_tape** out) {
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&t->ev_rev[b], cudaEventDisableTiming);
         }
     }
-    if (e == cudaSuccess) e = cudaMalloc((void**)&t->adj, 2 * kStateFields * fb);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&t->pk, 2 * ADJ_PACKET_FIELDS * fb);
+    if (e == cudaSuccess) e = cudaMalloc((void**)&t->adj, 2 * ADJ_FIELDS * fb);
     if (e == cudaSuccess) e = cudaMalloc((void**)&t->aux, kAuxFields * fb);
     if (e == cudaSuccess) e = cudaMalloc((void**)&t->dks, fb);
     if (e == cudaSuccess) e = cudaMalloc((void**)&t->d_step, sizeof(unsigned long long));
@@ -2290,31 +2293,16 @@ int hg_backward(hg_tape* t, const float* dL_drock_final, float* dL_dks, float* d
     const size_t c = cells(w), sf = kStateFields * c;
     const StepConsts cst = make_consts(w);
     const int th = w->tuning.th ? w->tuning.th : 16;
-    // state adjoints alternate between two buffers of own terms and packets
-    AdjFields own[2] = {fields_at(t->adj, c), fields_at(t->adj + sf, c)};
-    float* pkb[2] = {t->pk, t->pk + ADJ_PACKET_FIELDS * c};
-    auto view = [&](int k) {
-        AdjView v;
-        v.b = own[k].b;
-        v.d = own[k].d;
-        for (int d = 0; d < 4; ++d) {
-            v.f[d] = own[k].f[d];
-            v.pdh[d] = pkb[k] + (size_t)d * c;
-            v.pin[d] = pkb[k] + (size_t)(4 + d) * c;
-        }
-        v.pdx = pkb[k] + 8 * c;
-        v.pdz = pkb[k] + 9 * c;
-        return v;
-    };
+    // state adjoints alternate between two buffers
+    const AdjState adj[2] = {adj_at(t->adj, c), adj_at(t->adj + ADJ_FIELDS * c, c)};
     float* dse[2] = {t->aux, t->aux + c};
     float* du = t->aux + 2 * c;
     float* dv = t->aux + 3 * c;
     float* gbe = t->aux + 4 * c;  // adjoint of the eroded rock
-    // the final state's adjoint: rock only, no packets
-    HG_CUDA(cudaMemsetAsync(t->adj, 0, 2 * sf * sizeof(float), st));
-    HG_CUDA(cudaMemsetAsync(t->pk, 0, 2 * ADJ_PACKET_FIELDS * c * sizeof(float), st));
+    // the final state's adjoint: rock only (a step writes every field the next reads)
+    HG_CUDA(cudaMemcpyAsync(adj[0].b, dL_drock_final, c * sizeof(float), cudaMemcpyDeviceToDevice, st));
+    HG_CUDA(cudaMemsetAsync(adj[0].d, 0, (ADJ_FIELDS - 1) * c * sizeof(float), st));
     HG_CUDA(cudaMemsetAsync(t->aux, 0, 2 * c * sizeof(float), st));  // scatter targets start at zero
-    HG_CUDA(cudaMemcpyAsync(own[0].b, dL_drock_final, c * sizeof(float), cudaMemcpyDeviceToDevice, st));
     HG_CUDA(cudaMemsetAsync(t->dks, 0, c * sizeof(float), st));
     // segment s lives in buffer (nseg - 1 - s) % nbuf; with two buffers the
     // next segment's recompute runs on the recompute stream while this
@@ -2364,14 +2352,19 @@ int hg_backward(hg_tape* t, const float* dL_drock_final, float* dL_dks, float* d
             if (rc != HG_OK) return rc;
         }
         // the segment's last step: its sediment pass reversed on its own
-        launch_adjoint_sediment(cst, slot_of(len - 1), own[cur].s, dse[m & 1], du, dv, st);
+        launch_adjoint_sediment(cst, slot_of(len - 1), adj[cur].s, dse[m & 1], du, dv, st);
         for (int j = len - 1; j >= 0; --j, ++m) {
             const float* xin = j == 0 ? t->ckpt + (size_t)s * sf : seg_buf(t, bcur) + (size_t)j * sf;
             for (int f = 0; f < kStateFields; ++f)
                 if (!t->tma.get(xin + f * c, w->n, adjoint_box_rows(), &args.maps[f]))
                     return fail(HG_ERR_CUDA, "cuTensorMapEncodeTiled failed for a tape buffer");
             args.rain = make_rain(w, t->step0 + seg_start(t, s) + j + 1);
-            args.A = view(cur);
+            args.A = adj[cur];
+            const float* const af[7] = {args.A.h[0], args.A.h[1], args.A.h[2], args.A.h[3],
+                                        args.A.p,    args.A.gu,   args.A.gv};
+            for (int f = 0; f < 7; ++f)
+                if (!t->tma.get(af[f], w->n, adjoint_box_rows(), &args.maps[kStateFields + f]))
+                    return fail(HG_ERR_CUDA, "cuTensorMapEncodeTiled failed for a tape buffer");
             args.dse = dse[m & 1];
             args.dse_prev = dse[(m + 1) & 1];
             args.gbe = nullptr;
@@ -2380,30 +2373,19 @@ int hg_backward(hg_tape* t, const float* dL_drock_final, float* dL_dks, float* d
                 const float* be = slot_of(j).u + 3 * c;
                 if (!t->tma.get(be, w->n, adjoint_thermal_box_rows(), &mb))
                     return fail(HG_ERR_CUDA, "cuTensorMapEncodeTiled failed for a tape buffer");
-                launch_adjoint_thermal(cst, mb, view(cur), gbe, w->err, st);
+                launch_adjoint_thermal(cst, mb, adj[cur], gbe, w->err, st);
                 args.gbe = gbe;
             }
             args.scatter_prev = j > 0 ? 1 : 0;
             args.prev = j > 0 ? slot_of(j - 1) : AdjSlot{nullptr, nullptr, nullptr};
-            const AdjFields& R = own[cur ^ 1];
-            args.rb = R.b;
-            args.rd = R.d;
-            args.rs = R.s;
-            AdjView rv = view(cur ^ 1);
-            for (int d = 0; d < 4; ++d) {
-                args.rf[d] = R.f[d];
-                args.pdh[d] = const_cast<float*>(rv.pdh[d]);
-                args.pin[d] = const_cast<float*>(rv.pin[d]);
-            }
-            args.pdx = const_cast<float*>(rv.pdx);
-            args.pdz = const_cast<float*>(rv.pdz);
+            args.R = adj[cur ^ 1];
             launch_adjoint_cell(args, w->err, st);
             cur ^= 1;
         }
         if (overlap) HG_CUDA(cudaEventRecord(t->ev_rev[bcur], st));
     }
     if (t->nseg > t->nbuf) t->last_ready = false;  // other segments' recomputes reused buffer 0
-    if (dL_drock0) launch_adjoint_final(w->n, view(cur), dL_drock0, st);
+    if (dL_drock0) launch_adjoint_final(cst, adj[cur], dL_drock0, st);
     if (dL_dks) HG_CUDA(cudaMemcpyAsync(dL_dks, t->dks, c * sizeof(float), cudaMemcpyDeviceToDevice, st));
     HG_CUDA(cudaGetLastError());
     return HG_OK;

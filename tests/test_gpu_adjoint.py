@@ -342,3 +342,26 @@ def test_gpu_adjoint_full_inverse_workload():
               f"({near.mean():.3f} of the area)")
         assert np.mean(rel <= 1e-3) >= 0.9
         assert share >= 0.75
+
+
+@pytest.mark.parametrize("n,depth", [(64, 1e-30), (192, 1e-38), (192, 1e-12)])
+def test_films_outside_the_newton_range_pass_nothing(n, depth):
+    """Two steps before the first rain on films of `depth` (quotients whose
+    operands leave the Newton forms' range, subnormal ones included) give the
+    gradients of the dry start: a film is below half an ulp of every depth and
+    flux that follows, and passes no adjoint itself.  Bar: the atomic adds'
+    order, 1e-5 as above."""
+    torch = torch_dev()
+    outs = []
+    for d in (0.0, depth):
+        w = make_world(n)
+        w.set_rain(H.rain_uniform(0.01, 3))
+        rock = w.download("rock")
+        rng = np.random.default_rng(n)
+        w.upload("water", (d * rng.random((n, n))).astype(np.float32))
+        target = rock - 0.02 * rng.random((n, n))
+        _, dks, db0, _ = gpu_gradients(w, target, 11, 4)
+        assert np.all(np.isfinite(dks)) and np.all(np.isfinite(db0))
+        outs.append((dks, db0))
+    assert rel_l2(outs[1][0], outs[0][0]) <= 1e-5
+    assert rel_l2(outs[1][1], outs[0][1]) <= 1e-5
