@@ -671,11 +671,28 @@ __global__ void k_mse_grad(const float* __restrict__ b, const float* __restrict_
     __shared__ double sh[256 / 32];
     double acc = 0.0;
     const double inv = 1.0 / (double)count;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
-        float e = b[i] - target[i];
-        acc += (double)e * (double)e;
-        if (grad) grad[i] = (float)(2.0 * (double)e * inv);
+    // the gradient is e times 2 / count in two floats: FP64 runs at a small
+    // fraction of the FP32 rate, so it is kept for the sum (the square of a
+    // float is exact in it)
+    const float hi = (float)(2.0 * inv), lo = (float)(2.0 * inv - (double)hi);
+    const size_t step = (size_t)gridDim.x * blockDim.x;
+    auto one = [&](size_t i, float e) {
+        const double d = (double)e;
+        acc = fma(d, d, acc);
+        if (grad) {
+            const float p = e * hi;
+            grad[i] = p + __fmaf_rn(e, lo, __fmaf_rn(e, hi, -p));
+        }
+    };
+    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (; i + 3 * step < count; i += 4 * step) {
+        float e[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) e[k] = b[i + k * step] - target[i + k * step];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) one(i + k * step, e[k]);
     }
+    for (; i < count; i += step) one(i, b[i] - target[i]);
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
     __syncthreads();
@@ -686,11 +703,18 @@ __global__ void k_mse_grad(const float* __restrict__ b, const float* __restrict_
     }
 }
 
-__global__ void k_sum_parts(const double* __restrict__ part, int nparts, double* __restrict__ out) {
-    if (threadIdx.x != 0) return;
+// the partials' sum, in a fixed order: each lane its share, then the lanes'
+// (one lane alone took 22 us for 304 partials, so 5)
+__device__ __forceinline__ double sum_parts(const double* __restrict__ part, int nparts) {
     double t = 0.0;
-    for (int k = 0; k < nparts; ++k) t += part[k];
-    *out = t;
+#pragma unroll 4
+    for (int k = threadIdx.x; k < nparts; k += 32) t += part[k];
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+}
+__global__ void k_sum_parts(const double* __restrict__ part, int nparts, double* __restrict__ out) {
+    const double t = sum_parts(part, nparts);
+    if (threadIdx.x == 0) *out = t;
 }
 
 // per-block sums of g^2 in FP64 (the gradient norm's accumulation)
@@ -711,10 +735,8 @@ __global__ void k_sumsq_part(const float* __restrict__ g, size_t count, double* 
 
 // *out += sum of the partials (fixed order)
 __global__ void k_add_parts(const double* __restrict__ part, int nparts, double* __restrict__ out) {
-    if (threadIdx.x != 0) return;
-    double t = 0.0;
-    for (int k = 0; k < nparts; ++k) t += part[k];
-    *out += t;
+    const double t = sum_parts(part, nparts);
+    if (threadIdx.x == 0) *out += t;
 }
 
 // per-block max |g| (max is order-free, so the result does not depend on the split)

@@ -254,8 +254,6 @@ struct AdjSlot {
     const float* v;
     const float* se;  // eroded sediment
 };
-// packet fields of a state adjoint: height-difference terms toward L, R, T,
-// B, inflow terms from L, R, T, B, terrain-normal x and z terms
 // Adjoint of a state, as twelve fields per cell.  b, d, s: what the cell passes
 // to its own rock, water and sediment.  h: the adjoint of its four outflows
 // before scaling, 0 where nothing flows (L, R, T, B); p: of its inflows' sum;
@@ -295,8 +293,8 @@ void launch_adjoint_sediment(const StepConsts& c, const AdjSlot& slot, const flo
 void launch_adjoint_cell(const AdjCellArgs& args, int* err, cudaStream_t st);
 // gathered rock adjoint of a state into out_b
 void launch_adjoint_final(const StepConsts& c, const AdjState& A, float* out_b, cudaStream_t st);
-// reverse of the talus passes: A (adjoint of the step's output, own terms and
-// packets; its rock part is gathered in the kernel) -> g (adjoint of the
+// reverse of the talus passes: A (adjoint of the step's output; its rock part
+// is gathered in the kernel) -> g (adjoint of the
 // eroded rock); map_b: boxes 72 x adjoint_thermal_box_rows() of the eroded rock
 int adjoint_thermal_box_rows();
 void launch_adjoint_thermal(const StepConsts& c, const CUtensorMap& map_b, const AdjState& A, float* g, int* err,
