@@ -465,14 +465,15 @@ __global__ void __launch_bounds__(NTH, 3) k_adj_cell(const __grid_constant__ Adj
 }
 
 // ---- k_adj_final -----------------------------------------------------------------
+template <bool EDGE>
 __device__ __forceinline__ float2 adj_rock_pair(const StepConsts1& c, const AdjState& A, int x, int y) {
     const size_t i = at(c.n, x, y);
-    const float2 nbw = adj_nbw<true>(c, A, x, y, i, ldg2(A.h[0] + i), ldg2(A.h[1] + i));
-    return add2(sub2(ldg2(A.b + i), nbw), adj_normal<true>(A, c.n, x, y, i));
+    const float2 nbw = adj_nbw<EDGE>(c, A, x, y, i, ldg2(A.h[0] + i), ldg2(A.h[1] + i));
+    return add2(sub2(ldg2(A.b + i), nbw), adj_normal<EDGE>(A, c.n, x, y, i));
 }
 __global__ void k_adj_final(StepConsts c, AdjState A, float* __restrict__ out_b) {
     const int x = 2 * (blockIdx.x * BX + threadIdx.x), y = blockIdx.y * BY + threadIdx.y;
-    st2(out_b + at(c.n, x, y), adj_rock_pair(c, A, x, y));
+    st2(out_b + at(c.n, x, y), adj_rock_pair<true>(c, A, x, y));
 }
 
 // ---- k_adj_thermal ---------------------------------------------------------------
@@ -485,11 +486,18 @@ __global__ void k_adj_final(StepConsts c, AdjState A, float* __restrict__ out_b)
 //   their derivative to the direction that attains them (the first one in
 //   direction order); the marks themselves are locally constant.
 // dh_j = b(c) - b(neighbour j): +dL/ddh_j to the cell, - to the neighbour.
-// 64 x 16 tiles of 512 threads (the ring's share of the recomputed cells is
-// 16 % against 29 % for 64 x 8: 3 % less time); the per-cell terms of the
-// tile and its one-cell ring go through shared memory (54 KB, dynamic), from
-// a TMA box of the eroded rock and the gathered A, both with a two-cell halo.
-constexpr int TT_H = 16, TT_NTH = 512;
+// 64 x 8 tiles of 256 threads; the per-cell terms of the tile and its one-cell
+// ring go through shared memory (dynamic), from a TMA box of the eroded rock
+// and the gathered A, both with a two-cell halo.  Bound by issue slots and the
+// barriers between its phases.  Marks are 1 / 0 factors, the directions that
+// attain a maximum are found by equality, and quotients are the Newton forms:
+// 310 instructions per cell against 445 for the one with an argmax chain and
+// built-in division, 20 us against 23 at 1024² with talus.  2048² with talus,
+// 12 steps forward and backward: 3287 us; 64 x 16 tiles of 512 threads at 64
+// registers 3332, at 40 (spills) 3423; five blocks per SM 3437; a row per warp
+// in pairs as the forward's talus pass 3545 (27 to 30 us a launch: a chain of
+// staging, gather and exchange per row, too few warps to hide it).
+constexpr int TT_H = 8, TT_NTH = 256;
 constexpr int TT_RW = TW + 2 * HX, TT_BH = TT_H + 4, TT_BOX = TT_RW * TT_BH;
 constexpr int TT_BRC = ((TT_BOX + 31) / 32) * 32;
 constexpr int TT_CW = TW + 2, TT_CH = TT_H + 2, TT_NC = TT_CW * TT_CH;  // tile + ring
@@ -504,20 +512,58 @@ struct ThermalArgs {
     float* g;           // out: adjoint of the eroded rock
 };
 
-__device__ __forceinline__ float adj_rock_at(const StepConsts1& c, const AdjState& A, int n, int x, int y, size_t i) {
-    const float w = c.dt * c.G;
-    float nbw = 0.0f;
-    if (x > 0) nbw += w * A.h[1][i - 1];
-    if (x < n - 1) nbw += w * A.h[0][i + 1];
-    if (y < n - 1) nbw += w * A.h[3][i + n];
-    if (y > 0) nbw += w * A.h[2][i - n];
-    float nrm = 0.0f;
-    if (x > 0) nrm += A.nx[i - 1];
-    if (x < n - 1) nrm -= A.nx[i + 1];
-    if (y > 0) nrm += A.nz[i - n];
-    if (y < n - 1) nrm -= A.nz[i + n];
-    return (A.b[i] - nbw) + nrm;
+// The derivatives of one cell's outflows: gdh[k] = dL/ddh_k, and the cell's own
+// term (dL/db through H, plus sum_k dL/ddh_k).  dh: its drops, a: A at its
+// neighbours, ac: at the cell.  Any operands; the kernel leaves ties,
+// infinities and what the Newton forms do not take to it.
+__device__ __noinline__ void thermal_lane(const StepConsts& c, float b, const float dh[8], const float a[8], float ac,
+                                          float gdh[8], float& own) {
+    float Hmax = 0.0f;
+    int jh = -1;
+    own = 0.0f;
+    for (int k = 0; k < 8; ++k) {
+        gdh[k] = 0.0f;
+        if (dh[k] > Hmax) { Hmax = dh[k]; jh = k; }
+    }
+    const float H = gmin(b, Hmax);
+    float bk = 0.0f, max_cross = 0.0f, max_diag = 0.0f;
+    int jc = -1, jd = -1;
+    auto marked = [&](int k) { return dh[k] >= (k < 4 ? c.talus_x_cross : c.talus_b_diag); };
+    for (int k = 0; k < 8; ++k) {
+        if (!marked(k)) continue;
+        bk += dh[k];
+        if (k < 4) { if (dh[k] > max_cross) { max_cross = dh[k]; jc = k; } }
+        else if (dh[k] > max_diag) { max_diag = dh[k]; jd = k; }
+    }
+    if (!(bk > 0.0f)) return;
+    const float sd = max_diag / SQRT2_F;
+    const float slope = fmaxf(max_cross, sd);
+    const int js = (jd >= 0 && sd > max_cross) ? jd : jc;
+    float s1 = 1.0f;
+    const float newsh = 1.0f + poly_atanf(slope) - c.Kalpha0;
+    const bool taken = newsh > s1;
+    if (taken) s1 = newsh;
+    const float sh3 = s1 * (s1 * s1);
+    const float S = c.dt * c.Kspeed0 * sh3 * H / 2.0f;
+    const float rbk = __frcp_rn(bk);
+    float gbar = 0.0f;
+    for (int k = 0; k < 8; ++k)
+        if (marked(k)) gbar += (a[k] - ac) * dh[k];
+    gbar *= rbk;
+    const float sb = S * rbk;
+    for (int k = 0; k < 8; ++k)
+        if (marked(k)) gdh[k] = sb * ((a[k] - ac) - gbar);
+    const float dH = gbar * (c.dt * c.Kspeed0 * sh3 * 0.5f);
+    if (taken && js >= 0) {
+        const float ds1 = gbar * (c.dt * c.Kspeed0 * H * 0.5f) * 3.0f * s1 * s1;
+        const float dslope = ds1 * __frcp_rn(1.0f + slope * slope);
+        gdh[js] += js < 4 ? dslope : dslope * RCP_SQRT2_F;
+    }
+    if (Hmax < b) gdh[jh] += dH;
+    else own += dH;
+    for (int k = 0; k < 8; ++k) own += gdh[k];
 }
+
 
 template <bool EDGE>
 __device__ __forceinline__ void thermal_tile(const ThermalArgs& ta, float* bs, float* as, float* gd, uint64_t* bar,
@@ -532,13 +578,14 @@ __device__ __forceinline__ void thermal_tile(const ThermalArgs& ta, float* bs, f
     // while the eroded rock flies: the gathered adjoint A of the output rock
     // over the region's columns 2 .. TT_RW - 3 (the tile, its ring and their
     // neighbours), 0 outside the grid
+    constexpr int GP = (TT_RW - 4) / 2;  // pairs per row
 #pragma unroll 1
-    for (int q = tid; q < (TT_RW - 4) * TT_BH; q += TT_NTH) {
-        const int rx = 2 + q % (TT_RW - 4), ry = q / (TT_RW - 4);
+    for (int q = tid; q < GP * TT_BH; q += TT_NTH) {
+        const int rx = 2 + 2 * (q % GP), ry = q / GP;
         const int x = gx0 + rx, y = gy0 + ry;
-        float v = 0.0f;
-        if (!EDGE || (x >= 0 && x < n && y >= 0 && y < n)) v = adj_rock_at(c, ta.A, n, x, y, (size_t)y * n + x);
-        as[ry * TT_RW + rx] = v;
+        float2 v = pf(0.0f);
+        if (!EDGE || (x >= 0 && x < n && y >= 0 && y < n)) v = adj_rock_pair<EDGE>(c, ta.A, x, y);
+        st2(as + ry * TT_RW + rx, v);
     }
     bool ok = __syncthreads_and(mbar_wait(bar, 0));
     if (!ok) {
@@ -556,73 +603,72 @@ __device__ __forceinline__ void thermal_tile(const ThermalArgs& ta, float* bs, f
         if (!EDGE || (x >= 0 && x < n && y >= 0 && y < n)) {
             const int si = (ry + 2) * TT_RW + HX + rx;
             const float b = bs[si];
+            auto nb = [&](const float* p, int k) { return p[si + tt_oy(k) * TT_RW + tt_ox(k)]; };
             float dh[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
                 bool out = EDGE && (x + tt_ox(k) < 0 || x + tt_ox(k) >= n || y + tt_oy(k) < 0 || y + tt_oy(k) >= n);
-                dh[k] = b - (out ? FAR_HEIGHT : bs[si + tt_oy(k) * TT_RW + tt_ox(k)]);
+                dh[k] = b - (out ? FAR_HEIGHT : nb(bs, k));
             }
-            // the forward's values (cell_thermal_outflows' operations)
-            float Hmax = 0.0f;
-            int jh = -1;
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-                if (dh[k] > Hmax) { Hmax = dh[k]; jh = k; }
-            const float H = gmin(b, Hmax);
-            float bk = 0.0f, max_cross = 0.0f, max_diag = 0.0f;
-            int jc = -1, jd = -1;
-            bool mk[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                mk[k] = dh[k] >= (k < 4 ? c.talus_x_cross : c.talus_b_diag);
-                if (mk[k]) {
-                    bk += dh[k];
-                    if (k < 4) { if (dh[k] > max_cross) { max_cross = dh[k]; jc = k; } }
-                    else if (dh[k] > max_diag) { max_diag = dh[k]; jd = k; }
-                }
-            }
-            if (bk > 0.0f) {
-                const float sd = max_diag / SQRT2_F;
-                const float slope = fmaxf(max_cross, sd);
-                const int js = (jd >= 0 && sd > max_cross) ? jd : jc;
-                const float alph = poly_atanf(slope);
-                float s1 = 1.0f;
-                const float newsh = 1.0f + alph - c.Kalpha0;
-                const bool taken = newsh > s1;
-                if (taken) s1 = newsh;
-                const float sh3 = s1 * (s1 * s1);
-                const float S = c.dt * c.Kspeed0 * sh3 * H / 2.0f;
-                // reverse
-                const float ac = as[si];
-                const float rbk = __frcp_rn(bk);
-                float g[8], gbar = 0.0f;
+            float mc = fmaxf(fmax3(dh[0], dh[1], dh[2]), dh[3]), md = fmaxf(fmax3(dh[4], dh[5], dh[6]), dh[7]);
+            if ((mc >= c.talus_x_cross) | (md >= c.talus_b_diag)) {
+                // the forward's values (cell_thermal_outflows_dh2)
+                const float Hmax = fmax3(mc, md, 0.0f), H = fminf(b, Hmax);
+                mc = mc >= c.talus_x_cross ? mc : 0.0f;
+                md = md >= c.talus_b_diag ? md : 0.0f;
+                float m[8], bk = 0.0f;  // 1 where marked
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
-                    g[k] = mk[k] ? as[si + tt_oy(k) * TT_RW + tt_ox(k)] - ac : 0.0f;
-                    gbar += g[k] * dh[k];
+                    m[k] = set_ge(dh[k], k < 4 ? c.talus_x_cross : c.talus_b_diag);
+                    bk = __fmaf_rn(dh[k], m[k], bk);  // (the product is exact)
+                }
+                const float sd = div_recip(md, SQRT2_F, RCP_SQRT2_F);
+                const float slope = fmaxf(mc, sd);
+                const float newsh = 1.0f + poly_atanf(slope) - c.Kalpha0, s1 = fmaxf(newsh, 1.0f);
+                const float sh3 = s1 * (s1 * s1), dtK = c.dt * c.Kspeed0;
+                const float S = dtK * sh3 * H * 0.5f;
+                // reverse: differences of A in the marked directions
+                const float ac = as[si];
+                const float rbk = rcp_newton(bk);
+                float gbar = 0.0f;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    gdh[k] = (nb(as, k) - ac) * m[k];
+                    gbar += gdh[k] * dh[k];
                 }
                 gbar *= rbk;
                 const float sb = S * rbk;
+                const float dH = gbar * (dtK * sh3 * 0.5f), dHn = Hmax < b ? dH : 0.0f;
+                // the steepest marked slope's direction, where it sets the sharpness
+                const float ds1 = gbar * (dtK * H * 0.5f) * 3.0f * s1 * s1;
+                const float ds = newsh > 1.0f ? ds1 * rcp_newton(1.0f + slope * slope) : 0.0f;
+                const float dsd = ds * RCP_SQRT2_F;
+                const float NONE = __int_as_float(0x7fc00000);  // equal to nothing
+                const float kc = sd > mc ? NONE : mc, kd = sd > mc ? md : NONE;
+                float hits = 0.0f;  // directions that attain the two maxima: 2, more in a tie
+                own = Hmax < b ? 0.0f : dH;
 #pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    if (mk[k]) gdh[k] = sb * (g[k] - gbar);
-                const float dH = gbar * (c.dt * c.Kspeed0 * sh3 * 0.5f);
-                if (taken && js >= 0) {
-                    const float ds1 = gbar * (c.dt * c.Kspeed0 * H * 0.5f) * 3.0f * s1 * s1;
-                    const float dslope = ds1 * __frcp_rn(1.0f + slope * slope);
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)  // static indices keep gdh in registers
-                        if (k == js) gdh[k] += k < 4 ? dslope : dslope * RCP_SQRT2_F;
+                for (int k = 0; k < 8; ++k) {
+                    const float ts = set_eq(dh[k], k < 4 ? kc : kd), th = set_eq(dh[k], Hmax);
+                    hits += ts + th;
+                    const float v = sb * (gdh[k] - gbar) * m[k];
+                    gdh[k] = __fmaf_rn(th, dHn, __fmaf_rn(ts, k < 4 ? ds : dsd, v));  // (products with 0 and 1 are exact)
+                    own += gdh[k];
                 }
-                if (Hmax < b) {
+                // else: outside the Newton forms' range, several directions at a maximum, sums not finite
+                if (!((c.fast_div != 0) & (bk <= 0x1p40f) & (S >= 0x1p-50f) & (S <= 0x1p40f) & (hits == 2.0f) &
+                      (fabsf(own) < 0x1p126f))) {
+                    float al[8];
 #pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        if (k == jh) gdh[k] += dH;
-                } else {
-                    own += dH;
+                    for (int k = 0; k < 8; ++k) al[k] = nb(as, k);
+                    float dl[8], gl[8], ol;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) dl[k] = dh[k];
+                    thermal_lane(c, b, dl, al, ac, gl, ol);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) gdh[k] = gl[k];
+                    own = ol;
                 }
-#pragma unroll
-                for (int k = 0; k < 8; ++k) own += gdh[k];
             }
         }
 #pragma unroll
@@ -649,7 +695,7 @@ __device__ __forceinline__ void thermal_tile(const ThermalArgs& ta, float* bs, f
 
 constexpr size_t TT_SMEM = (2 * TT_BRC + 9 * TT_NC) * sizeof(float) + 8;
 
-__global__ void __launch_bounds__(TT_NTH) k_adj_thermal(const __grid_constant__ ThermalArgs ta, int* err) {
+__global__ void __launch_bounds__(TT_NTH, 4) k_adj_thermal(const __grid_constant__ ThermalArgs ta, int* err) {
     extern __shared__ __align__(128) float tdyn[];
     float* bs = tdyn;
     float* as = tdyn + TT_BRC;

@@ -365,3 +365,21 @@ def test_films_outside_the_newton_range_pass_nothing(n, depth):
         outs.append((dks, db0))
     assert rel_l2(outs[1][0], outs[0][0]) <= 1e-5
     assert rel_l2(outs[1][1], outs[0][1]) <= 1e-5
+
+
+@pytest.mark.parametrize("n", [64, 192])
+def test_thermal_adjoint_on_a_ramp(n):
+    """One step on a ramp of equal steps: every cell's largest drop and steepest
+    slope are attained by several directions at once, of which the first takes
+    the derivative.  (From the second step on the float and the FP64 model
+    break the ties differently.)  Bar as for the small sizes above."""
+    torch_dev()
+    w = make_world(n, thermal=True)
+    b0 = np.broadcast_to(2.0 * np.arange(n), (n, n)).astype(np.float64)
+    w.upload("rock", np.ascontiguousarray(b0, dtype=np.float32))
+    ks = w.download("ks")
+    rng = np.random.default_rng(n)
+    target = b0 - 0.02 * rng.random((n, n))
+    _, _, db0, _ = gpu_gradients(w, target, 1, 1)
+    _, _, rdb0 = O.adjoint_ref(ref_settings(True), 0.01, 1, b0, ks, target, 1)
+    assert rel_l2(db0, rdb0) <= 1e-3
