@@ -105,19 +105,17 @@ struct Drops {
     uint32_t* iters;
     int32_t* kill;
 };
-// Counting-sort and per-record buffers of one particle world.
+// Bucket and per-record buffers of one particle world.
 struct ParticleBufs {
     Drops d;
-    uint32_t* cnt;         // n*n records per texel
-    uint32_t* offs;        // n*n + 1 exclusive prefix
-    uint32_t* cursor;      // n*n scatter cursors
-    uint32_t* block_sums;  // particle_scan_blocks(n*n)
-    uint32_t* keys;        // 4*count records (droplet * 4 + corner), bucketed by texel
-    uint32_t* sorted;      // 4*count: hot texels' buckets in droplet-id order
-    uint32_t* hot;         // 2 + 2*hot_cap: counts of mid and big texels, then their indices
-    uint32_t hot_cap;      // particle_hot_capacity(n*n, count)
-    float* rec;            // 8*count: per record the dirt and rock sediment it left
-    uint8_t* rec_mask;     // 4*count: which layers a record set
+    uint32_t* cnt;      // n*n records per texel, then particle_counters() counters
+    uint32_t* offs;     // n*n: where a texel's bucket begins
+    uint32_t* keys;     // 4*count records (droplet * 4 + corner), bucketed by texel
+    uint32_t* sorted;   // 4*count: the largest buckets' chunks in droplet-id order
+    uint32_t* list[4];  // texels by record count, particle_list_capacity() each
+    uint4* rank;        // count: the places of a droplet's records in their buckets
+    float4* pack;       // 2*count: what a record reads of its droplet
+    float2* rec;        // 4*count: what a record left for its droplet
 };
 // The fields a particle pass reads or writes; mom = momentum (x, y, z, w).
 struct PWorld {
@@ -126,8 +124,9 @@ struct PWorld {
     float* water;
     float* mom[4];
 };
-size_t particle_scan_blocks(size_t cells);
-size_t particle_hot_capacity(size_t cells, int count);
+size_t particle_counters();
+int particle_lists();
+size_t particle_list_capacity(int list, size_t cells, int count);
 // movement, counting sort, erosion in droplet-id order, sediment replay
 void launch_particle_step(const StepConsts& c, const hg_erosion_settings& es, const ParticleBufs& pb,
                           const PWorld& pw, uint32_t step1, uint64_t seed, bool should_rain, cudaStream_t st);

@@ -6,16 +6,20 @@
 // The shader serialises the droplets' updates of a texel with a spinlock per
 // texel, in whatever order the droplets win it.  Here the order is fixed and
 // no thread waits on another:
-//   k_pcount / scan / k_pscatter   counting sort of the droplets' four corner
-//                                  records by texel
-//   k_papply / _mid / _big         each texel applies its records in
+//   k_pmove                        moves the droplets, counts their four corner
+//                                  records per texel (a record's place in its
+//                                  texel's bucket is what the count was) and
+//                                  packs what a record reads of its droplet
+//   k_palloc / k_pscatter          give each texel a bucket, and the texels to
+//                                  lists by record count; keys into the buckets
+//   k_papply                       each texel applies its records in
 //                                  droplet-id order (a texel update needs only
 //                                  the droplet's state from before the pass)
 //                                  and stores what each corner left for the
 //                                  droplet's sediment; a texel with up to 8
 //                                  records sorts them in its thread's
-//                                  registers, up to 32 across a warp's lanes,
-//                                  more in a warp's shared memory
+//                                  registers, one with more across a warp's
+//                                  lanes
 //   k_pfinal                       each droplet replays its corners 0..3
 // which is a sequential pass over droplets in id order, corners in order.
 // Spawn positions come from Philox4x32-10 (counter: droplet id, step,
@@ -44,6 +48,22 @@ __device__ __forceinline__ float bilin(const float* f, int n, float sx, float sy
     return gmix(v1, v2, fy);
 }
 
+// corner k of a droplet: texel (cx, cy) and the droplet's offset in its texel.
+// A live droplet sits in (1, n - 2) on both axes (movement reverts steps that
+// leave it), so the clamp only keeps a non-finite position's texels inside the map.
+__device__ __forceinline__ void corner(float px, float py, int k, int n, int& cx, int& cy, float& ofx, float& ofy) {
+    const int bx = min(max((int)(px * 1.0f), 0), n - 2), by = min(max((int)(py * 1.0f), 0), n - 2);
+    ofx = fract_(px * 1.0f);
+    ofy = fract_(py * 1.0f);
+    cx = (k == 1 || k == 2) ? bx + 1 : bx;
+    cy = (k >= 2) ? by + 1 : by;
+}
+__device__ __forceinline__ float corner_weight(float ofx, float ofy, int k) {
+    const float wx = (k == 1 || k == 2) ? ofx : 1.0f - ofx;
+    const float wy = (k >= 2) ? ofy : 1.0f - ofy;
+    return wx * wy;
+}
+
 struct MoveArgs {
     StepConsts c;
     hg_erosion_settings es;
@@ -56,9 +76,83 @@ struct MoveArgs {
     uint32_t step1;
     uint32_t seed_lo, seed_hi;
     int should_rain;
+    uint32_t* cnt;  // records per texel, zero before
+    uint4* rank;    // per droplet: its records' places in their buckets
+    float4* pack;   // per droplet, two: offset x (sign bit: kill), offset y, capacity, volume; sediments, velocity
 };
 
-__global__ void k_pmove(const MoveArgs a) {
+// Terrain normal's height differences and the samples at (px, py), see k_pmove
+struct Around {
+    float rr, rg, lr, lg, br, bg, tr, tg, mx, my, water;
+};
+__device__ __forceinline__ Around look_around(const MoveArgs& a, int n, float px, float py) {
+    Around o;
+    o.rr = bilin(a.rock, n, px + 1.0f, py); o.rg = bilin(a.dirt, n, px + 1.0f, py);
+    o.lr = bilin(a.rock, n, px - 1.0f, py); o.lg = bilin(a.dirt, n, px - 1.0f, py);
+    o.br = bilin(a.rock, n, px, py - 1.0f); o.bg = bilin(a.dirt, n, px, py - 1.0f);
+    o.tr = bilin(a.rock, n, px, py + 1.0f); o.tg = bilin(a.dirt, n, px, py + 1.0f);
+    o.mx = bilin(a.mx, n, px, py);
+    o.my = bilin(a.my, n, px, py);
+    o.water = bilin(a.water, n, px, py);
+    return o;
+}
+// The same from 16-byte loads.  A warp's droplets lie anywhere, so a load costs
+// a cache line per lane whatever its width, and the kernel is bound by those:
+// 44 loads of a texel each against about 20 of an aligned quad, of which a row's
+// four neighbouring texels need one or two (n is a multiple of 8: rows are whole
+// quads).  Needs the whole cross of texels inside the map.
+// With the count (9 us by itself before) and the packing the launch takes 41 us
+// (262144 droplets on 1024²), without them it took as long from single texels.
+__device__ __forceinline__ Around look_around_quads(const MoveArgs& a, int n, float px, float py, int ix, int iy) {
+    // texels first .. first + M - 1 of a row
+    const int s1 = (ix - 1) & 3, q1 = (ix - 1) & ~3, s0 = ix & 3, q0 = ix & ~3;
+    auto row4 = [&](const float* f, int y, float t[4]) {
+        const float4* p = reinterpret_cast<const float4*>(f + (size_t)y * n + q1);
+        const float4 u = __ldg(p);
+        float4 v = u;
+        if (s1) v = __ldg(p + 1);
+        t[0] = s1 == 0 ? u.x : s1 == 1 ? u.y : s1 == 2 ? u.z : u.w;
+        t[1] = s1 == 0 ? u.y : s1 == 1 ? u.z : s1 == 2 ? u.w : v.x;
+        t[2] = s1 == 0 ? u.z : s1 == 1 ? u.w : s1 == 2 ? v.x : v.y;
+        t[3] = s1 == 0 ? u.w : s1 == 1 ? v.x : s1 == 2 ? v.y : v.z;
+    };
+    auto row2 = [&](const float* f, int y, float t[2]) {
+        const float4* p = reinterpret_cast<const float4*>(f + (size_t)y * n + q0);
+        const float4 u = __ldg(p);
+        float v = 0.0f;
+        if (s0 == 3) v = __ldg(reinterpret_cast<const float*>(p + 1));
+        t[0] = s0 == 0 ? u.x : s0 == 1 ? u.y : s0 == 2 ? u.z : u.w;
+        t[1] = s0 == 0 ? u.y : s0 == 1 ? u.z : s0 == 2 ? u.w : v;
+    };
+    const float fx = fract_(px), fy = fract_(py), fr = fract_(px + 1.0f), fl = fract_(px - 1.0f),
+                ft = fract_(py + 1.0f), fb = fract_(py - 1.0f);
+    Around o;
+    auto cross = [&](const float* f, float& r, float& l, float& b, float& t) {
+        float c0[4], c1[4], dn[2], up[2];
+        row4(f, iy, c0);
+        row4(f, iy + 1, c1);
+        row2(f, iy - 1, dn);
+        row2(f, iy + 2, up);
+        r = gmix(gmix(c0[2], c0[3], fr), gmix(c1[2], c1[3], fr), fy);
+        l = gmix(gmix(c0[0], c0[1], fl), gmix(c1[0], c1[1], fl), fy);
+        b = gmix(gmix(dn[0], dn[1], fx), gmix(c0[1], c0[2], fx), fb);
+        t = gmix(gmix(c1[1], c1[2], fx), gmix(up[0], up[1], fx), ft);
+    };
+    cross(a.rock, o.rr, o.lr, o.br, o.tr);
+    cross(a.dirt, o.rg, o.lg, o.bg, o.tg);
+    auto here = [&](const float* f) {
+        float c0[2], c1[2];
+        row2(f, iy, c0);
+        row2(f, iy + 1, c1);
+        return gmix(gmix(c0[0], c0[1], fx), gmix(c1[0], c1[1], fx), fy);
+    };
+    o.mx = here(a.mx);
+    o.my = here(a.my);
+    o.water = here(a.water);
+    return o;
+}
+
+__global__ void __launch_bounds__(PB, 4) k_pmove(const MoveArgs a) {
     const int id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= a.d.count) return;
     const int n = a.c.n;
@@ -86,17 +180,17 @@ __global__ void k_pmove(const MoveArgs a) {
     }
     if (!done) {
         // get_terr_normal (:48-60)
-        const float rr = bilin(a.rock, n, px + 1.0f, py), rg = bilin(a.dirt, n, px + 1.0f, py);
-        const float lr = bilin(a.rock, n, px - 1.0f, py), lg = bilin(a.dirt, n, px - 1.0f, py);
-        const float br = bilin(a.rock, n, px, py - 1.0f), bg = bilin(a.dirt, n, px, py - 1.0f);
-        const float tr = bilin(a.rock, n, px, py + 1.0f), tg = bilin(a.dirt, n, px, py + 1.0f);
-        const float dx = rr + rg - lr - lg;
-        const float dz = tr + tg - br - bg;
+        const int ix = (int)px, iy = (int)py;
+        const bool quads = ix >= 1 && ix <= n - 3 && iy >= 1 && iy <= n - 3 &&
+                           (int)(px + 1.0f) == ix + 1 && (int)(px - 1.0f) == ix - 1 && (int)(py + 1.0f) == iy + 1 &&
+                           (int)(py - 1.0f) == iy - 1;
+        const Around o = quads ? look_around_quads(a, n, px, py, ix, iy) : look_around(a, n, px, py);
+        const float dx = o.rr + o.rg - o.lr - o.lg;
+        const float dz = o.tr + o.tg - o.br - o.bg;
         const float cx = dx * 2.0f - 0.0f * dz, cy = 0.0f * 0.0f - 2.0f * 2.0f, cz = 2.0f * dz - dx * 0.0f;
         const float len = sqrtf(cx * cx + cy * cy + cz * cz);
         const float nx = cx / len, ny = cy / len, nz = cz / len;
-        const float mxv = bilin(a.mx, n, px, py), myv = bilin(a.my, n, px, py);
-        const float water = bilin(a.water, n, px, py);
+        const float mxv = o.mx, myv = o.my, water = o.water;
         vx -= (dt * nx) / vol * a.es.G;
         vy -= (dt * nz) / vol * a.es.G;
         const float lm = sqrtf(mxv * mxv + myv * myv);
@@ -130,46 +224,25 @@ __global__ void k_pmove(const MoveArgs a) {
     }
     a.d.px[id] = px; a.d.py[id] = py; a.d.vx[id] = vx; a.d.vy[id] = vy; a.d.vol[id] = vol;
     a.d.s0[id] = s0; a.d.s1[id] = s1; a.d.sc[id] = sc; a.d.iters[id] = iters; a.d.kill[id] = kill;
-}
-
-// corner k of a droplet: texel (cx, cy) and weight.  A live droplet sits in
-// (1, n - 2) on both axes (movement reverts steps that leave it), so the
-// clamp only keeps a non-finite position's texels inside the map.
-__device__ __forceinline__ void corner(float px, float py, int k, int n, int& cx, int& cy, float& wgt) {
-    const int bx = min(max((int)(px * 1.0f), 0), n - 2), by = min(max((int)(py * 1.0f), 0), n - 2);
-    const float ofx = fract_(px * 1.0f), ofy = fract_(py * 1.0f);
-    cx = (k == 1 || k == 2) ? bx + 1 : bx;
-    cy = (k >= 2) ? by + 1 : by;
-    const float wx = (k == 1 || k == 2) ? ofx : 1.0f - ofx;
-    const float wy = (k >= 2) ? ofy : 1.0f - ofy;
-    wgt = wx * wy;
-}
-
-__global__ void k_pcount(Drops d, int n, uint32_t* __restrict__ cnt) {
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= d.count || d.iters[id] == 0) return;
+    if (iters == 0) return;
+    uint32_t rank[4];
+    float ofx, ofy;
     for (int k = 0; k < 4; ++k) {
         int cx, cy;
-        float wgt;
-        corner(d.px[id], d.py[id], k, n, cx, cy, wgt);
-        atomicAdd(cnt + (size_t)cy * n + cx, 1u);
+        corner(px, py, k, n, cx, cy, ofx, ofy);
+        rank[k] = atomicAdd(a.cnt + (size_t)cy * n + cx, 1u);
     }
+    a.pack[2 * id] = make_float4(copysignf(ofx, kill ? -1.0f : 1.0f), ofy, sc, vol);
+    a.pack[2 * id + 1] = make_float4(s0, s1, vx, vy);
+    a.rank[id] = make_uint4(rank[0], rank[1], rank[2], rank[3]);
 }
 
-__global__ void k_pscatter(Drops d, int n, uint32_t* __restrict__ cursor, uint32_t* __restrict__ keys) {
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= d.count || d.iters[id] == 0) return;
-    for (int k = 0; k < 4; ++k) {
-        int cx, cy;
-        float wgt;
-        corner(d.px[id], d.py[id], k, n, cx, cy, wgt);
-        const uint32_t slot = atomicAdd(cursor + (size_t)cy * n + cx, 1u);
-        keys[slot] = (uint32_t)id * 4u + (uint32_t)k;
-    }
-}
-
-// exclusive scan of up to 4096 x 4096 counts: blocks of 4096, then the block sums
-constexpr int SCAN_T = 1024, SCAN_E = 4;
+constexpr int SMALL = 8;       // records a texel's own thread sorts and applies
+constexpr int HALF = 4;        // of those, the ones with a network of half the size
+constexpr int MID = 32;        // records a warp sorts in registers, one per lane
+constexpr int HOT_KEYS = 512;  // records a warp sorts at a time in a busier texel
+enum { L_BIG = 0, L_MID, L_SMALL, L_HALF, LISTS };
+enum { C_TOTAL = LISTS, C_NEXT, COUNTERS };  // records in all; next work item of k_papply
 
 __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* warp_sums, uint32_t& total) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -196,77 +269,83 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* w
     return before + x - v;
 }
 
-__global__ void k_scan_blocks(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, size_t count,
-                              uint32_t* __restrict__ block_sums) {
-    __shared__ uint32_t ws[32];
-    const size_t base = (size_t)blockIdx.x * SCAN_T * SCAN_E + (size_t)threadIdx.x * SCAN_E;
-    uint32_t v[SCAN_E], sum = 0;
+struct TexelLists {
+    uint32_t* counters;      // COUNTERS of them: texels per list, then C_*; zero before
+    uint32_t* list[LISTS];
+    uint32_t cap[LISTS];
+};
+
+// Buckets for the texels' records, in whatever order the blocks come (a texel
+// sorts its own), and the texels by record count: 4096 texels per block, one
+// counter update per block and list.  One pass over the counts in place of a
+// scan's three (17 us at 1024², now 9).
+constexpr int AL_T = 1024, AL_E = 4;
+__global__ void __launch_bounds__(AL_T) k_palloc(const uint32_t* __restrict__ cnt, uint32_t* __restrict__ offs,
+                                                 size_t count, TexelLists tl) {
+    __shared__ uint32_t ws[32], num[LISTS], first[LISTS], base_sh;
+    const size_t base = ((size_t)blockIdx.x * AL_T + threadIdx.x) * AL_E;
+    if (threadIdx.x < LISTS) num[threadIdx.x] = 0;
+    __syncthreads();
+    uint32_t v[AL_E] = {0, 0, 0, 0}, sum = 0, place[AL_E];
+    if (base < count) {  // (n is a multiple of 8: whole quads)
+        const uint4 q = *reinterpret_cast<const uint4*>(cnt + base);
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    }
+    auto which = [](uint32_t k) { return k > MID ? L_BIG : k > SMALL ? L_MID : k > HALF ? L_SMALL : L_HALF; };
 #pragma unroll
-    for (int e = 0; e < SCAN_E; ++e) {
-        v[e] = base + e < count ? in[base + e] : 0u;
+    for (int e = 0; e < AL_E; ++e) {
         sum += v[e];
+        if (v[e]) place[e] = atomicAdd(&num[which(v[e])], 1u);
     }
     uint32_t total;
-    uint32_t run = block_exclusive_scan(sum, ws, total);
+    uint32_t run = block_exclusive_scan(sum, ws, total);  // (its barriers order num)
+    if (threadIdx.x < LISTS) first[threadIdx.x] = num[threadIdx.x] ? atomicAdd(tl.counters + threadIdx.x, num[threadIdx.x]) : 0u;
+    if (threadIdx.x == LISTS) base_sh = total ? atomicAdd(tl.counters + C_TOTAL, total) : 0u;
+    __syncthreads();
+    run += base_sh;
 #pragma unroll
-    for (int e = 0; e < SCAN_E; ++e) {
-        if (base + e < count) out[base + e] = run;
+    for (int e = 0; e < AL_E; ++e) {
+        if (v[e]) {
+            offs[base + e] = run;
+            const int w = which(v[e]);
+            const uint32_t slot = first[w] + place[e];
+            if (slot < tl.cap[w]) tl.list[w][slot] = (uint32_t)(base + e);
+        }
         run += v[e];
     }
-    if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
 }
 
-// one block: exclusive scan of the block sums in place, chunk by chunk; grand total into *total_out
-__global__ void k_scan_sums(uint32_t* __restrict__ sums, int nb, uint32_t* __restrict__ total_out) {
-    __shared__ uint32_t ws[32];
-    uint32_t carry = 0;
-    for (int chunk = 0; chunk < nb; chunk += SCAN_T * SCAN_E) {
-        const int base = chunk + threadIdx.x * SCAN_E;
-        uint32_t v[SCAN_E], sum = 0;
+__global__ void k_pscatter(Drops d, int n, const uint32_t* __restrict__ offs, const uint4* __restrict__ rank,
+                           uint32_t* __restrict__ keys) {
+    const int id = blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= d.count || d.iters[id] == 0) return;
+    const float px = d.px[id], py = d.py[id];
+    const uint4 r = rank[id];
+    const uint32_t rk[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
-        for (int e = 0; e < SCAN_E; ++e) {
-            v[e] = base + e < nb ? sums[base + e] : 0u;
-            sum += v[e];
-        }
-        uint32_t total;
-        uint32_t run = carry + block_exclusive_scan(sum, ws, total);
-#pragma unroll
-        for (int e = 0; e < SCAN_E; ++e) {
-            if (base + e < nb) sums[base + e] = run;
-            run += v[e];
-        }
-        carry += total;
-        __syncthreads();  // ws is reused by the next chunk
+    for (int k = 0; k < 4; ++k) {
+        int cx, cy;
+        float ofx, ofy;
+        corner(px, py, k, n, cx, cy, ofx, ofy);
+        keys[offs[(size_t)cy * n + cx] + rk[k]] = (uint32_t)id * 4u + (uint32_t)k;
     }
-    if (threadIdx.x == 0) *total_out = carry;
-}
-
-__global__ void k_scan_add(uint32_t* __restrict__ out, uint32_t* __restrict__ cursor, size_t count,
-                           const uint32_t* __restrict__ sums) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const uint32_t v = out[i] + sums[i / (SCAN_T * SCAN_E)];
-    out[i] = v;
-    cursor[i] = v;
 }
 
 struct ApplyArgs {
     hg_erosion_settings es;
-    Drops d;
-    int n;
-    const uint32_t* offs;  // n*n + 1
+    const float4* pack;
+    const uint32_t* cnt;
+    const uint32_t* offs;
     uint32_t* keys;        // records bucketed by texel, any order within a bucket
     uint32_t* sorted;      // big texels: their bucket in droplet-id order
-    uint32_t* hot;         // [0], [1]: mid and big texel counts; then mid texels
-                           // from [2], big texels from [2 + hot_cap]
-    uint32_t hot_cap;
+    TexelLists tl;
     float* rock;
     float* dirt;
     float* water;
     float* mz;
     float* mw;
-    float* rec;            // per record (droplet * 4 + corner): s1 of dirt, s1 of rock
-    uint8_t* rec_mask;     // bit 1: dirt layer handled, bit 0: rock layer handled
+    float2* rec;           // per record (droplet * 4 + corner): the sediment it left of dirt and of
+                           // rock, UNSET for a layer it did not reach
 };
 
 // A record's inputs: all from before the pass
@@ -279,16 +358,15 @@ struct Rec {
 __device__ __forceinline__ Rec load_rec(const ApplyArgs& a, uint32_t key) {
     Rec r;
     r.key = key;
-    const int id = (int)(key >> 2), k = (int)(key & 3u);
-    int cx, cy;
-    corner(a.d.px[id], a.d.py[id], k, a.n, cx, cy, r.multipl);
-    r.sc = a.d.sc[id];
-    r.vol = a.d.vol[id];
-    r.s0 = a.d.s0[id];
-    r.s1 = a.d.s1[id];
-    r.vx = a.d.vx[id];
-    r.vy = a.d.vy[id];
-    r.kill = a.d.kill[id];
+    const float4 p = __ldg(a.pack + 2 * (size_t)(key >> 2)), q = __ldg(a.pack + 2 * (size_t)(key >> 2) + 1);
+    r.multipl = corner_weight(fabsf(p.x), p.y, (int)(key & 3u));
+    r.kill = __float_as_int(p.x) < 0;
+    r.sc = p.z;
+    r.vol = p.w;
+    r.s0 = q.x;
+    r.s1 = q.y;
+    r.vx = q.z;
+    r.vy = q.w;
     return r;
 }
 
@@ -296,7 +374,9 @@ struct Texel {
     float terr[2], wat, mz, mw;
 };
 
-// what a record leaves for its droplet's sediment replay
+// A NaN that no arithmetic gives (that is 0x7fffffff), and every sediment stored comes from an add.
+constexpr uint32_t UNSET = 0x7fc0dead;
+// what a record leaves for its droplet's sediment replay (mask bit 1: dirt, bit 0: rock)
 struct RecOut {
     float s_dirt, s_rock;
     uint32_t mask;
@@ -428,9 +508,7 @@ __device__ __forceinline__ bool apply_prepared(const Pre& p, Texel& T, RecOut& o
 }
 
 __device__ __forceinline__ void store_rec(const ApplyArgs& a, uint32_t key, const RecOut& o) {
-    a.rec[2 * key + 0] = o.s_dirt;
-    a.rec[2 * key + 1] = o.s_rock;
-    a.rec_mask[key] = (uint8_t)o.mask;
+    a.rec[key] = make_float2(o.mask & 2u ? o.s_dirt : __uint_as_float(UNSET), o.mask & 1u ? o.s_rock : __uint_as_float(UNSET));
 }
 
 __device__ __forceinline__ Texel load_texel(const ApplyArgs& a, size_t t) {
@@ -444,46 +522,71 @@ __device__ __forceinline__ void store_texel(const ApplyArgs& a, size_t t, const 
     a.mw[t] = T.mw;
 }
 
-constexpr int SMALL = 8;  // records a texel's own thread sorts and applies
-constexpr int MID = 32;   // records a warp sorts in registers
-
-// each texel with at most SMALL records applies them in droplet-id order;
-// busier texels go to the mid (up to MID records) or big lists
-__global__ void k_papply(const ApplyArgs a) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int n = a.n;
-    if (x >= n || y >= n) return;
-    const size_t t = (size_t)y * n + x;
-    const uint32_t lo = a.offs[t], hi = a.offs[t + 1];
-    if (lo == hi) return;
-    const uint32_t k = hi - lo;
-    if (k > SMALL) {
-        const int big = k > (uint32_t)MID ? 1 : 0;
-        const uint32_t slot = atomicAdd(a.hot + big, 1u);
-        if (slot < a.hot_cap) a.hot[2 + big * a.hot_cap + slot] = (uint32_t)t;
-        return;
-    }
-    uint32_t kk[SMALL];
+// A texel with k <= S records, by one thread: sorting network on registers
+// (odd-even transposition, S rounds), then the records in droplet-id order
+// (each loaded when its turn comes: two or four loaded ahead cost registers, so
+// warps: 1193 and 1248 us for 8 steps against 1161).
+template <int S>
+__device__ __forceinline__ void apply_small(const ApplyArgs& a, size_t t) {
+    const uint32_t lo = a.offs[t], k = a.cnt[t];
+    uint32_t kk[S];
 #pragma unroll
-    for (int i = 0; i < SMALL; ++i) kk[i] = (uint32_t)i < k ? a.keys[lo + i] : 0xffffffffu;
-    // sorting network on registers (odd-even transposition, SMALL rounds)
+    for (int i = 0; i < S; ++i) kk[i] = (uint32_t)i < k ? a.keys[lo + i] : 0xffffffffu;
+    Texel T = load_texel(a, t);
 #pragma unroll
-    for (int r = 0; r < SMALL; ++r)
+    for (int r = 0; r < S; ++r)
 #pragma unroll
-        for (int i = r & 1; i + 1 < SMALL; i += 2) {
+        for (int i = r & 1; i + 1 < S; i += 2) {
             const uint32_t u = min(kk[i], kk[i + 1]), v = max(kk[i], kk[i + 1]);
             kk[i] = u;
             kk[i + 1] = v;
         }
-    Texel T = load_texel(a, t);
 #pragma unroll
-    for (int i = 0; i < SMALL; ++i)
+    for (int i = 0; i < S; ++i)
         if ((uint32_t)i < k) store_rec(a, kk[i], apply_record(a, load_rec(a, kk[i]), T));
     store_texel(a, t, T);
 }
 
-constexpr int HOT_WARPS = 4;     // warps per block of the mid / big kernels
-constexpr int HOT_KEYS = 1024;   // bucket size a warp sorts in shared memory
+constexpr int AP_WARPS = 4, AP_BLOCKS = 7;  // warps per block of k_papply, blocks per SM
+
+// Bitonic network over a warp's 32 * E keys, element lane * E + e in k[e]: the
+// smaller strides between a lane's registers, the others between lanes.
+template <int E>
+__device__ __forceinline__ void warp_sort(uint32_t (&k)[E], int lane) {
+#pragma unroll
+    for (int size = 2; size <= 32 * E; size <<= 1)
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            const bool lane_up = (lane & (size / E)) == 0;  // (size >= E: a lane's keys go one way)
+            if (stride >= E) {
+                const bool low = ((lane & (stride / E)) == 0) == lane_up;
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    const uint32_t other = __shfl_xor_sync(0xffffffffu, k[e], stride / E);
+                    k[e] = low ? min(k[e], other) : max(k[e], other);
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < E; ++e)
+                    if ((e & stride) == 0) {
+                        const bool up = size < E ? (e & size) == 0 : lane_up;
+                        const uint32_t u = min(k[e], k[e + stride]), v = max(k[e], k[e + stride]);
+                        k[e] = up ? u : v;
+                        k[e + stride] = up ? v : u;
+                    }
+            }
+        }
+}
+// len <= 32 * E keys of src, sorted into sk
+template <int E>
+__device__ __forceinline__ void sort_chunk(const uint32_t* src, uint32_t len, uint32_t* sk, int lane) {
+    uint32_t k[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) k[e] = 32u * e + lane < len ? src[32 * e + lane] : 0xffffffffu;
+    warp_sort<E>(k, lane);
+#pragma unroll
+    for (int e = 0; e < E; ++e) sk[lane * E + e] = k[e];
+}
 
 // A warp applies up to 32 records of one texel in order.  With no layer
 // exhausted each of the texel's five values is a plain running sum of amounts
@@ -572,125 +675,123 @@ __device__ __forceinline__ void warp_apply(const ApplyArgs& a, WarpSums& ws, int
     acc = lane == 0 ? T.terr[1] : lane == 1 ? T.terr[0] : lane == 2 ? T.wat : lane == 3 ? T.mz : T.mw;
 }
 
-// one warp per mid texel (SMALL < records <= 32): lane i holds record i; a
-// bitonic network over the lanes sorts the keys by droplet id, each lane loads
-// its record
-__global__ void __launch_bounds__(32 * HOT_WARPS) k_papply_mid(const ApplyArgs a) {
-    const unsigned FULL = 0xffffffffu;
-    __shared__ __align__(16) WarpSums sums[HOT_WARPS];
-    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-    const uint32_t nmid = min(a.hot[0], a.hot_cap);
-    for (uint32_t h = blockIdx.x * HOT_WARPS + wl; h < nmid; h += gridDim.x * HOT_WARPS) {
-        const size_t t = a.hot[2 + h];
-        const uint32_t lo = a.offs[t], k = a.offs[t + 1] - lo;
-        uint32_t key = (uint32_t)lane < k ? a.keys[lo + lane] : 0xffffffffu;
-#pragma unroll
-        for (int size = 2; size <= 32; size <<= 1)
-#pragma unroll
-            for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                const uint32_t other = __shfl_xor_sync(FULL, key, stride);
-                const bool up = (lane & size) == 0, lower = (lane & stride) == 0;
-                key = (lower == up) ? min(key, other) : max(key, other);
-            }
-        Rec mine{};
-        if ((uint32_t)lane < k) mine = load_rec(a, key);
-        float* f = texel_sum(a, min(lane, SUMS - 1)) + t;
-        float acc = *f;
-        warp_apply(a, sums[wl], lane, k, mine, acc);
-        if (lane < SUMS) *f = acc;
-    }
+// a texel of SMALL + 1 to MID records, by a warp: lane i holds record i; a
+// bitonic network over the lanes sorts the keys by droplet id
+__device__ __forceinline__ void apply_mid(const ApplyArgs& a, WarpSums& ws, int lane, size_t t) {
+    const uint32_t lo = a.offs[t], k = a.cnt[t];
+    uint32_t key[1] = {(uint32_t)lane < k ? a.keys[lo + lane] : 0xffffffffu};
+    float* f = texel_sum(a, min(lane, SUMS - 1)) + t;
+    float acc = *f;
+    warp_sort<1>(key, lane);
+    Rec mine{};
+    if ((uint32_t)lane < k) mine = load_rec(a, key[0]);
+    warp_apply(a, ws, lane, k, mine, acc);
+    if (lane < SUMS) *f = acc;
 }
 
-// one warp per big texel (more than 32 records): sort the bucket by droplet
-// id (bitonic network in shared memory, chunks of HOT_KEYS merged by rank),
-// then apply it 32 records at a time
-__global__ void __launch_bounds__(32 * HOT_WARPS) k_papply_big(const ApplyArgs a) {
-    __shared__ uint32_t sk[HOT_WARPS][HOT_KEYS];
-    __shared__ __align__(16) WarpSums sums[HOT_WARPS];
-    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-    const uint32_t nbig = min(a.hot[1], a.hot_cap);
-    for (uint32_t h = blockIdx.x * HOT_WARPS + wl; h < nbig; h += gridDim.x * HOT_WARPS) {
-        const size_t t = a.hot[2 + a.hot_cap + h];
-        const uint32_t lo = a.offs[t], hi = a.offs[t + 1], k = hi - lo;
-        // sort chunks of up to HOT_KEYS records in shared memory into
-        // `sorted`; a bucket of several chunks is then merged into `keys` by
-        // each record's rank (its place in its chunk plus, per other chunk,
-        // the records below it found by binary search)
-        for (uint32_t c0 = 0; c0 < k; c0 += HOT_KEYS) {
-            const uint32_t len = min((uint32_t)HOT_KEYS, k - c0);
-            uint32_t P = 32;
-            while (P < len) P <<= 1;
-            for (uint32_t i = lane; i < P; i += 32) sk[wl][i] = i < len ? a.keys[lo + c0 + i] : 0xffffffffu;
-            __syncwarp();
-            for (uint32_t size = 2; size <= P; size <<= 1)
-                for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-                    for (uint32_t q = lane; q < P / 2; q += 32) {
-                        const uint32_t pos = 2 * stride * (q / stride) + (q % stride), par = pos + stride;
-                        const bool up = (pos & size) == 0;
-                        const uint32_t u = sk[wl][pos], v = sk[wl][par];
-                        if ((u > v) == up) {
-                            sk[wl][pos] = v;
-                            sk[wl][par] = u;
-                        }
-                    }
-                    __syncwarp();
-                }
-            for (uint32_t i = lane; i < len; i += 32) a.sorted[lo + c0 + i] = sk[wl][i];
-            __syncwarp();
-        }
-        const bool merged = k > (uint32_t)HOT_KEYS;
-        if (merged) {
-            for (uint32_t i = lane; i < k; i += 32) {
-                const uint32_t key = a.sorted[lo + i];
-                const uint32_t own = i / HOT_KEYS * HOT_KEYS;
-                uint32_t rank = i - own;
-                for (uint32_t c0 = 0; c0 < k; c0 += HOT_KEYS) {
-                    if (c0 == own) continue;
-                    uint32_t l = 0, h = min((uint32_t)HOT_KEYS, k - c0);  // records of chunk c0 below key
-                    const uint32_t* ch = a.sorted + lo + c0;
-                    while (l < h) {
-                        const uint32_t m = (l + h) >> 1;
-                        if (ch[m] < key) l = m + 1; else h = m;
-                    }
-                    rank += l;
-                }
-                a.keys[lo + rank] = key;
-            }
-        }
-        const uint32_t* order = merged ? a.keys : a.sorted;
+// a texel of more than MID records, by a warp: sort the bucket by droplet id,
+// chunks of HOT_KEYS merged by rank, then apply it 32 records at a time
+__device__ __noinline__ void apply_big(const ApplyArgs& a, WarpSums& ws, uint32_t* sk, int lane, size_t t) {
+    const uint32_t lo = a.offs[t], k = a.cnt[t], hi = lo + k;
+    float* f = texel_sum(a, min(lane, SUMS - 1)) + t;
+    float acc = *f;
+    for (uint32_t c0 = 0; c0 < k; c0 += HOT_KEYS) {
+        const uint32_t len = min((uint32_t)HOT_KEYS, k - c0);
+        const uint32_t* src = a.keys + lo + c0;
+        if (len <= 64) sort_chunk<2>(src, len, sk, lane);
+        else if (len <= 128) sort_chunk<4>(src, len, sk, lane);
+        else if (len <= 256) sort_chunk<8>(src, len, sk, lane);
+        else sort_chunk<16>(src, len, sk, lane);
         __syncwarp();
-        float* f = texel_sum(a, min(lane, SUMS - 1)) + t;
-        float acc = *f;
-        for (uint32_t base = lo; base < hi; base += 32) {
-            const uint32_t m = min(32u, hi - base);
-            Rec mine{};
-            if ((uint32_t)lane < m) mine = load_rec(a, order[base + lane]);
-            warp_apply(a, sums[wl], lane, m, mine, acc);
+        if (k > HOT_KEYS) {
+            for (uint32_t i = lane; i < len; i += 32) a.sorted[lo + c0 + i] = sk[i];
+            __syncwarp();
         }
-        if (lane < SUMS) *f = acc;
+    }
+    if (k > HOT_KEYS) {
+        // merge into `keys` by each record's rank: its place in its chunk plus,
+        // per other chunk, the records below it (binary search)
+        for (uint32_t i = lane; i < k; i += 32) {
+            const uint32_t key = a.sorted[lo + i];
+            const uint32_t own = i / HOT_KEYS * HOT_KEYS;
+            uint32_t rank = i - own;
+            for (uint32_t c0 = 0; c0 < k; c0 += HOT_KEYS) {
+                if (c0 == own) continue;
+                uint32_t l = 0, h = min((uint32_t)HOT_KEYS, k - c0);  // records of chunk c0 below key
+                const uint32_t* ch = a.sorted + lo + c0;
+                while (l < h) {
+                    const uint32_t m = (l + h) >> 1;
+                    if (ch[m] < key) l = m + 1; else h = m;
+                }
+                rank += l;
+            }
+            a.keys[lo + rank] = key;
+        }
+        __syncwarp();
+    }
+    const uint32_t* order = k > HOT_KEYS ? a.keys + lo : sk;
+    for (uint32_t base = lo; base < hi; base += 32) {
+        const uint32_t m = min(32u, hi - base);
+        Rec mine{};
+        if ((uint32_t)lane < m) mine = load_rec(a, order[base - lo + lane]);
+        warp_apply(a, ws, lane, m, mine, acc);
+    }
+    __syncwarp();  // sk is read: the warp's next texel may sort
+    if (lane < SUMS) *f = acc;
+}
+
+// Every texel with records: warps take the next item until none is left, the
+// busiest texels first (they are the longest), then those of a warp each, then
+// 32 at a time those of a thread each.  Bound by latency: the records' droplets
+// lie anywhere, two loads of 16 bytes each (nine of 4 bytes before).  262144
+// droplets on 1024² after 100 steps (buckets up to 317 records): one launch over
+// all texels and one each over the busier two kinds took 33, 40 and 130 us, this
+// 60.  8 steps, three worlds in turn / alone: 7 blocks per SM 1143 / 1289 us, 6
+// 1161 / 1292, 8 1135 / 1328.
+__global__ void __launch_bounds__(32 * AP_WARPS, AP_BLOCKS) k_papply(const ApplyArgs a) {
+    __shared__ __align__(16) WarpSums sums[AP_WARPS];
+    __shared__ uint32_t sk[AP_WARPS][HOT_KEYS];
+    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+    uint32_t num[LISTS];
+#pragma unroll
+    for (int l = 0; l < LISTS; ++l) num[l] = min(a.tl.counters[l], a.tl.cap[l]);
+    const uint32_t small = (num[L_SMALL] + 31) / 32, half = (num[L_HALF] + 31) / 32;
+    for (;;) {
+        uint32_t i = lane == 0 ? atomicAdd(a.tl.counters + C_NEXT, 1u) : 0u;
+        i = __shfl_sync(0xffffffffu, i, 0);
+        if (i < num[L_BIG]) {
+            apply_big(a, sums[wl], sk[wl], lane, a.tl.list[L_BIG][i]);
+        } else if ((i -= num[L_BIG]) < num[L_MID]) {
+            apply_mid(a, sums[wl], lane, a.tl.list[L_MID][i]);
+        } else if ((i -= num[L_MID]) < small) {
+            if (32 * i + lane < num[L_SMALL]) apply_small<SMALL>(a, a.tl.list[L_SMALL][32 * i + lane]);
+        } else if ((i -= small) < half) {
+            if (32 * i + lane < num[L_HALF]) apply_small<HALF>(a, a.tl.list[L_HALF][32 * i + lane]);
+        } else {
+            return;
+        }
+        __syncwarp();
     }
 }
 
 // each droplet replays its corners 0..3 for its sediment
-__global__ void k_pfinal(const hg_erosion_settings es, Drops d, int n, const float* __restrict__ rec,
-                         const uint8_t* __restrict__ rec_mask) {
+__global__ void k_pfinal(const hg_erosion_settings es, Drops d, const float2* __restrict__ rec) {
     const int id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= d.count || d.iters[id] == 0) return;
     const float old_sed[2] = {d.s0[id], d.s1[id]};
     float sed[2] = {old_sed[0], old_sed[1]};
     const bool kill = d.kill[id] != 0;
+    const float ofx = fract_(d.px[id] * 1.0f), ofy = fract_(d.py[id] * 1.0f);
+#pragma unroll
     for (int k = 0; k < 4; ++k) {
-        int cx, cy;
-        float multipl;
-        corner(d.px[id], d.py[id], k, n, cx, cy, multipl);
-        const uint32_t key = (uint32_t)id * 4u + (uint32_t)k;
         if (kill) {
+            const float multipl = corner_weight(ofx, ofy, k);
             sed[1] -= old_sed[1] * multipl;
             sed[0] -= old_sed[0] * multipl;
         } else {
-            const uint32_t m = rec_mask[key];
-            if (m & 2u) sed[1] = rec[2 * key + 0];
-            if (m & 1u) sed[0] = rec[2 * key + 1];
+            const float2 r = rec[(size_t)id * 4 + k];
+            if (__float_as_uint(r.x) != UNSET) sed[1] = r.x;
+            if (__float_as_uint(r.y) != UNSET) sed[0] = r.y;
         }
         const float conv = sed[0] * es.Kconv * es.d_t;
         sed[1] += conv;
@@ -749,9 +850,12 @@ __global__ void k_psmooth(const SmoothArgs a) {
 
 }  // namespace
 
-size_t particle_scan_blocks(size_t cells) { return (cells + SCAN_T * SCAN_E - 1) / (SCAN_T * SCAN_E); }
-size_t particle_hot_capacity(size_t cells, int count) {
-    return std::min(cells, (size_t)4 * (size_t)count / (SMALL + 1) + 1);
+size_t particle_counters() { return COUNTERS; }
+int particle_lists() { return LISTS; }
+size_t particle_list_capacity(int list, size_t cells, int count) {
+    static_assert(LISTS == 4, "one capacity per list");
+    const size_t least[LISTS] = {MID + 1, SMALL + 1, HALF + 1, 1};  // records of its texels
+    return std::min(cells, (size_t)4 * (size_t)count / least[list] + 1);
 }
 
 void launch_particle_step(const StepConsts& c, const hg_erosion_settings& es, const ParticleBufs& pb,
@@ -760,24 +864,22 @@ void launch_particle_step(const StepConsts& c, const hg_erosion_settings& es, co
     const size_t cells = (size_t)n * n;
     const int pgrid = (pb.d.count + PB - 1) / PB;
     MoveArgs ma{c, es, pb.d, pw.rock, pw.dirt, pw.water, pw.mom[0], pw.mom[1], step1, (uint32_t)seed,
-                (uint32_t)(seed >> 32), should_rain ? 1 : 0};
+                (uint32_t)(seed >> 32), should_rain ? 1 : 0, pb.cnt, pb.rank, pb.pack};
+    TexelLists tl;
+    tl.counters = pb.cnt + cells;
+    for (int l = 0; l < LISTS; ++l) {
+        tl.list[l] = pb.list[l];
+        tl.cap[l] = (uint32_t)particle_list_capacity(l, cells, pb.d.count);
+    }
+    cudaMemsetAsync(pb.cnt, 0, (cells + COUNTERS) * sizeof(uint32_t), st);
     k_pmove<<<pgrid, PB, 0, st>>>(ma);
-    cudaMemsetAsync(pb.cnt, 0, cells * sizeof(uint32_t), st);
-    k_pcount<<<pgrid, PB, 0, st>>>(pb.d, n, pb.cnt);
-    const size_t nb = particle_scan_blocks(cells);
-    k_scan_blocks<<<(unsigned)nb, SCAN_T, 0, st>>>(pb.cnt, pb.offs, cells, pb.block_sums);
-    k_scan_sums<<<1, SCAN_T, 0, st>>>(pb.block_sums, (int)nb, pb.offs + cells);
-    k_scan_add<<<(unsigned)((cells + 255) / 256), 256, 0, st>>>(pb.offs, pb.cursor, cells, pb.block_sums);
-    k_pscatter<<<pgrid, PB, 0, st>>>(pb.d, n, pb.cursor, pb.keys);
-    ApplyArgs aa{es, pb.d, n, pb.offs, pb.keys, pb.sorted, pb.hot, pb.hot_cap, pw.rock, pw.dirt, pw.water,
-                 pw.mom[2], pw.mom[3], pb.rec, pb.rec_mask};
-    cudaMemsetAsync(pb.hot, 0, 2 * sizeof(uint32_t), st);
-    dim3 g((n + BX - 1) / BX, (n + BY - 1) / BY);
-    k_papply<<<g, dim3(BX, BY), 0, st>>>(aa);
-    k_papply_mid<<<152 * 12, 32 * HOT_WARPS, 0, st>>>(aa);
-    k_papply_big<<<152 * 8, 32 * HOT_WARPS, 0, st>>>(aa);
-    k_pfinal<<<pgrid, PB, 0, st>>>(es, pb.d, n, pb.rec, pb.rec_mask);
-    count_launch(10);
+    k_palloc<<<(unsigned)((cells + AL_T * AL_E - 1) / (AL_T * AL_E)), AL_T, 0, st>>>(pb.cnt, pb.offs, cells, tl);
+    k_pscatter<<<pgrid, PB, 0, st>>>(pb.d, n, pb.offs, pb.rank, pb.keys);
+    ApplyArgs aa{es, pb.pack, pb.cnt, pb.offs, pb.keys, pb.sorted, tl, pw.rock, pw.dirt, pw.water,
+                 pw.mom[2], pw.mom[3], pb.rec};
+    k_papply<<<152 * AP_BLOCKS, 32 * AP_WARPS, 0, st>>>(aa);
+    k_pfinal<<<pgrid, PB, 0, st>>>(es, pb.d, pb.rec);
+    count_launch(5);
 }
 
 void launch_particle_smooth(const StepConsts& c, float count, const PWorld& in, const PWorld& out, cudaStream_t st) {

@@ -1253,16 +1253,15 @@ int hg_particles_init(hg_world* w, int count) {
     for (float** f : fs) *f = (float*)take(cnt * sizeof(float));
     d.iters = (uint32_t*)take(cnt * sizeof(uint32_t));
     d.kill = (int32_t*)take(cnt * sizeof(int32_t));
-    P->b.cnt = (uint32_t*)take(cl * sizeof(uint32_t));
-    P->b.offs = (uint32_t*)take((cl + 1) * sizeof(uint32_t));
-    P->b.cursor = (uint32_t*)take(cl * sizeof(uint32_t));
-    P->b.block_sums = (uint32_t*)take(particle_scan_blocks(cl) * sizeof(uint32_t));
+    P->b.cnt = (uint32_t*)take((cl + particle_counters()) * sizeof(uint32_t));
+    P->b.offs = (uint32_t*)take(cl * sizeof(uint32_t));
     P->b.keys = (uint32_t*)take(4 * cnt * sizeof(uint32_t));
     P->b.sorted = (uint32_t*)take(4 * cnt * sizeof(uint32_t));
-    P->b.hot_cap = (uint32_t)particle_hot_capacity(cl, count);
-    P->b.hot = (uint32_t*)take((2 + 2 * (size_t)P->b.hot_cap) * sizeof(uint32_t));
-    P->b.rec = (float*)take(8 * cnt * sizeof(float));
-    P->b.rec_mask = (uint8_t*)take(4 * cnt);
+    for (int l = 0; l < particle_lists(); ++l)
+        P->b.list[l] = (uint32_t*)take(particle_list_capacity(l, cl, count) * sizeof(uint32_t));
+    P->b.rank = (uint4*)take(cnt * sizeof(uint4));
+    P->b.pack = (float4*)take(2 * cnt * sizeof(float4));
+    P->b.rec = (float2*)take(4 * cnt * sizeof(float2));
     for (int k = 0; k < 2; ++k)
         for (int c = 0; c < 4; ++c) P->mom[k][c] = (float*)take(cl * sizeof(float));
     if (e != cudaSuccess) {
@@ -1389,8 +1388,7 @@ int hg_world_poison_scratch(hg_world* w) {
         // momentum map's alternate is not scratch: border texels keep it
         // from two steps back, as the reference's ping-pong does
         const Particles& P = *w->parts;
-        HG_CUDA(cudaMemsetAsync(P.b.rec, 0xFF, 8 * (size_t)P.count * sizeof(float), w->stream));
-        HG_CUDA(cudaMemsetAsync(P.b.rec_mask, 0xFF, 4 * (size_t)P.count, w->stream));
+        HG_CUDA(cudaMemsetAsync(P.b.rec, 0xFF, 4 * (size_t)P.count * sizeof(float2), w->stream));
     }
     return HG_OK;
 }

@@ -127,3 +127,21 @@ def test_particles_checkpoint_resume_is_bitwise(tmp_path):
     assert np.array_equal(ka, kb)
     for f in ("rock", "dirt", "water", "momentum_x", "momentum_y"):
         assert np.array_equal(a.download(f), b.download(f)), f
+
+
+@pytest.mark.parametrize("n,count", [(16, 40), (16, 300), (16, 900), (16, 2500), (24, 9000), (16, 40000), (40, 6000)])
+@pytest.mark.parametrize("dirt", [0.0, 2.0])
+def test_particles_at_every_bucket_size(n, count, dirt):
+    """Buckets from a record to thousands per texel (a thread's networks of 4
+    and 8, a warp's of 32, up to 512 and merged chunks), with dirt and without,
+    where every dissolving record meets an exhausted layer."""
+    s = H.settings_particles()
+    w, ow, os_, oo = make(n, count, s, seed=n)
+    if dirt == 0.0:
+        z = np.zeros((n, n), np.float32)
+        w.upload("dirt", z)
+        ow.set("dirt", z)
+    for k in range(5):
+        w.step(1, H.MODE_PARTICLES)
+        ow.particle_step(os_, oo, 1)
+    check(w, ow, f"n={n} count={count} dirt={dirt}")
