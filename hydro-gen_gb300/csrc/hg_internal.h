@@ -27,6 +27,17 @@ void launch_rain(const StepConsts& c, const RainStep& r, float* water, cudaStrea
 void launch_flux(const StepConsts& c, const float* rock, const float* water, const float* fl, const float* fr,
                  const float* ft, const float* fb, float* water_o, float* fl_o, float* fr_o, float* ft_o,
                  float* fb_o, float* u, float* v, float* vz, cudaStream_t st);
+// launch_flux and launch_erosion of the state `in` in one kernel, after `rain`
+// on every cell (-0: none) and with the evaporation; sed in place
+void launch_flux_erosion(const StepConsts& c, float rain, const float* const in[S_COUNT], float* const out[S_COUNT], float* sed,
+                         float* u, float* v, float* vz, cudaStream_t st);
+// sediment transport without the evaporation
+void launch_gather(const StepConsts& c, const float* u, const float* v, const float* sed, float* sed_o,
+                   cudaStream_t st);
+// sediment transport without the evaporation and both talus passes of a whole
+// map's layer 0
+void launch_gather_talus(const StepConsts& c, const float* rock, float* rock_o, const float* u, const float* v,
+                  const float* sed, float* sed_o, cudaStream_t st);
 void launch_erosion(const StepConsts& c, const float* u, const float* v, const float* vz, const float* rock,
                     float* rock_o, float* sed_inout, cudaStream_t st);
 void launch_sediment(const StepConsts& c, const float* u, const float* v, const float* sed, float* sed_o,

@@ -2,11 +2,14 @@
 // structure-of-arrays fields, two adjacent cells per thread (rows of 64 cells
 // per warp, 8-byte accesses, both cells in f32x2 instructions; the maps' side
 // is even), Jacobi ping-pong between passes as in the reference
-// (src/erosion.cpp:158-200).  Bound by issue slots (flux, talus outflows: 83
-// and 86 % busy with one cell per thread and built-in divisions) or by the
-// launch at sides around 1000; a step with talus at 1000²: 52 us with one
-// cell per thread, 35 with two.
+// (src/erosion.cpp:158-200).  A step of whole maps joins passes that need
+// nothing of their neighbours' results: uniform rain, flux, erosion and
+// evaporation in one kernel, both talus passes in another.  Bound by issue slots
+// and, at sides around 1000, by launches.  A step with Bernoulli rain and talus
+// at 1000²: 52 us with one cell per thread and built-in divisions (flux and
+// talus outflows 83 and 86 % busy), 35 with two, 30 with the passes joined.
 #include "hg_internal.h"
+#include "hg_tile.cuh"
 
 namespace hg {
 
@@ -39,38 +42,52 @@ __device__ __forceinline__ bool pair_at(const StepConsts& c, int& x, int& y, siz
     i = at(c.n, x, y);
     return x < c.n && y >= c.row_lo && y < c.row_hi;
 }
-__device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
-__device__ __forceinline__ void st2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
 
-// glsl/hydro_flux.glsl:77-166
-__global__ void k_flux(StepConsts c, const float* __restrict__ rock, const float* __restrict__ water,
-                       const float* __restrict__ fl, const float* __restrict__ fr,
-                       const float* __restrict__ ft, const float* __restrict__ fb,
-                       float* __restrict__ water_o, float* __restrict__ fl_o, float* __restrict__ fr_o,
-                       float* __restrict__ ft_o, float* __restrict__ fb_o, float* __restrict__ u_o,
-                       float* __restrict__ v_o, float* __restrict__ vz_o) {
+// glsl/hydro_flux.glsl:77-166; ERODE: and glsl/hydro_erosion.glsl:37-92, which
+// needs nothing of the neighbours' flux, and the step's evaporation
+struct FluxArgs {
+    const float *rock, *water, *fl, *fr, *ft, *fb;
+    float *water_o, *fl_o, *fr_o, *ft_o, *fb_o, *u, *v, *vz;
+    float *rock_o, *sed;  // ERODE: eroded rock; sediment, in place
+    float rain;           // falls on every cell before the step (-0: none, which leaves a depth's bits)
+};
+template <bool ERODE>
+__global__ void k_flux(StepConsts c, const FluxArgs a) {
     int x, y;
     size_t i;
     if (!pair_at(c, x, y, i)) return;
     const int n = c.n;
     const bool hl = x > 0, hr = x + 2 < n, hb = y > 0, ht = y < n - 1;
-    const float2 d1 = ld2(water + i), w = add2(ld2(rock + i), d1);
-    const float2 f_l = ld2(fl + i), f_r = ld2(fr + i);
-    const float2 wl = make_float2(hl ? rock[i - 1] + water[i - 1] : FAR_HEIGHT, w.x);
-    const float2 wr = make_float2(w.y, hr ? rock[i + 2] + water[i + 2] : FAR_HEIGHT);
-    const float2 wt = ht ? add2(ld2(rock + i + n), ld2(water + i + n)) : pf(FAR_HEIGHT);
-    const float2 wb = hb ? add2(ld2(rock + i - n), ld2(water + i - n)) : pf(FAR_HEIGHT);
-    const float2 inl = make_float2(hl ? fr[i - 1] : 0.0f, f_r.x), inr = make_float2(f_l.y, hr ? fl[i + 2] : 0.0f);
-    const Flux2 o = cell_flux2(c, x, y, true, w, d1, f_l, f_r, ld2(ft + i), ld2(fb + i), wl, wr, wt, wb, inl, inr,
-                               ht ? ld2(fb + i + n) : pf(0.0f), hb ? ld2(ft + i - n) : pf(0.0f));
-    st2(fl_o + i, o.fl);
-    st2(fr_o + i, o.fr);
-    st2(ft_o + i, o.ft);
-    st2(fb_o + i, o.fb);
-    st2(water_o + i, o.d2);
-    st2(u_o + i, o.u);
-    st2(v_o + i, o.v);
-    st2(vz_o + i, o.vz);
+    const float2 rain = pf(a.rain), d1 = add2(ldg2(a.water + i), rain), f_l = ldg2(a.fl + i), f_r = ldg2(a.fr + i);
+    // heights of the neighbours: 0 outside, as the erosion's normal has it
+    float2 b = ldg2(a.rock + i);
+    const float2 bl = make_float2(hl ? __ldg(a.rock + i - 1) : 0.0f, b.x);
+    const float2 br = make_float2(b.y, hr ? __ldg(a.rock + i + 2) : 0.0f);
+    const float2 bt = ht ? ldg2(a.rock + i + n) : pf(0.0f), bb = hb ? ldg2(a.rock + i - n) : pf(0.0f);
+    const float2 w = add2(b, d1);
+    const float2 wl = make_float2(hl ? bl.x + (__ldg(a.water + i - 1) + a.rain) : FAR_HEIGHT, w.x);
+    const float2 wr = make_float2(w.y, hr ? br.y + (__ldg(a.water + i + 2) + a.rain) : FAR_HEIGHT);
+    const float2 wt = ht ? add2(bt, add2(ldg2(a.water + i + n), rain)) : pf(FAR_HEIGHT);
+    const float2 wb = hb ? add2(bb, add2(ldg2(a.water + i - n), rain)) : pf(FAR_HEIGHT);
+    const float2 inl = make_float2(hl ? __ldg(a.fr + i - 1) : 0.0f, f_r.x);
+    const float2 inr = make_float2(f_l.y, hr ? __ldg(a.fl + i + 2) : 0.0f);
+    const Flux2 o = cell_flux2(c, x, y, true, w, d1, f_l, f_r, ldg2(a.ft + i), ldg2(a.fb + i), wl, wr, wt, wb, inl, inr,
+                               ht ? ldg2(a.fb + i + n) : pf(0.0f), hb ? ldg2(a.ft + i - n) : pf(0.0f));
+    st2(a.fl_o + i, o.fl);
+    st2(a.fr_o + i, o.fr);
+    st2(a.ft_o + i, o.ft);
+    st2(a.fb_o + i, o.fb);
+    st2(a.water_o + i, ERODE ? mul2(o.d2, pf(c.evap)) : o.d2);
+    st2(a.u + i, o.u);
+    st2(a.v + i, o.v);
+    st2(a.vz + i, o.vz);
+    if (ERODE) {
+        float2 s = ld2(a.sed + i);
+        const float2 Kls0 = c.ks_field ? mul2(pf(c.dt), ldg2(c.ks_field + i)) : pf(c.Kls0);
+        cell_erosion_pair(c, Kls0, o.vz, o.len, b, s, br, bl, bb, bt);
+        st2(a.rock_o + i, b);
+        st2(a.sed + i, s);
+    }
 }
 
 // glsl/hydro_erosion.glsl:37-92
@@ -91,6 +108,7 @@ __global__ void k_erosion(StepConsts c, const float* __restrict__ u, const float
 }
 
 // glsl/sediment_transport.glsl:66-93
+template <bool EVAPORATE>
 __global__ void k_sediment(StepConsts c, const float* __restrict__ u, const float* __restrict__ v,
                            const float* __restrict__ sed, float* __restrict__ sed_o,
                            float* __restrict__ water) {
@@ -98,7 +116,7 @@ __global__ void k_sediment(StepConsts c, const float* __restrict__ u, const floa
     size_t i;
     if (!pair_at(c, x, y, i)) return;
     st2(sed_o + i, gather_sediment(c, sed, x, y, ld2(u + i), ld2(v + i)));
-    st2(water + i, mul2(ld2(water + i), pf(c.evap)));
+    if (EVAPORATE) st2(water + i, mul2(ld2(water + i), pf(c.evap)));
 }
 
 // glsl/thermal_erosion.glsl:28-115, layer 0
@@ -150,6 +168,28 @@ __global__ void k_thermal_in(StepConsts c, const float* __restrict__ rock, const
     rock_o[i] = cell_thermal_apply(rock[i], own, in);
 }
 
+// Both talus passes of layer 0 in one launch (see talus_rows; two launches with
+// the outflows in memory between them took 15 us at 1000²), SED: with the
+// sediment gather.  Steps with talus, gather in the same launch / in its own, in
+// three worlds in turn: 136² 9.9 / 11.6 us, 520² 10.6 / 12.6, 1000² 32.6 / 29.6,
+// 1496² 71 / 60; ROWS_MAX_N is the line here too.
+template <bool SED>
+__global__ void __launch_bounds__(32 * R_WARPS, SED ? 2 : 3) k_talus(StepConsts c, const float* __restrict__ rock,
+                                                                   float* __restrict__ rock_o, const float* __restrict__ u,
+                                                                   const float* __restrict__ v, const float* __restrict__ sed,
+                                                                   float* __restrict__ sed_o) {
+    Taps<1> taps;
+    talus_rows(
+        c, rock, rock_o, blockIdx.x, blockIdx.y * R_ROWS,
+        [&](int x, int y, size_t i) {
+            const float* const se[1] = {sed};
+            if (SED) load_taps<1>(c, se, x, y, ldg2(u + i), ldg2(v + i), taps);
+        },
+        [&](int, int, size_t i) {
+            if (SED) st2(sed_o + i, mix_taps(taps, 0));
+        });
+}
+
 // glsl/smoothing.glsl:22-103, rock channel (see cell_smooth)
 __global__ void k_smooth(StepConsts c, const float* __restrict__ rock, float* __restrict__ rock_o) {
     int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -178,8 +218,34 @@ void launch_rain(const StepConsts& c, const RainStep& r, float* water, cudaStrea
 void launch_flux(const StepConsts& c, const float* rock, const float* water, const float* fl, const float* fr,
                  const float* ft, const float* fb, float* water_o, float* fl_o, float* fr_o, float* ft_o,
                  float* fb_o, float* u, float* v, float* vz, cudaStream_t st) {
-    k_flux<<<pairs_for(c.n), dim3(BX, BY), 0, st>>>(c, rock, water, fl, fr, ft, fb, water_o, fl_o, fr_o, ft_o,
-                                                   fb_o, u, v, vz);
+    const FluxArgs a{rock, water, fl, fr, ft, fb, water_o, fl_o, fr_o, ft_o, fb_o, u, v, vz, nullptr, nullptr,
+                     -0.0f};
+    k_flux<false><<<pairs_for(c.n), dim3(BX, BY), 0, st>>>(c, a);
+    count_launch();
+}
+
+void launch_flux_erosion(const StepConsts& c, float rain, const float* const in[S_COUNT], float* const out[S_COUNT],
+                         float* sed, float* u, float* v, float* vz, cudaStream_t st) {
+    const FluxArgs a{in[S_ROCK],  in[S_WATER], in[S_FL],  in[S_FR],  in[S_FT],  in[S_FB], out[S_WATER], out[S_FL],
+                     out[S_FR],   out[S_FT],   out[S_FB], u,         v,         vz,       out[S_ROCK],  sed,
+                     rain};
+    k_flux<true><<<pairs_for(c.n), dim3(BX, BY), 0, st>>>(c, a);
+    count_launch();
+}
+
+void launch_gather(const StepConsts& c, const float* u, const float* v, const float* sed, float* sed_o,
+                   cudaStream_t st) {
+    k_sediment<false><<<pairs_for(c.n), dim3(BX, BY), 0, st>>>(c, u, v, sed, sed_o, nullptr);
+    count_launch();
+}
+
+void launch_gather_talus(const StepConsts& c, const float* rock, float* rock_o, const float* u, const float* v,
+                  const float* sed, float* sed_o, cudaStream_t st) {
+    const dim3 grid(strips(c.n), c.n / R_ROWS);
+    const bool together = c.n <= ROWS_MAX_N;
+    if (!together) launch_gather(c, u, v, sed, sed_o, st);
+    if (together) k_talus<true><<<grid, 32 * R_WARPS, 0, st>>>(c, rock, rock_o, u, v, sed, sed_o);
+    else k_talus<false><<<grid, 32 * R_WARPS, 0, st>>>(c, rock, rock_o, nullptr, nullptr, nullptr, nullptr);
     count_launch();
 }
 
@@ -191,7 +257,7 @@ void launch_erosion(const StepConsts& c, const float* u, const float* v, const f
 
 void launch_sediment(const StepConsts& c, const float* u, const float* v, const float* sed, float* sed_o,
                      float* water_inout, cudaStream_t st) {
-    k_sediment<<<pairs_for(c.n), dim3(BX, BY), 0, st>>>(c, u, v, sed, sed_o, water_inout);
+    k_sediment<true><<<pairs_for(c.n), dim3(BX, BY), 0, st>>>(c, u, v, sed, sed_o, water_inout);
     count_launch();
 }
 

@@ -1623,21 +1623,27 @@ int hg_step(hg_world* w, int nsteps, int mode) {
         }
         if (nsteps > 0) w->dev_step_valid = false;
     } else if (mode == HG_MODE_PLAIN) {
+        const bool whole = !rows_restricted(w);
         for (int k = 0; k < nsteps; ++k) {
-            rain_pass(w, c, w->step + 1, w->cur[S_ROCK], nullptr, w->cur[S_WATER], st);
-            launch_flux(c, w->cur[S_ROCK], w->cur[S_WATER], w->cur[S_FL], w->cur[S_FR], w->cur[S_FT],
-                        w->cur[S_FB], w->alt[S_WATER], w->alt[S_FL], w->alt[S_FR], w->alt[S_FT], w->alt[S_FB],
-                        w->u, w->v, w->vz, st);
+            const RainStep r = make_rain(w, w->step + 1);
+            // uniform rain falls in the flux kernel (a slab's border rows come rained on)
+            const bool uniform = whole && r.active && !r.bernoulli && w->opt.rain_mode != HG_RAIN_REFERENCE;
+            if (!uniform) rain_pass(w, c, w->step + 1, w->cur[S_ROCK], nullptr, w->cur[S_WATER], st);
+            launch_flux_erosion(c, uniform ? r.amount : -0.0f, w->cur, w->alt, w->cur[S_SED], w->u, w->v, w->vz, st);
             swap(S_WATER); swap(S_FL); swap(S_FR); swap(S_FT); swap(S_FB);
-            launch_erosion(c, w->u, w->v, w->vz, w->cur[S_ROCK], w->alt[S_ROCK], w->cur[S_SED], st);
             swap(S_ROCK);
-            launch_sediment(c, w->u, w->v, w->cur[S_SED], w->alt[S_SED], w->cur[S_WATER], st);
-            swap(S_SED);
-            if (c.thermal) {
-                launch_thermal_out(c, w->cur[S_ROCK], w->tc, w->td, st);
-                launch_thermal_in(c, w->cur[S_ROCK], w->tc, w->td, w->alt[S_ROCK], st);
+            if (c.thermal && whole) {
+                launch_gather_talus(c, w->cur[S_ROCK], w->alt[S_ROCK], w->u, w->v, w->cur[S_SED], w->alt[S_SED], st);
                 swap(S_ROCK);
+            } else {
+                launch_gather(c, w->u, w->v, w->cur[S_SED], w->alt[S_SED], st);
+                if (c.thermal) {  // a slab's border rows need outflows of rows beyond it
+                    launch_thermal_out(c, w->cur[S_ROCK], w->tc, w->td, st);
+                    launch_thermal_in(c, w->cur[S_ROCK], w->tc, w->td, w->alt[S_ROCK], st);
+                    swap(S_ROCK);
+                }
             }
+            swap(S_SED);
             // the dirt layer's talus pass moves nothing (its H is min(0, .) == 0);
             // smoothing changes rock when Kspeed[1] != 0
             if (c.smooth_m != 0.0f) {
