@@ -229,46 +229,11 @@ struct Layer1Args {
     Talus1 t1;
     int thermal1;              // layer-1 talus pass on (Kspeed[1] != 0)
     float *rock_o, *dirt_o;
-    // particle mode: smoothing's particle branch (glsl/smoothing.glsl:76-95),
-    // per cell: momentum fold and water decay
-    float count;               // droplets
-    const float* water;
-    float* water_o;
-    const float* mom[4];
-    float* mom_o[4];
+    ParticleCells pc;          // particle mode
 };
 constexpr int L_RH = TH + 6, L_BOX = RW * L_RH, L_RC = ((L_BOX + 31) / 32) * 32;  // 3-row halo
 constexpr int P_W = TW + 4, P_H = TH + 4, P_C = P_W * P_H;                        // outflows of the tile plus 2
 constexpr size_t LAYER1_SMEM = (2 * L_RC + 8 * P_C) * sizeof(float) + 16;
-
-// smoothing's particle branch at the cells (x, y), (x + 1, y): border texels
-// copy their water and leave the momentum map's write buffer as it was
-__device__ __forceinline__ void particle_cells(const Layer1Args& a, size_t gi, int x, int y) {
-    const int n = a.c.n;
-    const bool row = y == 0 || y == n - 1;
-    const bool b0 = row || x == 0, b1 = row || x + 2 == n;
-    const float2 wat = ldg2(a.water + gi);
-    float2 w = mul2(wat, pf(gclamp(1.0f - 8e-8f * a.count, 0.0f, 1.0f)));
-    w = make_float2(w.x < 1e-6f ? 0.0f : w.x, w.y < 1e-6f ? 0.0f : w.y);
-    st2(a.water_o + gi, make_float2(b0 ? wat.x : w.x, b1 ? wat.y : w.y));
-    const float2 keep = pf(gclamp(1.0f - 1e-12f * a.count, 0.0f, 1.0f)), take = pf(1e-12f * a.count);
-    float2 mx = add2(mul2(ldg2(a.mom[0] + gi), keep), mul2(take, ldg2(a.mom[2] + gi)));
-    float2 my = add2(mul2(ldg2(a.mom[1] + gi), keep), mul2(take, ldg2(a.mom[3] + gi)));
-    const float2 len = sqrt_newton2(add2(mul2(mx, mx), mul2(my, my)));  // (below 2^-100 it stays far below 1e-12)
-    const bool zx = len.x < 1e-12f, zy = len.y < 1e-12f;
-    mx = make_float2(zx ? 0.0f : mx.x, zy ? 0.0f : mx.y);
-    my = make_float2(zx ? 0.0f : my.x, zy ? 0.0f : my.y);
-    const float2 z = pf(0.0f), v[4] = {mx, my, z, z};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        if (!b0 && !b1) {
-            st2(a.mom_o[k] + gi, v[k]);
-        } else {
-            if (!b0) a.mom_o[k][gi] = v[k].x;
-            if (!b1) a.mom_o[k][gi + 1] = v[k].y;
-        }
-    }
-}
 
 // A 64 x 16 tile of rock and dirt staged with a 3-row, 4-column halo; pairs of
 // cells throughout: outflows of the tile plus two rings into shared memory,
@@ -403,7 +368,7 @@ __global__ void __launch_bounds__(NT, 4) k2f_layer1(const __grid_constant__ Laye
         }
         st2(a.rock_o + gi, nr);
         st2(a.dirt_o + gi, ng);
-        if (PARTICLE) particle_cells(a, gi, x, y);
+        if (PARTICLE) particle_cells(a.pc, n, gi, x, y);
     }
 }
 
@@ -499,13 +464,7 @@ int launch_particle_thermal_smooth(const StepConsts& c, const Talus1& t1, float 
     la.thermal1 = c.Kspeed1 != 0.0f ? 1 : 0;
     la.rock_o = out.rock;
     la.dirt_o = out.dirt;
-    la.count = count;
-    la.water = in.water;
-    la.water_o = out.water;
-    for (int k = 0; k < 4; ++k) {
-        la.mom[k] = in.mom[k];
-        la.mom_o[k] = out.mom[k];
-    }
+    la.pc = particle_cells_of(count, in, out);
     return launch_layer1(la, rock_l0, in.dirt, true, tma, err, st);
 }
 

@@ -34,6 +34,8 @@ void launch_flux_erosion(const StepConsts& c, float rain, const float* const in[
 // sediment transport without the evaporation
 void launch_gather(const StepConsts& c, const float* u, const float* v, const float* sed, float* sed_o,
                    cudaStream_t st);
+// both talus passes of a whole map's layer 0
+void launch_talus(const StepConsts& c, const float* rock, float* rock_o, cudaStream_t st);
 // sediment transport without the evaporation and both talus passes of a whole
 // map's layer 0
 void launch_gather_talus(const StepConsts& c, const float* rock, float* rock_o, const float* u, const float* v,
@@ -57,16 +59,16 @@ void launch_ref_rain(const hg_rain_settings& rs, const hg_map_settings& map, flo
                      const float* dirt, float* water, cudaStream_t st);
 
 // ---- two-layer per-pass kernels (hg_layers.cu) -----------------------------------
-void launch_flux2(const StepConsts& c, const float* rock, const float* dirt, const float* water, const float* fl,
-                  const float* fr, const float* ft, const float* fb, float* water_o, float* fl_o, float* fr_o,
-                  float* ft_o, float* fb_o, float* u, float* v, float* vz, cudaStream_t st);
-void launch_erosion2(const StepConsts& c, const float* u, const float* v, const float* vz, const float* rock,
-                     const float* dirt, float* rock_o, float* dirt_o, float* s0, float* s1, cudaStream_t st);
-void launch_sediment2(const StepConsts& c, const float* u, const float* v, const float* s0, const float* s1,
-                      float* s0_o, float* s1_o, float* water, cudaStream_t st);
-// thermal_erosion for layer 1 (dirt); thermal_transport reuses launch_thermal_in on the dirt field
-void launch_thermal_out1(const StepConsts& c, const float* rock, const float* dirt, float4* tc, float4* td,
-                         cudaStream_t st);
+// flux, erosion of both layers and evaporation of the state (in, dirt); sediments in place
+void launch_flux_erosion2(const StepConsts& c, const float* const in[S_COUNT], const float* dirt,
+                          float* const out[S_COUNT], float* dirt_o, float* s0, float* s1, float* u, float* v, float* vz,
+                          cudaStream_t st);
+// sediment transport of both channels without the evaporation
+void launch_gather2(const StepConsts& c, const float* u, const float* v, const float* s0, const float* s1, float* s0_o,
+                    float* s1_o, cudaStream_t st);
+// both talus passes of layer 1 (dirt)
+void launch_talus1(const StepConsts& c, const Talus1& t1, const float* rock, const float* dirt, float* dirt_o,
+                   cudaStream_t st);
 void launch_smooth2(const StepConsts& c, const float* rock, const float* dirt, float* rock_o, float* dirt_o,
                     cudaStream_t st);
 

@@ -3,166 +3,171 @@
 // sediment in sedimap.r and dirt sediment in sedimap.g
 // (glsl/heightmap.glsl:138-146, src/rendering.cpp:214); the total height the
 // flux pass compares is (rock + dirt) + water, the order in which every pass
-// before it leaves the total channel.  Rain reuses k_rain; thermal layer 0
-// reuses k_thermal_out / k_thermal_in (its drops involve rock only).
+// before it leaves the total channel.  Rain reuses k_rain.  As in the one-layer
+// step (hg_plain.cu) a thread has a pair of cells and passes that need nothing
+// of their neighbours' results are joined: flux, erosion and evaporation in one
+// kernel, each layer's two talus passes in another.  Bound by issue slots and
+// launches: 8 steps with the reference's defaults at 1000² took 697 us in eight
+// launches a step of one cell per thread with built-in divisions, 381 so.
 #include "hg_internal.h"
+#include "hg_tile.cuh"
 
 namespace hg {
 
 namespace {
 
 constexpr int BX = 32, BY = 8;
-__device__ __forceinline__ size_t at(int n, int x, int y) { return (size_t)y * n + x; }
-__device__ __forceinline__ bool inside(int n, int x, int y) { return x >= 0 && x < n && y >= 0 && y < n; }
 
-// glsl/hydro_flux.glsl:77-166 with the two-layer total
-__global__ void k2_flux(StepConsts c, const float* __restrict__ rock, const float* __restrict__ dirt,
-                        const float* __restrict__ water, const float* __restrict__ fl, const float* __restrict__ fr,
-                        const float* __restrict__ ft, const float* __restrict__ fb, float* __restrict__ water_o,
-                        float* __restrict__ fl_o, float* __restrict__ fr_o, float* __restrict__ ft_o,
-                        float* __restrict__ fb_o, float* __restrict__ u_o, float* __restrict__ v_o,
-                        float* __restrict__ vz_o) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int n = c.n;
-    if (x >= n || y >= n) return;
-    size_t i = at(n, x, y);
-    auto total = [&](int xx, int yy) -> float {
-        if (!inside(n, xx, yy)) return FAR_HEIGHT;
-        size_t j = at(n, xx, yy);
-        return rock[j] + dirt[j] + water[j];
-    };
-    float d1 = water[i];
-    float inl = x > 0 ? fr[i - 1] : 0.0f;
-    float inr = x < n - 1 ? fl[i + 1] : 0.0f;
-    float int_ = y < n - 1 ? fb[i + n] : 0.0f;
-    float inb = y > 0 ? ft[i - n] : 0.0f;
-    FluxOut o = cell_flux(c, x, y, total(x, y), d1, fl[i], fr[i], ft[i], fb[i], total(x - 1, y), total(x + 1, y),
-                          total(x, y + 1), total(x, y - 1), inl, inr, int_, inb);
-    fl_o[i] = o.fl; fr_o[i] = o.fr; ft_o[i] = o.ft; fb_o[i] = o.fb;
-    water_o[i] = o.d2;
-    u_o[i] = o.u; v_o[i] = o.v; vz_o[i] = o.vz;
+// the thread's pair of cells (x, y), (x + 1, y); false past the map
+__device__ __forceinline__ bool pair_at(int n, int& x, int& y, size_t& i) {
+    x = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    y = blockIdx.y * blockDim.y + threadIdx.y;
+    i = (size_t)y * n + x;
+    return x < n && y < n;
 }
 
-// glsl/hydro_erosion.glsl:23-92, both layers
-__global__ void k2_erosion(StepConsts c, const float* __restrict__ u, const float* __restrict__ v,
-                           const float* __restrict__ vz, const float* __restrict__ rock,
-                           const float* __restrict__ dirt, float* __restrict__ rock_o, float* __restrict__ dirt_o,
-                           float* __restrict__ s0, float* __restrict__ s1) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y * blockDim.y + threadIdx.y;
+// glsl/hydro_flux.glsl:77-166 with the two-layer total, glsl/hydro_erosion.glsl:23-92
+// on both layers and the step's evaporation
+struct Flux2Args {
+    const float *rock, *dirt, *water, *fl, *fr, *ft, *fb;
+    float *water_o, *fl_o, *fr_o, *ft_o, *fb_o, *u, *v, *vz, *rock_o, *dirt_o;
+    float *s0, *s1;  // in place
+};
+__global__ void k2_flux_erosion(StepConsts c, const Flux2Args a) {
+    int x, y;
+    size_t i;
     const int n = c.n;
-    if (x >= n || y >= n) return;
-    size_t i = at(n, x, y);
-    auto R = [&](int xx, int yy) { return inside(n, xx, yy) ? rock[at(n, xx, yy)] : 0.0f; };
-    auto D = [&](int xx, int yy) { return inside(n, xx, yy) ? dirt[at(n, xx, yy)] : 0.0f; };
-    float r = rock[i], g = dirt[i], a = s0[i], b = s1[i];
-    float Kls0 = c.ks_field ? c.dt * c.ks_field[i] : c.Kls0;
-    cell_erosion2(c, Kls0, u[i], v[i], vz[i], r, g, a, b, R(x + 1, y), D(x + 1, y), R(x - 1, y), D(x - 1, y),
-                  R(x, y + 1), D(x, y + 1), R(x, y - 1), D(x, y - 1));
-    rock_o[i] = r;
-    dirt_o[i] = g;
-    s0[i] = a;
-    s1[i] = b;
+    if (!pair_at(n, x, y, i)) return;
+    const bool hl = x > 0, hr = x + 2 < n, hb = y > 0, ht = y < n - 1;
+    const float2 z = pf(0.0f);
+    const float2 d1 = ldg2(a.water + i), f_l = ldg2(a.fl + i), f_r = ldg2(a.fr + i);
+    // heights of the neighbours: 0 outside, as the erosion's normal has them
+    auto row = [&](const float* f, float2& m, float2& l, float2& r, float2& t, float2& b) {
+        m = ldg2(f + i);
+        l = make_float2(hl ? __ldg(f + i - 1) : 0.0f, m.x);
+        r = make_float2(m.y, hr ? __ldg(f + i + 2) : 0.0f);
+        t = ht ? ldg2(f + i + n) : z;
+        b = hb ? ldg2(f + i - n) : z;
+    };
+    float2 r, rl, rr, rt, rb, g, gl, gr, gt, gb;
+    row(a.rock, r, rl, rr, rt, rb);
+    row(a.dirt, g, gl, gr, gt, gb);
+    const float2 w = add2(add2(r, g), d1);
+    const float2 wl = make_float2(hl ? (rl.x + gl.x) + __ldg(a.water + i - 1) : FAR_HEIGHT, w.x);
+    const float2 wr = make_float2(w.y, hr ? (rr.y + gr.y) + __ldg(a.water + i + 2) : FAR_HEIGHT);
+    const float2 wt = ht ? add2(add2(rt, gt), ldg2(a.water + i + n)) : pf(FAR_HEIGHT);
+    const float2 wb = hb ? add2(add2(rb, gb), ldg2(a.water + i - n)) : pf(FAR_HEIGHT);
+    const float2 inl = make_float2(hl ? __ldg(a.fr + i - 1) : 0.0f, f_r.x);
+    const float2 inr = make_float2(f_l.y, hr ? __ldg(a.fl + i + 2) : 0.0f);
+    const Flux2 o = cell_flux2(c, x, y, true, w, d1, f_l, f_r, ldg2(a.ft + i), ldg2(a.fb + i), wl, wr, wt, wb, inl, inr,
+                               ht ? ldg2(a.fb + i + n) : z, hb ? ldg2(a.ft + i - n) : z);
+    st2(a.fl_o + i, o.fl);
+    st2(a.fr_o + i, o.fr);
+    st2(a.ft_o + i, o.ft);
+    st2(a.fb_o + i, o.fb);
+    st2(a.water_o + i, mul2(o.d2, pf(c.evap)));
+    st2(a.u + i, o.u);
+    st2(a.v + i, o.v);
+    st2(a.vz + i, o.vz);
+    float2 s0 = ld2(a.s0 + i), s1 = ld2(a.s1 + i);
+    const float2 Kls0 = c.ks_field ? mul2(pf(c.dt), ldg2(c.ks_field + i)) : pf(c.Kls0);
+    cell_erosion2_pair(c, Kls0, o.vz, o.len, r, g, s0, s1, rr, gr, rl, gl, rt, gt, rb, gb);
+    st2(a.rock_o + i, r);
+    st2(a.dirt_o + i, g);
+    st2(a.s0 + i, s0);
+    st2(a.s1 + i, s1);
 }
 
 // glsl/sediment_transport.glsl:66-93, both sediment channels
-__global__ void k2_sediment(StepConsts c, const float* __restrict__ u, const float* __restrict__ v,
-                            const float* __restrict__ s0, const float* __restrict__ s1, float* __restrict__ s0_o,
-                            float* __restrict__ s1_o, float* __restrict__ water) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int n = c.n;
-    if (x >= n || y >= n) return;
-    size_t i = at(n, x, y);
-    float px, py;
-    backtrace(c, x, y, u[i], v[i], px, py);
-    int ix = (int)px, iy = (int)py;
-    auto tap = [&](const float* s, int xx, int yy) -> float { return inside(n, xx, yy) ? s[at(n, xx, yy)] : 0.0f; };
-    s0_o[i] = bilinear_mix(px, py, tap(s0, ix, iy), tap(s0, ix + 1, iy), tap(s0, ix, iy + 1), tap(s0, ix + 1, iy + 1));
-    s1_o[i] = bilinear_mix(px, py, tap(s1, ix, iy), tap(s1, ix + 1, iy), tap(s1, ix, iy + 1), tap(s1, ix + 1, iy + 1));
-    water[i] = water[i] * c.evap;
+__global__ void k2_gather(StepConsts c, const float* __restrict__ u, const float* __restrict__ v,
+                          const float* __restrict__ s0, const float* __restrict__ s1, float* __restrict__ s0_o,
+                          float* __restrict__ s1_o) {
+    int x, y;
+    size_t i;
+    if (!pair_at(c.n, x, y, i)) return;
+    float2 q0, q1;
+    gather_sediment2(c, s0, s1, x, y, ldg2(u + i), ldg2(v + i), q0, q1);
+    st2(s0_o + i, q0);
+    st2(s1_o + i, q1);
 }
 
-__constant__ int c2_ox[8] = {-1, 1, 0, 0, -1, 1, -1, 1};
-__constant__ int c2_oy[8] = {0, 0, 1, -1, 1, 1, -1, -1};
-
-// glsl/thermal_erosion.glsl:28-109, layer 1: drops summed over rock and
-// dirt ((0 + (r - nr)) + (g - ng)), H capped by the dirt height
-__global__ void k2_thermal_out1(StepConsts c, const float* __restrict__ rock, const float* __restrict__ dirt,
-                                float4* __restrict__ tc, float4* __restrict__ td) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int n = c.n;
-    if (x >= n || y >= n) return;
-    size_t i = at(n, x, y);
-    const float r = rock[i], g = dirt[i];
-    float dh[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        int xx = x + c2_ox[k], yy = y + c2_oy[k];
-        bool in = inside(n, xx, yy);
-        float nr = in ? rock[at(n, xx, yy)] : FAR_HEIGHT;
-        float ng = in ? dirt[at(n, xx, yy)] : FAR_HEIGHT;
-        dh[k] = (0.0f + (r - nr)) + (g - ng);
-    }
-    ThermalOut t = cell_thermal_dh(c.dt, c.Kalpha1, c.Kspeed1, g, dh);
-    float o[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) o[k] = (t.mask >> k & 1u) ? t.S * dh[k] / t.bk : 0.0f;
-    tc[i] = make_float4(o[0], o[1], o[2], o[3]);
-    td[i] = make_float4(o[4], o[5], o[6], o[7]);
+// Both talus passes of layer 1 in one launch (glsl/thermal_erosion.glsl:28-109,
+// glsl/thermal_transport.glsl:31-65): drops summed over rock and dirt, H capped
+// by the dirt height, dirt moves
+__global__ void __launch_bounds__(32 * R_WARPS, 2) k2_talus1(StepConsts c, Talus1 t1, const float* __restrict__ rock,
+                                                             const float* __restrict__ dirt, float* __restrict__ dirt_o) {
+    talus_rows<true>(
+        c, TalusRates{c.Kalpha1, c.Kspeed1, t1.x_cross, t1.b_diag, t1.fast_div}, rock, dirt, dirt_o, blockIdx.x,
+        blockIdx.y * R_ROWS, [](int, int, size_t) {}, [](int, int, size_t) {});
 }
 
-// glsl/smoothing.glsl:22-103, both channels
+// glsl/smoothing.glsl:22-103, both channels; PARTICLE: with the particle branch
+// (:76-95); border texels are copied (:27-33)
+template <bool PARTICLE>
 __global__ void k2_smooth(StepConsts c, const float* __restrict__ rock, const float* __restrict__ dirt,
-                          float* __restrict__ rock_o, float* __restrict__ dirt_o) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y * blockDim.y + threadIdx.y;
+                          float* __restrict__ rock_o, float* __restrict__ dirt_o, const ParticleCells pc) {
+    int x, y;
+    size_t i;
     const int n = c.n;
-    if (x >= n || y >= n) return;
-    size_t i = at(n, x, y);
-    float r = rock[i], g = dirt[i];
-    if (!(x == 0 || y == 0 || x == n - 1 || y == n - 1))  // border texels are copied (:27-33)
-        cell_smooth2(c.smooth_m, r, g, rock[i - 1], dirt[i - 1], rock[i + 1], dirt[i + 1], rock[i + n], dirt[i + n],
-                     rock[i - n], dirt[i - n]);
-    rock_o[i] = r;
-    dirt_o[i] = g;
+    if (!pair_at(n, x, y, i)) return;
+    const float2 r0 = ldg2(rock + i), g0 = ldg2(dirt + i);
+    float2 r = r0, g = g0;
+    if (y > 0 && y < n - 1) {
+        const bool hl = x > 0, hr = x + 2 < n;
+        cell_smooth2_pair(c.smooth_m, r, g, make_float2(hl ? __ldg(rock + i - 1) : 0.0f, r0.x),
+                          make_float2(hl ? __ldg(dirt + i - 1) : 0.0f, g0.x),
+                          make_float2(r0.y, hr ? __ldg(rock + i + 2) : 0.0f),
+                          make_float2(g0.y, hr ? __ldg(dirt + i + 2) : 0.0f), ldg2(rock + i + n), ldg2(dirt + i + n),
+                          ldg2(rock + i - n), ldg2(dirt + i - n));
+        if (!hl) {
+            r.x = r0.x;
+            g.x = g0.x;
+        }
+        if (!hr) {
+            r.y = r0.y;
+            g.y = g0.y;
+        }
+    }
+    st2(rock_o + i, r);
+    st2(dirt_o + i, g);
+    if (PARTICLE) particle_cells(pc, n, i, x, y);
 }
 
-dim3 grid_for(int n) { return dim3((n + BX - 1) / BX, (n + BY - 1) / BY); }
+dim3 pairs_for(int n) { return dim3((n / 2 + BX - 1) / BX, (n + BY - 1) / BY); }
 
 }  // namespace
 
-void launch_flux2(const StepConsts& c, const float* rock, const float* dirt, const float* water, const float* fl,
-                  const float* fr, const float* ft, const float* fb, float* water_o, float* fl_o, float* fr_o,
-                  float* ft_o, float* fb_o, float* u, float* v, float* vz, cudaStream_t st) {
-    k2_flux<<<grid_for(c.n), dim3(BX, BY), 0, st>>>(c, rock, dirt, water, fl, fr, ft, fb, water_o, fl_o, fr_o, ft_o,
-                                                     fb_o, u, v, vz);
+void launch_flux_erosion2(const StepConsts& c, const float* const in[S_COUNT], const float* dirt,
+                          float* const out[S_COUNT], float* dirt_o, float* s0, float* s1, float* u, float* v, float* vz,
+                          cudaStream_t st) {
+    const Flux2Args a{in[S_ROCK], dirt,      in[S_WATER], in[S_FL],  in[S_FR], in[S_FT], in[S_FB],    out[S_WATER], out[S_FL],
+                      out[S_FR],  out[S_FT], out[S_FB],   u,         v,        vz,       out[S_ROCK], dirt_o,       s0,
+                      s1};
+    k2_flux_erosion<<<pairs_for(c.n), dim3(BX, BY), 0, st>>>(c, a);
     count_launch();
 }
 
-void launch_erosion2(const StepConsts& c, const float* u, const float* v, const float* vz, const float* rock,
-                     const float* dirt, float* rock_o, float* dirt_o, float* s0, float* s1, cudaStream_t st) {
-    k2_erosion<<<grid_for(c.n), dim3(BX, BY), 0, st>>>(c, u, v, vz, rock, dirt, rock_o, dirt_o, s0, s1);
+void launch_gather2(const StepConsts& c, const float* u, const float* v, const float* s0, const float* s1, float* s0_o,
+                    float* s1_o, cudaStream_t st) {
+    k2_gather<<<pairs_for(c.n), dim3(BX, BY), 0, st>>>(c, u, v, s0, s1, s0_o, s1_o);
     count_launch();
 }
 
-void launch_sediment2(const StepConsts& c, const float* u, const float* v, const float* s0, const float* s1,
-                      float* s0_o, float* s1_o, float* water, cudaStream_t st) {
-    k2_sediment<<<grid_for(c.n), dim3(BX, BY), 0, st>>>(c, u, v, s0, s1, s0_o, s1_o, water);
-    count_launch();
-}
-
-void launch_thermal_out1(const StepConsts& c, const float* rock, const float* dirt, float4* tc, float4* td,
-                         cudaStream_t st) {
-    k2_thermal_out1<<<grid_for(c.n), dim3(BX, BY), 0, st>>>(c, rock, dirt, tc, td);
+void launch_talus1(const StepConsts& c, const Talus1& t1, const float* rock, const float* dirt, float* dirt_o,
+                   cudaStream_t st) {
+    k2_talus1<<<dim3(strips(c.n), c.n / R_ROWS), 32 * R_WARPS, 0, st>>>(c, t1, rock, dirt, dirt_o);
     count_launch();
 }
 
 void launch_smooth2(const StepConsts& c, const float* rock, const float* dirt, float* rock_o, float* dirt_o,
                     cudaStream_t st) {
-    k2_smooth<<<grid_for(c.n), dim3(BX, BY), 0, st>>>(c, rock, dirt, rock_o, dirt_o);
+    k2_smooth<false><<<pairs_for(c.n), dim3(BX, BY), 0, st>>>(c, rock, dirt, rock_o, dirt_o, ParticleCells{});
+    count_launch();
+}
+
+void launch_particle_smooth(const StepConsts& c, float count, const PWorld& in, const PWorld& out, cudaStream_t st) {
+    const ParticleCells pc = particle_cells_of(count, in, out);
+    k2_smooth<true><<<pairs_for(c.n), dim3(BX, BY), 0, st>>>(c, in.rock, in.dirt, out.rock, out.dirt, pc);
     count_launch();
 }
 

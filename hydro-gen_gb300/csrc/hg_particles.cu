@@ -33,7 +33,7 @@ namespace hg {
 
 namespace {
 
-constexpr int BX = 32, BY = 8, PB = 256;
+constexpr int PB = 256;
 
 __device__ __forceinline__ float fract_(float x) { return x - floorf(x); }
 __device__ __forceinline__ bool inb(int n, int x, int y) { return x >= 0 && x < n && y >= 0 && y < n; }
@@ -801,53 +801,6 @@ __global__ void k_pfinal(const hg_erosion_settings es, Drops d, const float2* __
     d.s1[id] = sed[1];
 }
 
-struct SmoothArgs {
-    float m;       // clamp(Kspeed[1] * d_t, 0, 1)
-    float count;   // droplets
-    int n;
-    const float* rock;
-    const float* dirt;
-    const float* water;
-    float* rock_o;
-    float* dirt_o;
-    float* water_o;
-    const float* mom[4];
-    float* mom_o[4];
-};
-
-// glsl/smoothing.glsl:22-103 with the particle branch (:76-95); border texels
-// copy their height and leave the momentum map's write buffer untouched
-__global__ void k_psmooth(const SmoothArgs a) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int n = a.n;
-    if (x >= n || y >= n) return;
-    const size_t i = (size_t)y * n + x;
-    float r = a.rock[i], g = a.dirt[i], wat = a.water[i];
-    if (x == 0 || y == 0 || x == n - 1 || y == n - 1) {
-        a.rock_o[i] = r;
-        a.dirt_o[i] = g;
-        a.water_o[i] = wat;
-        return;
-    }
-    cell_smooth2(a.m, r, g, a.rock[i - 1], a.dirt[i - 1], a.rock[i + 1], a.dirt[i + 1], a.rock[i + n], a.dirt[i + n],
-                 a.rock[i - n], a.dirt[i - n]);
-    float mx = a.mom[0][i], my = a.mom[1][i], mz = a.mom[2][i], mw = a.mom[3][i];
-    const float keep = gclamp(1.0f - 1e-12f * a.count, 0.0f, 1.0f);
-    mx *= keep;
-    my *= keep;
-    mx += 1e-12f * a.count * mz;
-    my += 1e-12f * a.count * mw;
-    mz = 0.0f;
-    mw = 0.0f;
-    wat *= gclamp(1.0f - 8e-8f * a.count, 0.0f, 1.0f);
-    if (wat < 1e-6f) wat = 0.0f;
-    if (sqrtf(mx * mx + my * my) < 1e-12f) { mx = 0.0f; my = 0.0f; }
-    a.mom_o[0][i] = mx; a.mom_o[1][i] = my; a.mom_o[2][i] = mz; a.mom_o[3][i] = mw;
-    a.rock_o[i] = r;
-    a.dirt_o[i] = g;
-    a.water_o[i] = wat;
-}
-
 }  // namespace
 
 size_t particle_counters() { return COUNTERS; }
@@ -880,22 +833,6 @@ void launch_particle_step(const StepConsts& c, const hg_erosion_settings& es, co
     k_papply<<<152 * AP_BLOCKS, 32 * AP_WARPS, 0, st>>>(aa);
     k_pfinal<<<pgrid, PB, 0, st>>>(es, pb.d, pb.rec);
     count_launch(5);
-}
-
-void launch_particle_smooth(const StepConsts& c, float count, const PWorld& in, const PWorld& out, cudaStream_t st) {
-    SmoothArgs sa;
-    sa.m = c.smooth_m;
-    sa.count = count;
-    sa.n = c.n;
-    sa.rock = in.rock; sa.dirt = in.dirt; sa.water = in.water;
-    sa.rock_o = out.rock; sa.dirt_o = out.dirt; sa.water_o = out.water;
-    for (int k = 0; k < 4; ++k) {
-        sa.mom[k] = in.mom[k];
-        sa.mom_o[k] = out.mom[k];
-    }
-    dim3 g((c.n + BX - 1) / BX, (c.n + BY - 1) / BY);
-    k_psmooth<<<g, dim3(BX, BY), 0, st>>>(sa);
-    count_launch();
 }
 
 }  // namespace hg

@@ -239,13 +239,20 @@ void launch_gather(const StepConsts& c, const float* u, const float* v, const fl
     count_launch();
 }
 
+void launch_talus(const StepConsts& c, const float* rock, float* rock_o, cudaStream_t st) {
+    k_talus<false><<<dim3(strips(c.n), c.n / R_ROWS), 32 * R_WARPS, 0, st>>>(c, rock, rock_o, nullptr, nullptr, nullptr,
+                                                                            nullptr);
+    count_launch();
+}
+
 void launch_gather_talus(const StepConsts& c, const float* rock, float* rock_o, const float* u, const float* v,
-                  const float* sed, float* sed_o, cudaStream_t st) {
-    const dim3 grid(strips(c.n), c.n / R_ROWS);
-    const bool together = c.n <= ROWS_MAX_N;
-    if (!together) launch_gather(c, u, v, sed, sed_o, st);
-    if (together) k_talus<true><<<grid, 32 * R_WARPS, 0, st>>>(c, rock, rock_o, u, v, sed, sed_o);
-    else k_talus<false><<<grid, 32 * R_WARPS, 0, st>>>(c, rock, rock_o, nullptr, nullptr, nullptr, nullptr);
+                         const float* sed, float* sed_o, cudaStream_t st) {
+    if (c.n > ROWS_MAX_N) {
+        launch_gather(c, u, v, sed, sed_o, st);
+        launch_talus(c, rock, rock_o, st);
+        return;
+    }
+    k_talus<true><<<dim3(strips(c.n), c.n / R_ROWS), 32 * R_WARPS, 0, st>>>(c, rock, rock_o, u, v, sed, sed_o);
     count_launch();
 }
 

@@ -2,6 +2,7 @@
 // and the talus pass with a row of a strip per warp.
 #pragma once
 #include "hg_device.cuh"
+#include "hg_internal.h"
 
 namespace hg {
 
@@ -61,10 +62,16 @@ __host__ __device__ constexpr int strips(int n) { return (n + SW - 1) / SW; }
 // the outflows, in lanes whose pair this block delivers: a sediment gather
 // leaves its taps in flight between them.
 constexpr int R_ROWS = 8, R_WARPS = R_ROWS + 2;
-template <class Begin, class End>
-__device__ __forceinline__ void talus_rows(const StepConsts1& c, const float* __restrict__ in_rock,
-                                           float* __restrict__ out_rock, int strip, int y0, Begin begin,
-                                           End end) {
+struct TalusRates {
+    float Kalpha, Kspeed, x_cross, b_diag;
+    int fast_div;
+};
+// DIRT: layer 1, whose drops are rock's plus dirt's and whose dirt moves;
+// else in_dirt is not read and rock moves
+template <bool DIRT, class Begin, class End>
+__device__ __forceinline__ void talus_rows(const StepConsts1& c, const TalusRates& t, const float* __restrict__ in_rock,
+                                           const float* __restrict__ in_dirt, float* __restrict__ out, int strip, int y0,
+                                           Begin begin, End end) {
     __shared__ float2 to_up[R_WARPS][3][32], to_down[R_WARPS][3][32];  // T, RT, LT / B, RB, LB at the receiving column
     const int n = c.n;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -72,22 +79,36 @@ __device__ __forceinline__ void talus_rows(const StepConsts1& c, const float* __
     const bool in = x >= 0 && x < n;
     const bool own = in && lane >= 1 && lane <= SW / 2 && warp >= 1 && warp <= R_ROWS;
     const size_t gi = (size_t)y * n + x;
-    if (!c.thermal) {
+    if (!DIRT && !c.thermal) {
         if (own) {
             begin(x, y, gi);
             end(x, y, gi);
         }
         return;
     }
-    auto rock = [&](int r) { return in && r >= 0 && r < n ? ldg2(in_rock + (size_t)r * n + x) : pf(FAR_HEIGHT); };
-    const float2 c0 = rock(y - 1), c1 = rock(y), c2 = rock(y + 1);
+    auto height = [&](const float* f, int r) {
+        return in && r >= 0 && r < n ? ldg2(f + (size_t)r * n + x) : pf(FAR_HEIGHT);
+    };
+    const float2 c0 = height(in_rock, y - 1), c1 = height(in_rock, y), c2 = height(in_rock, y + 1);
+    float2 g0, g1, g2;
+    if (DIRT) {
+        g0 = height(in_dirt, y - 1);
+        g1 = height(in_dirt, y);
+        g2 = height(in_dirt, y + 1);
+    }
     if (own) begin(x, y, gi);
     float2 o[8];
     if (y >= 0 && y < n) {
         const RockRow dn = rock_row(c0), md = rock_row(c1), up = rock_row(c2);
         float2 dm[8] = {sub2(md.c, md.l), sub2(md.c, md.r), sub2(md.c, up.c), sub2(md.c, dn.c),
                         sub2(md.c, up.l), sub2(md.c, up.r), sub2(md.c, dn.l), sub2(md.c, dn.r)};
-        cell_thermal_outflows_dh2(c.dt, c.Kalpha0, c.Kspeed0, c.talus_x_cross, c.talus_b_diag, c.fast_div, md.c, dm, o);
+        if (DIRT) {
+            const RockRow dg = rock_row(g0), mg = rock_row(g1), ug = rock_row(g2);
+            const float2 ng[8] = {mg.l, mg.r, ug.c, dg.c, ug.l, ug.r, dg.l, dg.r};
+#pragma unroll
+            for (int k = 0; k < 8; ++k) dm[k] = add2(dm[k], sub2(mg.c, ng[k]));
+        }
+        cell_thermal_outflows_dh2(c.dt, t.Kalpha, t.Kspeed, t.x_cross, t.b_diag, t.fast_div, DIRT ? g1 : md.c, dm, o);
     }
     if (!in || y < 0 || y >= n) {
 #pragma unroll
@@ -110,7 +131,13 @@ __device__ __forceinline__ void talus_rows(const StepConsts1& c, const float* __
     float2 inf = add2(add2(lr, to_down[warp + 1][0][lane]), to_up[warp - 1][0][lane]);
     inf = add2(add2(inf, to_down[warp + 1][1][lane]), to_down[warp + 1][2][lane]);
     inf = add2(add2(inf, to_up[warp - 1][1][lane]), to_up[warp - 1][2][lane]);
-    st2(out_rock + gi, add2(c1, add2(osum, inf)));
+    st2(out + gi, add2(DIRT ? g1 : c1, add2(osum, inf)));
+}
+template <class Begin, class End>
+__device__ __forceinline__ void talus_rows(const StepConsts1& c, const float* __restrict__ in_rock,
+                                           float* __restrict__ out_rock, int strip, int y0, Begin begin, End end) {
+    const TalusRates t{c.Kalpha0, c.Kspeed0, c.talus_x_cross, c.talus_b_diag, c.fast_div};
+    talus_rows<false>(c, t, in_rock, nullptr, out_rock, strip, y0, begin, end);
 }
 // Worlds up to this side run talus_rows: a one-layer step with talus takes, in
 // three worlds in turn / alone, 3.4 / 8.3 us at 256² (marching: 4.6 / 11.2),
@@ -118,5 +145,50 @@ __device__ __forceinline__ void talus_rows(const StepConsts1& c, const float* __
 // 1024² marching takes 19.8 / 29.1 against 22.8 / 26.1, from 1536² on less
 // both ways.
 constexpr int ROWS_MAX_N = 768;
+
+// smoothing's particle branch (glsl/smoothing.glsl:76-95), per cell: momentum
+// fold and water decay
+struct ParticleCells {
+    float count;  // droplets
+    const float* water;
+    float* water_o;
+    const float* mom[4];
+    float* mom_o[4];
+};
+inline ParticleCells particle_cells_of(float count, const PWorld& in, const PWorld& out) {
+    ParticleCells p{count, in.water, out.water, {}, {}};
+    for (int k = 0; k < 4; ++k) {
+        p.mom[k] = in.mom[k];
+        p.mom_o[k] = out.mom[k];
+    }
+    return p;
+}
+// smoothing's particle branch at the cells (x, y), (x + 1, y): border texels
+// copy their water and leave the momentum map's write buffer as it was
+__device__ __forceinline__ void particle_cells(const ParticleCells& a, int n, size_t gi, int x, int y) {
+    const bool row = y == 0 || y == n - 1;
+    const bool b0 = row || x == 0, b1 = row || x + 2 == n;
+    const float2 wat = ldg2(a.water + gi);
+    float2 w = mul2(wat, pf(gclamp(1.0f - 8e-8f * a.count, 0.0f, 1.0f)));
+    w = make_float2(w.x < 1e-6f ? 0.0f : w.x, w.y < 1e-6f ? 0.0f : w.y);
+    st2(a.water_o + gi, make_float2(b0 ? wat.x : w.x, b1 ? wat.y : w.y));
+    const float2 keep = pf(gclamp(1.0f - 1e-12f * a.count, 0.0f, 1.0f)), take = pf(1e-12f * a.count);
+    float2 mx = add2(mul2(ldg2(a.mom[0] + gi), keep), mul2(take, ldg2(a.mom[2] + gi)));
+    float2 my = add2(mul2(ldg2(a.mom[1] + gi), keep), mul2(take, ldg2(a.mom[3] + gi)));
+    const float2 len = sqrt_newton2(add2(mul2(mx, mx), mul2(my, my)));  // (below 2^-100 it stays far below 1e-12)
+    const bool zx = len.x < 1e-12f, zy = len.y < 1e-12f;
+    mx = make_float2(zx ? 0.0f : mx.x, zy ? 0.0f : mx.y);
+    my = make_float2(zx ? 0.0f : my.x, zy ? 0.0f : my.y);
+    const float2 z = pf(0.0f), v[4] = {mx, my, z, z};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (!b0 && !b1) {
+            st2(a.mom_o[k] + gi, v[k]);
+        } else {
+            if (!b0) a.mom_o[k][gi] = v[k].x;
+            if (!b1) a.mom_o[k][gi + 1] = v[k].y;
+        }
+    }
+}
 
 }  // namespace hg

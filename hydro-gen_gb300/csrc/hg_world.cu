@@ -1563,13 +1563,11 @@ int hg_step(hg_world* w, int nsteps, int mode) {
                 continue;
             }
             if (c.thermal) {
-                launch_thermal_out(c, w->cur[S_ROCK], w->tc, w->td, st);
-                launch_thermal_in(c, w->cur[S_ROCK], w->tc, w->td, w->alt[S_ROCK], st);
+                launch_talus(c, w->cur[S_ROCK], w->alt[S_ROCK], st);
                 swap(S_ROCK);
             }
             if (c.Kspeed1 != 0.0f) {
-                launch_thermal_out1(c, w->cur[S_ROCK], w->dirt[0], w->tc, w->td, st);
-                launch_thermal_in(c, w->dirt[0], w->tc, w->td, w->dirt[1], st);
+                launch_talus1(c, t1, w->cur[S_ROCK], w->dirt[0], w->dirt[1], st);
                 swap2(w->dirt);
             }
             PWorld in{w->cur[S_ROCK], w->dirt[0], w->cur[S_WATER], {P.mom[0][0], P.mom[0][1], P.mom[0][2], P.mom[0][3]}};
@@ -1589,29 +1587,24 @@ int hg_step(hg_world* w, int nsteps, int mode) {
         // the reference's two-layer step (src/erosion.cpp:158-200): thermal
         // and smoothing passes for layers whose slippage rate is 0 are
         // identities and are skipped
+        const Talus1 t1 = make_talus1(w);
         auto swap2 = [](float** f) { float* t = f[0]; f[0] = f[1]; f[1] = t; };
         for (int k = 0; k < nsteps; ++k) {
             rain_pass(w, c, w->step + 1, w->cur[S_ROCK], w->dirt[0], w->cur[S_WATER], st);
-            launch_flux2(c, w->cur[S_ROCK], w->dirt[0], w->cur[S_WATER], w->cur[S_FL], w->cur[S_FR], w->cur[S_FT],
-                         w->cur[S_FB], w->alt[S_WATER], w->alt[S_FL], w->alt[S_FR], w->alt[S_FT], w->alt[S_FB],
-                         w->u, w->v, w->vz, st);
+            launch_flux_erosion2(c, w->cur, w->dirt[0], w->alt, w->dirt[1], w->cur[S_SED], w->sdirt[0], w->u, w->v,
+                                 w->vz, st);
             swap(S_WATER); swap(S_FL); swap(S_FR); swap(S_FT); swap(S_FB);
-            launch_erosion2(c, w->u, w->v, w->vz, w->cur[S_ROCK], w->dirt[0], w->alt[S_ROCK], w->dirt[1],
-                            w->cur[S_SED], w->sdirt[0], st);
             swap(S_ROCK);
             swap2(w->dirt);
-            launch_sediment2(c, w->u, w->v, w->cur[S_SED], w->sdirt[0], w->alt[S_SED], w->sdirt[1], w->cur[S_WATER],
-                             st);
+            launch_gather2(c, w->u, w->v, w->cur[S_SED], w->sdirt[0], w->alt[S_SED], w->sdirt[1], st);
             swap(S_SED);
             swap2(w->sdirt);
             if (c.thermal) {  // layer 0: drops of rock only
-                launch_thermal_out(c, w->cur[S_ROCK], w->tc, w->td, st);
-                launch_thermal_in(c, w->cur[S_ROCK], w->tc, w->td, w->alt[S_ROCK], st);
+                launch_talus(c, w->cur[S_ROCK], w->alt[S_ROCK], st);
                 swap(S_ROCK);
             }
             if (c.Kspeed1 != 0.0f) {  // layer 1: drops of rock + dirt, dirt moves
-                launch_thermal_out1(c, w->cur[S_ROCK], w->dirt[0], w->tc, w->td, st);
-                launch_thermal_in(c, w->dirt[0], w->tc, w->td, w->dirt[1], st);
+                launch_talus1(c, t1, w->cur[S_ROCK], w->dirt[0], w->dirt[1], st);
                 swap2(w->dirt);
             }
             if (c.smooth_m != 0.0f) {

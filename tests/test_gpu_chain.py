@@ -95,3 +95,34 @@ def test_two_layer_chain_against_per_pass(n, thermal, dirt_talus):
         for f in H.STATE_FIELDS + ["dirt", "sediment_dirt"]:
             x, y = a.download(f), b.download(f)
             assert np.array_equal(x, y), f"{f} after {a.step_count}: {np.count_nonzero(x != y)} cells differ"
+
+
+@pytest.mark.parametrize("n", [72, 760, 776])
+@pytest.mark.parametrize("rain", ["uniform", "bernoulli"])
+def test_joined_passes_against_single_ones(n, rain):
+    """The per-pass step joins passes (the gather in the talus launch up to a
+    side of 768, in its own above): the bits of the passes run one by one."""
+    worlds = []
+    for _ in range(2):
+        w = H.World(n)
+        w.init_heightmap(H.noise(seed=5))
+        H.configure(w, "config2")
+        if rain == "uniform":
+            w.set_rain(H.rain_uniform(0.01, 2))
+            w.set_options(H.options(H.RAIN_UNIFORM))
+        else:
+            w.set_options(H.options(H.RAIN_BERNOULLI, p=0.05, seed=3))
+        worlds.append(w)
+    a, b = worlds
+    for k in range(4):
+        a.step(1, H.MODE_PLAIN)
+        b.run_pass("rain")
+        b.run_pass("flux")
+        b.run_pass("erosion")
+        b.run_pass("sediment")
+        b.run_pass("thermal_flux")
+        b.run_pass("thermal_transport")
+        b.step_count = k + 1
+    for f in ("rock", "water", "sediment", "flux_l", "flux_r", "flux_t", "flux_b", "vel_u", "vel_v", "vel_z"):
+        x, y = a.download(f), b.download(f)
+        assert np.array_equal(x, y), f"{f}: {np.count_nonzero(x != y)} cells differ"
