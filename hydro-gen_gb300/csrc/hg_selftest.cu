@@ -1,4 +1,5 @@
-// Device self-test of div_recip (hg_device.cuh) against IEEE division.
+// Device self-test of div_recip, rcp_newton and sqrt_newton (hg_device.cuh)
+// against IEEE division, reciprocal and square root.
 //
 // No counterpart in the reference: it checks an arithmetic shortcut of this
 // library.  Operands are drawn with Philox from the range div_recip's callers
