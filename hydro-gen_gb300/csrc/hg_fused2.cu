@@ -1,5 +1,5 @@
 // Fused step of a two-layer (rock + dirt) world, the reference's own model,
-// in three kernels per step (four in a chain's last) instead of the nine
+// in three kernels per step (up to four in a chain's last) instead of the nine
 // per-pass launches:
 //   k2f_hydro   [the previous step's sediment gather, both channels ->] rain ->
 //               hydro_flux -> hydro_erosion (both layers, Kconv) ->
@@ -8,7 +8,7 @@
 //   k2f_rock    the rock talus pass (thermal_erosion/thermal_transport, layer
 //               0), a row per warp
 //   k2f_gather  a chain's last step (or a single step): the sediment gather of
-//               both channels on its own
+//               both channels on its own (up to 768² within k2f_rock)
 //   k2f_layer1  the dirt talus pass (layer 1: cumulative rock + dirt drops,
 //               capped by the dirt height) and smoothing of both channels, on
 //               64 x 16 tiles staged with a 3-cell halo
@@ -208,8 +208,24 @@ struct RockArgs {
 // share the SMs with the other kernels of worlds stepped together.  (Warps
 // marching up strips take 32 us against 40 at 2048², but 8 steps of three
 // worlds in turn 1.28 ms against 1.18; of one world 1.34 against 1.38.)
-__global__ void __launch_bounds__(32 * R_WARPS, 3) k2f_rock(const __grid_constant__ RockArgs a) {
-    talus_rows(a.c, a.rock, a.rock_o, blockIdx.x, blockIdx.y * R_ROWS, [](int, int, size_t) {}, [](int, int, size_t) {});
+// SED: with the sediment gather of both channels (a chain's last step of a small
+// world, see ROWS_MAX_N: one launch less; at 2048² the pair takes 45 us together,
+// 40 and 12 apart, but a single step 215 us together, 200 apart)
+template <bool SED>
+__global__ void __launch_bounds__(32 * R_WARPS, SED ? 2 : 3) k2f_rock(const __grid_constant__ RockArgs a) {
+    Taps<2> taps;
+    talus_rows(
+        a.c, a.rock, a.rock_o, blockIdx.x, blockIdx.y * R_ROWS,
+        [&](int x, int y, size_t gi) {
+            const float* const se[2] = {a.s0, a.s1};
+            if (SED) load_taps<2>(a.c, se, x, y, ldg2(a.u + gi), ldg2(a.v + gi), taps);
+        },
+        [&](int, int, size_t gi) {
+            if (SED) {
+                st2(a.s0_o + gi, mix_taps(taps, 0));
+                st2(a.s1_o + gi, mix_taps(taps, 1));
+            }
+        });
 }
 
 // sediment_transport of both channels, for a chain's last step.
@@ -372,8 +388,10 @@ __global__ void __launch_bounds__(NT, 4) k2f_layer1(const __grid_constant__ Laye
     }
 }
 
-void launch_rock(const RockArgs& a, cudaStream_t st) {
-    k2f_rock<<<dim3(strips(a.c.n), a.c.n / R_ROWS), 32 * R_WARPS, 0, st>>>(a);
+void launch_rock(const RockArgs& a, bool gather, cudaStream_t st) {
+    const dim3 grid(strips(a.c.n), a.c.n / R_ROWS);
+    if (gather) k2f_rock<true><<<grid, 32 * R_WARPS, 0, st>>>(a);
+    else k2f_rock<false><<<grid, 32 * R_WARPS, 0, st>>>(a);
     count_launch();
 }
 
@@ -429,8 +447,9 @@ int launch_fused2_step(const StepConsts& c, const Talus1& t1, const RainStep& r,
         ra.s0_o = b.s0_o; ra.s1_o = b.s1_o;
         ra.rock = b.b_ero;
         ra.rock_o = rock_l0;
-        if (l0) launch_rock(ra, st);
-        if (pos.last) {
+        const bool together = l0 && pos.last && n <= ROWS_MAX_N;
+        if (l0) launch_rock(ra, together, st);
+        if (pos.last && !together) {
             k2f_gather<<<dim3(n / 64, n / (NT / 32)), NT, 0, st>>>(ra);
             count_launch();
         }
@@ -455,7 +474,7 @@ int launch_particle_thermal_smooth(const StepConsts& c, const Talus1& t1, float 
         ra.c = c;
         ra.rock = in.rock;
         ra.rock_o = rock_mid;
-        launch_rock(ra, st);
+        launch_rock(ra, false, st);
         rock_l0 = rock_mid;
     }
     Layer1Args la{};
