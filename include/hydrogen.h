@@ -164,8 +164,8 @@ typedef struct hg_noise_settings {
 #define HG_FIELD_MOMENTUM_Y 14    /* momentmap.y */
 #define HG_FIELD_COUNT 15
 
-#define HG_MODE_PLAIN 0           /* one kernel per GLSL pass */
-#define HG_MODE_FUSED 1           /* fused, tiled kernels: two per step (three in two-layer worlds) */
+#define HG_MODE_PLAIN 0           /* per-pass kernels (whole maps join passes that need no neighbour's result) */
+#define HG_MODE_FUSED 1           /* fused, tiled kernels: up to two per step (three or four in two-layer worlds) */
 #define HG_MODE_FUSED_PER_WORLD 2 /* batches only: each world's own fused launches */
 #define HG_MODE_PARTICLES 3       /* droplet erosion (hg_particles_init; two-layer worlds) */
 
@@ -407,8 +407,8 @@ int hg_world_tuning(const hg_world* w, int* tile_y, int* graph, double ms[4]);
 /* No counterpart in the reference (one map per process, src/main.cpp:222).
  * A batch steps several worlds of any sizes (multiples of 64 for the fused
  * mode) and settings together: in HG_MODE_FUSED one launch of each fused
- * kernel covers every tile of every world (a table of per-world descriptors),
- * optionally replayed from a captured CUDA graph; HG_MODE_FUSED_PER_WORLD and
+ * kernel covers every tile of every world (a table of per-world descriptors;
+ * large batches run as two such groups side by side), optionally replayed from a captured CUDA graph; HG_MODE_FUSED_PER_WORLD and
  * HG_MODE_PLAIN run each world's own launches (the one-launch-per-terrain
  * baseline).  The batch has its own stream, ordered after and before the
  * worlds' streams; the worlds stay usable on their own between batch steps. */
