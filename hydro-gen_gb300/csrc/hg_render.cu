@@ -172,18 +172,22 @@ __device__ __forceinline__ float4 tex_bilinear(const Scene& S, float px, float p
 // issue slots (72 %): it reads a plane of totals or of (rock, dirt) pairs, a
 // quarter or half of the texel, and takes the texel index from an add of 2^23
 // that rounds toward zero (an index outside [0, n - 2], a negative or NaN
-// coordinate too, fails the unsigned test and goes the general way).
+// coordinate too, fails the unsigned test and goes the general way), both
+// coordinates in one f32x2 pair (502 -> 492 us a 1920x1080 frame with three
+// worlds in turn; the mix of two rows as a pair on top takes as long).
 __device__ __forceinline__ float plane_mix(float a, float b, float fx) { return gmix(a, b, fx); }
 __device__ __forceinline__ float2 plane_mix(float2 a, float2 b, float fx) { return gmix2(a, b, pf(fx)); }
 template <class T>
-__device__ __forceinline__ T plane_bilinear(const T* __restrict__ plane, int n, float px, float py, T zero) {
-    const float wx = __fadd_rz(px, 0x1p23f), wy = __fadd_rz(py, 0x1p23f);
-    const uint32_t ix = __float_as_uint(wx) - 0x4b000000u, iy = __float_as_uint(wy) - 0x4b000000u;
+__device__ __forceinline__ T plane_bilinear(const T* __restrict__ plane, int n, float2 at, T zero) {
+    const float2 w = add_rz2(at, pf(0x1p23f));
+    const uint32_t ix = __float_as_uint(w.x) - 0x4b000000u, iy = __float_as_uint(w.y) - 0x4b000000u;
     T a, b, c, d;
+    const float px = at.x, py = at.y;
     float fx, fy;
     if ((ix < (uint32_t)(n - 1)) & (iy < (uint32_t)(n - 1))) {  // all four taps inside
-        fx = px - (wx - 0x1p23f);
-        fy = py - (wy - 0x1p23f);
+        const float2 f = sub2(at, add2(w, pf(-0x1p23f)));
+        fx = f.x;
+        fy = f.y;
         const T* p = plane + (size_t)iy * n + ix;
         a = __ldg(p);
         b = __ldg(p + 1);
@@ -204,10 +208,10 @@ __device__ __forceinline__ T plane_bilinear(const T* __restrict__ plane, int n, 
     return plane_mix(plane_mix(a, b, fx), plane_mix(c, d, fx), fy);
 }
 __device__ __forceinline__ float2 tex_ground(const Scene& S, float px, float py) {
-    return plane_bilinear(S.ground, S.n, px, py, make_float2(0.0f, 0.0f));
+    return plane_bilinear(S.ground, S.n, make_float2(px, py), make_float2(0.0f, 0.0f));
 }
 __device__ __forceinline__ float tex_total(const Scene& S, float px, float py) {
-    return plane_bilinear(S.total, S.n, px, py, 0.0f);
+    return plane_bilinear(S.total, S.n, make_float2(px, py), 0.0f);
 }
 template <bool TERRAIN>
 __device__ __forceinline__ float tex_height(const Scene& S, float px, float py) {
@@ -249,6 +253,7 @@ __device__ __noinline__ Ray raymarch(const Scene S, V3 o, V3 d, float max_d, int
     float dist = TERRAIN ? 0.0f : 0.001f, d_dist = TERRAIN ? 0.1e-12f : 0.1f;
     float min_sdf = 1.0f, dh = 0.0f;
     V3 sp = o;
+    const float2 oxz = make_float2(o.x, o.z), dxz = make_float2(d.x, d.z);
     bool out = true;  // left the height range, or ran out of steps
     auto penumbra = [&]() {
         const float num = 12.0f * d_dist;
@@ -258,7 +263,8 @@ __device__ __noinline__ Ray raymarch(const Scene S, V3 o, V3 d, float max_d, int
     };
 #pragma unroll 1
     for (int i = 0; i < max_iter; ++i) {
-        sp = add(o, scl(d, dist));
+        const float2 xz = add2(oxz, mul2(dxz, pf(dist)));
+        sp = v3(xz.x, o.y + d.y * dist, xz.y);
         dh = sp.y - tex_height<TERRAIN>(S, sp.x, sp.z);
         out = (sp.y > top) | (sp.y <= bottom);
         if (out | (dh <= 0.05f) | (dist > max_d)) break;  // (a NaN height goes on)
