@@ -473,7 +473,10 @@ __device__ __forceinline__ float2 adj_rock_pair(const StepConsts1& c, const AdjS
 }
 __global__ void k_adj_final(StepConsts c, AdjState A, float* __restrict__ out_b) {
     const int x = 2 * (blockIdx.x * BX + threadIdx.x), y = blockIdx.y * BY + threadIdx.y;
-    st2(out_b + at(c.n, x, y), adj_rock_pair<true>(c, A, x, y));
+    const float2 v = adj_rock_pair<true>(c, A, x, y);
+    float* o = out_b + at(c.n, x, y);  // the caller's buffer: on any float's boundary
+    o[0] = v.x;
+    o[1] = v.y;
 }
 
 // ---- k_adj_thermal ---------------------------------------------------------------

@@ -383,3 +383,25 @@ def test_thermal_adjoint_on_a_ramp(n):
     _, _, db0, _ = gpu_gradients(w, target, 1, 1)
     _, _, rdb0 = O.adjoint_ref(ref_settings(True), 0.01, 1, b0, ks, target, 1)
     assert rel_l2(db0, rdb0) <= 1e-3
+
+
+def test_buffers_on_any_float_boundary():
+    """Targets and gradients one float past a 16-byte boundary give the aligned
+    buffers' values (the atomic adds' order aside)."""
+    torch = torch_dev()
+    n = 64
+    outs = []
+    for off in (0, 1):
+        w = make_world(n, thermal=True)
+        buf = [torch.zeros(n * n + 4, dtype=torch.float32, device="cuda")[off:off + n * n] for _ in range(4)]
+        target, g, dks, db0 = buf
+        target.copy_(torch.from_numpy(w.download("rock") * 0.99).flatten())
+        torch.cuda.synchronize()
+        tape = H.Tape(w, 4, 2)
+        tape.forward()
+        loss = H.mse(w, target.data_ptr(), g.data_ptr())
+        tape.backward(g.data_ptr(), dks.data_ptr(), db0.data_ptr())
+        w.sync()
+        outs.append((loss, g.cpu().numpy(), dks.cpu().numpy(), db0.cpu().numpy()))
+    assert outs[0][0] == outs[1][0] and np.array_equal(outs[0][1], outs[1][1])
+    assert rel_l2(outs[1][2], outs[0][2]) <= 1e-5 and rel_l2(outs[1][3], outs[0][3]) <= 1e-5
