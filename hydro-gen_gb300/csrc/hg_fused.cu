@@ -567,6 +567,18 @@ void launch_transport1(const TerrainDesc& td, bool last, int steps, cudaStream_t
 }
 }  // namespace
 
+void launch_talus_march(const StepConsts& c, const float* rock, float* rock_o, cudaStream_t st) {
+    TerrainDesc td{};
+    td.h.c = c;
+    td.h.b_ero = const_cast<float*>(rock);  // (read only)
+    td.h.out[S_ROCK] = rock_o;
+    td.h.t_rows = chunk_rows(&c.n, 1);
+    td.row_hi = c.n;
+    const int tasks = transport_tasks(c.n, c.n, td.h.t_rows);
+    k_transport1<false><<<task_blocks(tasks), 32 * T_WARPS, 0, st>>>(td, tasks, 0);
+    count_launch();
+}
+
 void launch_fused_table(const BatchParams& bp, const CUtensorMap* maps, int total_tiles, int th, bool thermal,
                         ChainPos pos, int* err, cudaStream_t st) {
     if (th == 16) launch_hydro_table<16>(bp, maps, total_tiles, pos.index, err, st);

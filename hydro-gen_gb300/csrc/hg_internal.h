@@ -36,6 +36,8 @@ void launch_gather(const StepConsts& c, const float* u, const float* v, const fl
                    cudaStream_t st);
 // both talus passes of a whole map's layer 0
 void launch_talus(const StepConsts& c, const float* rock, float* rock_o, cudaStream_t st);
+// the same by k_transport's marching warps (hg_fused.cu)
+void launch_talus_march(const StepConsts& c, const float* rock, float* rock_o, cudaStream_t st);
 // sediment transport without the evaporation and both talus passes of a whole
 // map's layer 0
 void launch_gather_talus(const StepConsts& c, const float* rock, float* rock_o, const float* u, const float* v,

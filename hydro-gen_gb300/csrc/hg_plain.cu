@@ -239,7 +239,14 @@ void launch_gather(const StepConsts& c, const float* u, const float* v, const fl
     count_launch();
 }
 
+// From this side up warps march (hg_fused.cu): steps with talus, a row per warp /
+// marching, in three worlds in turn and (alone): 1496² 60 / 58 us (81 / 86), 1752²
+// 72 / 67 (93 / 94), 2296² 123 / 111 (149 / 148), 3000² 234 / 210 (274 / 270);
+// 1000² 29.3 / 30.1 (45 / 50).
+constexpr int MARCH_MIN_N = 2048;
+
 void launch_talus(const StepConsts& c, const float* rock, float* rock_o, cudaStream_t st) {
+    if (c.n >= MARCH_MIN_N) return launch_talus_march(c, rock, rock_o, st);
     k_talus<false><<<dim3(strips(c.n), c.n / R_ROWS), 32 * R_WARPS, 0, st>>>(c, rock, rock_o, nullptr, nullptr, nullptr,
                                                                             nullptr);
     count_launch();

@@ -97,11 +97,12 @@ def test_two_layer_chain_against_per_pass(n, thermal, dirt_talus):
             assert np.array_equal(x, y), f"{f} after {a.step_count}: {np.count_nonzero(x != y)} cells differ"
 
 
-@pytest.mark.parametrize("n", [72, 760, 776])
+@pytest.mark.parametrize("n", [72, 760, 776, 2040, 2056])
 @pytest.mark.parametrize("rain", ["uniform", "bernoulli"])
 def test_joined_passes_against_single_ones(n, rain):
     """The per-pass step joins passes (the gather in the talus launch up to a
-    side of 768, in its own above): the bits of the passes run one by one."""
+    side of 768, in its own above; marching talus warps from 2048 up): the bits
+    of the passes run one by one."""
     worlds = []
     for _ in range(2):
         w = H.World(n)
