@@ -688,6 +688,15 @@ int fork_groups(FusedGroup* groups, int ngroups, cudaEvent_t ev) {
     return HG_OK;
 }
 
+// The first group's stream goes on after the others'.
+int join_groups(FusedGroup* groups, int ngroups, cudaEvent_t ev) {
+    for (int g = 1; g < ngroups; ++g) {
+        HG_CUDA(cudaEventRecord(ev, groups[g].st));
+        HG_CUDA(cudaStreamWaitEvent(groups[0].st, ev, 0));
+    }
+    return HG_OK;
+}
+
 int check_groups(const FusedGroup* groups, int ngroups) {
     for (int g = 0; g < ngroups; ++g)
         for (const hg_world* w : groups[g].worlds) {
@@ -698,13 +707,17 @@ int check_groups(const FusedGroup* groups, int ngroups) {
 }
 
 // Builds the groups' plans of both tile heights and captures their graphs.
+// Preparing a plan sets its worlds' device step counters on the group's
+// stream, so the groups are joined before anything else uses them.
 int fused_prepare(FusedGroup* groups, int ngroups, cudaEvent_t ev, int* err) {
     int rc = check_groups(groups, ngroups), dir = 0;
     if (rc == HG_OK) rc = fork_groups(groups, ngroups, ev);
+    if (rc != HG_OK) return rc;
     for (int g = 0; g < ngroups && rc == HG_OK; ++g)
         for (int th : {16, 8})
             if (rc == HG_OK) rc = prepare_plan(plan_for(groups[g], th, err), true, &dir);
-    return rc;
+    const int joined = join_groups(groups, ngroups, ev);
+    return rc != HG_OK ? rc : joined;
 }
 
 // Fused steps over the groups' worlds with the autotuned (or requested) variant.  The
@@ -731,11 +744,8 @@ int fused_run(FusedGroup* groups, int ngroups, cudaEvent_t ev, Tuning& tune, int
     auto run_all = [&](int th, int count, bool graph) -> int {
         int rc = fork_groups(groups, ngroups, ev);
         for (int g = 0; g < ngroups && rc == HG_OK; ++g) rc = run_plan(plan_for(groups[g], th, err), count, graph);
-        for (int g = 1; g < ngroups; ++g) {
-            HG_CUDA(cudaEventRecord(ev, groups[g].st));
-            HG_CUDA(cudaStreamWaitEvent(st, ev, 0));
-        }
-        return rc;
+        const int joined = join_groups(groups, ngroups, ev);
+        return rc != HG_OK ? rc : joined;
     };
     if (req_th == HG_AUTO && req_graph == HG_AUTO && tune.th == 0 && nsteps >= 8) {
         // tiles of 8 rows give a launch more blocks and each thread one pair:
@@ -927,6 +937,7 @@ int hg_world_create(int n, int layers, hg_world** out) {
     if (e == cudaSuccess) e = alloc((void**)&w->err, sizeof(int));
     if (e == cudaSuccess) e = alloc((void**)&w->d_step, sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemsetAsync(w->err, 0, sizeof(int), w->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(w->d_step, 0, sizeof(unsigned long long), w->stream);
     if (e == cudaSuccess) e = alloc((void**)&w->red_f, sizeof(float) * (2 * reduction_parts() + 2));
     if (e == cudaSuccess) e = alloc((void**)&w->red_d, sizeof(double) * (8 * reduction_parts() + 8));
     if (e != cudaSuccess) {

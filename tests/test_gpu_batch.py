@@ -163,3 +163,38 @@ def test_largest_batch_in_one_launch():
     assert e.value.code == -5  # HG_ERR_UNSUPPORTED
     for w in ref + ws + extra:
         w.close()
+
+
+@pytest.mark.parametrize("sides", [(2048, 2048), (2048, 1024, 1024, 1024, 1024)])
+def test_two_groups_take_the_worlds_step_counters_over(sides):
+    """Batches large enough for two concurrent groups of worlds, one of them
+    (or both) a single world, created over worlds with steps still in flight:
+    the tuned first call and a later one equal per-pass steps bit for bit.
+    The rain's cells follow from the step counter alone, so a counter that is
+    set out of turn shows in the water."""
+    ts = H.config3_terrains(count=len(sides), seed=3)
+    for t, n in zip(ts, sides):
+        t["n"] = n
+
+    def worlds():
+        out = []
+        for i, t in enumerate(ts):
+            w = H.make_config3_world(t, terrain_id=i)
+            w.set_options(H.options(H.RAIN_BERNOULLI, p=0.02, seed=t["seed"], terrain_id=i))
+            out.append(w)
+        return out
+    ref, ws = worlds(), worlds()
+    b = H.Batch(ws)
+    for w in ws:
+        w.step(6, H.MODE_PLAIN)  # not waited for
+    b.step(16, H.MODE_FUSED)  # builds, times the launch forms, steps
+    b.step(5, H.MODE_FUSED)
+    for w in ref:
+        w.step(27, H.MODE_PLAIN)
+    b.sync()
+    for a, c in zip(ref, ws):
+        same(a, c)
+        assert c.step_count == 27
+    b.close()
+    for w in ref + ws:
+        w.close()
