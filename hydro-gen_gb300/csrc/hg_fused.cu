@@ -478,17 +478,17 @@ bool fused_tile_ok(int n, int th) { return (th == 16 || th == 8) && n % TW == 0 
 
 int fused_tiles(int n, int th) { return (n / TW) * (n / th); }
 
-int chunk_rows(const int* sides, int count) {
+int chunk_rows(const int* sides, const int* rows, int count) {
     int most = 0;
     size_t cells = 0;
     for (int i = 0; i < count; ++i) {
-        most = sides[i] > most ? sides[i] : most;
-        cells += (size_t)sides[i] * sides[i];
+        most = rows[i] > most ? rows[i] : most;
+        cells += (size_t)sides[i] * rows[i];
     }
     size_t r = cells / SW / T_FILL;
     for (r = r < 4 ? 4 : r; r < (size_t)most; ++r) {
         size_t tasks = 0;
-        for (int i = 0; i < count; ++i) tasks += transport_tasks(sides[i], sides[i], (int)r);
+        for (int i = 0; i < count; ++i) tasks += transport_tasks(sides[i], rows[i], (int)r);
         if (tasks <= (size_t)T_FILL) break;
     }
     return (int)r;
@@ -514,7 +514,7 @@ bool fill_desc(TerrainDesc& d, const TerrainSrc& s, int th, TmaCache& cache) {
     h.uv_prev = s.uv_prev;
     h.step = s.step;
     h.tiles_x = s.c.n / TW;
-    h.t_rows = chunk_rows(&s.c.n, 1);
+    h.t_rows = chunk_rows(&s.c.n, &s.c.n, 1);
     d.row_lo = 0;
     d.row_hi = s.c.n;
     const int in_fields[H_N] = {S_ROCK, S_WATER, S_FL, S_FR, S_FT, S_FB, S_SED};
@@ -572,7 +572,7 @@ void launch_talus_march(const StepConsts& c, const float* rock, float* rock_o, c
     td.h.c = c;
     td.h.b_ero = const_cast<float*>(rock);  // (read only)
     td.h.out[S_ROCK] = rock_o;
-    td.h.t_rows = chunk_rows(&c.n, 1);
+    td.h.t_rows = chunk_rows(&c.n, &c.n, 1);
     td.row_hi = c.n;
     const int tasks = transport_tasks(c.n, c.n, td.h.t_rows);
     k_transport1<false><<<task_blocks(tasks), 32 * T_WARPS, 0, st>>>(td, tasks, 0);

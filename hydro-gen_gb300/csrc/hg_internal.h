@@ -246,8 +246,9 @@ bool fused_tile_ok(int n, int th);
 int fused_tiles(int n, int th);
 // Fills a descriptor (tensor maps from the cache); false if a map cannot be encoded.
 bool fill_desc(TerrainDesc& d, const TerrainSrc& s, int th, TmaCache& cache);
-// Rows a warp of k_transport marches in a launch over terrains of these sides.
-int chunk_rows(const int* sides, int count);
+// Rows a warp of k_transport marches in a launch over rows[i] rows of each terrain
+// of side sides[i].
+int chunk_rows(const int* sides, const int* rows, int count);
 // Warps it runs for `rows` rows of an n x n terrain.
 int transport_tasks(int n, int rows, int t_rows);
 // One fused step (k_hydro, k_transport) over every tile of the batch's

@@ -497,7 +497,7 @@ int build_plan(Plan* p) {
             bp.tasks = 0;
             std::vector<int> sides;
             for (hg_world* w : p->worlds) sides.push_back(w->n);
-            const int rows = chunk_rows(sides.data(), (int)nt);
+            const int rows = chunk_rows(sides.data(), sides.data(), (int)nt);
             std::vector<CUtensorMap> maps(nt * MAPS_PER_TERRAIN);
             for (size_t i = 0; i < nt; ++i) {
                 bp.tile0[i] = tile0[i];
@@ -1768,6 +1768,10 @@ int hg_fused_pass(hg_world* w, int which) {
     if (!fill_desc(td, src, th, w->tma)) return fail(HG_ERR_CUDA, "cuTensorMapEncodeTiled failed for a world buffer");
     td.row_lo = w->row_lo;
     td.row_hi = w->row_hi;
+    const int rows = w->row_hi - w->row_lo;
+    // a slab's warps march fewer rows than the whole map's would, so that it
+    // fills the GPU too (an eighth of 8192²: k_transport 243 us, now 104)
+    td.h.t_rows = chunk_rows(&w->n, &rows, 1);
     launch_fused_half(td, th, which, w->err, st);
     if (which == 1) {  // the step's outputs become the state (k_transport advanced the device counter)
         for (int f = 0; f < S_COUNT; ++f) std::swap(w->cur[f], w->alt[f]);

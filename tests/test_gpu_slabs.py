@@ -8,6 +8,7 @@ blocks, under uniform rain and under thin films (back-traces past the halo:
 all-gathers and roll-backs), every rank's own rows equal one world stepped
 whole with the per-pass kernels, bit for bit."""
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -176,3 +177,57 @@ def test_gpu_fused_slabs_equal_one_world(nranks, films):
     assert (gathers > 0) == films
     for w in worlds:
         w.close()
+
+
+def eroded(n, lo=0, hi=-1):
+    """A world after a few fused steps and the next step's k_hydro on all its
+    rows, restricted to rows [lo, hi) for the k_transport to come."""
+    w = make_fused(True, n)
+    w.step(4, H.MODE_FUSED)
+    if hi >= 0:
+        w.fused_pass(0)
+        w.restrict_rows(lo, hi)
+    return w
+
+
+@pytest.mark.parametrize("n,cut", [(1024, 320), (4608, 3712)])
+def test_transport_on_unequal_row_ranges_equals_the_whole_map(n, cut):
+    """k_transport over [0, cut) and [cut, n): the rows of a whole step, bit for
+    bit, at sides whose ranges take its forms for larger launches."""
+    ref = eroded(n)
+    ref.step(1, H.MODE_FUSED)
+    for lo, hi in ((0, cut), (cut, n)):
+        w = eroded(n, lo, hi)
+        w.fused_pass(1)
+        w.sync()
+        assert w.step_count == ref.step_count == 5
+        for f in ("rock", "sediment"):
+            a, b = w.get_rows(f, lo, hi), ref.get_rows(f, lo, hi)
+            assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), f"{f} of rows [{lo}, {hi})"
+        w.close()
+    ref.close()
+
+
+def test_transport_of_a_slab_takes_a_slabs_share_of_the_time():
+    """An eighth of an 8192² map's rows is an eighth of the work; a launch whose
+    warps marched as many rows as the whole map's took a third of its time."""
+    n = 8192
+    w = eroded(n)
+
+    def us(k=12):
+        best = 1e9
+        for _ in range(5):
+            w.sync()
+            t0 = time.perf_counter()
+            for _ in range(k):
+                w.fused_pass(1)
+            w.sync()
+            best = min(best, (time.perf_counter() - t0) / k)
+        return best * 1e6
+
+    us()
+    whole = us()
+    w.restrict_rows(n // 2, n // 2 + n // 8)
+    slab = us()
+    w.close()
+    assert slab < 0.25 * whole, f"{slab:.0f} us of {whole:.0f} us"
