@@ -27,10 +27,9 @@
 // latter for batches and worlds below 4096² (see hydro_block).
 //
 // Both kernels are table driven: one launch covers any number of worlds
-// ("terrains") of different sizes and settings.  A block (k_hydro) or warp
-// (k_transport) finds its terrain by binary search and reads the terrain's
-// record (step constants, rain settings, buffers, step counter; TMA tensor
-// maps in global memory).  A single world takes its whole descriptor, tensor
+// ("terrains") of different sizes and settings.  A block (a marching warp)
+// finds its terrain by binary search and reads the terrain's record (step constants, rain settings, buffers, step counter;
+// TMA tensor maps in global memory).  A single world takes its whole descriptor, tensor
 // maps included, as a kernel parameter.  The rain step number is the
 // terrain's device step counter (advanced at a chain's end) plus the step's
 // place in the chain, so a captured CUDA graph of a few steps can be replayed
@@ -42,7 +41,8 @@
 //   and gather the sediment.  Each thread computes pairs of adjacent cells,
 //   one per iteration, a warp covering a row of the tile.
 //   k_transport marches warps up strips of columns, the talus pass in
-//   registers (see below).
+//   registers; smaller launches run it by tiles in shared memory, the
+//   smallest worlds by a row per warp (see below).
 //
 // Per-cell arithmetic is the code of the per-pass kernels (hg_device.cuh),
 // evaluated two cells per f32x2 instruction where cells pair up, so the
@@ -289,9 +289,9 @@ __global__ void __launch_bounds__(Geo<TH>::NTH, 4) k_hydro1(const __grid_constan
 }
 
 // ---------------------------------------------------------------------------
-// k_transport: sediment_transport, then thermal_erosion/thermal_transport
-// (layer 0).  A warp marches up a strip of columns, two adjacent cells per
-// lane (one f32x2 pair), and keeps the talus pass in registers: the eroded
+// k_transport of large launches: sediment_transport, then
+// thermal_erosion/thermal_transport (layer 0).  A warp marches up a strip of
+// columns, two adjacent cells per lane (one f32x2 pair), and keeps the talus pass in registers: the eroded
 // rock of three rows, the current row's eight outflows, and of the row below
 // what its neighbours need.  Neighbours across lanes come by shuffle, so
 // there is no shared memory and no block barrier.
@@ -417,6 +417,147 @@ __global__ void __launch_bounds__(32 * T_WARPS, SED ? T_BLOCKS_SED : T_BLOCKS)
     if (w < tasks) transport_task<SED>(td.h, w, td.row_lo, td.row_hi, steps);
 }
 
+// ---------------------------------------------------------------------------
+// k_transport_tile: the same by 64 x 16 tiles, 256 threads with a row group of
+// four cells (two pairs) each: the eroded rock of the tile and a two-row halo
+// and the outflows of the tile and a ring of one go through shared memory.  A
+// block is short and the SM holds 32 warps of it, where a marching warp works
+// through its rows one after the other at 20 to 24 warps per SM: the form for
+// launches whose time is latency.  The marching form recomputes less once it can
+// march far, and leaves the SMs room for other worlds' kernels.
+// Bound by issue slots and the barriers.
+// ---------------------------------------------------------------------------
+constexpr int TT_H = 16, TT_NTH = 256, TT_BH = TT_H + 4, TT_OC = RW * (TT_H + 2);
+struct TileShared {
+    float rock[RW * TT_BH];  // region (rx, ry): global (tx0 - HX + rx, ty0 - 2 + ry)
+    float out[8 * TT_OC];    // outflows at (rx, ry), ry in [1, TT_H + 2]: index (ry - 1) * RW + rx
+};
+
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+
+// outflows of the pair at index si of the staged rock
+__device__ __forceinline__ void tile_outflows(const StepConsts1& c, const float* rock, int si, float2 o[8]) {
+    const float2 m = ld2(rock + si), up = ld2(rock + si + RW), dn = ld2(rock + si - RW);
+    auto left = [&](int i, float2 v) { return make_float2(rock[i - 1], v.x); };
+    auto right = [&](int i, float2 v) { return make_float2(v.y, rock[i + 2]); };
+    float2 dm[8] = {sub2(m, left(si, m)),       sub2(m, right(si, m)),       sub2(m, up),
+                    sub2(m, dn),                sub2(m, left(si + RW, up)),  sub2(m, right(si + RW, up)),
+                    sub2(m, left(si - RW, dn)), sub2(m, right(si - RW, dn))};
+    cell_thermal_outflows_dh2(c.dt, c.Kalpha0, c.Kspeed0, c.talus_x_cross, c.talus_b_diag, c.fast_div, m, dm, o);
+}
+
+template <bool SED>
+__device__ __forceinline__ void transport_tile(const TerrainHot& td, TileShared& sm, int tx0, int ty0) {
+    const StepConsts1& c = td.c;
+    const int n = c.n, tid = threadIdx.x;
+    const int gx0 = tx0 - HX, gy0 = ty0 - 2;
+    const int ix = 4 * (tid % (TW / 4)), iy = tid / (TW / 4);
+    const size_t gi = (size_t)(ty0 + iy) * n + tx0 + ix;
+    // the rock (the shader's out-of-range height outside the grid) and the
+    // sediment taps are in flight together
+    constexpr int BP = RW / 2 * TT_BH, BK = (BP + TT_NTH - 1) / TT_NTH;
+    float2 box[BK];
+    if (c.thermal) {
+#pragma unroll
+        for (int k = 0; k < BK; ++k) {
+            const int q = tid + k * TT_NTH, gx = gx0 + 2 * (q % (RW / 2)), gy = gy0 + q / (RW / 2);
+            const bool in = q < BP && gx >= 0 && gx < n && gy >= 0 && gy < n;
+            box[k] = in ? ldg2(td.b_ero + (size_t)gy * n + gx) : pf(FAR_HEIGHT);
+        }
+    }
+    Taps<1> taps[2];
+    if (SED) {
+        const float4 u = __ldg(reinterpret_cast<const float4*>(td.u + gi));
+        const float4 v = __ldg(reinterpret_cast<const float4*>(td.v + gi));
+        const float* const se[1] = {td.s_ero};
+        load_taps<1>(c, se, tx0 + ix, ty0 + iy, make_float2(u.x, u.y), make_float2(v.x, v.y), taps[0]);
+        load_taps<1>(c, se, tx0 + ix + 2, ty0 + iy, make_float2(u.z, u.w), make_float2(v.z, v.w), taps[1]);
+    }
+    if (c.thermal) {
+#pragma unroll
+        for (int k = 0; k < BK; ++k) {
+            const int q = tid + k * TT_NTH;
+            if (q < BP) st2(sm.rock + 2 * q, box[k]);
+        }
+        __syncthreads();
+    }
+    if (SED) {
+        const float2 a = mix_taps(taps[0], 0), b = mix_taps(taps[1], 0);
+        *reinterpret_cast<float4*>(td.out[S_SED] + gi) = make_float4(a.x, a.y, b.x, b.y);
+    }
+    if (!c.thermal) return;
+    // outflows of the ring: 34 pairs in the row below and above the tile (from
+    // two columns before it), a pair at either end of its rows
+    constexpr int CAP = TW / 2 + 2, RING = 2 * CAP + 2 * TT_H;
+    if (tid < RING) {
+        const bool cap = tid < 2 * CAP;
+        const int rx = cap ? HX - 2 + 2 * (tid % CAP) : tid & 1 ? HX + TW : HX - 2;
+        const int ry = cap ? (tid < CAP ? 1 : TT_H + 2) : 2 + (tid - 2 * CAP) / 2;
+        float2 o[8];
+        tile_outflows(c, sm.rock, ry * RW + rx, o);
+        const int gx = gx0 + rx, gy = gy0 + ry;
+        const bool in = gx >= 0 && gx < n && gy >= 0 && gy < n;  // (a pair lies inside the grid or outside it)
+#pragma unroll
+        for (int d = 0; d < 8; ++d) st2(sm.out + d * TT_OC + (ry - 1) * RW + rx, in ? o[d] : pf(0.0f));
+    }
+    const int si = (iy + 2) * RW + HX + ix, oi = si - RW;
+    float2 osum[2];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        float2 o[8];
+        tile_outflows(c, sm.rock, si + 2 * p, o);
+        osum[p] = pf(0.0f);
+#pragma unroll
+        for (int d = 0; d < 8; ++d) {
+            osum[p] = sub2(osum[p], o[d]);
+            st2(sm.out + d * TT_OC + oi + 2 * p, o[d]);
+        }
+    }
+    __syncthreads();
+    // inflows in the shader's order: L, R, T, B, LT, RT, LB, RB
+    float2 inf[2] = {pf(0.0f), pf(0.0f)};
+    auto add = [&](float2 a, float2 b) {
+        inf[0] = add2(inf[0], a);
+        inf[1] = add2(inf[1], b);
+    };
+    auto sides = [&](int dl, int dr, int off) {  // left neighbour's dl, right neighbour's dr
+        const float *a = sm.out + dl * TT_OC + oi + off, *b = sm.out + dr * TT_OC + oi + off;
+        const float4 l = ld4(a), r = ld4(b);
+        add(make_float2(a[-1], l.x), make_float2(l.y, l.z));
+        add(make_float2(r.y, r.z), make_float2(r.w, b[4]));
+    };
+    auto above = [&](int d, int off) {
+        const float4 v = ld4(sm.out + d * TT_OC + oi + off);
+        add(make_float2(v.x, v.y), make_float2(v.z, v.w));
+    };
+    sides(1, 0, 0);
+    above(3, RW);
+    above(2, -RW);
+    sides(7, 6, RW);
+    sides(5, 4, -RW);
+    const float4 b = ld4(sm.rock + si);
+    const float2 r0 = add2(make_float2(b.x, b.y), add2(osum[0], inf[0]));
+    const float2 r1 = add2(make_float2(b.z, b.w), add2(osum[1], inf[1]));
+    *reinterpret_cast<float4*>(td.out[S_ROCK] + gi) = make_float4(r0.x, r0.y, r1.x, r1.y);
+}
+
+template <bool SED>
+__global__ void __launch_bounds__(TT_NTH, 4) k_transport_tile1(const __grid_constant__ TerrainDesc td, int steps) {
+    __shared__ __align__(16) TileShared sm;
+    transport_tile<SED>(td.h, sm, blockIdx.x * TW, td.row_lo + blockIdx.y * TT_H);
+    if (SED && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *td.h.step += (unsigned long long)steps;
+}
+
+// shift: 0 when k_hydro's tiles have 16 rows as these, 1 when they have 8
+template <bool SED>
+__global__ void __launch_bounds__(TT_NTH, 4) k_transport_tile(const __grid_constant__ BatchParams bp, int shift, int steps) {
+    __shared__ __align__(16) TileShared sm;
+    const int t = find_terrain(bp.tile0, bp.nterr, blockIdx.x << shift);
+    const unsigned tile = blockIdx.x - (bp.tile0[t] >> shift), tiles_x = bp.t[t].tiles_x;
+    transport_tile<SED>(bp.t[t], sm, (tile % tiles_x) * TW, (tile / tiles_x) * TT_H);
+    if (SED && tile == 0 && threadIdx.x == 0) *bp.t[t].step += (unsigned long long)steps;
+}
+
 template <bool SED>
 __global__ void __launch_bounds__(32 * R_WARPS, SED ? 2 : 3) k_transport_rows(const __grid_constant__ TerrainDesc td, int steps) {
     const TerrainHot& h = td.h;
@@ -530,6 +671,21 @@ namespace {
 // path.
 constexpr int SPLIT_MIN_N = 4096;
 
+// Forms of the talus launch: a single world up to this side runs talus_rows, a
+// larger one and batches tiles up to the cells below, above them warps march.
+// One step with talus of one world, alone / three worlds in turn, us, by tiles,
+// marching: 1024² 46 / 20, 54 / 25; 2048² 111 / 79, 124 / 85; 3072² 209 / 177,
+// 230 / 180; 4096² 347 / 315, 377 / 312.  Eight chained steps, of which one
+// gathers: 1024² 199 / 156, 255 / 182; 2048² 707 / 600, 784 / 616; 3072² 1444 /
+// 1346, 1555 / 1317.  By rows, tiles: 256² 68 / 25, 76 / 28; 384² 80 / 31, 82 / 36;
+// 448² 87 / 39, 92 / 40; four worlds of 448² on their own streams 164 / 166, 152 /
+// 140.
+constexpr int ROWS1_MAX_N = 384;
+bool tiled(size_t cells, bool thermal, bool last) {
+    if (!thermal) return true;  // the gather alone, nothing to march for
+    return last ? cells < (size_t)4096 * 4096 : cells <= (size_t)2048 * 2048;
+}
+
 template <int TH>
 void launch_hydro1(const TerrainDesc& td, int index, int* err, cudaStream_t st) {
     const dim3 tiles(td.h.tiles_x, (td.row_hi - td.row_lo) / TH);
@@ -553,14 +709,22 @@ void launch_hydro_table(const BatchParams& bp, const CUtensorMap* maps, int tile
 }
 
 void launch_transport1(const TerrainDesc& td, bool last, int steps, cudaStream_t st) {
-    if (td.h.c.n <= ROWS_MAX_N) {
-        const dim3 grid(strips(td.h.c.n), (td.row_hi - td.row_lo) / R_ROWS);
+    const int rows = td.row_hi - td.row_lo;
+    if (td.h.c.thermal && td.h.c.n <= ROWS1_MAX_N) {
+        const dim3 grid(strips(td.h.c.n), rows / R_ROWS);
         if (last) k_transport_rows<true><<<grid, 32 * R_WARPS, 0, st>>>(td, steps);
         else k_transport_rows<false><<<grid, 32 * R_WARPS, 0, st>>>(td, 0);
         count_launch();
         return;
     }
-    const int tasks = transport_tasks(td.h.c.n, td.row_hi - td.row_lo, td.h.t_rows);
+    if (tiled((size_t)td.h.c.n * rows, td.h.c.thermal, last)) {
+        const dim3 grid(td.h.tiles_x, rows / TT_H);
+        if (last) k_transport_tile1<true><<<grid, TT_NTH, 0, st>>>(td, steps);
+        else k_transport_tile1<false><<<grid, TT_NTH, 0, st>>>(td, 0);
+        count_launch();
+        return;
+    }
+    const int tasks = transport_tasks(td.h.c.n, rows, td.h.t_rows);
     if (last) k_transport1<true><<<task_blocks(tasks), 32 * T_WARPS, 0, st>>>(td, tasks, steps);
     else k_transport1<false><<<task_blocks(tasks), 32 * T_WARPS, 0, st>>>(td, tasks, 0);
     count_launch();
@@ -584,6 +748,13 @@ void launch_fused_table(const BatchParams& bp, const CUtensorMap* maps, int tota
     if (th == 16) launch_hydro_table<16>(bp, maps, total_tiles, pos.index, err, st);
     else launch_hydro_table<8>(bp, maps, total_tiles, pos.index, err, st);
     if (!pos.last && !thermal) return;
+    if (tiled((size_t)total_tiles * TW * th, thermal, pos.last)) {
+        const int shift = th == TT_H ? 0 : 1, tiles = total_tiles >> shift;
+        if (pos.last) k_transport_tile<true><<<tiles, TT_NTH, 0, st>>>(bp, shift, pos.index + 1);
+        else k_transport_tile<false><<<tiles, TT_NTH, 0, st>>>(bp, shift, 0);
+        count_launch();
+        return;
+    }
     if (pos.last) k_transport<true><<<task_blocks(bp.tasks), 32 * T_WARPS, 0, st>>>(bp, pos.index + 1);
     else k_transport<false><<<task_blocks(bp.tasks), 32 * T_WARPS, 0, st>>>(bp, 0);
     count_launch();

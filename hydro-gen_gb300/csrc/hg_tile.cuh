@@ -79,13 +79,6 @@ __device__ __forceinline__ void talus_rows(const StepConsts1& c, const TalusRate
     const bool in = x >= 0 && x < n;
     const bool own = in && lane >= 1 && lane <= SW / 2 && warp >= 1 && warp <= R_ROWS;
     const size_t gi = (size_t)y * n + x;
-    if (!DIRT && !c.thermal) {
-        if (own) {
-            begin(x, y, gi);
-            end(x, y, gi);
-        }
-        return;
-    }
     auto height = [&](const float* f, int r) {
         return in && r >= 0 && r < n ? ldg2(f + (size_t)r * n + x) : pf(FAR_HEIGHT);
     };
@@ -139,11 +132,9 @@ __device__ __forceinline__ void talus_rows(const StepConsts1& c, const float* __
     const TalusRates t{c.Kalpha0, c.Kspeed0, c.talus_x_cross, c.talus_b_diag, c.fast_div};
     talus_rows<false>(c, t, in_rock, nullptr, out_rock, strip, y0, begin, end);
 }
-// Worlds up to this side run talus_rows: a one-layer step with talus takes, in
-// three worlds in turn / alone, 3.4 / 8.3 us at 256² (marching: 4.6 / 11.2),
-// 5.0 / 10.4 at 448² (6.0 / 12.4), 11.7 / 18.3 at 768² (12.4 / 21.8); at
-// 1024² marching takes 19.8 / 29.1 against 22.8 / 26.1, from 1536² on less
-// both ways.
+// Maps up to this side gather the sediment within the rock's talus launch: one
+// launch less (two layers, one step: 384² 109 us apart, 103 together; 2048² 200
+// apart, 215 together).
 constexpr int ROWS_MAX_N = 768;
 
 // smoothing's particle branch (glsl/smoothing.glsl:76-95), per cell: momentum

@@ -3,6 +3,8 @@ in the next step's first kernel) against the same steps one call at a time,
 bit for bit, with and without talus passes, by direct launches and by graph,
 for batches of unlike worlds, and where k_transport's strips and chunks end
 unevenly."""
+import time
+
 import numpy as np
 import pytest
 
@@ -127,3 +129,60 @@ def test_joined_passes_against_single_ones(n, rain):
     for f in ("rock", "water", "sediment", "flux_l", "flux_r", "flux_t", "flux_b", "vel_u", "vel_v", "vel_z"):
         x, y = a.download(f), b.download(f)
         assert np.array_equal(x, y), f"{f}: {np.count_nonzero(x != y)} cells differ"
+
+
+@pytest.mark.parametrize("n", [384, 448, 2112, 4160])
+def test_forms_of_the_talus_launch_against_per_pass(n):
+    """Either side of the lines between rows, tiles and marching warps: a chain
+    (launches with and without the gather) and a single step."""
+    a, b = make(n, seed=6), make(n, seed=6)
+    a.step(3, H.MODE_FUSED)
+    a.step(1, H.MODE_FUSED)
+    b.step(4, H.MODE_PLAIN)
+    assert_same(a, b, f"{n}")
+    a.close()
+    b.close()
+
+
+def test_marching_batch_against_per_pass():
+    """Two groups of two worlds, each group large enough for marching warps
+    with the gather too."""
+    def worlds():
+        return [make(2944, seed=k, thermal=k != 2, graph=0) for k in range(4)]
+
+    a, b = worlds(), worlds()
+    batch = H.Batch(a)
+    batch.step(3)
+    batch.step(1)
+    batch.sync()
+    for w in b:
+        w.step(4, H.MODE_PLAIN)
+    for i, (x, y) in enumerate(zip(a, b)):
+        assert_same(x, y, f"terrain {i}")
+    batch.close()
+    for w in a + b:
+        w.close()
+
+
+def test_talus_launch_of_a_middle_sized_world():
+    """At 1024² the talus passes with the sediment gather take about as long as
+    the rest of the step; a warp per strip of four rows took 1.75 times that."""
+    w = make(1024)
+    w.set_options(H.options(H.RAIN_UNIFORM))
+    w.step(8, H.MODE_FUSED)
+
+    def us(which, k=40):
+        best = 1e9
+        for _ in range(10):
+            w.sync()
+            t0 = time.perf_counter()
+            for _ in range(k):
+                w.fused_pass(which)
+            w.sync()
+            best = min(best, (time.perf_counter() - t0) / k)
+        return best * 1e6
+
+    us(0), us(1)
+    hydro, transport = us(0), us(1)
+    w.close()
+    assert transport < 1.45 * hydro, f"{transport:.1f} us, {hydro:.1f} us"
