@@ -1954,9 +1954,10 @@ int hg_batch_step(hg_batch* b, int nsteps, int mode) {
         if (rc != HG_OK) return rc == HG_ERR_CUDA ? cuda_fail(cudaGetLastError(), "batch tuning") : rc;
         b->tuning.ms_per_world = ms / 2.0;
         nsteps -= 12;
-        double best = 1e30;
-        for (double m : b->tuning.ms) best = std::min(best, m);
-        b->tuning.per_world = b->tuning.ms_per_world < best ? 1 : 0;
+        // against the table variant that would run: a faster one that is not
+        // eligible (tiles of 8 rows in large launches) decides nothing
+        const double table = b->tuning.ms[(b->tuning.th == 16 ? 0 : 2) + b->tuning.graph];
+        b->tuning.per_world = b->tuning.ms_per_world < table ? 1 : 0;
         char m[120];
         std::snprintf(m, sizeof m, "autotuner: batch of %zu worlds, %s (%.4f ms/step per world's launches)",
                       b->worlds.size(), b->tuning.per_world ? "per-world launches" : "one table launch",

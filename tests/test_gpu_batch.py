@@ -165,6 +165,27 @@ def test_largest_batch_in_one_launch():
         w.close()
 
 
+@pytest.mark.parametrize("sides", [(512, 512), (640, 512, 256), (1024, 512), (768, 768, 768)])
+def test_launch_form_is_chosen_against_the_table_variant_that_runs(sides):
+    """Batches above 640² cells in all, where tiles of 8 rows are timed but not
+    chosen: the worlds' own launches are compared with the chosen variant."""
+    for seed in range(4):
+        ws = [H.World(n) for n in sides]
+        for i, w in enumerate(ws):
+            w.init_heightmap(H.noise(seed=seed + i))
+            H.configure(w, "config2")
+        b = H.Batch(ws)
+        b.step(12, H.MODE_FUSED)
+        b.sync()
+        th, graph, ms = b.tuning()
+        per_world, ms_pw = b.launch_form()
+        assert th == 16 and ms[graph] == min(ms[:2])
+        assert per_world == (ms_pw < ms[graph]), (per_world, ms_pw, ms)
+        b.close()
+        for w in ws:
+            w.close()
+
+
 @pytest.mark.parametrize("sides", [(2048, 2048), (2048, 1024, 1024, 1024, 1024)])
 def test_two_groups_take_the_worlds_step_counters_over(sides):
     """Batches large enough for two concurrent groups of worlds, one of them
