@@ -720,18 +720,12 @@ __global__ void k_mse_grad(const float* __restrict__ b, const float* __restrict_
     __shared__ double sh[256 / 32];
     double acc = 0.0;
     const double inv = 1.0 / (double)count;
-    // the gradient is e times 2 / count in two floats: FP64 runs at a small
-    // fraction of the FP32 rate, so it is kept for the sum (the square of a
-    // float is exact in it)
-    const float hi = (float)(2.0 * inv), lo = (float)(2.0 * inv - (double)hi);
+    const double twice = 2.0 * inv;
     const size_t step = (size_t)gridDim.x * blockDim.x;
     auto one = [&](size_t i, float e) {
         const double d = (double)e;
         acc = fma(d, d, acc);
-        if (grad) {
-            const float p = e * hi;
-            grad[i] = p + __fmaf_rn(e, lo, __fmaf_rn(e, hi, -p));
-        }
+        if (grad) grad[i] = (float)(d * twice);  // (in two floats 9 us less at 1024², but inf - inf and fewer bits)
     };
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     for (; i + 3 * step < count; i += 4 * step) {

@@ -405,3 +405,29 @@ def test_buffers_on_any_float_boundary():
         outs.append((loss, g.cpu().numpy(), dks.cpu().numpy(), db0.cpu().numpy()))
     assert outs[0][0] == outs[1][0] and np.array_equal(outs[0][1], outs[1][1])
     assert rel_l2(outs[1][2], outs[0][2]) <= 1e-5 and rel_l2(outs[1][3], outs[0][3]) <= 1e-5
+
+
+def test_mse_gradient_is_the_fp64_product_rounded_once():
+    """2 (rock - target) / count in FP64, rounded to float, for a count that is
+    not a power of two; infinite differences keep their infinite gradient."""
+    torch = torch_dev()
+    n = 200
+    rng = np.random.default_rng(4)
+    rock = (rng.random((n, n)) * 100).astype(np.float32)
+    target = (rng.random((n, n)) * 100).astype(np.float32)
+    rock[3, :4], target[3, :4] = (3e38, -3e38, np.inf, 1.0), (-3e38, 3e38, 1.0, np.nan)
+    w = H.World(n)
+    w.upload("rock", rock)
+    t = torch.from_numpy(target).cuda()
+    g = torch.empty((n, n), dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    loss = H.mse(w, t.data_ptr(), g.data_ptr())
+    w.sync()
+    with np.errstate(over="ignore", invalid="ignore"):
+        e = rock - target
+    want = (2.0 * e.astype(np.float64) / float(n * n)).astype(np.float32)
+    got = g.cpu().numpy()
+    assert np.array_equal(got, want, equal_nan=True), np.argwhere((got != want) & (want == want))[:5]
+    assert got[3, 0] == np.inf and got[3, 1] == -np.inf and got[3, 2] == np.inf and np.isnan(got[3, 3])
+    assert np.isnan(loss)
+    w.close()
