@@ -510,7 +510,7 @@ __host__ __device__ constexpr int tt_oy(int k) { return (k == 2 || k == 4 || k =
 
 struct ThermalArgs {
     CUtensorMap map_b;  // eroded rock of the step (box TT_RW x TT_BH)
-    AdjState A;          // adjoint of the step's output (own terms + packets)
+    AdjState A;         // adjoint of the step's output
     StepConsts c;
     float* g;           // out: adjoint of the eroded rock
 };

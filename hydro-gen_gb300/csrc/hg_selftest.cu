@@ -2,11 +2,12 @@
 // against IEEE division, reciprocal and square root.
 //
 // No counterpart in the reference: it checks an arithmetic shortcut of this
-// library.  Operands are drawn with Philox from the range div_recip's callers
-// guarantee (a = 0 or |a| in [2^-80, 2^80], b in [2^-30, 2^40]); a third of
+// library.  The quotient's operands are drawn with Philox from the range its callers
+// guarantee (a = 0 or |a| in [2^-80, 2^80], b in [2^-40, 2^40]); a third of
 // them are built so that a/b lies next to a float (a = RN(q*b) nudged by up to
 // two ulps) and a third next to the midpoint between two floats, the cases
-// where a quotient rounds wrongly first.
+// where a quotient rounds wrongly first.  The reciprocal and the square root
+// run over every float of their ranges.
 #include "hg_internal.h"
 #include "hg_tma.cuh"
 
@@ -25,7 +26,7 @@ __global__ void k_selftest_division(uint32_t seed_lo, uint32_t seed_hi, unsigned
     for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
         uint32_t w[4] = {(uint32_t)i, (uint32_t)(i >> 32), 0x5eedu, 0u};
         philox4x32_10(w, seed_lo, seed_hi);
-        const float b = uniform_exp_float(w[0], w[1], -30, 39);
+        const float b = uniform_exp_float(w[0], w[1], -40, 39);
         float a;
         const uint32_t kind = w[3] % 3u;
         if (kind == 0) {
@@ -50,13 +51,24 @@ __global__ void k_selftest_division(uint32_t seed_lo, uint32_t seed_hi, unsigned
         const float dd = uniform_exp_float(w[2], w[0], -30, 39);
         if (__float_as_uint(div_recip(dd, SQRT2_F, RCP_SQRT2_F)) != __float_as_uint(__fdiv_rn(dd, SQRT2_F)))
             ++local;
-        // the Newton reciprocal and square root the quotients and roots start from
-        const float rr = uniform_exp_float(w[1], w[2], -100, 99);
-        if (__float_as_uint(rcp_newton(rr)) != __float_as_uint(__frcp_rn(rr))) ++local;
-        if (__float_as_uint(sqrt_newton(rr)) != __float_as_uint(__fsqrt_rn(rr))) ++local;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0 && __float_as_uint(__frcp_rn(SQRT2_F)) != __float_as_uint(RCP_SQRT2_F))
         ++local;
+    if (local) atomicAdd(bad, local);
+}
+
+// The Newton reciprocal and square root that the quotients and roots start
+// from, over every float of their callers' ranges: [2^-125, 2^125] and
+// [2^-100, 2^100] and 0.
+__global__ void k_selftest_newton(unsigned long long* bad) {
+    unsigned long long local = 0;
+    const uint32_t lo = __float_as_uint(0x1p-125f), hi = __float_as_uint(0x1p125f), stride = gridDim.x * blockDim.x;
+    for (uint32_t bits = lo + blockIdx.x * blockDim.x + threadIdx.x; bits <= hi; bits += stride) {
+        const float x = __uint_as_float(bits);
+        if (__float_as_uint(rcp_newton(x)) != __float_as_uint(__frcp_rn(x))) ++local;
+        if (x >= 0x1p-100f && x <= 0x1p100f && __float_as_uint(sqrt_newton(x)) != __float_as_uint(__fsqrt_rn(x))) ++local;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0 && __float_as_uint(sqrt_newton(0.0f)) != 0u) ++local;
     if (local) atomicAdd(bad, local);
 }
 
@@ -166,7 +178,8 @@ extern "C" int hg_selftest_division(uint64_t seed, uint64_t count, uint64_t* mis
     if (e == cudaSuccess) e = cudaMemset(d, 0, sizeof(*d));
     if (e == cudaSuccess) {
         k_selftest_division<<<4 * 152, 256>>>((uint32_t)seed, (uint32_t)(seed >> 32), count, d);
-        count_launch();
+        k_selftest_newton<<<8 * 152, 256>>>(d);
+        count_launch(2);
         e = cudaGetLastError();
     }
     unsigned long long h = 0;

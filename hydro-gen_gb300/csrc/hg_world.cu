@@ -576,9 +576,6 @@ void launch_steps(Plan* p, int dir, int count) {
         launch_dir(p, (dir + k) & 1, chain ? ChainPos{k, k + 1 == count} : ChainPos{0, true});
 }
 
-// Brings a plan up to date (tables, device step counters, the graph that
-// starts with the next direction) without running a step; *dir gets the
-// next direction.
 // Steps per replay of a plan's long graph: long runs replay kLongGraph
 // steps at a time (an even count: the buffers are back in their roles
 // after it), a quarter of the host's graph launches.
@@ -603,6 +600,9 @@ int capture_steps(Plan* p, int dir, int which) {
     return HG_OK;
 }
 
+// Brings a plan up to date (tables, device step counters, the graphs that
+// start with the next direction) without running a step; *dir_out gets the
+// next direction.
 int prepare_plan(Plan* p, bool use_graph, int* dir_out) {
     int dir = plan_dir(p);
     if (dir < 0) {

@@ -538,7 +538,8 @@ int hg_field_totals_noalloc(const float* const* fields, int nfields, size_t coun
 /* No counterpart in the reference.  Draws `count` operand pairs (seeded) in
  * the range where the fused kernel divides through a shared reciprocal
  * (Markstein's correction) and counts results that differ in any bit from
- * IEEE division; 0 is the only passing answer.  Synchronises. */
+ * IEEE division, and so for the reciprocal and the square root of every float
+ * in their ranges; 0 is the only passing answer.  Synchronises. */
 int hg_selftest_division(uint64_t seed, uint64_t count, uint64_t* mismatches);
 /* The kernels' bounded barrier wait (a TMA tile that never arrives) run on a
  * barrier phase that nothing completes, with no copy in flight: `polls`
