@@ -708,28 +708,28 @@ __device__ __noinline__ void apply_big(const ApplyArgs& a, WarpSums& ws, uint32_
             __syncwarp();
         }
     }
-    if (k > HOT_KEYS) {
-        // merge into `keys` by each record's rank: its place in its chunk plus,
-        // per other chunk, the records below it (binary search)
+    // merge the sorted chunks, two neighbouring runs at a time: a record's place is
+    // its place in its run plus the records of the other run below it
+    // (every chunk searched by every record took 16.3 ms a step at 64² with 262144
+    // droplets after 80 steps, so 9.0)
+    uint32_t *src = a.sorted + lo, *dst = a.keys + lo;
+    for (uint32_t run = HOT_KEYS; run < k; run *= 2) {
         for (uint32_t i = lane; i < k; i += 32) {
-            const uint32_t key = a.sorted[lo + i];
-            const uint32_t own = i / HOT_KEYS * HOT_KEYS;
-            uint32_t rank = i - own;
-            for (uint32_t c0 = 0; c0 < k; c0 += HOT_KEYS) {
-                if (c0 == own) continue;
-                uint32_t l = 0, h = min((uint32_t)HOT_KEYS, k - c0);  // records of chunk c0 below key
-                const uint32_t* ch = a.sorted + lo + c0;
-                while (l < h) {
-                    const uint32_t m = (l + h) >> 1;
-                    if (ch[m] < key) l = m + 1; else h = m;
-                }
-                rank += l;
+            const uint32_t key = src[i], own = i & ~(run - 1), pair = i & ~(2 * run - 1);
+            const uint32_t other = pair + (own == pair ? run : 0u), len = other < k ? min(run, k - other) : 0u;
+            uint32_t l = 0, h = len;  // records of the other run below key
+            while (l < h) {
+                const uint32_t m = (l + h) >> 1;
+                if (src[other + m] < key) l = m + 1; else h = m;
             }
-            a.keys[lo + rank] = key;
+            dst[pair + (i - own) + l] = key;
         }
         __syncwarp();
+        uint32_t* t2 = src;
+        src = dst;
+        dst = t2;
     }
-    const uint32_t* order = k > HOT_KEYS ? a.keys + lo : sk;
+    const uint32_t* order = k > HOT_KEYS ? src : sk;
     for (uint32_t base = lo; base < hi; base += 32) {
         const uint32_t m = min(32u, hi - base);
         Rec mine{};

@@ -2,6 +2,8 @@
 sequential restatement (droplets in id order, corners 0..3), bit for bit:
 droplet state, rock, dirt, water and the momentum map, with the reference's
 particle defaults and with denser droplets sharing texels."""
+import time
+
 import numpy as np
 import pytest
 
@@ -145,3 +147,28 @@ def test_particles_at_every_bucket_size(n, count, dirt):
         w.step(1, H.MODE_PARTICLES)
         ow.particle_step(os_, oo, 1)
     check(w, ow, f"n={n} count={count} dirt={dirt}")
+
+
+def us_per_step(n, count, warm, steps=16):
+    w = H.World(n, layers=2)
+    w.init_reference_heightmap(H.map_settings(hmap_dims=(n, n), seed=0.3, scale=0.01))
+    w.particles_init(count)
+    w.set_erosion(H.settings_particles())
+    w.set_options(H.options(H.RAIN_UNIFORM, seed=3))
+    w.step(warm, H.MODE_PARTICLES)
+    w.sync()
+    t0 = time.perf_counter()
+    w.step(steps, H.MODE_PARTICLES)
+    w.sync()
+    us = (time.perf_counter() - t0) / steps * 1e6
+    w.close()
+    return us
+
+
+def test_time_of_buckets_of_many_chunks():
+    """262144 droplets gathered on 64², tens of thousands of records in a texel:
+    against the same droplets spread over 1024², the sorting of a bucket must not
+    grow with the square of its records (105 times so, 58 by merging runs)."""
+    spread = us_per_step(1024, 262144, 16)
+    crowded = us_per_step(64, 262144, 80)
+    assert crowded < 90 * spread, f"{crowded:.0f} us, {spread:.0f} us"
