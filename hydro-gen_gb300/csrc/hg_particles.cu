@@ -424,12 +424,10 @@ __device__ __forceinline__ RecOut apply_record(const ApplyArgs& a, const Rec& r,
     return RecOut{s_out[1], s_out[0], mask};
 }
 
-// A record's update with its texel-independent parts computed ahead (in
-// parallel across a warp's lanes): the dirt step with no layer exhausted,
-// then the rock step.  mode 0: kill (both layers take their share back);
-// 1: dirt dissolves and the loop breaks; 2: dirt deposits, rock dissolves;
-// 3: both deposit.  Only an exhausted dirt layer (mode 1 going below zero)
-// needs the full update, apply_record.
+// A record's amounts with no layer exhausted, which do not depend on the texel
+// (computed in parallel across a warp's lanes): the dirt step, then the rock step.
+// mode 0: kill (both layers take their share back); 1: dirt dissolves and the
+// loop breaks; 2: dirt deposits, rock dissolves; 3: both deposit.
 struct Pre {
     uint32_t key;
     int mode;
@@ -472,39 +470,6 @@ __device__ __forceinline__ Pre prep_record(const ApplyArgs& a, const Rec& r) {
         p.s0n = r.s0 - p.d0;
     }
     return p;
-}
-
-// the texel-dependent rest of a prepared record; false (texel untouched)
-// when the dirt layer would be exhausted
-__device__ __forceinline__ bool apply_prepared(const Pre& p, Texel& T, RecOut& o) {
-    if (p.mode == 1) {
-        const float t = T.terr[1] - p.d1;
-        if (t < 0.0f) return false;
-        T.terr[1] = t;
-        o = RecOut{p.s1n, 0.0f, 2u};
-    } else if (p.mode == 0) {
-        T.terr[1] += p.d1;
-        T.terr[0] += p.d0;
-        o = RecOut{0.0f, 0.0f, 0u};
-    } else if (p.mode == 2) {
-        T.terr[1] += p.d1;
-        const float t = T.terr[0] - p.d0;
-        if (t < 0.0f) {
-            o = RecOut{p.s1n, p.s0n + t, 3u};
-            T.terr[0] = 0.0f;
-        } else {
-            o = RecOut{p.s1n, p.s0n, 3u};
-            T.terr[0] = t;
-        }
-    } else {
-        T.terr[1] += p.d1;
-        T.terr[0] += p.d0;
-        o = RecOut{p.s1n, p.s0n, 3u};
-    }
-    T.wat += p.wi;
-    T.mz += p.mzi;
-    T.mw += p.mwi;
-    return true;
 }
 
 __device__ __forceinline__ void store_rec(const ApplyArgs& a, uint32_t key, const RecOut& o) {
@@ -593,13 +558,17 @@ __device__ __forceinline__ void sort_chunk(const uint32_t* src, uint32_t len, ui
 // that do not depend on the texel, and so is what a record leaves for its
 // droplet: lane c keeps sum c (dirt, rock, water, mz, mw) and adds the records'
 // amounts, transposed through shared memory, one add per record for all five.
-// A sum that gets below zero may mean an exhausted layer: then the batch runs
-// again from the values it started with, record by record.
-// Bound by the latency of that chain: about 10 cycles per record against 100
-// for a lane that applies whole records.
+// A dirt or rock sum that gets below zero may mean an exhausted layer: then every
+// lane runs these two again from the values they started with, a record at a
+// time without a branch, and keeps those its own record met; from them it works
+// out what the record leaves.
+// Bound by the latency of the two chains: about 10 cycles a record, and 60 where
+// layers are exhausted (790 when the whole record went from lane to lane).
 constexpr int SUMS = 5, SUM_PITCH = 36;  // (16-byte rows, lanes 0 to 4 on different banks)
 struct WarpSums {
     float v[SUMS][SUM_PITCH];
+    float4 w[2][32];  // exhausted layers: dirt and rock amounts, capacity, rock sediment; rock's
+                      // rates, whether the record dissolves dirt, rock
 };
 __device__ __forceinline__ float* texel_sum(const ApplyArgs& a, int c) {
     return c == 0 ? a.dirt : c == 1 ? a.rock : c == 2 ? a.water : c == 3 ? a.mz : a.mw;
@@ -639,40 +608,35 @@ __device__ __forceinline__ void warp_apply(const ApplyArgs& a, WarpSums& ws, int
         }
         return;
     }
-    Texel T;
-    T.terr[1] = __shfl_sync(FULL, acc, 0);
-    T.terr[0] = __shfl_sync(FULL, acc, 1);
-    T.wat = __shfl_sync(FULL, acc, 2);
-    T.mz = __shfl_sync(FULL, acc, 3);
-    T.mw = __shfl_sync(FULL, acc, 4);
+    ws.w[0][lane] = make_float4(p.mode == 1 ? -p.d1 : p.d1, p.mode == 1 ? -0.0f : p.mode == 2 ? -p.d0 : p.d0, mine.sc, mine.s0);
+    ws.w[1][lane] = make_float4(mine.multipl * (a.es.d_t * a.es.Ks[0]), mine.multipl * (a.es.d_t * a.es.Kd[0]),
+                                p.mode == 1 ? 1.0f : 0.0f, p.mode == 2 ? 1.0f : 0.0f);
+    __syncwarp();
+    float dirt = __shfl_sync(FULL, acc, 0), rock = __shfl_sync(FULL, acc, 1), met_dirt = 0.0f, met_rock = 0.0f;
+#pragma unroll 4
     for (uint32_t i = 0; i < m; ++i) {
-        Pre q;
-        q.key = __shfl_sync(FULL, p.key, i);
-        q.mode = __shfl_sync(FULL, p.mode, i);
-        q.d1 = __shfl_sync(FULL, p.d1, i);
-        q.d0 = __shfl_sync(FULL, p.d0, i);
-        q.s1n = __shfl_sync(FULL, p.s1n, i);
-        q.s0n = __shfl_sync(FULL, p.s0n, i);
-        q.wi = __shfl_sync(FULL, p.wi, i);
-        q.mzi = __shfl_sync(FULL, p.mzi, i);
-        q.mwi = __shfl_sync(FULL, p.mwi, i);
-        RecOut o;
-        if (!apply_prepared(q, T, o)) {  // uniform: every lane holds the same texel state
-            Rec r;
-            r.key = q.key;
-            r.multipl = __shfl_sync(FULL, mine.multipl, i);
-            r.sc = __shfl_sync(FULL, mine.sc, i);
-            r.vol = __shfl_sync(FULL, mine.vol, i);
-            r.s0 = __shfl_sync(FULL, mine.s0, i);
-            r.s1 = __shfl_sync(FULL, mine.s1, i);
-            r.vx = __shfl_sync(FULL, mine.vx, i);
-            r.vy = __shfl_sync(FULL, mine.vy, i);
-            r.kill = __shfl_sync(FULL, mine.kill, i);
-            o = apply_record(a, r, T);
-        }
-        if ((uint32_t)lane == i) store_rec(a, q.key, o);
+        const float4 u = ws.w[0][i], v = ws.w[1][i];
+        const bool here = (uint32_t)lane == i;
+        met_dirt = here ? dirt : met_dirt;
+        met_rock = here ? rock : met_rock;
+        const float d = dirt + u.x;
+        const bool gone = (v.z != 0.0f) & (d < 0.0f);
+        // the rock below an exhausted dirt layer: what the dirt held counts
+        // against the capacity
+        const float c = gmax(0.0f, u.z - dirt);
+        const bool more = c > u.w;
+        const float e = (more ? v.x : v.y) * (more ? c - u.w : u.w - c);
+        const float r = rock + (gone ? (more ? -e : e) : u.y);
+        dirt = gone ? 0.0f : d;
+        rock = ((gone ? more : v.w != 0.0f) & (r < 0.0f)) ? 0.0f : r;
     }
-    acc = lane == 0 ? T.terr[1] : lane == 1 ? T.terr[0] : lane == 2 ? T.wat : lane == 3 ? T.mz : T.mw;
+    __syncwarp();  // the rows are read
+    if (have) {
+        Texel T{{met_rock, met_dirt}, 0.0f, 0.0f, 0.0f};
+        const RecOut o = apply_record(a, mine, T);
+        store_rec(a, p.key, o);
+    }
+    acc = lane == 0 ? dirt : lane == 1 ? rock : sum;  // (no layer enters the water's and the momentum's sums)
 }
 
 // a texel of SMALL + 1 to MID records, by a warp: lane i holds record i; a

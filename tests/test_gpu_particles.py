@@ -172,3 +172,12 @@ def test_time_of_buckets_of_many_chunks():
     spread = us_per_step(1024, 262144, 16)
     crowded = us_per_step(64, 262144, 80)
     assert crowded < 90 * spread, f"{crowded:.0f} us, {spread:.0f} us"
+
+
+def test_time_of_exhausted_layers():
+    """Droplets gathered in pits without dirt: nearly every record meets an
+    exhausted layer (19 times the spread droplets' step when such a record went
+    through the warp's lanes whole, 7 now)."""
+    spread = us_per_step(1024, 262144, 16)
+    crowded = us_per_step(128, 262144, 40)
+    assert crowded < 13 * spread, f"{crowded:.0f} us, {spread:.0f} us"
