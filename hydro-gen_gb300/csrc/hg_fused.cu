@@ -62,10 +62,13 @@ namespace {
 
 enum { H_B = 0, H_D, H_FL, H_FR, H_FT, H_FB, H_S, H_N };
 
-// Geometry of a 64 x TH tile, TH = 16 or 8: 256 threads with two pairs of cells or one.
-template <int TH>
+// Geometry of a 64 x TH tile, TH = 16 or 8, of NT threads: two pairs of cells per
+// thread, or one in small launches' 8-row tiles (256 threads), where the time is
+// latency.  4096² by 8 rows, one step without talus / eight with it: 282 / 2800 us
+// with one pair per thread, 243 / 2611 with two (16 rows: 246 / 2673).
+template <int TH, int NT>
 struct Geo {
-    static constexpr int NTH = 256;
+    static constexpr int NTH = NT, BLOCKS = 1024 / NT;  // (64 registers)
     static constexpr int H_RH = TH + 2, H_BOX = RW * H_RH;
     static constexpr int H_RC = ((H_BOX + 31) / 32) * 32;  // 128-byte aligned array stride
     static constexpr int CPT = TW * TH / NTH;             // cells per thread in k_hydro (4)
@@ -106,11 +109,11 @@ __device__ __forceinline__ RainStep rain_for(const RainBase& rb, unsigned long l
 // ---------------------------------------------------------------------------
 // EM: 0 inner tile, 1 edge tile (each its own code), 2 either, told at run
 // time by edge_rt (one code path for both)
-template <int TH, int EM, bool CHAIN>
+template <int TH, int NT, int EM, bool CHAIN>
 __device__ __forceinline__ void hydro_tile(const TerrainHot& td, const CUtensorMap* maps, float* sm, uint64_t* bar,
                                            int tx0, int ty0, int index, bool edge_rt, int* err) {
     const bool EDGE = EM == 2 ? edge_rt : EM == 1;
-    using G = Geo<TH>;
+    using G = Geo<TH, NT>;
     constexpr int NTH = G::NTH, H_RC = G::H_RC, H_RH = G::H_RH;
     const StepConsts1& c = td.c;
     const int n = c.n;
@@ -250,10 +253,10 @@ __device__ __forceinline__ void hydro_tile(const TerrainHot& td, const CUtensorM
     }
 }
 
-template <int TH, bool SPLIT, bool CHAIN>
+template <int TH, int NT, bool SPLIT, bool CHAIN>
 __device__ __forceinline__ void hydro_block(const TerrainHot& td, const CUtensorMap* maps, int tx0, int ty0, int index,
                                             int* err) {
-    using G = Geo<TH>;
+    using G = Geo<TH, NT>;
     __shared__ __align__(128) float sm[(CHAIN ? H_S : H_N) * G::H_RC];
     __shared__ __align__(8) uint64_t bar;
     if (threadIdx.x == 0) mbar_init(&bar, 1);
@@ -265,27 +268,27 @@ __device__ __forceinline__ void hydro_block(const TerrainHot& td, const CUtensor
     // missed in the instruction cache: 4.6 stalls per issue on an empty
     // instruction buffer, 11 % more time at 256²).  A large world is almost
     // all inner tiles and keeps a copy specialised for them (SPLIT).
-    if (!SPLIT) hydro_tile<TH, 2, CHAIN>(td, maps, sm, &bar, tx0, ty0, index, !inner, err);
-    else if (inner) hydro_tile<TH, 0, CHAIN>(td, maps, sm, &bar, tx0, ty0, index, false, err);
-    else hydro_tile<TH, 1, CHAIN>(td, maps, sm, &bar, tx0, ty0, index, true, err);
+    if (!SPLIT) hydro_tile<TH, NT, 2, CHAIN>(td, maps, sm, &bar, tx0, ty0, index, !inner, err);
+    else if (inner) hydro_tile<TH, NT, 0, CHAIN>(td, maps, sm, &bar, tx0, ty0, index, false, err);
+    else hydro_tile<TH, NT, 1, CHAIN>(td, maps, sm, &bar, tx0, ty0, index, true, err);
 }
 
 // Batch form: the terrain records are a kernel parameter (constant bank),
 // the block finds its terrain by binary search.
-template <int TH, bool CHAIN>
-__global__ void __launch_bounds__(Geo<TH>::NTH, 4) k_hydro(const __grid_constant__ BatchParams bp,
+template <int TH, int NT, bool CHAIN>
+__global__ void __launch_bounds__(NT, Geo<TH, NT>::BLOCKS) k_hydro(const __grid_constant__ BatchParams bp,
                                                         const CUtensorMap* __restrict__ maps, int index, int* err) {
     const int t = find_terrain(bp.tile0, bp.nterr, blockIdx.x);
     const unsigned tile = blockIdx.x - bp.tile0[t], tiles_x = bp.t[t].tiles_x;
-    hydro_block<TH, false, CHAIN>(bp.t[t], maps + MAPS_PER_TERRAIN * t, (tile % tiles_x) * TW, (tile / tiles_x) * TH,
+    hydro_block<TH, NT, false, CHAIN>(bp.t[t], maps + MAPS_PER_TERRAIN * t, (tile % tiles_x) * TW, (tile / tiles_x) * TH,
                                   index, err);
 }
 
 // Single-world form: the whole descriptor, tensor maps included, is a kernel
 // parameter.  SPLIT as for hydro_block: the host picks it by world size.
-template <int TH, bool SPLIT, bool CHAIN>
-__global__ void __launch_bounds__(Geo<TH>::NTH, 4) k_hydro1(const __grid_constant__ TerrainDesc td, int index, int* err) {
-    hydro_block<TH, SPLIT, CHAIN>(td.h, td.maps, blockIdx.x * TW, td.row_lo + blockIdx.y * TH, index, err);
+template <int TH, int NT, bool SPLIT, bool CHAIN>
+__global__ void __launch_bounds__(NT, Geo<TH, NT>::BLOCKS) k_hydro1(const __grid_constant__ TerrainDesc td, int index, int* err) {
+    hydro_block<TH, NT, SPLIT, CHAIN>(td.h, td.maps, blockIdx.x * TW, td.row_lo + blockIdx.y * TH, index, err);
 }
 
 // ---------------------------------------------------------------------------
@@ -686,25 +689,32 @@ bool tiled(size_t cells, bool thermal, bool last) {
     return last ? cells < (size_t)4096 * 4096 : cells <= (size_t)2048 * 2048;
 }
 
-template <int TH>
+template <int TH, int NT>
 void launch_hydro1(const TerrainDesc& td, int index, int* err, cudaStream_t st) {
     const dim3 tiles(td.h.tiles_x, (td.row_hi - td.row_lo) / TH);
     const bool split = td.h.c.n >= SPLIT_MIN_N;
     if (index > 0) {
-        if (split) k_hydro1<TH, true, true><<<tiles, Geo<TH>::NTH, 0, st>>>(td, index, err);
-        else k_hydro1<TH, false, true><<<tiles, Geo<TH>::NTH, 0, st>>>(td, index, err);
+        if (split) k_hydro1<TH, NT, true, true><<<tiles, NT, 0, st>>>(td, index, err);
+        else k_hydro1<TH, NT, false, true><<<tiles, NT, 0, st>>>(td, index, err);
     } else {
-        if (split) k_hydro1<TH, true, false><<<tiles, Geo<TH>::NTH, 0, st>>>(td, 0, err);
-        else k_hydro1<TH, false, false><<<tiles, Geo<TH>::NTH, 0, st>>>(td, 0, err);
+        if (split) k_hydro1<TH, NT, true, false><<<tiles, NT, 0, st>>>(td, 0, err);
+        else k_hydro1<TH, NT, false, false><<<tiles, NT, 0, st>>>(td, 0, err);
     }
     count_launch();
 }
+// (a launch of 8-row tiles is small up to the cells where the tuner takes them)
+bool small_launch(size_t cells) { return cells <= (size_t)640 * 640; }
+void launch_hydro1(const TerrainDesc& td, int th, int index, int* err, cudaStream_t st) {
+    if (th == 16) launch_hydro1<16, 256>(td, index, err, st);
+    else if (small_launch((size_t)td.h.c.n * (td.row_hi - td.row_lo))) launch_hydro1<8, 256>(td, index, err, st);
+    else launch_hydro1<8, 128>(td, index, err, st);
+}
 
-template <int TH>
+template <int TH, int NT>
 void launch_hydro_table(const BatchParams& bp, const CUtensorMap* maps, int tiles, int index, int* err,
                         cudaStream_t st) {
-    if (index > 0) k_hydro<TH, true><<<tiles, Geo<TH>::NTH, 0, st>>>(bp, maps, index, err);
-    else k_hydro<TH, false><<<tiles, Geo<TH>::NTH, 0, st>>>(bp, maps, 0, err);
+    if (index > 0) k_hydro<TH, NT, true><<<tiles, NT, 0, st>>>(bp, maps, index, err);
+    else k_hydro<TH, NT, false><<<tiles, NT, 0, st>>>(bp, maps, 0, err);
     count_launch();
 }
 
@@ -745,10 +755,12 @@ void launch_talus_march(const StepConsts& c, const float* rock, float* rock_o, c
 
 void launch_fused_table(const BatchParams& bp, const CUtensorMap* maps, int total_tiles, int th, bool thermal,
                         ChainPos pos, int* err, cudaStream_t st) {
-    if (th == 16) launch_hydro_table<16>(bp, maps, total_tiles, pos.index, err, st);
-    else launch_hydro_table<8>(bp, maps, total_tiles, pos.index, err, st);
+    const size_t cells = (size_t)total_tiles * TW * th;
+    if (th == 16) launch_hydro_table<16, 256>(bp, maps, total_tiles, pos.index, err, st);
+    else if (small_launch(cells)) launch_hydro_table<8, 256>(bp, maps, total_tiles, pos.index, err, st);
+    else launch_hydro_table<8, 128>(bp, maps, total_tiles, pos.index, err, st);
     if (!pos.last && !thermal) return;
-    if (tiled((size_t)total_tiles * TW * th, thermal, pos.last)) {
+    if (tiled(cells, thermal, pos.last)) {
         const int shift = th == TT_H ? 0 : 1, tiles = total_tiles >> shift;
         if (pos.last) k_transport_tile<true><<<tiles, TT_NTH, 0, st>>>(bp, shift, pos.index + 1);
         else k_transport_tile<false><<<tiles, TT_NTH, 0, st>>>(bp, shift, 0);
@@ -763,13 +775,11 @@ void launch_fused_table(const BatchParams& bp, const CUtensorMap* maps, int tota
 void launch_fused_half(const TerrainDesc& td, int th, int which, int* err, cudaStream_t st) {
     if (td.row_hi <= td.row_lo) return;
     if (which == 1) launch_transport1(td, true, 1, st);
-    else if (th == 16) launch_hydro1<16>(td, 0, err, st);
-    else launch_hydro1<8>(td, 0, err, st);
+    else launch_hydro1(td, th, 0, err, st);
 }
 
 void launch_fused_one(const TerrainDesc& td, int th, ChainPos pos, int* err, cudaStream_t st) {
-    if (th == 16) launch_hydro1<16>(td, pos.index, err, st);
-    else launch_hydro1<8>(td, pos.index, err, st);
+    launch_hydro1(td, th, pos.index, err, st);
     if (pos.last || td.h.c.thermal) launch_transport1(td, pos.last, pos.index + 1, st);
 }
 

@@ -186,3 +186,50 @@ def test_talus_launch_of_a_middle_sized_world():
     hydro, transport = us(0), us(1)
     w.close()
     assert transport < 1.45 * hydro, f"{transport:.1f} us, {hydro:.1f} us"
+
+
+@pytest.mark.parametrize("graph", [0, 1])
+@pytest.mark.parametrize("n", [640, 704, 4160])
+def test_tiles_of_8_rows_either_side_of_the_small_launch(n, graph):
+    """Tiles of 8 rows on request: a block of 256 threads in small launches, of
+    128 in larger ones, a world alone and in a batch."""
+    def world(k):
+        w = make(n, seed=k)
+        w.set_options(H.options(H.RAIN_BERNOULLI, p=0.02, seed=k, tile=(64, 8), graph=graph))
+        return w
+
+    a, b = world(7), world(7)
+    a.step(3, H.MODE_FUSED)
+    a.step(1, H.MODE_FUSED)
+    b.step(4, H.MODE_PLAIN)
+    assert_same(a, b, f"{n}")
+    if n < 4096:
+        ws, small = [world(8), make(64, seed=9)], [world(8), make(64, seed=9)]
+        batch = H.Batch(ws)
+        batch.step(3)
+        batch.sync()
+        for x, y in zip(ws, small):
+            y.step(3, H.MODE_PLAIN)
+            assert_same(x, y, f"batch {n}")
+        batch.close()
+    a.close()
+    b.close()
+
+
+def test_tiles_of_8_rows_keep_up_at_4096():
+    """Single steps without talus by tiles of 8 and of 16 rows (1.15 times when a
+    thread of an 8-row tile had one pair of cells at every size)."""
+    w = make(4096, thermal=False)
+    us = {}
+    for rows in (16, 8):
+        w.set_options(H.options(H.RAIN_UNIFORM, tile=(64, rows), graph=0))
+        us[rows] = 1e9
+        for _ in range(6):
+            w.sync()
+            t0 = time.perf_counter()
+            for _ in range(12):
+                w.step(1, H.MODE_FUSED)
+            w.sync()
+            us[rows] = min(us[rows], (time.perf_counter() - t0) / 12 * 1e6)
+    w.close()
+    assert us[8] < 1.07 * us[16], us
