@@ -729,13 +729,8 @@ int fused_prepare(FusedGroup* groups, int ngroups, cudaEvent_t ev, int* err) {
 // first group's (ev: one event, reused).
 int fused_run(FusedGroup* groups, int ngroups, cudaEvent_t ev, Tuning& tune, int req_th, int req_graph, int* err,
               int nsteps) {
-    size_t all = 0;
     int nworlds = 0;
-    for (int g = 0; g < ngroups; ++g)
-        for (hg_world* w : groups[g].worlds) {
-            all += cells(w);
-            nworlds += 1;
-        }
+    for (int g = 0; g < ngroups; ++g) nworlds += (int)groups[g].worlds.size();
     const int checked = check_groups(groups, ngroups);
     if (checked != HG_OK) return checked;
     if (req_th != HG_AUTO && req_th != 16 && req_th != 8)
@@ -748,11 +743,6 @@ int fused_run(FusedGroup* groups, int ngroups, cudaEvent_t ev, Tuning& tune, int
         return rc != HG_OK ? rc : joined;
     };
     if (req_th == HG_AUTO && req_graph == HG_AUTO && tune.th == 0 && nsteps >= 8) {
-        // tiles of 8 rows give a launch more blocks and each thread one pair:
-        // less latency, which is what a small launch takes, but more halo to
-        // load (1024² without talus: 12.2 us a step at 16 rows, 15.2 at 8,
-        // three worlds in turn), so larger ones stay at 16.
-        const bool small = all <= (size_t)640 * 640;
         // Host work (plans, graph captures) first; then the candidates are
         // queued without a wait between them, so that each one's launches
         // overlap the steps before it as they do in a run.
@@ -772,7 +762,6 @@ int fused_run(FusedGroup* groups, int ngroups, cudaEvent_t ev, Tuning& tune, int
             float ms = 0;
             cudaEventElapsedTime(&ms, mark[cand], mark[cand + 1]);
             tune.ms[cand] = ms / 2.0;
-            if (cand >= 2 && !small) continue;
             if (tune.ms[cand] < best) {
                 best = tune.ms[cand];
                 tune.th = cand < 2 ? 16 : 8;
@@ -1954,8 +1943,7 @@ int hg_batch_step(hg_batch* b, int nsteps, int mode) {
         if (rc != HG_OK) return rc == HG_ERR_CUDA ? cuda_fail(cudaGetLastError(), "batch tuning") : rc;
         b->tuning.ms_per_world = ms / 2.0;
         nsteps -= 12;
-        // against the table variant that would run: a faster one that is not
-        // eligible (tiles of 8 rows in large launches) decides nothing
+        // against the table variant that would run
         const double table = b->tuning.ms[(b->tuning.th == 16 ? 0 : 2) + b->tuning.graph];
         b->tuning.per_world = b->tuning.ms_per_world < table ? 1 : 0;
         char m[120];
