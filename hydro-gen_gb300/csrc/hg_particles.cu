@@ -562,8 +562,8 @@ __device__ __forceinline__ void sort_chunk(const uint32_t* src, uint32_t len, ui
 // lane runs these two again from the values they started with, a record at a
 // time without a branch, and keeps those its own record met; from them it works
 // out what the record leaves.
-// Bound by the latency of the two chains: about 10 cycles a record, and 60 where
-// layers are exhausted (790 when the whole record went from lane to lane).
+// Bound by the latency of the chains: about 25 cycles a record, and 105 more where
+// a layer is exhausted (790 when the whole record went from lane to lane).
 constexpr int SUMS = 5, SUM_PITCH = 36;  // (16-byte rows, lanes 0 to 4 on different banks)
 struct WarpSums {
     float v[SUMS][SUM_PITCH];
@@ -710,7 +710,7 @@ __device__ __noinline__ void apply_big(const ApplyArgs& a, WarpSums& ws, uint32_
 // lie anywhere, two loads of 16 bytes each (nine of 4 bytes before).  262144
 // droplets on 1024² after 100 steps (buckets up to 317 records): one launch over
 // all texels and one each over the busier two kinds took 33, 40 and 130 us, this
-// 60.  8 steps, three worlds in turn / alone: 7 blocks per SM 1143 / 1289 us, 6
+// 46.  8 steps, three worlds in turn / alone: 7 blocks per SM 1143 / 1289 us, 6
 // 1161 / 1292, 8 1135 / 1328.
 __global__ void __launch_bounds__(32 * AP_WARPS, AP_BLOCKS) k_papply(const ApplyArgs a) {
     __shared__ __align__(16) WarpSums sums[AP_WARPS];
