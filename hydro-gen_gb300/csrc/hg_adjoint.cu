@@ -187,7 +187,7 @@ __device__ __forceinline__ FluxFwd2 flux_fwd2(const StepConsts& c, int x, int y,
     if (!(fullx & fully)) {
         const float2 dn = make_float2(fullx ? 1.0f : den.x, fully ? 1.0f : den.y);
         float2 q;
-        if (num_range(d1.x) & num_range(d1.y) & den_range(dn.x) & den_range(dn.y)) {
+        if (depth_range(d1) & den_range(dn.x) & den_range(dn.y)) {
             o.rden = rcp_newton2(dn);
             q = div_recip2(d1, make_float2(-dn.x, -dn.y), o.rden);
         } else {

@@ -83,3 +83,30 @@ def test_steps_over_the_float_range(kind, n, thermal, ks1):
             for name, x, y in pairs:
                 assert np.array_equal(x, y, equal_nan=True), \
                     f"step {step + 1} {name} {k}: {np.count_nonzero(~((x == y) | (np.isnan(x) & np.isnan(y))))} differ"
+
+
+@pytest.mark.parametrize("layers", [1, 2])
+@pytest.mark.parametrize("mode", [H.MODE_PLAIN, H.MODE_FUSED])
+def test_flux_scale_of_a_hugely_negative_depth(mode, layers):
+    """A depth of -3e38 over an outflow of less than one: the quotient is minus
+    infinity, and so is the scale min(1, quotient)."""
+    n = 64
+    f = fields("ordinary", n, seed=5)
+    f["water"][::7, ::5] = -3e38
+    s = H.settings_config1()
+    s.G = 0.0  # outflows from the old flux, whatever the depth
+    w = H.World(n, layers=layers)
+    w.set_erosion(s)
+    w.set_options(H.options(H.RAIN_OFF))
+    ref = O.OracleWorld(n, 32)
+    for k, v in f.items():
+        w.upload(k, v)
+        ref.set(k, v)
+    w.step(1, mode)
+    ref.step(O.erosion_from(s), O.options(0, 1, 0.0), 1)
+    hit = 0
+    for k in ("water", "flux_l", "flux_r", "flux_t", "flux_b", "vel_u", "vel_v"):
+        a, b = w.download(k), ref.get(k)
+        hit += np.count_nonzero(~np.isfinite(b))
+        assert np.array_equal(a, b, equal_nan=True), f"{k}: {np.count_nonzero(~((a == b) | (np.isnan(a) & np.isnan(b))))} differ"
+    assert hit > 0
