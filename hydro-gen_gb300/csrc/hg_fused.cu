@@ -676,17 +676,17 @@ constexpr int SPLIT_MIN_N = 4096;
 
 // Forms of the talus launch: a single world up to this side runs talus_rows, a
 // larger one and batches tiles up to the cells below, above them warps march.
-// One step with talus of one world, alone / three worlds in turn, us, by tiles,
-// marching: 1024² 46 / 20, 54 / 25; 2048² 111 / 79, 124 / 85; 3072² 209 / 177,
-// 230 / 180; 4096² 347 / 315, 377 / 312.  Eight chained steps, of which one
-// gathers: 1024² 199 / 156, 255 / 182; 2048² 707 / 600, 784 / 616; 3072² 1444 /
-// 1346, 1555 / 1317.  By rows, tiles: 256² 68 / 25, 76 / 28; 384² 80 / 31, 82 / 36;
-// 448² 87 / 39, 92 / 40; four worlds of 448² on their own streams 164 / 166, 152 /
-// 140.
+// One step of one world, alone / three worlds in turn, us, by tiles, marching:
+// 1024² 37 / 20, 44 / 24; 2048² 98 / 76, 106 / 77; 3072² 188 / 166, 198 / 158
+// (smoothing, 16 such steps: 3596 / 3424, 3887 / 3383); 4096² 347 / 315, 377 / 312.
+// 16 chained steps, of which two gather: 1024² 372 / 297, 462 / 325; 1536² 825 / 646,
+// 892 / 645; 1792² 1071 / 876, 1158 / 847; 2048² 1322 / 1131, 1409 / 1078.  Eight by
+// rows, tiles: 256² 68 / 25, 76 / 28; 384² 80 / 31, 82 / 36; 448² 87 / 39, 92 / 40,
+// four worlds of 448² on their own streams 164 / 166, 152 / 140.
 constexpr int ROWS1_MAX_N = 384;
 bool tiled(size_t cells, bool thermal, bool last) {
     if (!thermal) return true;  // the gather alone, nothing to march for
-    return last ? cells < (size_t)4096 * 4096 : cells <= (size_t)2048 * 2048;
+    return last ? cells < (size_t)4096 * 4096 : cells <= (size_t)1536 * 1536;
 }
 
 template <int TH, int NT>
