@@ -768,6 +768,12 @@ int fused_run(FusedGroup* groups, int ngroups, cudaEvent_t ev, Tuning& tune, int
                 tune.graph = cand & 1;
             }
         }
+        // Within 2 % tiles of 16 rows stay: that is how far the steps' cost
+        // drifts over the candidates, and they load less halo, which worlds
+        // stepped in turn pay for (8192² with talus and uniform rain, alone /
+        // three in turn, us a step: 16 rows 1026 / 917, 8 rows 1024 / 925; with
+        // Bernoulli rain 1084 / 976, 1055 / 953; 4096² 297 / 257, 286 / 248).
+        if (rc == HG_OK && tune.th == 8 && tune.ms[tune.graph] <= 1.02 * best) tune.th = 16;
         for (cudaEvent_t e : mark)
             if (e) cudaEventDestroy(e);
         if (rc != HG_OK) return rc == HG_ERR_CUDA ? cuda_fail(cudaGetLastError(), "autotuning") : rc;
@@ -1943,9 +1949,9 @@ int hg_batch_step(hg_batch* b, int nsteps, int mode) {
         if (rc != HG_OK) return rc == HG_ERR_CUDA ? cuda_fail(cudaGetLastError(), "batch tuning") : rc;
         b->tuning.ms_per_world = ms / 2.0;
         nsteps -= 12;
-        // against the table variant that would run
-        const double table = b->tuning.ms[(b->tuning.th == 16 ? 0 : 2) + b->tuning.graph];
-        b->tuning.per_world = b->tuning.ms_per_world < table ? 1 : 0;
+        // (the table variant that would run is the fastest, or within 2 % of it)
+        const double* m4 = b->tuning.ms;
+        b->tuning.per_world = b->tuning.ms_per_world < *std::min_element(m4, m4 + 4) ? 1 : 0;
         char m[120];
         std::snprintf(m, sizeof m, "autotuner: batch of %zu worlds, %s (%.4f ms/step per world's launches)",
                       b->worlds.size(), b->tuning.per_world ? "per-world launches" : "one table launch",

@@ -167,8 +167,9 @@ def test_largest_batch_in_one_launch():
 
 @pytest.mark.parametrize("sides", [(512, 512), (640, 512, 256), (1024, 512), (768, 768, 768)])
 def test_launch_form_is_chosen_against_the_table_variant_that_runs(sides):
-    """Batches above 640² cells in all: the table variant is the fastest of the
-    four timed, and the worlds' own launches are compared with that one."""
+    """Batches above 640² cells in all: the table variant that runs is the fastest
+    of the four timed or within 2 % of it, and the worlds' own launches are
+    compared with it."""
     for seed in range(4):
         ws = [H.World(n) for n in sides]
         for i, w in enumerate(ws):
@@ -180,8 +181,8 @@ def test_launch_form_is_chosen_against_the_table_variant_that_runs(sides):
         th, graph, ms = b.tuning()
         per_world, ms_pw = b.launch_form()
         table = ms[(0 if th == 16 else 2) + graph]
-        assert table == min(ms)
-        assert per_world == (ms_pw < table), (per_world, ms_pw, ms)
+        assert table <= 1.02 * min(ms) and (th == 16 or table == min(ms)), (th, graph, ms)
+        assert per_world == (ms_pw < min(ms)), (per_world, ms_pw, ms)
         b.close()
         for w in ws:
             w.close()
