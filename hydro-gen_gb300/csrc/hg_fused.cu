@@ -702,8 +702,10 @@ void launch_hydro1(const TerrainDesc& td, int index, int* err, cudaStream_t st) 
     }
     count_launch();
 }
-// (a launch of 8-row tiles is small up to the cells where the tuner takes them)
-bool small_launch(size_t cells) { return cells <= (size_t)640 * 640; }
+// 8-row tiles have 256 threads up to these cells, 128 above: 16 steps without talus,
+// alone / three worlds in turn, us, by 256 and 128 threads: 256² 75 / 28 and 87 / 31,
+// 448² 93 / 39 and 99 / 41, 640² 134 / 78 and 125 / 62, 1024² 235 / 244 and 212 / 193.
+bool small_launch(size_t cells) { return cells <= (size_t)512 * 512; }
 void launch_hydro1(const TerrainDesc& td, int th, int index, int* err, cudaStream_t st) {
     if (th == 16) launch_hydro1<16, 256>(td, index, err, st);
     else if (small_launch((size_t)td.h.c.n * (td.row_hi - td.row_lo))) launch_hydro1<8, 256>(td, index, err, st);

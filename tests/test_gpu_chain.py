@@ -189,7 +189,7 @@ def test_talus_launch_of_a_middle_sized_world():
 
 
 @pytest.mark.parametrize("graph", [0, 1])
-@pytest.mark.parametrize("n", [640, 704, 4160])
+@pytest.mark.parametrize("n", [512, 576, 4160])
 def test_tiles_of_8_rows_either_side_of_the_small_launch(n, graph):
     """Tiles of 8 rows on request: a block of 256 threads in small launches, of
     128 in larger ones, a world alone and in a batch."""
